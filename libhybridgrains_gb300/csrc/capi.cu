@@ -1365,7 +1365,8 @@ hg_status hg_dem_destroy(hg_dem *d) {
     DeviceGuard g(ctx);
     if (d->own) cudaStreamSynchronize(d->own);
     cudaStreamSynchronize(ctx->stream);
-    if (d->pair_exec) cudaGraphExecDestroy(d->pair_exec);
+    for (auto &pg : d->pair)
+      if (pg.exec) cudaGraphExecDestroy(pg.exec);
     if (d->own) cudaStreamDestroy(d->own);
     if (d->own_ev) cudaEventDestroy(d->own_ev);
     if (d->ctx_ev) cudaEventDestroy(d->ctx_ev);
@@ -1392,10 +1393,11 @@ hg_status hg_dem_set_concurrent(hg_dem *d, int32_t on) {
     HG_CUDA_TRY(cudaStreamWaitEvent(d->own, d->ctx_ev, 0));
   } else if (!on && d->own) {
     HG_CUDA_TRY(cudaStreamSynchronize(d->own));
-    if (d->pair_exec) { // captured on the own stream; rebuilt on the next step
-      cudaGraphExecDestroy(d->pair_exec);
-      d->pair_exec = nullptr;
-    }
+    for (auto &pg : d->pair) // captured on the own stream; rebuilt on the next step
+      if (pg.exec) {
+        cudaGraphExecDestroy(pg.exec);
+        pg.exec = nullptr;
+      }
     cudaStreamDestroy(d->own);
     cudaEventDestroy(d->own_ev);
     cudaEventDestroy(d->ctx_ev);
@@ -1465,6 +1467,8 @@ static hg_status dem_upload_impl(hg_dem *d, int64_t n, const double *q, const do
   cudaStream_t s = dem_stream(d);
   d->n = n;
   d->inv_valid = false;
+  d->desc_valid = false;
+  dem_bodies_changed(d);
   hg_status st;
   if ((st = h2d(s, d->q.p, q, 3 * n)) || (st = h2d(s, d->v.p, v, 3 * n)) ||
       (st = h2d(s, d->r.p, r, n)) || (st = h2d(s, d->m0.p, mass, n)) ||
@@ -1549,6 +1553,7 @@ hg_status hg_dem_set_state(hg_dem *d, const double *q, const double *v) {
   DeviceGuard g(d->ctx);
   AllocScope dem_scope(dem_stream(d)); // temporaries on the DEM's stream
   hg_status st;
+  if (q) dem_bodies_changed(d);
   if (q && (st = h2d(dem_stream(d), d->q.p, q, 3 * d->n))) return st;
   if (v && (st = h2d(dem_stream(d), d->v.p, v, 3 * d->n))) return st;
   HG_CUDA_TRY(cudaStreamSynchronize(dem_stream(d)));
@@ -1567,28 +1572,28 @@ hg_status hg_dem_download(hg_dem *d, double *q, double *v) {
   return HG_OK;
 }
 
-// Captures two consecutive DEM steps on the context's stream into a graph
-// (once per state: n, dt, weighting, live contact buffer, broadphase cell).
+// Captures two consecutive DEM steps on the DEM's stream into a graph (once
+// per live contact buffer and state: n, dt, weighting, broadphase cell). The
+// bodies are binned and the contact lists known, as after any step.
 static hg_status dem_pair_graph(hg_dem *d, double dt, int weighted) {
-  if (d->pair_exec && d->pair_n == d->n && d->pair_dt == dt && d->pair_weighted == weighted &&
-      d->pair_cc == d->cc && d->pair_cell == d->cell_h)
+  hg_dem::PairGraph &g = d->pair[d->cc];
+  if (g.exec && g.n == d->n && g.dt == dt && g.weighted == weighted && g.cell == d->cell_h)
     return HG_OK;
-  if (d->pair_exec) {
-    cudaGraphExecDestroy(d->pair_exec);
-    d->pair_exec = nullptr;
+  if (g.exec) {
+    cudaGraphExecDestroy(g.exec);
+    g.exec = nullptr;
   }
   cudaStream_t s = dem_stream(d);
-  const int cc0 = d->cc;
-  const bool hv0 = d->history_valid;
   const int64_t l0 = g_launches.load();
   HG_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-  hg_status st = dem_step(d, dt, weighted);
-  if (st == HG_OK) st = dem_step(d, dt, weighted);
+  // (the host's bookkeeping after two steps is what it was before them)
+  const int cc0 = d->cc, bins0 = d->bins;
+  hg_status st = dem_step(d, dt, weighted, true);
+  if (st == HG_OK) st = dem_step(d, dt, weighted, true);
+  d->cc = cc0;
+  d->bins = bins0;
   cudaGraph_t graph = nullptr;
   const cudaError_t e = cudaStreamEndCapture(s, &graph);
-  // capturing ran no step: restore the host-side bookkeeping it advanced
-  d->cc = cc0;
-  d->history_valid = hv0;
   const int64_t launches = g_launches.load() - l0;
   g_launches.fetch_sub(launches, std::memory_order_relaxed);
   if (st != HG_OK) {
@@ -1596,20 +1601,17 @@ static hg_status dem_pair_graph(hg_dem *d, double dt, int weighted) {
     return st;
   }
   if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
-  const cudaError_t ei = cudaGraphInstantiate(&d->pair_exec, graph, 0);
+  const cudaError_t ei = cudaGraphInstantiate(&g.exec, graph, 0);
   cudaGraphDestroy(graph);
   if (ei != cudaSuccess) {
-    d->pair_exec = nullptr;
+    g.exec = nullptr;
     return cuda_fail(ei, "cudaGraphInstantiate");
   }
-  d->pair_n = d->n;
-  d->pair_dt = dt;
-  d->pair_weighted = weighted;
-  d->pair_cc = cc0;
-  d->pair_cell = d->cell_h;
-  d->pair_launches = launches;
-  // a pair of replays leaves the live buffer where it started
-  d->history_valid = true;
+  g.n = d->n;
+  g.dt = dt;
+  g.weighted = weighted;
+  g.cell = d->cell_h;
+  g.launches = launches;
   return HG_OK;
 }
 
@@ -1621,20 +1623,24 @@ hg_status hg_dem_step(hg_dem *d, double dt, int32_t nsteps, int32_t weighted) {
   DeviceGuard g(d->ctx);
   AllocScope dem_scope(dem_stream(d)); // temporaries on the DEM's stream
   int k = 0;
+  hg_status st;
   if (nsteps >= 4 && d->n > 0) {
-    // Repeated steps replay a captured pair of steps: one graph launch in
-    // place of about 40 kernel launches and memsets.
-    hg_status st = dem_prepare(d, dt);
-    if (st == HG_OK) st = dem_pair_graph(d, dt, weighted);
-    if (st != HG_OK) return st;
+    // Repeated steps replay a captured pair of steps, which starts from
+    // binned bodies and known contact lists: a plain step first where the
+    // bodies changed.
+    if (d->bins != hg_dem::BINS_FILLED || !d->desc_valid) {
+      if ((st = dem_step(d, dt, weighted, true))) return st;
+      k = 1;
+    }
+    if ((st = dem_prepare(d, dt)) || (st = dem_pair_graph(d, dt, weighted))) return st;
+    const hg_dem::PairGraph &pg = d->pair[d->cc];
     for (; k + 2 <= nsteps; k += 2) {
-      HG_CUDA_TRY(cudaGraphLaunch(d->pair_exec, dem_stream(d)));
-      g_launches.fetch_add(d->pair_launches, std::memory_order_relaxed);
+      HG_CUDA_TRY(cudaGraphLaunch(pg.exec, dem_stream(d)));
+      g_launches.fetch_add(pg.launches, std::memory_order_relaxed);
     }
   }
   for (; k < nsteps; ++k) {
-    hg_status st = dem_step(d, dt, weighted);
-    if (st != HG_OK) return st;
+    if ((st = dem_step(d, dt, weighted, true))) return st;
   }
   return HG_OK;
 }

@@ -248,11 +248,11 @@ __global__ void kc_transfer(GridGeom G, int64_t nb, const int32_t *__restrict__ 
 }
 
 template <bool W32>
-__global__ void kc_hstress(GridGeom G, int64_t nb, const int32_t *__restrict__ off,
+__global__ void kc_hstress(GridGeom G, const int2 *__restrict__ range,
                            const double *__restrict__ rec, const double *__restrict__ q,
                            double *hs) {
-  // circle-circle contacts occupy [off[nb], off[2 nb]) of the contact list
-  const int s = off[nb], e = off[2 * nb];
+  // the circle-circle contacts of the contact list
+  const int s = range->x, e = range->y;
   const double cw = G.h;
   const double area = cw * cw;
   const double hl = cw * 0.25;
@@ -448,7 +448,8 @@ hg_status hybrid_step_impl(hg_hybrid *h, double dt, int flags) {
   h->packed_valid = false;
   h->step_bodies = nb;
   // DiscreteIntegrator::step -> flowWithWeight (DiscreteIntegrator.cpp:99-116)
-  if ((st = dem_step(d, dt, 1))) return st;
+  // (kc_transfer moves the grains after it, so it bins none for the next step)
+  if ((st = dem_step(d, dt, 1, false))) return st;
   if ((st = mixed ? mixed_grid_update(m, dt) : mpm64_phase1(m, dt))) return st;
   // rasterizeGrainMom
   HG_CUDA_TRY(cudaMemsetAsync(h->dem_mom.p, 0, sizeof(double) * 2 * nn, s));
@@ -470,7 +471,7 @@ hg_status hybrid_step_impl(hg_hybrid *h, double dt, int flags) {
   HG_CHECK_LAUNCH();
   if ((st = mixed ? mixed_particles(m, dt) : mpm64_phase2(m, dt))) return st;
   if ((flags & HG_HYBRID_HOMOGENIZE_STRESS) && nb > 0) {
-    HG_LAUNCH(kc_hstress<W32>, gs, 128, 0, s, G, nb, d->per_body_off.p, d->crec[d->cc].p, d->q.p,
+    HG_LAUNCH(kc_hstress<W32>, gs, 128, 0, s, G, d->cc_range.p, d->crec[d->cc].p, d->q.p,
               h->hstress.p);
     HG_CHECK_LAUNCH();
   }

@@ -8,30 +8,37 @@
 // instead of atomics. The step is therefore deterministic and matches a serial
 // FP64 evaluation of the reference bit for bit.
 //
-// Kernels per step:
-//   kd_bodies_home / kd_fill broadphase: hash-grid counting sort of the disks
-//                            by the cell of their AABB minimum. The cell width
-//                            is 2 r_max (1 + 1e-6), so the partners of a disk
-//                            lie in 3x3 cells; the result is the reference's
-//                            candidate set {i < j : AABBs overlap}
-//                            (SpatialGrid.cpp:14-19, 90-118), independent of
-//                            the reference's own cell width.
-//   kd_pairs_count / _emit   narrow phase (RigidBody2DSim.cpp:270-336 with
-//                            q0 == q1, CollisionDetectionUtilities.cpp:3-101)
-//                            and body-plane tests (RigidBody2DSim.cpp:777-842);
-//                            count (keeping short partner lists), then emit
-//                            sorted per-body contact lists. Candidates are
-//                            filtered in FP32 on cell-relative offsets before
-//                            the exact FP64 tests: FP64 runs at 1/64 of the
-//                            FP32 rate on this part, and the filter leaves
-//                            about one FP64 test per contact.
-//   kd_contacts              collision-cache update with tangential-spring
-//                            carry (PenaltyImpactFrictionMap.cpp:296-599) and
-//                            the penalty force with Coulomb projection
-//                            (616-1081, secondRootOfQuadratic 601-614).
-//   kd_in_count / kd_in_fill incoming circle-circle contact lists per body.
-//   kd_integrate             force gather, fixed-body zeroing and symplectic
-//                            Euler (PenaltyImpactFrictionMap.cpp:1101-1114).
+// Kernels per step (in one of two ways to the tile sums):
+//   kd_bin         broadphase: a hash grid of linked lists over the disks'
+//                  centres, only in the first step after the bodies changed
+//                  (later ones are binned by the integration). The cell width
+//                  is 2 r_max (1 + 1e-6), so the partners of a disk lie in
+//                  3x3 cells; the result is the reference's candidate set
+//                  {i < j : AABBs overlap} (SpatialGrid.cpp:14-19, 90-118),
+//                  independent of the reference's own cell width.
+//   kd_pairs       narrow phase (RigidBody2DSim.cpp:270-336 with q0 == q1,
+//                  CollisionDetectionUtilities.cpp:3-101) and body-plane
+//                  tests (RigidBody2DSim.cpp:777-842): counts, keeping short
+//                  partner lists. Candidates are filtered in FP32 on
+//                  cell-relative offsets before the exact FP64 tests; the
+//                  filter leaves about one FP64 test per contact at the
+//                  filter's edge.
+//   kd_pairs_emit  offsets and sorted per-body contact lists
+//   kd_contacts    collision-cache update with tangential-spring carry
+//                  (PenaltyImpactFrictionMap.cpp:296-599) and the penalty
+//                  force with Coulomb projection (616-1081,
+//                  secondRootOfQuadratic 601-614); incoming contact lists per
+//                  body.
+//   kd_integrate   force gather, fixed-body zeroing and symplectic Euler
+//                  (PenaltyImpactFrictionMap.cpp:1101-1114), then the binning
+//                  for the next step.
+// Small scenes are bound by the chain of dependent launches and loads, the
+// contact law by the FP64 pipe, a million disks by the records' 176 bytes per
+// contact. Against a counting sort of the grid, scans for every offset list
+// and records stored by their lanes (14 launches per step), per step: 1,000
+// disks stepped one call at a time 63.6 -> 28.3 us; 10,000 disks at 2.8
+// contacts each, FP64, 68.3 -> 39.0 us; 1,000,000 such disks, mixed, 889 ->
+// 434 us.
 #include "hg_internal.cuh"
 
 #include <algorithm>
@@ -123,57 +130,156 @@ __device__ __forceinline__ void sort_small(int *keys, int n) {
   }
 }
 
-// Per body, for the pair search: the home cell (the cell of the AABB
-// minimum) and, in FP32, the offset of the centre from the home cell's
-// corner and the radius, with the fixed flag and the active static planes
+// ---- FP64 values through the integer pipe -----------------------------------
+//
+// FP64 instructions, conversions to and from FP64 included, issue at about two
+// lanes per cycle and SM on this part (17-21 cycles per warp instruction
+// measured, with 65 cycles of latency; a 32-bit integer instruction takes
+// 0.3), so conversions and decisions that integer arithmetic can make exactly
+// are made there.
+
+// (float)x, rounded to nearest even, for a double in FP32's normal range;
+// other values take the conversion instruction.
+__device__ __noinline__ float narrow_slow(double x) { return (float)x; }
+__device__ __forceinline__ float narrow(double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const uint32_t e = (hi >> 20) & 0x7FFu;
+  if (e - 897u < 253u) { // 2^-126 <= |x| < 2^127
+    const uint64_t b = ((uint64_t)(hi & 0x7FFFFFFFu) << 32) | lo;
+    const uint64_t r = b + 0x0FFFFFFFull + ((b >> 29) & 1u); // ties to even at bit 29
+    return __uint_as_float(((uint32_t)(r >> 29) - (896u << 23)) | (hi & 0x80000000u));
+  }
+  if (((hi << 1) | lo) == 0u) return __uint_as_float(hi); // a zero keeps its sign
+  return narrow_slow(x);
+}
+// The same truncated, for FP32 estimates.
+__device__ __forceinline__ float narrow_trunc(double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const uint32_t e = (hi >> 20) & 0x7FFu;
+  if (e - 897u < 253u)
+    return __uint_as_float((((hi & 0x7FFFFFFFu) - (896u << 20)) << 3) | (lo >> 29) |
+                           (hi & 0x80000000u));
+  if (((hi << 1) | lo) == 0u) return 0.0f;
+  return narrow_slow(x);
+}
+// (double)f
+__device__ __noinline__ double widen_slow(float f) { return (double)f; }
+__device__ __forceinline__ double widen(float f) {
+  const uint32_t b = __float_as_uint(f), m = b & 0x7FFFFFFFu;
+  if (m - 0x00800000u < 0x7F000000u) // normal
+    return __hiloint2double((int)(((m >> 3) + (896u << 20)) | (b & 0x80000000u)), (int)(b << 29));
+  if (m == 0u) return __hiloint2double((int)b, 0);
+  return widen_slow(f);
+}
+// (double)i for 0 <= i < 2^30
+__device__ __forceinline__ double index_f64(int i) {
+  if (i == 0) return 0.0;
+  const int e = 31 - __clz(i);
+  const uint64_t m = (uint64_t)(uint32_t)i << (52 - e); // leading bit at 52
+  return __longlong_as_double((int64_t)(m + ((uint64_t)(e + 1022) << 52)));
+}
+// min(0, x); 0 for a NaN
+__device__ __forceinline__ double min_zero(double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const bool nan = (hi & 0x7FFFFFFFu) > 0x7FF00000u ||
+                   ((hi & 0x7FFFFFFFu) == 0x7FF00000u && lo != 0u);
+  return (hi >> 31) && !nan ? x : 0.0;
+}
+
+// Per body, for the pair search: the home cell (the cell of its centre) and,
+// in FP32, the offset of the centre from the home cell's corner and the
+// radius, with the fixed flag and the active static planes
 // (StaticPlaneCircleConstraint::isActive, StaticPlaneCircleConstraint.cpp:
-// 12-17, in FP64) as bits. The FP64 arithmetic per body is a few operations;
-// per candidate pair the search needs FP32 only, except for the exact tests
-// of the pairs that survive the FP32 filter. Active static drums take the
-// bits after the planes'. The home cell only has to be a
-// consistent binning (the search covers the neighbouring cells), so it is
-// floor(x_min / H) computed as x_min * (1 / H).
-struct HomeArgs {
+// 12-17) as bits; active static drums take the bits after the planes'. Per
+// candidate pair the search needs FP32 only, except for the exact tests of
+// the pairs that survive the FP32 filter.
+//
+// The bodies of a hash bucket are a linked list (head per bucket, the next
+// body in the record), built with one exchange per body: the search needs no
+// bucket counts, so no scan and no second pass over the bodies. The order of
+// a list does not matter: the emission pass sorts what the search finds.
+struct BinArgs {
   int64_t n;
   double H, invH;
   uint32_t mask;
   int nplanes;
   double px[HG_MAX_PLANES][2], pn[HG_MAX_PLANES][2];
+  float pxf[HG_MAX_PLANES][2], pnf[HG_MAX_PLANES][2];
   int ndrums;
   double dx[HG_MAX_DRUMS][2], dr[HG_MAX_DRUMS];
-  const double *q, *r;
+  const double *r;
   const uint8_t *fixed;
-  float4 *rec; // 2 per body: (offset x, offset y, radius, flags), (home cell x, y)
-  int32_t *bucket_count;
-  // this step's per-body counters, zeroed here in place of memsets: contact
-  // counts (3n + 1), pair fill (n), incoming counts (n + 1) and cursors (n)
-  int32_t *per_body, *pfill, *in_count, *in_cursor;
+  float4 *rec; // 2 per body: (offset x, offset y, radius, flags), (home cell x, y, next, -)
+  int32_t *heads;
+  unsigned long long *pc; // contact counts by kind (PC_*)
+  int32_t *in_count;      // contacts in which the body is the second
+  int32_t *tiles;         // sums of the four counts per tile, or nullptr
+  int tile_shift;
 };
 
 enum : uint32_t { REL_FIXED = 1u, REL_PLANE0 = 2u };
 static_assert(1 + HG_MAX_PLANES + HG_MAX_DRUMS <= 32, "static-object bits of the body record");
 
-__global__ void kd_bodies_home(HomeArgs A) {
-  // (launched with programmatic dependence on the kernel before it)
-  pdl_wait();
-  pdl_trigger();
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= A.n) return;
-  A.per_body[3 * i] = A.per_body[3 * i + 1] = A.per_body[3 * i + 2] = 0;
-  A.pfill[i] = 0;
-  A.in_count[i] = 0;
-  A.in_cursor[i] = 0;
-  if (i == 0) {
-    A.per_body[3 * A.n] = 0;
-    A.in_count[A.n] = 0;
+// Contact counts of a first body in one word: static objects in bits 0-7,
+// circle-circle in 8-35, kinematic in 36-63. The search adds to it with one
+// atomic per contact, which also gives the partner's slot. The last two are
+// the partners found; at most MAXP of each kind are kept.
+constexpr int PC_CC = 8, PC_KIN = 36;
+__device__ __forceinline__ int pc_static(unsigned long long p) { return (int)(p & 0xFFu); }
+__device__ __forceinline__ int pc_found_cc(unsigned long long p) {
+  return (int)((p >> PC_CC) & 0xFFFFFFFu);
+}
+__device__ __forceinline__ int pc_found_kin(unsigned long long p) { return (int)(p >> PC_KIN); }
+__device__ __forceinline__ int pc_cc(unsigned long long p) { return min(pc_found_cc(p), MAXP); }
+__device__ __forceinline__ int pc_kin(unsigned long long p) { return min(pc_found_kin(p), MAXP); }
+
+// Cell floor(x / H) of a coordinate and the FP32 offset from the cell's lower
+// edge. x / H is formed in fixed point with 24 fraction bits by one FP64 FMA
+// (adding 3 * 2^27 leaves an ulp of 2^-24), so the split is integer work; the
+// binning only has to be the same for every body and monotone. Rounding moves
+// a coordinate by at most 2^-25 cells, and contacts are at most
+// H / (1 + 1e-6) apart, so the cells of a contact's centres differ by at most
+// one. Coordinates beyond 2^27 cells and non-finite ones take the FP64 path.
+__device__ __noinline__ float2 bin_slow(double x, double H, double invH) {
+  const int c = (int)floor(x * invH);
+  return make_float2(__int_as_float(c), (float)(x - (double)c * H));
+}
+__device__ __forceinline__ void bin_axis(double x, double H, double invH, int &c, float &off) {
+  constexpr uint32_t BIAS_HI = 0x41B80000u; // 1.5 * 2^28
+  const double u = fma(x, invH, __hiloint2double((int)BIAS_HI, 0));
+  const uint32_t hi = (uint32_t)__double2hiint(u), lo = (uint32_t)__double2loint(u);
+  if ((hi >> 20) == (BIAS_HI >> 20)) {
+    c = (int)__funnelshift_r(lo, hi - BIAS_HI, 24);
+    off = (float)(lo & 0xFFFFFFu) * (1.0f / 16777216.0f) * (float)H;
+    return;
   }
-  // CircleGeometry::computeCollisionAABB (CircleGeometry.cpp:22-30), q0 == q1
-  const double x = A.q[3 * i], y = A.q[3 * i + 1], ri = A.r[i];
-  const int cx = (int)floor((x - ri) * A.invH), cy = (int)floor((y - ri) * A.invH);
+  const float2 s = bin_slow(x, H, invH);
+  c = __float_as_int(s.x);
+  off = s.y;
+}
+
+// The body's record and its entry in the hash grid; counters set for the
+// step's search. x, y: the centre.
+__device__ __forceinline__ void bin_body(const BinArgs &A, int64_t i, double x, double y) {
+  const double ri = A.r[i];
+  const float rf = narrow_trunc(ri), xf = narrow_trunc(x), yf = narrow_trunc(y);
   uint32_t flags = A.fixed[i] ? REL_FIXED : 0u;
   for (int k = 0; k < A.nplanes; ++k) {
-    const double d = A.pn[k][0] * (x - A.px[k][0]) + A.pn[k][1] * (y - A.px[k][1]);
-    if (d <= ri) flags |= REL_PLANE0 << k;
+    // n . (x - x_plane) <= r: decided in FP32 when the margin exceeds the
+    // error of truncated coordinates and FP32 sums (under 1e-6 of the terms),
+    // else in FP64 as the reference does
+    const float ex = xf - A.pxf[k][0], ey = yf - A.pxf[k][1];
+    const float gap = A.pnf[k][0] * ex + A.pnf[k][1] * ey - rf;
+    const float err = 1.0e-6f * (fabsf(xf) + fabsf(A.pxf[k][0]) + fabsf(yf) +
+                                 fabsf(A.pxf[k][1]) + rf);
+    bool on;
+    if (fabsf(gap) > err) {
+      on = gap < 0.0f;
+    } else {
+      const double d = A.pn[k][0] * (x - A.px[k][0]) + A.pn[k][1] * (y - A.px[k][1]);
+      on = d <= ri;
+    }
+    if (on) flags |= REL_PLANE0 << k;
   }
   // StaticDrumCircleConstraint::isActive (StaticDrumCircleConstraint.cpp:7-13):
   // |x_drum - x|^2 >= (r_drum - r)^2; drum k is static object nplanes + k
@@ -181,26 +287,30 @@ __global__ void kd_bodies_home(HomeArgs A) {
     const double ex = A.dx[k][0] - x, ey = A.dx[k][1] - y, g = A.dr[k] - ri;
     if (ex * ex + ey * ey >= g * g) flags |= REL_PLANE0 << (A.nplanes + k);
   }
-  // one 32-byte record: the FP32 part, then the home cell
-  A.rec[2 * i] = make_float4((float)(x - (double)cx * A.H), (float)(y - (double)cy * A.H),
-                             (float)ri, __uint_as_float(flags));
-  A.rec[2 * i + 1] = make_float4(__int_as_float(cx), __int_as_float(cy), 0.0f, 0.0f);
-  atomicAdd(&A.bucket_count[cell_hash(cx, cy, A.mask)], 1);
+  int cx, cy;
+  float ox, oy;
+  bin_axis(x, A.H, A.invH, cx, ox);
+  bin_axis(y, A.H, A.invH, cy, oy);
+  const int next = atomicExch(&A.heads[cell_hash(cx, cy, A.mask)], (int)i);
+  A.rec[2 * i] = make_float4(ox, oy, rf, __uint_as_float(flags));
+  A.rec[2 * i + 1] =
+      make_float4(__int_as_float(cx), __int_as_float(cy), __int_as_float(next), 0.0f);
+  // fixed bodies have no contacts of their own
+  const int ns = (flags & REL_FIXED) ? 0 : __popc(flags >> 1);
+  A.pc[i] = (unsigned long long)ns;
+  A.in_count[i] = 0;
+  if (A.tiles && ns) atomicAdd(A.tiles + 4 * (i >> A.tile_shift), ns);
 }
 
-// Places each body in its bucket. bucket_pos holds the bucket starts and
-// ends up holding the bucket ends (start + count).
-__global__ void kd_fill_ends(int64_t n, uint32_t mask, const float4 *__restrict__ rec,
-                             int32_t *bucket_pos, int32_t *items, uint32_t *status) {
-  // (launched with programmatic dependence on the kernel before it)
+// Bins every body: the first step after the bodies changed. Later steps find
+// the bins made by the integration of the step before.
+__global__ void __launch_bounds__(128) kd_bin(const __grid_constant__ BinArgs A,
+                                              const double *__restrict__ q) {
   pdl_wait();
   pdl_trigger();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float4 h = rec[2 * i + 1];
-  const int p = atomicAdd(&bucket_pos[cell_hash(__float_as_int(h.x), __float_as_int(h.y), mask)], 1);
-  if (!HG_INDEX_OK(p, n, status)) return;
-  items[p] = (int32_t)i;
+  if (i >= A.n) return;
+  bin_body(A, i, q[3 * i], q[3 * i + 1]);
 }
 
 // The per-body terms of kd_integrate that change only with the masses, the
@@ -217,27 +327,32 @@ __global__ void kd_body_terms(int64_t n, double dt, double gx, double gy,
   terms[j] = make_double4(0.0 + M * gx, 0.0 + M * gy, dt * (1.0 / M), dt * (1.0 / Mi));
 }
 
-constexpr int PW = 8; // partners per body kept by the counting pass
+constexpr int PW = 8; // partners per body kept by the search
 
 struct PairArgs {
   int64_t n;
   uint32_t mask;
-  const float4 *rec; // body records of kd_bodies_home
+  const float4 *rec; // body records of bin_body
   float Hf;  // cell width in FP32
   float tol; // FP32 filter slack
-  const int32_t *bucket_end;
-  const int32_t *bucket_count;
-  const int32_t *items;
+  const int32_t *heads;
   const double *q;
   const double *r;
-  int nstatic;        // static objects: the planes, then the drums
-  int32_t *cnt;       // 3N counts [kind][body]
-  uint32_t *plist;    // PW partners per body (fixed partners flagged by bit 31)
-  int32_t *pfill;     // partners credited to each body (counting pass)
-  const int32_t *off; // 3N+1 offsets (emit pass)
-  int64_t *keys;      // emit pass output
+  int nstatic;            // static objects: the planes, then the drums
+  unsigned long long *pc; // contact counts per first body
+  int32_t *in_count;      // contacts per second body
+  uint32_t *plist;        // PW partners per body (fixed partners flagged by bit 31)
+  int4 *desc;   // per body: offsets of its static, circle-circle and kinematic
+                // contacts and of its incoming list
+  int32_t *descn; // per body: the three counts, 8 bits each
+  int32_t *in_cursor;
+  int32_t *tiles; // sums of the four counts over tiles of 2^tile_shift bodies
+  int tile_shift, ntiles;
+  bool add_tiles; // the search adds to tiles (else kd_tile_sums forms them)
+  int64_t *keys; // contact keys, sorted
   int64_t ccap;
-  const int32_t *overflow; // emit pass: set when the contacts do not fit
+  int32_t *count; // total number of contacts
+  int2 *range;    // [x, y): the circle-circle contacts
   uint32_t *status;
 };
 
@@ -268,122 +383,103 @@ __device__ __forceinline__ bool is_contact(const PairArgs &A, float4 pa, float4 
   return c0 <= 0.0;
 }
 
-// Contact enumeration for body a as the first index: circle-circle with
-// b > a non-fixed, kinematic with b fixed (any index; the reference swaps the
-// fixed body into the second slot). Fixed bodies emit none.
-//
-// A partner b overlapping a's AABB has its home cell within one cell of a's
-// (the cell width is at least every AABB's width), so the 3x3 cells around
-// a's home cell hold every candidate.
+// Walks the bucket list of cell (cx, cy) over the bodies whose home cell it
+// is (a bucket may be shared by other cells).
 template <class F>
-__device__ __forceinline__ void for_each_partner(const PairArgs &A, int a, F &&found) {
-  const float4 pa = A.rec[2 * a], ca = A.rec[2 * a + 1];
-  const int2 ha = make_int2(__float_as_int(ca.x), __float_as_int(ca.y));
-  // the nine bucket ranges first: independent loads instead of a chain
-  int bs[9], be[9];
-#pragma unroll
-  for (int c = 0; c < 9; ++c) {
-    const uint32_t bk = cell_hash(ha.x + c % 3 - 1, ha.y + c / 3 - 1, A.mask);
-    be[c] = A.bucket_end[bk];
-    bs[c] = be[c] - A.bucket_count[bk];
-  }
-#pragma unroll
-  for (int c = 0; c < 9; ++c) {
-    const int dx = c % 3 - 1, dy = c / 3 - 1;
-    const int cx = ha.x + dx, cy = ha.y + dy;
-    for (int k = bs[c]; k < be[c]; ++k) {
-      if (!HG_INDEX_OK(k, A.n, A.status)) break;
-      const int b = A.items[k];
-      if (!HG_INDEX_OK(b, A.n, A.status)) continue;
-      if (b == a) continue;
-      const float4 pb = A.rec[2 * b], cb = A.rec[2 * b + 1];
-      if (__float_as_int(cb.x) != cx || __float_as_int(cb.y) != cy)
-        continue; // bucket shared by another cell
-      const bool bf = (__float_as_uint(pb.w) & REL_FIXED) != 0u;
-      if (!(b > a || bf)) continue;
-      if (!is_contact(A, pa, pb, dx, dy, a, b)) continue;
-      found(b, bf);
-    }
+__device__ __forceinline__ void for_each_in_cell(const PairArgs &A, int cx, int cy, F &&body) {
+  int b = A.heads[cell_hash(cx, cy, A.mask)];
+  // (a list holds each body once: the bound on the steps is never reached)
+  for (int64_t left = A.n; b >= 0 && left > 0; --left) {
+    if (!HG_INDEX_OK(b, A.n, A.status)) return;
+    const float4 pb = A.rec[2 * b], cb = A.rec[2 * b + 1];
+    if (__float_as_int(cb.x) == cx && __float_as_int(cb.y) == cy) body(b, pb);
+    b = __float_as_int(cb.z);
   }
 }
 
-// Counting pass over half of each neighbourhood: the home cell and the four
-// cells after it in (dy, dx) order. A pair of bodies in different cells is
-// met from exactly one of them (the offset from one home cell to the other is
-// in the half, its negative is not); a pair within one cell is met from both
-// and kept from the lower index. Each contact is credited to its first body
-// (the lower index of two free bodies, the free body of a free-fixed pair,
-// none for two fixed bodies) with atomics: per-kind counts, capped at MAXP,
-// and the first PW partners in plist (in no particular order; the emission
-// pass sorts them). The survivors of the FP32 filter take the same FP64 tests
-// as the full search, which are symmetric in the two bodies.
+// Contact enumeration for body a as the first index: circle-circle with
+// b > a non-fixed, kinematic with b fixed (any index; the reference swaps the
+// fixed body into the second slot). Fixed bodies emit none. The 3x3 cells
+// around a's home cell hold every candidate.
+template <class F>
+__device__ __forceinline__ void for_each_partner(const PairArgs &A, int a, F &&found) {
+  const float4 pa = A.rec[2 * a], ca = A.rec[2 * a + 1];
+  for (int dy = -1; dy <= 1; ++dy)
+    for (int dx = -1; dx <= 1; ++dx)
+      for_each_in_cell(A, __float_as_int(ca.x) + dx, __float_as_int(ca.y) + dy,
+                       [&](int b, float4 pb) {
+                         if (b == a) return;
+                         const bool bf = (__float_as_uint(pb.w) & REL_FIXED) != 0u;
+                         if (!(b > a || bf)) return;
+                         if (is_contact(A, pa, pb, dx, dy, a, b)) found(b, bf);
+                       });
+}
+
+// Search over half of each neighbourhood: the home cell and the four cells
+// after it in (dy, dx) order. A pair of bodies in different cells is met from
+// exactly one of them (the offset from one home cell to the other is in the
+// half, its negative is not); a pair within one cell is met from both and
+// kept from the lower index. Each contact is credited to its first body (the
+// lower index of two free bodies, the free body of a free-fixed pair, none
+// for two fixed bodies): the count of its kind and the first PW partners in
+// plist (in no particular order; the emission pass sorts them).
+// Circle-circle contacts also count as incoming at their second body.
 
 __device__ __forceinline__ void credit(const PairArgs &A, int first, int second, bool kin,
                                        bool &overflow) {
   if (!HG_INDEX_OK(first, A.n, A.status)) return;
-  int32_t *c = A.cnt + (kin ? 2 : 1) * A.n + first;
-  if (atomicAdd(c, 1) >= MAXP) {
-    atomicSub(c, 1);
-    overflow = true;
-    return;
+  const unsigned long long p = atomicAdd(A.pc + first, 1ull << (kin ? PC_KIN : PC_CC));
+  const int ncc = pc_found_cc(p), nkin = pc_found_kin(p);
+  const bool kept = (kin ? nkin : ncc) < MAXP;
+  overflow |= !kept;
+  if (ncc + nkin < PW)
+    A.plist[(int64_t)first * PW + ncc + nkin] = (uint32_t)second | (kin ? 0x80000000u : 0u);
+  if (!kin) atomicAdd(A.in_count + second, 1);
+  if (A.add_tiles) {
+    if (kept) atomicAdd(A.tiles + 4 * (int64_t)(first >> A.tile_shift) + (kin ? 2 : 1), 1);
+    if (!kin) atomicAdd(A.tiles + 4 * (int64_t)(second >> A.tile_shift) + 3, 1);
   }
-  const int slot = atomicAdd(A.pfill + first, 1);
-  if (slot < PW) A.plist[(int64_t)first * PW + slot] = (uint32_t)second | (kin ? 0x80000000u : 0u);
 }
 
 // cell c of the half neighbourhood: (0, 0), (1, 0), (-1, 1), (0, 1), (1, 1)
 __device__ __forceinline__ int half_dx(int c) { return c == 0 ? 0 : (c == 1 ? 1 : c - 3); }
 __device__ __forceinline__ int half_dy(int c) { return c >= 2 ? 1 : 0; }
 
+__device__ __forceinline__ void search_cell(const PairArgs &A, int a, int c, float4 pa, float4 ca,
+                                            bool &overflow) {
+  const bool af = (__float_as_uint(pa.w) & REL_FIXED) != 0u;
+  const int dx = half_dx(c), dy = half_dy(c);
+  for_each_in_cell(A, __float_as_int(ca.x) + dx, __float_as_int(ca.y) + dy,
+                   [&](int b, float4 pb) {
+                     if (b == a || (c == 0 && b < a)) return;
+                     const bool bf = (__float_as_uint(pb.w) & REL_FIXED) != 0u;
+                     if (af && bf) return;
+                     if (!is_contact(A, pa, pb, dx, dy, a, b)) return;
+                     if (af) credit(A, b, a, true, overflow);
+                     else if (bf) credit(A, a, b, true, overflow);
+                     else credit(A, min(a, b), max(a, b), false, overflow);
+                   });
+}
+
 // One thread per body over its five cells: fewer loads of the body's own
-// record than kd_pairs_count when the bodies alone fill the GPU.
-__global__ void kd_pairs_count_body(PairArgs A) {
+// record than kd_pairs when the bodies alone fill the GPU.
+__global__ void kd_pairs_body(PairArgs A) {
   // (launched with programmatic dependence on the kernel before it)
   pdl_wait();
   pdl_trigger();
-  const int64_t n = A.n;
   const int a = (int)(blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
-  if (a >= n) return;
+  if (a >= A.n) return;
   const float4 pa = A.rec[2 * a], ca = A.rec[2 * a + 1];
-  const uint32_t flags = __float_as_uint(pa.w);
-  const bool af = (flags & REL_FIXED) != 0u;
-  if (!af) A.cnt[a] = __popc(flags >> 1); // static planes
-  const int2 ha = make_int2(__float_as_int(ca.x), __float_as_int(ca.y));
-  int bs[5], be[5];
-#pragma unroll
-  for (int c = 0; c < 5; ++c) {
-    const uint32_t bk = cell_hash(ha.x + half_dx(c), ha.y + half_dy(c), A.mask);
-    be[c] = A.bucket_end[bk];
-    bs[c] = be[c] - A.bucket_count[bk];
-  }
   bool overflow = false;
 #pragma unroll
-  for (int c = 0; c < 5; ++c) {
-    const int dx = half_dx(c), dy = half_dy(c);
-    const int cx = ha.x + dx, cy = ha.y + dy;
-    for (int k = bs[c]; k < be[c]; ++k) {
-      if (!HG_INDEX_OK(k, n, A.status)) break;
-      const int b = A.items[k];
-      if (!HG_INDEX_OK(b, n, A.status)) continue;
-      if (b == a || (c == 0 && b < a)) continue;
-      const float4 pb = A.rec[2 * b], cb = A.rec[2 * b + 1];
-      if (__float_as_int(cb.x) != cx || __float_as_int(cb.y) != cy)
-        continue; // bucket shared by another cell
-      const bool bf = (__float_as_uint(pb.w) & REL_FIXED) != 0u;
-      if (af && bf) continue;
-      if (!is_contact(A, pa, pb, dx, dy, a, b)) continue;
-      if (af) credit(A, b, a, true, overflow);
-      else if (bf) credit(A, a, b, true, overflow);
-      else credit(A, min(a, b), max(a, b), false, overflow);
-    }
-  }
+  for (int c = 0; c < 5; ++c) search_cell(A, a, c, pa, ca, overflow);
   if (overflow) atomicOr(A.status, (uint32_t)HG_STATUS_CELL_OVERFLOW);
 }
 
 // One thread per (body, cell of the half neighbourhood): thread t takes cell
 // t / n of body t % n, so a warp's lanes read consecutive bodies' records and
-// each thread follows one bucket instead of five.
-__global__ void kd_pairs_count(PairArgs A) {
+// each thread follows one list instead of five.
+__global__ void kd_pairs(PairArgs A) {
   // (launched with programmatic dependence on the kernel before it)
   pdl_wait();
   pdl_trigger();
@@ -392,47 +488,150 @@ __global__ void kd_pairs_count(PairArgs A) {
   if (t >= 5 * n) return;
   const int c = (int)(t / n);
   const int a = (int)(t - (int64_t)c * n);
-  const float4 pa = A.rec[2 * a], ca = A.rec[2 * a + 1];
-  const uint32_t flags = __float_as_uint(pa.w);
-  const bool af = (flags & REL_FIXED) != 0u;
-  if (c == 0 && !af) A.cnt[a] = __popc(flags >> 1); // static planes
-  const int dx = half_dx(c), dy = half_dy(c);
-  const int cx = __float_as_int(ca.x) + dx, cy = __float_as_int(ca.y) + dy;
-  const uint32_t bk = cell_hash(cx, cy, A.mask);
-  const int be = A.bucket_end[bk], bs = be - A.bucket_count[bk];
-  if (bs >= be) return;
   bool overflow = false;
-  for (int k = bs; k < be; ++k) {
-    if (!HG_INDEX_OK(k, n, A.status)) break;
-    const int b = A.items[k];
-    if (!HG_INDEX_OK(b, n, A.status)) continue;
-    if (b == a || (c == 0 && b < a)) continue;
-    const float4 pb = A.rec[2 * b], cb = A.rec[2 * b + 1];
-    if (__float_as_int(cb.x) != cx || __float_as_int(cb.y) != cy)
-      continue; // bucket shared by another cell
-    const bool bf = (__float_as_uint(pb.w) & REL_FIXED) != 0u;
-    if (af && bf) continue;
-    if (!is_contact(A, pa, pb, dx, dy, a, b)) continue;
-    if (af) credit(A, b, a, true, overflow);
-    else if (bf) credit(A, a, b, true, overflow);
-    else credit(A, min(a, b), max(a, b), false, overflow);
-  }
+  search_cell(A, a, c, A.rec[2 * a], A.rec[2 * a + 1], overflow);
   if (overflow) atomicOr(A.status, (uint32_t)HG_STATUS_CELL_OVERFLOW);
 }
 
-// Emission pass: sorted per-body contact keys at the scanned offsets. Lists
-// of at most PW partners come from the counting pass; longer ones are
-// searched again (the same partners, the first MAXP of each kind).
-__global__ void kd_pairs_emit(PairArgs A) {
+__device__ __forceinline__ int warp_sum(int x) {
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
+  return x;
+}
+
+// Sums of the contact counts (static, circle-circle, kinematic, incoming)
+// over tiles of 2^shift bodies, one CTA per tile.
+__global__ void __launch_bounds__(256) kd_tile_sums(int64_t n, int shift,
+                                                    const unsigned long long *__restrict__ pc,
+                                                    const int32_t *__restrict__ in_count,
+                                                    int32_t *tiles) {
   // (launched with programmatic dependence on the kernel before it)
   pdl_wait();
   pdl_trigger();
+  __shared__ int s_sum[8][4];
+  const int64_t b0 = (int64_t)blockIdx.x << shift;
+  const int64_t b1 = min(n, b0 + ((int64_t)1 << shift));
+  int s[4] = {0, 0, 0, 0};
+  for (int64_t i = b0 + threadIdx.x; i < b1; i += 256) {
+    const unsigned long long p = pc[i];
+    s[0] += pc_static(p);
+    s[1] += pc_cc(p);
+    s[2] += pc_kin(p);
+    s[3] += in_count[i];
+  }
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int t = warp_sum(s[k]);
+    if (lane == 0) s_sum[wid][k] = t;
+  }
+  __syncthreads();
+  if (threadIdx.x < 4) {
+    int t = 0;
+    for (int w = 0; w < 8; ++w) t += s_sum[w][threadIdx.x];
+    tiles[4 * (int64_t)blockIdx.x + threadIdx.x] = t;
+  }
+}
+
+// Emission pass, one CTA per NT bodies: the offsets of their contacts, then
+// their sorted contact keys. The offsets need no scan launches: a CTA sums
+// the tile counts before its bodies itself (at most MAX_TILES of them), then
+// the bodies between its tile's start and its first body, and scans its own.
+// When the total exceeds the contact capacity the step keeps no contacts and
+// reports HG_STATUS_CONTACT_OVERFLOW instead of writing past the buffers.
+// Partner lists of at most PW bodies come from the search; longer ones are
+// searched again (the same partners, the first MAXP of each kind).
+constexpr int MAX_TILES = 1024;
+template <int NT> __global__ void __launch_bounds__(NT) kd_pairs_emit(PairArgs A) {
+  // (launched with programmatic dependence on the kernel before it)
+  pdl_wait();
+  pdl_trigger();
+  constexpr int NW = NT / 32;
+  __shared__ int s_sum[NW][7];
+  __shared__ unsigned long long s_scan[NW];
+  __shared__ int s_in[NW];
   const int64_t n = A.n;
-  const int a = (int)(blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
-  if (a >= n) return;
-  const int npl = A.cnt[a], ncc = A.cnt[n + a], nkin = A.cnt[2 * n + a];
-  if (npl + ncc + nkin == 0 || *A.overflow) return;
-  const int64_t o0 = A.off[a], o1 = A.off[n + a], o2 = A.off[2 * n + a];
+  const int64_t b0 = blockIdx.x * (int64_t)NT;
+  const int64_t a64 = b0 + threadIdx.x;
+  const int a = (int)a64;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  unsigned long long p = a64 < n ? A.pc[a] : 0ull;
+  const int nin = a64 < n ? A.in_count[a] : 0;
+  // [0, 3): totals of the three kinds; [3, 7): counts before this CTA
+  int sum[7] = {0, 0, 0, 0, 0, 0, 0};
+  const int64_t t0 = b0 >> A.tile_shift;
+  for (int t = threadIdx.x; t < A.ntiles; t += NT) {
+    const int4 v = reinterpret_cast<const int4 *>(A.tiles)[t];
+    const bool before = t < t0;
+    sum[0] += v.x;
+    sum[1] += v.y;
+    sum[2] += v.z;
+    sum[3] += before ? v.x : 0;
+    sum[4] += before ? v.y : 0;
+    sum[5] += before ? v.z : 0;
+    sum[6] += before ? v.w : 0;
+  }
+  for (int64_t i = (t0 << A.tile_shift) + threadIdx.x; i < b0; i += NT) {
+    const unsigned long long pi = A.pc[i];
+    sum[3] += pc_static(pi);
+    sum[4] += pc_cc(pi);
+    sum[5] += pc_kin(pi);
+    sum[6] += A.in_count[i];
+  }
+  // the CTA's own counts: three 21-bit fields scanned in one word
+  const unsigned long long own = (unsigned long long)pc_static(p) |
+                                 (unsigned long long)pc_cc(p) << 21 |
+                                 (unsigned long long)pc_kin(p) << 42;
+  unsigned long long inc = own;
+  int inc_in = nin;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const unsigned long long x = __shfl_up_sync(0xffffffffu, inc, d);
+    const int y = __shfl_up_sync(0xffffffffu, inc_in, d);
+    if (lane >= d) {
+      inc += x;
+      inc_in += y;
+    }
+  }
+  if (lane == 31) {
+    s_scan[wid] = inc;
+    s_in[wid] = inc_in;
+  }
+#pragma unroll
+  for (int k = 0; k < 7; ++k) {
+    const int t = warp_sum(sum[k]);
+    if (lane == 0) s_sum[wid][k] = t;
+  }
+  __syncthreads();
+  unsigned long long ex = inc - own;
+  int ex_in = inc_in - nin;
+#pragma unroll
+  for (int k = 0; k < 7; ++k) sum[k] = 0;
+#pragma unroll
+  for (int w = 0; w < NW; ++w) {
+    if (w < wid) {
+      ex += s_scan[w];
+      ex_in += s_in[w];
+    }
+#pragma unroll
+    for (int k = 0; k < 7; ++k) sum[k] += s_sum[w][k];
+  }
+  const bool over = (int64_t)sum[0] + sum[1] + sum[2] > A.ccap;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (over) atomicOr(A.status, (uint32_t)HG_STATUS_CONTACT_OVERFLOW);
+    *A.count = over ? 0 : sum[0] + sum[1] + sum[2];
+    *A.range = over ? make_int2(0, 0) : make_int2(sum[0], sum[0] + sum[1]);
+  }
+  if (a64 >= n) return;
+  if (over) p = 0ull;
+  const int npl = pc_static(p), ncc = pc_cc(p), nkin = pc_kin(p);
+  const int64_t o0 = sum[3] + (int)(ex & 0x1FFFFFu);
+  const int64_t o1 = (int64_t)sum[0] + sum[4] + (int)((ex >> 21) & 0x1FFFFFu);
+  const int64_t o2 = (int64_t)sum[0] + sum[1] + sum[5] + (int)(ex >> 42);
+  A.desc[a] = over ? make_int4(0, 0, 0, 0) : make_int4((int)o0, (int)o1, (int)o2, sum[6] + ex_in);
+  A.descn[a] = npl | ncc << 8 | nkin << 16;
+  A.in_cursor[a] = 0;
+  if (npl + ncc + nkin == 0) return;
   if (o0 + npl > A.ccap || o1 + ncc > A.ccap || o2 + nkin > A.ccap) {
     atomicOr(A.status, (uint32_t)HG_STATUS_CONTACT_OVERFLOW);
     return;
@@ -440,7 +639,10 @@ __global__ void kd_pairs_emit(PairArgs A) {
   const uint32_t flags = __float_as_uint(A.rec[2 * a].w);
   int j = 0;
   for (int k = 0; k < A.nstatic; ++k)
-    if (flags & (REL_PLANE0 << k)) A.keys[o0 + j++] = ckey(K_PLANE, a, k);
+    if (flags & (REL_PLANE0 << k)) {
+      if (j < npl) A.keys[o0 + j] = ckey(K_PLANE, a, k);
+      ++j;
+    }
   if (ncc + nkin <= PW) {
     // odd-even transposition sort of the flagged indices: circle-circle
     // partners ascending, then the fixed ones ascending
@@ -474,36 +676,8 @@ __global__ void kd_pairs_emit(PairArgs A) {
   });
   sort_small(cc, mc);
   sort_small(kin, mk);
-  for (int k = 0; k < mc; ++k) A.keys[o1 + k] = ckey(K_CC, a, cc[k]);
-  for (int k = 0; k < mk; ++k) A.keys[o2 + k] = ckey(K_KIN, a, kin[k]);
-}
-
-// Capacity guard between the counting and the emission pass: when the total
-// exceeds the contact capacity the step keeps no contacts (and reports
-// HG_STATUS_CONTACT_OVERFLOW) instead of writing past the buffers.
-__global__ void kd_check_capacity(int64_t n, const int32_t *__restrict__ off, int64_t ccap,
-                                  int32_t *overflow, uint32_t *status) {
-  // (launched with programmatic dependence on the kernel before it)
-  pdl_wait();
-  pdl_trigger();
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    const bool over = (int64_t)off[3 * n] > ccap;
-    *overflow = over ? 1 : 0;
-    if (over) atomicOr(status, (uint32_t)HG_STATUS_CONTACT_OVERFLOW);
-  }
-}
-
-__global__ void kd_drop_if_overflow(int64_t n, const int32_t *__restrict__ overflow,
-                                    int32_t *cnt, int32_t *off) {
-  // (launched with programmatic dependence on the kernel before it)
-  pdl_wait();
-  pdl_trigger();
-  if (!*overflow) return;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= 3 * n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    cnt[i] = 0;
-    off[i] = 0;
-  }
+  for (int k = 0; k < min(mc, ncc); ++k) A.keys[o1 + k] = ckey(K_CC, a, cc[k]);
+  for (int k = 0; k < min(mk, nkin); ++k) A.keys[o2 + k] = ckey(K_KIN, a, kin[k]);
 }
 
 struct ContactArgs {
@@ -519,14 +693,36 @@ struct ContactArgs {
   const int32_t *count; // device count (total contacts)
   const int64_t *keys;
   double *rec;
+  // per contact, for the integration: the total force and its torques about
+  // the first and the second body (double4 in FP64, float4 in MIXED)
+  void *load;
+  const int4 *desc; // offsets of the bodies' contact lists (incoming: w)
+  int32_t *in_cursor, *in_list;
+  // the previous step's contacts; old_desc (with old_descn) gives each
+  // body's lists in them, or is nullptr when the bodies were renumbered since
   const int64_t *old_keys;
   const double *old_rec;
-  const int32_t *old_count; // device count of the previous step's contacts
+  const int32_t *old_count;
+  const int4 *old_desc;
+  const int32_t *old_descn;
+  // cleared for the next step: the search is done with them
+  int32_t *heads, *tiles;
+  int64_t nheads;
   int64_t ccap;
   uint32_t *status;
 };
 
-__device__ __forceinline__ int find_old(const ContactArgs &C, int64_t key) {
+// The previous step's contact with this key: among its first body's own
+// contacts of the kind (a few consecutive keys), or by binary search.
+__device__ __forceinline__ int find_old(const ContactArgs &C, int64_t key, int kind, int a) {
+  if (C.old_desc) {
+    const int4 d = C.old_desc[a];
+    const int n = (C.old_descn[a] >> (8 * kind)) & 0xFF;
+    const int o = kind == K_PLANE ? d.x : (kind == K_CC ? d.y : d.z);
+    for (int i = 0; i < n; ++i)
+      if (C.old_keys[o + i] == key) return o + i;
+    return -1;
+  }
   int lo = 0, hi = min((int64_t)*C.old_count, C.ccap) - 1;
   while (lo <= hi) {
     const int mid = (lo + hi) >> 1;
@@ -544,20 +740,89 @@ __device__ __forceinline__ double second_root(double a, double b, double c, doub
   return (-b + ds) / (2.0 * a);
 }
 
-__global__ void kd_contacts(ContactArgs C) {
+// Quotients by one divisor. With y = 1 / b rounded to nearest, the multiply
+// q = a y followed by the residual correction q + (a - q b) y in two FMAs
+// gives a / b rounded to nearest (P. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", 1990), three FP64
+// instructions in place of a division's eight. Operands near the ends of the
+// exponent range are divided.
+struct Divisor {
+  double b, y;
+  bool ok;
+};
+__device__ __forceinline__ Divisor divisor(double b) {
+  const uint32_t e = ((uint32_t)__double2hiint(b) >> 20) & 0x7FFu;
+  return {b, 1.0 / b, e - 823u <= 400u};
+}
+__device__ __noinline__ double divide(double a, double b) { return a / b; }
+__device__ __forceinline__ double quot(double a, const Divisor &d) {
+  const uint32_t hi = (uint32_t)__double2hiint(a);
+  const double q = a * d.y;
+  const double z = fma(fma(-q, d.b, a), d.y, q);
+  if (d.ok && ((hi >> 20) & 0x7FFu) - 300u <= 1400u) return z;
+  if (d.ok && (((hi << 1) | (uint32_t)__double2loint(a)) == 0u)) return q; // a zero's sign
+  return divide(a, d.b);
+}
+
+constexpr int CONTACT_THREADS = 128;
+constexpr int CONTACT_WARPS = CONTACT_THREADS / 32;
+constexpr int RW2 = RW / 2; // a record in 16-byte pieces
+static_assert(RW % 2 == 0, "records are moved in 16-byte pieces");
+
+// The contact law's grid-stride loop, shared by the two precisions. Contacts
+// go to the warps in chunks of 32, chunk c to CTA c mod gridDim, so that few
+// contacts spread over all SMs (the law is bound by each SM's FP64 pipe).
+// law(k, key, kind, a, b, out) computes contact k's record into out (the
+// caller's shared-memory row). A record is 176 bytes: written by its lane it
+// would be 22 stores of 8 bytes in 32 different sectors each, so the warp's
+// records are staged in shared memory and written as contiguous 16-byte pieces.
+template <class Law>
+__device__ __forceinline__ void for_each_contact(const ContactArgs &C, Law &&law) {
+  __shared__ __align__(16) double s_rec[CONTACT_WARPS][32 * RW];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t tid = blockIdx.x * (int64_t)CONTACT_THREADS + threadIdx.x;
+  const int64_t nthreads = (int64_t)gridDim.x * CONTACT_THREADS;
+  for (int64_t i = tid; i < C.nheads / 4; i += nthreads)
+    reinterpret_cast<int4 *>(C.heads)[i] = make_int4(-1, -1, -1, -1);
+  for (int64_t i = tid; i < MAX_TILES; i += nthreads)
+    reinterpret_cast<int4 *>(C.tiles)[i] = make_int4(0, 0, 0, 0);
+  const int64_t total = min((int64_t)*C.count, C.ccap);
+  double *out = s_rec[wid] + lane * RW;
+  for (int64_t c = blockIdx.x + (int64_t)gridDim.x * wid; 32 * c < total;
+       c += (int64_t)gridDim.x * CONTACT_WARPS) {
+    const int64_t k = 32 * c + lane;
+    if (k < total) {
+      const int64_t key = C.keys[k];
+      const int kind = (int)(key >> 60);
+      const int a = (int)((key >> 30) & 0x3FFFFFFF);
+      const int b = (int)(key & 0x3FFFFFFF);
+      if (HG_INDEX_OK(a, C.n, C.status) &&
+          HG_INDEX_OK(b, kind == K_PLANE ? (int64_t)(C.nplanes + C.ndrums) : C.n, C.status)) {
+        if (kind == K_CC) { // the second body's list of incoming contacts
+          const int64_t o = (int64_t)C.desc[b].w + atomicAdd(&C.in_cursor[b], 1);
+          if (o < C.ccap) C.in_list[o] = (int32_t)k;
+        }
+        law(k, key, kind, a, b, out);
+      }
+    }
+    __syncwarp();
+    const int pieces = (int)min((int64_t)32, total - 32 * c) * RW2;
+    const double2 *src = reinterpret_cast<const double2 *>(s_rec[wid]);
+    double2 *dst = reinterpret_cast<double2 *>(C.rec + 32 * c * RW);
+    for (int i = lane; i < pieces; i += 32) dst[i] = src[i];
+    __syncwarp();
+  }
+}
+
+__device__ __forceinline__ void put2(double *out, int i, double x, double y) {
+  reinterpret_cast<double2 *>(out)[i] = make_double2(x, y);
+}
+
+__global__ void __launch_bounds__(CONTACT_THREADS) kd_contacts(const __grid_constant__ ContactArgs C) {
   // (launched with programmatic dependence on the kernel before it)
   pdl_wait();
   pdl_trigger();
-  const int64_t total = min((int64_t)*C.count, C.ccap);
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t key = C.keys[k];
-    const int kind = (int)(key >> 60);
-    const int a = (int)((key >> 30) & 0x3FFFFFFF);
-    const int b = (int)(key & 0x3FFFFFFF);
-    if (!HG_INDEX_OK(a, C.n, C.status) ||
-        !HG_INDEX_OK(b, kind == K_PLANE ? (int64_t)(C.nplanes + C.ndrums) : C.n, C.status))
-      continue;
+  for_each_contact(C, [&](int64_t k, int64_t key, int kind, int a, int b, double *out) {
     const D2 qa{C.q[3 * a], C.q[3 * a + 1]};
     const D2 va{C.v[3 * a], C.v[3 * a + 1]};
     const double wa = C.v[3 * a + 2];
@@ -586,7 +851,7 @@ __global__ void kd_contacts(ContactArgs C) {
       n = D2{C.pn[b][0], C.pn[b][1]};
       cp = dsub(qa, dscl(ra, n));
       weight = C.weighted ? C.w[a] : 1.0;
-      depth = fmin(0.0, ddot(n, dsub(qa, xp)) - ra);
+      depth = min_zero(ddot(n, dsub(qa, xp)) - ra);
       r0 = dscl(-ra, n);
       const D2 t0{-r0.y, r0.x};
       const D2 arm = dsub(cp, xp);
@@ -596,12 +861,18 @@ __global__ void kd_contacts(ContactArgs C) {
     } else {
       const D2 qb{C.q[3 * b], C.q[3 * b + 1]};
       const double rb = C.r[b];
-      n = dnormalized(dsub(qa, qb));
-      depth = fmin(0.0, dnorm(dsub(qa, qb)) - ra - rb);
+      const D2 d = dsub(qa, qb);
+      const double d2 = dsq(d), dist = sqrt(d2);
+      n = d;
+      if (d2 > 0.0) {
+        const Divisor len = divisor(dist);
+        n = D2{quot(d.x, len), quot(d.y, len)};
+      }
+      depth = min_zero(dist - ra - rb);
       const D2 vb{C.v[3 * b], C.v[3 * b + 1]};
       const double wb = C.v[3 * b + 2];
       if (kind == K_CC) { // CircleCircleConstraint.cpp:171-233
-        cp = dadd(qa, dscl(ra / (ra + rb), dsub(qb, qa)));
+        cp = dadd(qa, dscl(ra / (ra + rb), D2{-d.x, -d.y}));
         weight = C.weighted ? (C.w[a] + C.w[b]) * 0.5 : 1.0;
         r0 = dsub(cp, qa);
         r1 = dsub(cp, qb);
@@ -620,123 +891,107 @@ __global__ void kd_contacts(ContactArgs C) {
     }
     // tangential spring carry
     D2 ds;
-    const int o = find_old(C, key);
+    const int o = find_old(C, key, kind, a);
     if (o >= 0) {
-      ds = D2{C.old_rec[(int64_t)o * RW + 6], C.old_rec[(int64_t)o * RW + 7]};
-      ds = dadd(ds, dscl(C.dt, vrel));
+      const double2 old = *reinterpret_cast<const double2 *>(C.old_rec + (int64_t)o * RW + 6);
+      ds = dadd(D2{old.x, old.y}, dscl(C.dt, vrel));
     } else {
       ds = dscl(C.dt, vrel);
     }
     ds = dsub(ds, dscl(ddot(n, ds), n));
     // penalty force (PenaltyImpactFrictionMap.cpp:616-1081)
     const double w = weight;
+    // (products with a weight of 1 are the products without it)
+    const bool one = w == 1.0;
+    const double nkn = one ? -C.kn : -C.kn * w, nkt = one ? -C.kt : -C.kt * w;
+    const double hgn = 0.5 * C.gn * w, hgt = 0.5 * C.gt * w;
     const D2 vt = dsub(vrel, dscl(ddot(n, vrel), n));
     const D2 vn = dsub(vrel, vt);
-    const D2 fn = dsub(dscl(-C.kn * w * depth, n), dscl(0.5 * C.gn * w, vn));
-    D2 ft = dsub(dscl(-C.kt * w, ds), dscl(0.5 * C.gt * w, vt));
-    const double mu_fn = C.mu * dnorm(fn);
-    const double ftn = dnorm(ft);
-    if (0.5 * C.gt * w * dnorm(vt) > mu_fn) {
-      ds = D2{0.0, 0.0};
-      ft = dscl(-0.5 * C.gt * w, vt);
-      ft = dnormalized(ft);
-      ft = dscl(mu_fn, ft);
-    } else if (ftn > mu_fn) {
-      const double qa_ = C.kt * w * C.kt * w * dsq(ds);
-      const double qb_ = C.kt * w * C.gt * w * ddot(ds, vt);
-      const double qc_ = 0.25 * C.gt * w * C.gt * w * ddot(vt, vt) - C.mu * C.mu * dsq(fn);
-      const double dscr = qb_ * qb_ - 4 * qa_ * qc_;
-      const double root1 = second_root(qa_, qb_, qc_, sqrt(dscr));
-      const D2 nds = dscl(root1, ds);
-      ft = dsub(dscl(-C.kt * w, nds), dscl(0.5 * C.gt * w, vt));
-      ds = nds;
+    const D2 fn = dsub(dscl(nkn * depth, n), dscl(hgn, vn));
+    D2 ft = dsub(dscl(nkt, ds), dscl(hgt, vt));
+    // Coulomb's law compares gamma_t w / 2 |vt| and |ft| with mu |fn|. FP32
+    // estimates of the three, within 1e-6 of them, decide all but close calls:
+    // a sticking contact then needs none of the three square roots, a sliding
+    // one none but the root of its quadratic.
+    const float vt2 = narrow_trunc(vt.x) * narrow_trunc(vt.x) + narrow_trunc(vt.y) * narrow_trunc(vt.y);
+    const float fn2 = narrow_trunc(fn.x) * narrow_trunc(fn.x) + narrow_trunc(fn.y) * narrow_trunc(fn.y);
+    const float ft2 = narrow_trunc(ft.x) * narrow_trunc(ft.x) + narrow_trunc(ft.y) * narrow_trunc(ft.y);
+    const float cap32 = narrow_trunc(C.mu) * sqrtf(fn2);
+    const float drag32 = narrow_trunc(hgt) * sqrtf(vt2), ft32 = sqrtf(ft2);
+    const bool sure = fn2 > 1.0e-24f && fn2 < 1.0e24f && vt2 > 1.0e-24f && vt2 < 1.0e24f &&
+                      ft2 > 1.0e-24f && ft2 < 1.0e24f && cap32 > 1.0e-12f;
+    const bool stick_drag = sure && drag32 < cap32 * 0.99999f; // not slipping
+    if (!(stick_drag && ft32 < cap32 * 0.99999f)) {
+      bool slip = false, slide = true;
+      double mu_fn = 0.0;
+      if (!(stick_drag && ft32 > cap32 * 1.00001f)) {
+        mu_fn = C.mu * dnorm(fn);
+        slip = hgt * dnorm(vt) > mu_fn;
+        slide = dnorm(ft) > mu_fn;
+      }
+      if (slip) {
+        ds = D2{0.0, 0.0};
+        ft = dscl(-0.5 * C.gt * w, vt);
+        ft = dnormalized(ft);
+        ft = dscl(mu_fn, ft);
+      } else if (slide) {
+        const double qa_ = C.kt * w * C.kt * w * dsq(ds);
+        const double qb_ = C.kt * w * C.gt * w * ddot(ds, vt);
+        const double qc_ = 0.25 * C.gt * w * C.gt * w * ddot(vt, vt) - C.mu * C.mu * dsq(fn);
+        const double dscr = qb_ * qb_ - 4 * qa_ * qc_;
+        const double root1 = second_root(qa_, qb_, qc_, sqrt(dscr));
+        const D2 nds = dscl(root1, ds);
+        ft = dsub(dscl(-C.kt * w, nds), dscl(0.5 * C.gt * w, vt));
+        ds = nds;
+      }
     }
-    double *o_ = C.rec + k * RW;
-    o_[0] = kind;
-    o_[1] = a;
-    o_[2] = b;
-    o_[3] = depth;
-    o_[4] = n.x;
-    o_[5] = n.y;
-    o_[6] = ds.x;
-    o_[7] = ds.y;
-    o_[8] = vrel.x;
-    o_[9] = vrel.y;
-    o_[10] = r0.x;
-    o_[11] = r0.y;
-    o_[12] = r1.x;
-    o_[13] = r1.y;
-    o_[14] = weight;
-    o_[15] = cp.x;
-    o_[16] = cp.y;
-    o_[17] = fn.x;
-    o_[18] = fn.y;
-    o_[19] = ft.x;
-    o_[20] = ft.y;
-    o_[21] = 0.0;
-  }
+    const D2 f = dadd(fn, ft);
+    reinterpret_cast<double4 *>(C.load)[k] =
+        make_double4(f.x, f.y, dcross(r0, f), kind == K_CC ? dcross(r1, f) : 0.0);
+    put2(out, 0, index_f64(kind), index_f64(a));
+    put2(out, 1, index_f64(b), depth);
+    put2(out, 2, n.x, n.y);
+    put2(out, 3, ds.x, ds.y);
+    put2(out, 4, vrel.x, vrel.y);
+    put2(out, 5, r0.x, r0.y);
+    put2(out, 6, r1.x, r1.y);
+    put2(out, 7, weight, cp.x);
+    put2(out, 8, cp.y, fn.x);
+    put2(out, 9, fn.y, ft.x);
+    put2(out, 10, ft.y, 0.0);
+  });
 }
 
-__global__ void kd_in_count(int64_t n, const int32_t *__restrict__ off,
-                            const int64_t *__restrict__ keys, int32_t *in_count) {
-  // (launched with programmatic dependence on the kernel before it)
-  pdl_wait();
-  pdl_trigger();
-  // circle-circle contacts occupy [off[n], off[2n])
-  const int s = off[n], e = off[2 * n];
-  for (int64_t k = s + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < e;
-       k += (int64_t)gridDim.x * blockDim.x)
-    atomicAdd(&in_count[keys[k] & 0x3FFFFFFF], 1);
-}
-
-__global__ void kd_in_fill(int64_t n, const int32_t *__restrict__ off,
-                           const int64_t *__restrict__ keys,
-                           const int32_t *__restrict__ in_off, int32_t *in_cursor,
-                           int32_t *in_list) {
-  // (launched with programmatic dependence on the kernel before it)
-  pdl_wait();
-  pdl_trigger();
-  const int s = off[n], e = off[2 * n];
-  for (int64_t k = s + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < e;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    const int b = (int)(keys[k] & 0x3FFFFFFF);
-    in_list[in_off[b] + atomicAdd(&in_cursor[b], 1)] = (int32_t)k;
-  }
-}
-
-__global__ void kd_integrate(int64_t n, double dt, double *q, double *v,
-                             const double4 *__restrict__ terms,
-                             const uint8_t *__restrict__ fixed,
-                             const int32_t *__restrict__ cnt, const int32_t *__restrict__ off,
-                             const double *__restrict__ rec, const int32_t *__restrict__ in_count,
-                             const int32_t *__restrict__ in_off, int32_t *in_list,
-                             uint32_t *status) {
-  // (launched with programmatic dependence on the kernel before it)
-  pdl_wait();
-  pdl_trigger();
-  const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  // gravity and dt / M, dt / Mi from kd_body_terms
-  const double4 bt = terms[j];
-  double Fx = bt.x, Fy = bt.y, T = 0.0;
-  auto total = [&](int64_t k, D2 &f) {
-    const double *r = rec + k * RW;
-    f = dadd(D2{r[17], r[18]}, D2{r[19], r[20]});
-  };
-  // circle vs plane
-  for (int64_t k = off[j], e = off[j] + cnt[j]; k < e; ++k) {
-    D2 f;
-    total(k, f);
-    Fx += f.x;
-    Fy += f.y;
-    T += dcross(D2{rec[k * RW + 10], rec[k * RW + 11]}, f);
-  }
-  // circle vs circle: contributions as the second body come from first
-  // indices below j, i.e. before j's own list in the reference's loop.
-  {
-    int *lst = in_list + in_off[j];
-    const int c = in_count[j];
-    for (int i = 1; i < c; ++i) { // contact indices sorted = first indices sorted
+// Body j's contacts in the reference's order: with static objects, as the
+// second body of circle-circle contacts (their first indices lie below j, so
+// they come before j's own list in the reference's loop), as the first body,
+// and with fixed disks. apply(contact, as_second). The incoming list, filled
+// in no particular order, is sorted first.
+template <class F>
+__device__ __forceinline__ void for_each_load(int j, int4 d, int counts, int nin, int32_t *in_list,
+                                              int64_t ccap, uint32_t *status, F &&apply) {
+  for (int k = 0; k < (counts & 0xFF); ++k) apply(d.x + k, false);
+  nin = (int)min((int64_t)nin, max((int64_t)0, ccap - d.w));
+  int32_t *lst = in_list + d.w;
+  if (nin <= 4) {
+    int L[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) L[k] = k < nin ? lst[k] : 0x7FFFFFFF;
+    auto order = [&](int x, int y) {
+      const int lo = min(L[x], L[y]), hi = max(L[x], L[y]);
+      L[x] = lo;
+      L[y] = hi;
+    };
+    order(0, 1);
+    order(2, 3);
+    order(0, 2);
+    order(1, 3);
+    order(1, 2);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (k < nin && HG_INDEX_OK(L[k], ccap, status)) apply(L[k], true);
+  } else {
+    for (int i = 1; i < nin; ++i) {
       const int key = lst[i];
       int t = i - 1;
       while (t >= 0 && lst[t] > key) {
@@ -745,45 +1000,70 @@ __global__ void kd_integrate(int64_t n, double dt, double *q, double *v,
       }
       lst[t + 1] = key;
     }
-    for (int i = 0; i < c; ++i) {
-      const int64_t k = lst[i];
-      if (!HG_INDEX_OK(k, off[3 * n], status)) continue;
-      D2 f;
-      total(k, f);
-      Fx -= f.x;
-      Fy -= f.y;
-      T -= dcross(D2{rec[k * RW + 12], rec[k * RW + 13]}, f);
-    }
+    for (int i = 0; i < nin; ++i)
+      if (HG_INDEX_OK(lst[i], ccap, status)) apply(lst[i], true);
   }
-  for (int64_t k = off[n + j], e = off[n + j] + cnt[n + j]; k < e; ++k) {
-    D2 f;
-    total(k, f);
-    Fx += f.x;
-    Fy += f.y;
-    T += dcross(D2{rec[k * RW + 10], rec[k * RW + 11]}, f);
-  }
-  // kinematic circle vs circle
-  for (int64_t k = off[2 * n + j], e = off[2 * n + j] + cnt[2 * n + j]; k < e; ++k) {
-    D2 f;
-    total(k, f);
-    Fx += f.x;
-    Fy += f.y;
-    T += dcross(D2{rec[k * RW + 10], rec[k * RW + 11]}, f);
-  }
-  if (fixed[j]) Fx = Fy = T = 0.0;
+  for (int k = 0; k < ((counts >> 8) & 0xFF); ++k) apply(d.y + k, false);
+  for (int k = 0; k < ((counts >> 16) & 0xFF); ++k) apply(d.z + k, false);
+}
+
+struct IntegrateArgs {
+  int64_t n, ccap;
+  double dt;
+  double *q, *v;
+  const double4 *terms;
+  const uint8_t *fixed;
+  const int4 *desc;
+  const int32_t *descn, *in_cursor;
+  int32_t *in_list;
+  const void *load;
+  uint32_t *status;
+};
+
+// Force gather and symplectic Euler. With BIN the body is binned at its new
+// position for the next step's search (the tables were cleared by the contact
+// law), which saves that step a pass over the bodies.
+template <bool BIN>
+__global__ void kd_integrate(const __grid_constant__ IntegrateArgs A,
+                             const __grid_constant__ BinArgs B) {
+  // (launched with programmatic dependence on the kernel before it)
+  pdl_wait();
+  pdl_trigger();
+  const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (j >= A.n) return;
+  // gravity and dt / M, dt / Mi from kd_body_terms
+  const double4 bt = A.terms[j];
+  const double4 *load = reinterpret_cast<const double4 *>(A.load);
+  double Fx = bt.x, Fy = bt.y, T = 0.0;
+  for_each_load((int)j, A.desc[j], A.descn[j], A.in_cursor[j], A.in_list, A.ccap, A.status,
+                [&](int k, bool second) {
+                  const double4 f = load[k];
+                  if (second) {
+                    Fx -= f.x;
+                    Fy -= f.y;
+                    T -= f.w;
+                  } else {
+                    Fx += f.x;
+                    Fy += f.y;
+                    T += f.z;
+                  }
+                });
+  if (A.fixed[j]) Fx = Fy = T = 0.0;
   // v1 = v0 + dt Minv F ; q1 = q0 + dt v1
-  const double v0 = v[3 * j] + bt.z * Fx;
-  const double v1 = v[3 * j + 1] + bt.z * Fy;
-  const double v2 = v[3 * j + 2] + bt.w * T;
-  v[3 * j] = v0;
-  v[3 * j + 1] = v1;
-  v[3 * j + 2] = v2;
-  const double q0 = q[3 * j] + dt * v0, q1 = q[3 * j + 1] + dt * v1, q2 = q[3 * j + 2] + dt * v2;
-  q[3 * j] = q0;
-  q[3 * j + 1] = q1;
-  q[3 * j + 2] = q2;
+  const double v0 = A.v[3 * j] + bt.z * Fx;
+  const double v1 = A.v[3 * j + 1] + bt.z * Fy;
+  const double v2 = A.v[3 * j + 2] + bt.w * T;
+  A.v[3 * j] = v0;
+  A.v[3 * j + 1] = v1;
+  A.v[3 * j + 2] = v2;
+  const double q0 = A.q[3 * j] + A.dt * v0, q1 = A.q[3 * j + 1] + A.dt * v1,
+               q2 = A.q[3 * j + 2] + A.dt * v2;
+  A.q[3 * j] = q0;
+  A.q[3 * j + 1] = q1;
+  A.q[3 * j + 2] = q2;
   if (!finite_bits(q0) || !finite_bits(q1) || !finite_bits(v0) || !finite_bits(v1))
-    atomicOr(status, (uint32_t)HG_STATUS_NONFINITE);
+    atomicOr(A.status, (uint32_t)HG_STATUS_NONFINITE);
+  if (BIN) bin_body(B, j, q0, q1);
 }
 
 // ---- mixed precision: the same contact law and integration with FP32
@@ -811,88 +1091,79 @@ __device__ __forceinline__ F2 fnormalized(F2 a) {
 }
 __device__ __forceinline__ float fcross(F2 a, F2 b) { return a.x * b.y - a.y * b.x; }
 
-__global__ void kdx_contacts(ContactArgs C) {
+__global__ void __launch_bounds__(CONTACT_THREADS) kdx_contacts(const __grid_constant__ ContactArgs C) {
   // (launched with programmatic dependence on the kernel before it)
   pdl_wait();
   pdl_trigger();
-  const int64_t total = min((int64_t)*C.count, C.ccap);
   const float dt = (float)C.dt, kn = (float)C.kn, kt = (float)C.kt, gn = (float)C.gn,
               gt = (float)C.gt, mu = (float)C.mu;
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t key = C.keys[k];
-    const int kind = (int)(key >> 60);
-    const int a = (int)((key >> 30) & 0x3FFFFFFF);
-    const int b = (int)(key & 0x3FFFFFFF);
-    if (!HG_INDEX_OK(a, C.n, C.status) ||
-        !HG_INDEX_OK(b, kind == K_PLANE ? (int64_t)(C.nplanes + C.ndrums) : C.n, C.status))
-      continue;
+  for_each_contact(C, [&](int64_t k, int64_t key, int kind, int a, int b, double *out) {
     const double qax = C.q[3 * a], qay = C.q[3 * a + 1];
-    const F2 va{(float)C.v[3 * a], (float)C.v[3 * a + 1]};
-    const float wa = (float)C.v[3 * a + 2];
-    const float ra = (float)C.r[a];
+    const F2 va{narrow(C.v[3 * a]), narrow(C.v[3 * a + 1])};
+    const float wa = narrow(C.v[3 * a + 2]);
+    const float ra = narrow(C.r[a]);
     float depth, weight;
     F2 n, r0, r1{0.0f, 0.0f}, vrel;
     double cpx, cpy;
     if (kind == K_PLANE && b >= C.nplanes) { // PenaltyImpactFrictionMap.cpp:361-401
       const int dk = b - C.nplanes;
       const double ex = C.dx[dk][0] - qax, ey = C.dx[dk][1] - qay; // FP64 difference
-      const F2 e{(float)ex, (float)ey};
+      const F2 e{narrow(ex), narrow(ey)};
       n = fnormalized(e); // towards the drum's centre
       // -(|e| - (R - r)) as ((R - r)^2 - |e|^2) / (|e| + R - r): the
       // cancelling difference in FP64, the rest in FP32
       const double g = C.dr[dk] - C.r[a];
       const double g2 = g * g - (ex * ex + ey * ey);
-      depth = g2 < 0.0 ? (float)g2 / (fnrm(e) + (float)g) : 0.0f;
-      weight = C.weighted ? (float)C.w[a] : 1.0f;
+      depth = g2 < 0.0 ? narrow(g2) / (fnrm(e) + narrow(g)) : 0.0f;
+      weight = C.weighted ? narrow(C.w[a]) : 1.0f;
       r0 = fscl(-ra, n);
-      cpx = qax + (double)r0.x;
-      cpy = qay + (double)r0.y;
+      cpx = qax + widen(r0.x);
+      cpy = qay + widen(r0.y);
       vrel = fadd(va, fscl(wa, F2{-r0.y, r0.x})); // the drum is static
     } else if (kind == K_PLANE) { // PenaltyImpactFrictionMap.cpp:316-359
-      n = F2{(float)C.pn[b][0], (float)C.pn[b][1]};
+      n = F2{narrow(C.pn[b][0]), narrow(C.pn[b][1])};
       // penetration from FP64 positions (a difference of nearly equal terms)
       const double dist = C.pn[b][0] * (qax - C.px[b][0]) + C.pn[b][1] * (qay - C.px[b][1]);
-      depth = (float)fmin(0.0, dist - C.r[a]);
-      weight = C.weighted ? (float)C.w[a] : 1.0f;
+      depth = narrow(min_zero(dist - C.r[a]));
+      weight = C.weighted ? narrow(C.w[a]) : 1.0f;
       r0 = fscl(-ra, n);
-      cpx = qax + (double)r0.x;
-      cpy = qay + (double)r0.y;
+      cpx = qax + widen(r0.x);
+      cpy = qay + widen(r0.y);
       vrel = fadd(va, fscl(wa, F2{-r0.y, r0.x})); // the plane is static
     } else {
       const double qbx = C.q[3 * b], qby = C.q[3 * b + 1];
-      const float rb = (float)C.r[b];
+      const float rb = narrow(C.r[b]);
       const double dx = qax - qbx, dy = qay - qby; // FP64 difference
-      const F2 d{(float)dx, (float)dy};
+      const F2 d{narrow(dx), narrow(dy)};
       n = fnormalized(d);
       // |d| - (ra + rb) as (|d|^2 - (ra + rb)^2) / (|d| + ra + rb): the
       // cancelling difference in FP64, the rest in FP32
       const double rs = C.r[a] + C.r[b];
       const double g2 = (dx * dx + dy * dy) - rs * rs;
-      depth = g2 < 0.0 ? (float)g2 / (fnrm(d) + (float)rs) : 0.0f;
-      const F2 vb{(float)C.v[3 * b], (float)C.v[3 * b + 1]};
-      const float wb = (float)C.v[3 * b + 2];
+      depth = g2 < 0.0 ? narrow(g2) / (fnrm(d) + narrow(rs)) : 0.0f;
+      const F2 vb{narrow(C.v[3 * b]), narrow(C.v[3 * b + 1])};
+      const float wb = narrow(C.v[3 * b + 2]);
       if (kind == K_CC) { // CircleCircleConstraint.cpp:171-233
-        weight = C.weighted ? (float)((C.w[a] + C.w[b]) * 0.5) : 1.0f;
+        weight = C.weighted ? narrow((C.w[a] + C.w[b]) * 0.5) : 1.0f;
         r0 = fscl(-(ra / (ra + rb)), d); // p - xa = ra/(ra+rb) (xb - xa)
         r1 = fadd(d, r0);                // p - xb
         vrel = fsub(fsub(fadd(va, fscl(wa, F2{-r0.y, r0.x})), vb), fscl(wb, F2{-r1.y, r1.x}));
       } else { // KinematicObjectCircleConstraint.cpp
-        weight = C.weighted ? (float)C.w[a] : 1.0f;
+        weight = C.weighted ? narrow(C.w[a]) : 1.0f;
         r0 = fscl(-ra, n);
         const F2 arm = fadd(d, r0); // p - xb
         const F2 vk = fadd(vb, fscl(wb, F2{-arm.y, arm.x}));
         vrel = fsub(fadd(va, fscl(wa, F2{-r0.y, r0.x})), vk);
       }
-      cpx = qax + (double)r0.x;
-      cpy = qay + (double)r0.y;
+      cpx = qax + widen(r0.x);
+      cpy = qay + widen(r0.y);
     }
     // tangential spring carry
     F2 ds;
-    const int o = find_old(C, key);
+    const int o = find_old(C, key, kind, a);
     if (o >= 0) {
-      ds = F2{(float)C.old_rec[(int64_t)o * RW + 6], (float)C.old_rec[(int64_t)o * RW + 7]};
-      ds = fadd(ds, fscl(dt, vrel));
+      const double2 old = *reinterpret_cast<const double2 *>(C.old_rec + (int64_t)o * RW + 6);
+      ds = fadd(F2{narrow(old.x), narrow(old.y)}, fscl(dt, vrel));
     } else {
       ds = fscl(dt, vrel);
     }
@@ -917,89 +1188,58 @@ __global__ void kdx_contacts(ContactArgs C) {
       ds = fscl(root1, ds);
       ft = fsub(fscl(-kt * w, ds), fscl(0.5f * gt * w, vt));
     }
-    double *o_ = C.rec + k * RW;
-    o_[0] = kind;
-    o_[1] = a;
-    o_[2] = b;
-    o_[3] = depth;
-    o_[4] = n.x;
-    o_[5] = n.y;
-    o_[6] = ds.x;
-    o_[7] = ds.y;
-    o_[8] = vrel.x;
-    o_[9] = vrel.y;
-    o_[10] = r0.x;
-    o_[11] = r0.y;
-    o_[12] = r1.x;
-    o_[13] = r1.y;
-    o_[14] = weight;
-    o_[15] = cpx;
-    o_[16] = cpy;
-    o_[17] = fn.x;
-    o_[18] = fn.y;
-    o_[19] = ft.x;
-    o_[20] = ft.y;
-    o_[21] = 0.0;
-  }
+    const F2 f = fadd(fn, ft);
+    reinterpret_cast<float4 *>(C.load)[k] = make_float4(f.x, f.y, fcross(r0, f), fcross(r1, f));
+    put2(out, 0, index_f64(kind), index_f64(a));
+    put2(out, 1, index_f64(b), widen(depth));
+    put2(out, 2, widen(n.x), widen(n.y));
+    put2(out, 3, widen(ds.x), widen(ds.y));
+    put2(out, 4, widen(vrel.x), widen(vrel.y));
+    put2(out, 5, widen(r0.x), widen(r0.y));
+    put2(out, 6, widen(r1.x), widen(r1.y));
+    put2(out, 7, widen(weight), cpx);
+    put2(out, 8, cpy, widen(fn.x));
+    put2(out, 9, widen(fn.y), widen(ft.x));
+    put2(out, 10, widen(ft.y), 0.0);
+  });
 }
 
 // Force gather (the FP64 kernel's summation order) and symplectic Euler in
 // FP32; q += dt v in FP64.
-__global__ void kdx_integrate(int64_t n, double dt, double *q, double *v,
-                              const double4 *__restrict__ terms,
-                              const uint8_t *__restrict__ fixed,
-                              const int32_t *__restrict__ cnt, const int32_t *__restrict__ off,
-                              const double *__restrict__ rec,
-                              const int32_t *__restrict__ in_count,
-                              const int32_t *__restrict__ in_off, int32_t *in_list,
-                              uint32_t *status) {
+template <bool BIN>
+__global__ void kdx_integrate(const __grid_constant__ IntegrateArgs A,
+                              const __grid_constant__ BinArgs B) {
   // (launched with programmatic dependence on the kernel before it)
   pdl_wait();
   pdl_trigger();
   const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const double4 bt = terms[j];
-  float Fx = (float)bt.x, Fy = (float)bt.y, T = 0.0f;
-  auto add = [&](int64_t k, int which, float sign) {
-    const double *r = rec + k * RW;
-    const F2 f = fadd(F2{(float)r[17], (float)r[18]}, F2{(float)r[19], (float)r[20]});
-    Fx += sign * f.x;
-    Fy += sign * f.y;
-    T += sign * fcross(F2{(float)r[10 + 2 * which], (float)r[11 + 2 * which]}, f);
-  };
-  for (int64_t k = off[j], e = off[j] + cnt[j]; k < e; ++k) add(k, 0, 1.0f);
-  {
-    int *lst = in_list + in_off[j];
-    const int c = in_count[j];
-    for (int i = 1; i < c; ++i) { // contact indices sorted = first indices sorted
-      const int key = lst[i];
-      int t = i - 1;
-      while (t >= 0 && lst[t] > key) {
-        lst[t + 1] = lst[t];
-        --t;
-      }
-      lst[t + 1] = key;
-    }
-    for (int i = 0; i < c; ++i)
-      if (HG_INDEX_OK(lst[i], off[3 * n], status)) add(lst[i], 1, -1.0f);
-  }
-  for (int64_t k = off[n + j], e = off[n + j] + cnt[n + j]; k < e; ++k) add(k, 0, 1.0f);
-  for (int64_t k = off[2 * n + j], e = off[2 * n + j] + cnt[2 * n + j]; k < e; ++k)
-    add(k, 0, 1.0f);
-  if (fixed[j]) Fx = Fy = T = 0.0f;
-  const float v0 = (float)v[3 * j] + (float)bt.z * Fx;
-  const float v1 = (float)v[3 * j + 1] + (float)bt.z * Fy;
-  const float v2 = (float)v[3 * j + 2] + (float)bt.w * T;
-  v[3 * j] = v0;
-  v[3 * j + 1] = v1;
-  v[3 * j + 2] = v2;
-  const double q0 = q[3 * j] + dt * (double)v0, q1 = q[3 * j + 1] + dt * (double)v1,
-               q2 = q[3 * j + 2] + dt * (double)v2;
-  q[3 * j] = q0;
-  q[3 * j + 1] = q1;
-  q[3 * j + 2] = q2;
+  if (j >= A.n) return;
+  const double4 bt = A.terms[j];
+  const float4 *load = reinterpret_cast<const float4 *>(A.load);
+  float Fx = narrow(bt.x), Fy = narrow(bt.y), T = 0.0f;
+  for_each_load((int)j, A.desc[j], A.descn[j], A.in_cursor[j], A.in_list, A.ccap, A.status,
+                [&](int k, bool second) {
+                  const float4 f = load[k];
+                  Fx += second ? -f.x : f.x;
+                  Fy += second ? -f.y : f.y;
+                  T += second ? -f.w : f.z;
+                });
+  if (A.fixed[j]) Fx = Fy = T = 0.0f;
+  const float v0 = narrow(A.v[3 * j]) + narrow(bt.z) * Fx;
+  const float v1 = narrow(A.v[3 * j + 1]) + narrow(bt.z) * Fy;
+  const float v2 = narrow(A.v[3 * j + 2]) + narrow(bt.w) * T;
+  const double w0 = widen(v0), w1 = widen(v1), w2 = widen(v2);
+  A.v[3 * j] = w0;
+  A.v[3 * j + 1] = w1;
+  A.v[3 * j + 2] = w2;
+  const double q0 = A.q[3 * j] + A.dt * w0, q1 = A.q[3 * j + 1] + A.dt * w1,
+               q2 = A.q[3 * j + 2] + A.dt * w2;
+  A.q[3 * j] = q0;
+  A.q[3 * j + 1] = q1;
+  A.q[3 * j + 2] = q2;
   if (!finite_bits(q0) || !finite_bits(q1) || !isfinite(v0) || !isfinite(v1))
-    atomicOr(status, (uint32_t)HG_STATUS_NONFINITE);
+    atomicOr(A.status, (uint32_t)HG_STATUS_NONFINITE);
+  if (BIN) bin_body(B, j, q0, q1);
 }
 
 
@@ -1073,31 +1313,43 @@ hg_status build_buckets(cudaStream_t s, BroadArgs &B, int32_t *bcount, int32_t *
 
 } // namespace
 
+namespace {
+
+// tiles of at least 64 bodies, at most MAX_TILES of them
+int tile_shift_for(int64_t n) {
+  int sh = 6;
+  while (((n - 1) >> sh) + 1 > MAX_TILES) ++sh;
+  return sh;
+}
+
+} // namespace
+
 hg_status dem_alloc(hg_dem *d) {
   const int64_t N = std::max<int64_t>(d->cap, 1);
   const int64_t C = std::max<int64_t>(d->ccap, 1);
   const uint32_t bits = table_bits(N);
   d->mask = (1u << bits) - 1u;
   const int64_t T = (int64_t)d->mask + 1;
-  int64_t tmp = std::max(scan_tmp_size(3 * N + 1), scan_tmp_size(T));
-  tmp = std::max(tmp, scan_tmp_size(N + 1));
+  const bool mixed = d->p.precision == HG_PRECISION_MIXED;
   hg_status st;
   if ((st = d->status.alloc(1)) || (st = d->q.alloc(3 * N)) || (st = d->v.alloc(3 * N)) ||
       (st = d->r.alloc(N)) || (st = d->m0.alloc(N)) || (st = d->I0.alloc(N)) ||
       (st = d->w.alloc(N)) || (st = d->minv.alloc(4 * N)) || (st = d->fixed.alloc(N)) ||
-      (st = d->brec.alloc(2 * N)) || (st = d->pfill.alloc(N)) || (st = d->plist.alloc(PW * N)) ||
-      (st = d->bcount.alloc(T)) || (st = d->bstart.alloc(T)) ||
-      (st = d->items.alloc(N)) || (st = d->scan_tmp.alloc(tmp)) ||
-      (st = d->c_count.alloc(2)) || (st = d->per_body.alloc(3 * N + 1)) ||
-      (st = d->per_body_off.alloc(3 * N + 1)) || (st = d->ckey[0].alloc(C)) ||
-      (st = d->ckey[1].alloc(C)) || (st = d->crec[0].alloc(C * RW)) ||
-      (st = d->crec[1].alloc(C * RW)) || (st = d->in_count.alloc(N + 1)) ||
-      (st = d->in_off.alloc(N + 1)) || (st = d->in_list.alloc(C)) ||
-      (st = d->in_cursor.alloc(N)) || (st = d->overflow.alloc(1)))
+      (st = d->brec.alloc(2 * N)) || (st = d->plist.alloc(PW * N)) || (st = d->heads.alloc(T)) ||
+      (st = d->pc.alloc(N)) || (st = d->in_count.alloc(N)) ||
+      (st = d->tiles.alloc(4 * (int64_t)MAX_TILES)) || (st = d->c_count.alloc(2)) ||
+      (st = d->cc_range.alloc(1)) || (st = d->in_list.alloc(C)) || (st = d->in_cursor.alloc(N)) ||
+      (st = d->load.alloc(C * (mixed ? 16 : 32))))
     return st;
+  for (int b = 0; b < 2; ++b)
+    if ((st = d->ckey[b].alloc(C)) || (st = d->crec[b].alloc(C * RW)) ||
+        (st = d->desc[b].alloc(N)) || (st = d->descn[b].alloc(N)))
+      return st;
   cudaStream_t s = dem_stream(d);
   HG_CUDA_TRY(cudaMemsetAsync(d->status.p, 0, sizeof(uint32_t), s));
   HG_CUDA_TRY(cudaMemsetAsync(d->c_count.p, 0, 2 * sizeof(int32_t), s));
+  d->bins = hg_dem::BINS_DIRTY;
+  d->desc_valid = false;
   HG_CUDA_TRY(cudaStreamSynchronize(s));
   return HG_OK;
 }
@@ -1105,7 +1357,14 @@ hg_status dem_alloc(hg_dem *d) {
 hg_status dem_reset_history(hg_dem *d) {
   HG_CUDA_TRY(cudaMemsetAsync(d->c_count.p, 0, 2 * sizeof(int32_t), dem_stream(d)));
   d->history_valid = false;
+  d->desc_valid = false;
   return HG_OK;
+}
+
+// The bodies' positions, radii, flags or number changed outside dem_step: the
+// next step bins them anew.
+void dem_bodies_changed(hg_dem *d) {
+  if (d->bins == hg_dem::BINS_FILLED) d->bins = hg_dem::BINS_DIRTY;
 }
 
 hg_status dem_prepare(hg_dem *d, double dt) {
@@ -1118,23 +1377,23 @@ hg_status dem_prepare(hg_dem *d, double dt) {
   return HG_OK;
 }
 
-// The contact law's grid: one resident wave (the SM count times the blocks
-// of 256 threads that fit on an SM at once: 3 for the FP64 law's registers,
-// 4 for the mixed one's), so that the grid-stride loop runs no partial
-// second wave.
+// The contact law's grid: one resident wave, so that the grid-stride loop runs
+// no partial second wave.
 void dem_set_launch_shapes(hg_dem *d) {
   int per_sm = 0;
   cudaError_t e = d->p.precision == HG_PRECISION_MIXED
-                      ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kdx_contacts, 256, 0)
-                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kd_contacts, 256, 0);
+                      ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kdx_contacts,
+                                                                      CONTACT_THREADS, 0)
+                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kd_contacts,
+                                                                      CONTACT_THREADS, 0);
   if (e != cudaSuccess || per_sm < 1) {
     (void)cudaGetLastError();
-    per_sm = 3;
+    per_sm = 4;
   }
   d->contact_grid = d->ctx->num_sms * per_sm;
 }
 
-hg_status dem_step(hg_dem *d, double dt, int weighted) {
+hg_status dem_step(hg_dem *d, double dt, int weighted, bool bin_next) {
   cudaStream_t s = dem_stream(d);
   const int64_t n = d->n;
   if (n == 0) return HG_OK;
@@ -1142,101 +1401,89 @@ hg_status dem_step(hg_dem *d, double dt, int weighted) {
   if ((st = dem_prepare(d, dt))) return st;
   // the hash table grows with the live body count (at most the capacity's)
   const uint32_t mask = (1u << table_bits(n)) - 1u;
-  {
-    // hash-grid counting sort of the bodies by home cell
-    const int64_t T = (int64_t)mask + 1;
-    HG_CUDA_TRY(cudaMemsetAsync(d->bcount.p, 0, sizeof(int32_t) * T, s));
-    HomeArgs H;
-    H.n = n;
-    H.H = d->cell_h;
-    H.invH = 1.0 / d->cell_h;
-    H.mask = mask;
-    H.nplanes = d->p.nplanes;
-    H.ndrums = d->p.ndrums;
-    for (int k = 0; k < HG_MAX_DRUMS; ++k) {
-      H.dx[k][0] = d->p.dx[k][0];
-      H.dx[k][1] = d->p.dx[k][1];
-      H.dr[k] = d->p.dr[k];
+  const int shift = tile_shift_for(n);
+  const int ntiles = (int)(((n - 1) >> shift) + 1);
+  // Below about one body per thread slot of the GPU, five threads per body
+  // hide the list walks' latency, and the search adds to the tile sums as it
+  // goes (a launch less); above it, one thread per body reads each body's
+  // record once, and the sums take a pass of their own (at a million disks
+  // under contact load the added atomics cost more than the pass).
+  const bool few = n < (int64_t)d->ctx->num_sms * 1024;
+  BinArgs H;
+  H.n = n;
+  H.H = d->cell_h;
+  H.invH = 1.0 / d->cell_h;
+  H.mask = mask;
+  H.nplanes = d->p.nplanes;
+  H.ndrums = d->p.ndrums;
+  for (int k = 0; k < HG_MAX_DRUMS; ++k) {
+    H.dx[k][0] = d->p.dx[k][0];
+    H.dx[k][1] = d->p.dx[k][1];
+    H.dr[k] = d->p.dr[k];
+  }
+  for (int k = 0; k < HG_MAX_PLANES; ++k)
+    for (int c = 0; c < 2; ++c) {
+      H.px[k][c] = d->p.px[k][c];
+      H.pn[k][c] = d->p.pn[k][c];
+      H.pxf[k][c] = (float)d->p.px[k][c];
+      H.pnf[k][c] = (float)d->p.pn[k][c];
     }
-    for (int k = 0; k < HG_MAX_PLANES; ++k)
-      for (int c = 0; c < 2; ++c) {
-        H.px[k][c] = d->p.px[k][c];
-        H.pn[k][c] = d->p.pn[k][c];
-      }
-    H.q = d->q.p;
-    H.r = d->r.p;
-    H.fixed = d->fixed.p;
-    H.rec = d->brec.p;
-    H.bucket_count = d->bcount.p;
-    H.per_body = d->per_body.p;
-    H.pfill = d->pfill.p;
-    H.in_count = d->in_count.p;
-    H.in_cursor = d->in_cursor.p;
-    HG_LAUNCH_PDL(kd_bodies_home, blocks_for(n, 256), 256, 0, s, H);
-    HG_CHECK_LAUNCH();
-    if ((st = exclusive_scan_i32(d->bcount.p, d->bstart.p, T, d->scan_tmp.p, s))) return st;
-    HG_LAUNCH_PDL(kd_fill_ends, blocks_for(n, 256), 256, 0, s, n, mask, d->brec.p, d->bstart.p,
-              d->items.p, d->status.p);
+  H.r = d->r.p;
+  H.fixed = d->fixed.p;
+  H.rec = d->brec.p;
+  H.heads = d->heads.p;
+  H.pc = d->pc.p;
+  H.in_count = d->in_count.p;
+  H.tiles = few ? d->tiles.p : nullptr;
+  H.tile_shift = shift;
+  const int bins = d->bins;
+  d->bins = hg_dem::BINS_DIRTY; // until the step is queued
+  if (bins == hg_dem::BINS_DIRTY) {
+    HG_CUDA_TRY(cudaMemsetAsync(d->heads.p, 0xFF, sizeof(int32_t) * ((int64_t)d->mask + 1), s));
+    HG_CUDA_TRY(cudaMemsetAsync(d->tiles.p, 0, sizeof(int32_t) * 4 * MAX_TILES, s));
+  }
+  if (bins != hg_dem::BINS_FILLED) {
+    HG_LAUNCH_PDL(kd_bin, blocks_for(n, 128), 128, 0, s, H, d->q.p);
     HG_CHECK_LAUNCH();
   }
+  const int nb = 1 - d->cc; // buffer receiving this step's contacts
   PairArgs A;
   A.n = n;
   A.mask = mask;
   A.rec = d->brec.p;
   A.Hf = (float)d->cell_h;
   A.tol = (float)(1.0e-4 * d->cell_h);
-  A.plist = d->plist.p;
-  A.bucket_end = d->bstart.p;
-  A.bucket_count = d->bcount.p;
-  A.items = d->items.p;
+  A.heads = d->heads.p;
   A.q = d->q.p;
   A.r = d->r.p;
   A.nstatic = d->p.nplanes + d->p.ndrums;
-  A.cnt = d->per_body.p;
-  A.off = d->per_body_off.p;
-  const int nb = 1 - d->cc; // buffer receiving this step's contacts
+  A.pc = d->pc.p;
+  A.in_count = d->in_count.p;
+  A.plist = d->plist.p;
+  A.desc = d->desc[nb].p;
+  A.descn = d->descn[nb].p;
+  A.in_cursor = d->in_cursor.p;
+  A.tiles = d->tiles.p;
+  A.tile_shift = shift;
+  A.ntiles = ntiles;
+  A.add_tiles = few;
   A.keys = d->ckey[nb].p;
   A.ccap = d->ccap;
-  A.overflow = d->overflow.p;
+  A.count = d->c_count.p + nb;
+  A.range = d->cc_range.p;
   A.status = d->status.p;
-  A.pfill = d->pfill.p;
-  // (per_body and pfill were zeroed by kd_bodies_home)
-  // Below about one body per thread slot of the GPU, five threads per body
-  // hide the bucket walks' latency; above it, one thread per body reads each
-  // body's record once.
-  if (n < (int64_t)d->ctx->num_sms * 1024)
-    HG_LAUNCH_PDL(kd_pairs_count, blocks_for(5 * n, 128), 128, 0, s, A);
-  else
-    HG_LAUNCH_PDL(kd_pairs_count_body, blocks_for(n, 128), 128, 0, s, A);
-  HG_CHECK_LAUNCH();
-  // offsets, the contact-capacity check (all contacts dropped when the list
-  // would overflow) and the contact count
-  const bool small = 3 * n + 1 <= small_scan_max();
-  if (small) {
-    ScanLimit lim;
-    lim.limit = d->ccap;
-    lim.overflow = d->overflow.p;
-    lim.status = d->status.p;
-    lim.status_bit = HG_STATUS_CONTACT_OVERFLOW;
-    lim.total = d->c_count.p + nb;
-    if ((st = exclusive_scan_i32_limited(d->per_body.p, d->per_body_off.p, 3 * n + 1, lim, s)))
-      return st;
+  if (few) {
+    HG_LAUNCH_PDL(kd_pairs, blocks_for(5 * n, 128), 128, 0, s, A);
+    HG_CHECK_LAUNCH();
+    HG_LAUNCH_PDL(kd_pairs_emit<64>, blocks_for(n, 64), 64, 0, s, A);
   } else {
-    if ((st = exclusive_scan_i32(d->per_body.p, d->per_body_off.p, 3 * n + 1, d->scan_tmp.p,
-                                 s)))
-      return st;
-    HG_LAUNCH_PDL(kd_check_capacity, 1, 32, 0, s, n, d->per_body_off.p, d->ccap, d->overflow.p,
-              d->status.p);
+    HG_LAUNCH_PDL(kd_pairs_body, blocks_for(n, 128), 128, 0, s, A);
     HG_CHECK_LAUNCH();
-    HG_LAUNCH_PDL(kd_drop_if_overflow, blocks_for(3 * n + 1, 256), 256, 0, s, n, d->overflow.p,
-              d->per_body.p, d->per_body_off.p);
+    HG_LAUNCH_PDL(kd_tile_sums, ntiles, 256, 0, s, n, shift, d->pc.p, d->in_count.p, d->tiles.p);
     HG_CHECK_LAUNCH();
+    HG_LAUNCH_PDL(kd_pairs_emit<256>, blocks_for(n, 256), 256, 0, s, A);
   }
-  HG_LAUNCH_PDL(kd_pairs_emit, blocks_for(n, 128), 128, 0, s, A);
   HG_CHECK_LAUNCH();
-  if (!small)
-    HG_CUDA_TRY(cudaMemcpyAsync(d->c_count.p + nb, d->per_body_off.p + 3 * n, sizeof(int32_t),
-                                cudaMemcpyDeviceToDevice, s));
   ContactArgs Cg;
   Cg.n = n;
   Cg.dt = dt;
@@ -1265,37 +1512,53 @@ hg_status dem_step(hg_dem *d, double dt, int weighted) {
   Cg.count = d->c_count.p + nb;
   Cg.keys = d->ckey[nb].p;
   Cg.rec = d->crec[nb].p;
+  Cg.load = d->load.p;
+  Cg.desc = d->desc[nb].p;
+  Cg.in_cursor = d->in_cursor.p;
+  Cg.in_list = d->in_list.p;
   Cg.old_keys = d->ckey[d->cc].p;
   Cg.old_rec = d->crec[d->cc].p;
   Cg.old_count = d->c_count.p + d->cc;
+  Cg.old_desc = d->desc_valid ? d->desc[d->cc].p : nullptr;
+  Cg.old_descn = d->descn[d->cc].p;
+  Cg.heads = d->heads.p;
+  Cg.nheads = (int64_t)mask + 1;
+  Cg.tiles = d->tiles.p;
   Cg.ccap = d->ccap;
   Cg.status = d->status.p;
-  // The contact law is launched in stream order: scheduled while
-  // kd_pairs_emit is still running, its one-wave grid-stride launch took
-  // 10 us longer per step on 28,000 contacts (2.8 per disk); every other
-  // launch of the step is programmatic.
-  const int cgrid = d->contact_grid > 0 ? d->contact_grid : d->ctx->num_sms * 3;
+  // one wave, or the CTAs that the contacts the buffers hold can fill
+  const int64_t chunks = std::max<int64_t>((d->ccap + 31) / 32, (n + 31) / 32);
+  const int cgrid = (int)std::min<int64_t>(d->contact_grid, chunks);
   if (d->p.precision == HG_PRECISION_MIXED)
-    HG_LAUNCH(kdx_contacts, cgrid, 256, 0, s, Cg);
+    HG_LAUNCH_PDL(kdx_contacts, cgrid, CONTACT_THREADS, 0, s, Cg);
   else
-    HG_LAUNCH(kd_contacts, cgrid, 256, 0, s, Cg);
+    HG_LAUNCH_PDL(kd_contacts, cgrid, CONTACT_THREADS, 0, s, Cg);
   HG_CHECK_LAUNCH();
-  // (in_count and in_cursor were zeroed by kd_bodies_home)
-  HG_LAUNCH_PDL(kd_in_count, d->ctx->num_sms * 2, 256, 0, s, n, d->per_body_off.p, d->ckey[nb].p,
-            d->in_count.p);
-  HG_CHECK_LAUNCH();
-  if ((st = exclusive_scan_i32(d->in_count.p, d->in_off.p, n + 1, d->scan_tmp.p, s))) return st;
-  HG_LAUNCH_PDL(kd_in_fill, d->ctx->num_sms * 2, 256, 0, s, n, d->per_body_off.p, d->ckey[nb].p,
-            d->in_off.p, d->in_cursor.p, d->in_list.p);
-  HG_CHECK_LAUNCH();
-  auto integrate = d->p.precision == HG_PRECISION_MIXED ? kdx_integrate : kd_integrate;
-  HG_LAUNCH_PDL(integrate, blocks_for(n, 128), 128, 0, s, n, dt, d->q.p, d->v.p,
-            reinterpret_cast<const double4 *>(d->minv.p), d->fixed.p, d->per_body.p,
-            d->per_body_off.p,
-            d->crec[nb].p, d->in_count.p, d->in_off.p, d->in_list.p, d->status.p);
+  IntegrateArgs I;
+  I.n = n;
+  I.ccap = d->ccap;
+  I.dt = dt;
+  I.q = d->q.p;
+  I.v = d->v.p;
+  I.terms = reinterpret_cast<const double4 *>(d->minv.p);
+  I.fixed = d->fixed.p;
+  I.desc = d->desc[nb].p;
+  I.descn = d->descn[nb].p;
+  I.in_cursor = d->in_cursor.p;
+  I.in_list = d->in_list.p;
+  I.load = d->load.p;
+  I.status = d->status.p;
+  auto integrate = d->p.precision == HG_PRECISION_MIXED
+                       ? (bin_next ? kdx_integrate<true> : kdx_integrate<false>)
+                       : (bin_next ? kd_integrate<true> : kd_integrate<false>);
+  // one warp per CTA spreads few bodies over all SMs' FP64 pipes
+  const int it = few ? 32 : 128;
+  HG_LAUNCH_PDL(integrate, blocks_for(n, it), it, 0, s, I, H);
   HG_CHECK_LAUNCH();
   d->cc = nb;
   d->history_valid = true;
+  d->desc_valid = true;
+  d->bins = bin_next ? hg_dem::BINS_FILLED : hg_dem::BINS_CLEAR;
   return HG_OK;
 }
 
@@ -1368,6 +1631,7 @@ hg_status dem_relabel_device(hg_dem *d, const int32_t *map, int64_t nmap) {
             d->crec[nb].p, d->c_count.p + nb);
   HG_CHECK_LAUNCH();
   d->cc = nb;
+  d->desc_valid = false; // the bodies' lists moved
   return HG_OK;
 }
 
@@ -1464,6 +1728,8 @@ hg_status dem_edit(hg_dem *d, int64_t n_old, const int32_t *map_host, int64_t n_
   }
   d->n = n_keep + n_add;
   d->inv_valid = false;
+  d->desc_valid = false;
+  dem_bodies_changed(d);
   return HG_OK;
 }
 

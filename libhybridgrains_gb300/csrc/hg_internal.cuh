@@ -500,35 +500,49 @@ struct hg_dem {
   bool inv_valid = false;  // minv matches m0, I0, w and terms_dt
   double terms_dt = 0.0;
   hg::DevBuf<uint8_t> fixed;
-  // broadphase: hash grid of cell width H over the AABB minima
+  // broadphase: hash grid of cell width H over the centres, linked lists
   double cell_h = 0.0;
   uint32_t mask = 0; // hash table size - 1 at the capacity
-  // per body, 32 bytes: FP32 offset from the home cell, radius, flags; home cell
+  // per body, 32 bytes: FP32 offset from the home cell, radius, flags; home
+  // cell, next body of the bucket
   hg::DevBuf<float4> brec;
-  hg::DevBuf<uint32_t> plist;  // partners kept by the counting pass
-  hg::DevBuf<int32_t> pfill;   // partners credited per body in the counting pass
-  hg::DevBuf<int32_t> bcount, bstart, items; // bstart holds bucket ends after the fill
-  hg::DevBuf<int32_t> scan_tmp;
+  hg::DevBuf<int32_t> heads;           // first body of each bucket, -1: none
+  hg::DevBuf<unsigned long long> pc;   // contact counts per first body
+  hg::DevBuf<int32_t> in_count;        // and per second body
+  hg::DevBuf<int32_t> tiles;           // sums of the counts over tiles of bodies
+  hg::DevBuf<uint32_t> plist;          // partners kept by the search
+  // heads, tiles and the counts between steps: of no use, cleared, or filled
+  // by the last step's integration for the bodies as they are
+  enum { BINS_DIRTY, BINS_CLEAR, BINS_FILLED };
+  int bins = BINS_DIRTY;
   // contacts: current and previous, sorted by (kind, first, second)
   hg::DevBuf<int32_t> c_count; // contacts in ckey[0], ckey[1] (device)
-  hg::DevBuf<int32_t> overflow; // set when this step's contacts exceed ccap
-  hg::DevBuf<int32_t> per_body, per_body_off; // emission counts / offsets
+  hg::DevBuf<int2> cc_range;    // the last step's circle-circle contacts [x, y)
   hg::DevBuf<int64_t> ckey[2];                 // kind << 60 | first << 30 | second
   hg::DevBuf<double> crec[2];                  // HG_DEM_RECORD_WIDTH per contact
   int cc = 0;                                  // live contact buffer
   int64_t ncontacts_host = 0;                  // count after the last step
   bool history_valid = false;
   int contact_grid = 0; // blocks of the contact law's grid-stride launch
-  // body gather lists for deterministic force accumulation
-  hg::DevBuf<int32_t> in_count, in_off, in_list, in_cursor;
-  hg::DevBuf<int32_t> out_off; // first contact index of each body
+  // per body: offsets of its contact lists and their counts, for each contact
+  // buffer; desc_valid while desc[cc] describes the live contacts
+  hg::DevBuf<int4> desc[2];
+  hg::DevBuf<int32_t> descn[2];
+  bool desc_valid = false;
+  // body gather lists for deterministic force accumulation, and the forces
+  // and torques per contact (double4 in FP64, float4 in MIXED)
+  hg::DevBuf<int32_t> in_list, in_cursor;
+  hg::DevBuf<unsigned char> load;
   // two steps captured as a CUDA graph (the contact buffers alternate, so a
-  // pair of steps returns to the same pointers); rebuilt when n, dt, the
-  // weighting, the live buffer or the broadphase cell change
-  cudaGraphExec_t pair_exec = nullptr;
-  int64_t pair_n = -1, pair_launches = 0;
-  double pair_dt = 0.0, pair_cell = 0.0;
-  int pair_weighted = -1, pair_cc = -1;
+  // pair of steps returns to the same pointers), one per live buffer; rebuilt
+  // when n, dt, the weighting or the broadphase cell change
+  struct PairGraph {
+    cudaGraphExec_t exec = nullptr;
+    int64_t n = -1, launches = 0;
+    double dt = 0.0, cell = 0.0;
+    int weighted = -1;
+  };
+  PairGraph pair[2];
 };
 
 namespace hg {
@@ -543,7 +557,10 @@ hg_status dem_relabel_device(hg_dem *d, const int32_t *old_to_new, int64_t nmap)
 hg_status dem_edit(hg_dem *d, int64_t n_old, const int32_t *old_to_new, int64_t n_keep,
                    int64_t n_add, const double *q, const double *v, const double *r,
                    const double *m, const double *I, const uint8_t *fixed);
-hg_status dem_step(hg_dem *d, double dt, int weighted);
+// bin_next: bin the bodies for the next step (wasted when they are moved in
+// between, as the hybrid step does)
+hg_status dem_step(hg_dem *d, double dt, int weighted, bool bin_next);
+void dem_bodies_changed(hg_dem *d);
 void dem_set_launch_shapes(hg_dem *d);
 // per-body terms that dem_step needs and that only change with the bodies
 // or the time step; called before a step is captured into a graph
@@ -568,21 +585,6 @@ constexpr int64_t scan_tmp_size(int64_t n) {
   }
   return total + 2;
 }
-// A capacity limit checked by the scan that produces the offsets: when the
-// total exceeds limit (>= 0), *overflow is set, status_bit raised in
-// *status and every count and offset written as zero; *total (when given)
-// receives the total, or 0 when the limit is exceeded.
-struct ScanLimit {
-  int64_t limit = -1;
-  int32_t *overflow = nullptr;
-  uint32_t *status = nullptr;
-  uint32_t status_bit = 0;
-  int32_t *total = nullptr;
-};
-// The largest n exclusive_scan_i32_limited takes (one CTA, one launch).
-int64_t small_scan_max();
-hg_status exclusive_scan_i32_limited(int32_t *in, int32_t *out, int64_t n, const ScanLimit &lim,
-                                     cudaStream_t s);
 } // namespace hg
 
 struct hg_hybrid {

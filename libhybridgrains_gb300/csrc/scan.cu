@@ -95,7 +95,7 @@ __global__ void k_tile_scan_summed(const int32_t *__restrict__ in, int64_t n,
   }
 }
 
-// Up to small_scan_max() elements: one CTA and one launch in place of three
+// Up to SMALL_N elements: one CTA and one launch in place of three
 // (in a captured step the launches, not the bytes, are the cost at these
 // sizes). Thread t owns the SMALL_ITEMS consecutive elements from
 // t * SMALL_ITEMS: it reads them as 16-byte vectors (all loads in flight at
@@ -110,7 +110,7 @@ constexpr int SMALL_N = SMALL_THREADS * SMALL_ITEMS;
 static_assert(SMALL_ITEMS % 4 == 0, "runs are read as int4");
 
 __global__ void __launch_bounds__(SMALL_THREADS)
-    k_small_scan(int32_t *__restrict__ in, int64_t n64, int32_t *__restrict__ out, ScanLimit lim) {
+    k_small_scan(const int32_t *__restrict__ in, int64_t n64, int32_t *__restrict__ out) {
   // (launched with programmatic dependence on the kernel before it)
   pdl_wait();
   pdl_trigger();
@@ -153,13 +153,6 @@ __global__ void __launch_bounds__(SMALL_THREADS)
   // exclusive prefix is the sum of the warps before its own
   int total;
   const int off = block_excl_scan<SMALL_THREADS>(lane == 31 ? carry : 0, &total);
-  // the same decision in every thread: the total is block-wide
-  const bool over = lim.limit >= 0 && (int64_t)total > lim.limit;
-  if (threadIdx.x == 0) {
-    if (lim.overflow) *lim.overflow = over ? 1 : 0;
-    if (over && lim.status) atomicOr(lim.status, lim.status_bit);
-    if (lim.total) *lim.total = over ? 0 : total;
-  }
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) {
     const int i = wbase + 128 * r + 4 * lane;
@@ -169,38 +162,16 @@ __global__ void __launch_bounds__(SMALL_THREADS)
     o[2] = o[1] + v[r][1];
     o[3] = o[2] + v[r][2];
     if (vec) {
-      *reinterpret_cast<int4 *>(out + i) =
-          over ? make_int4(0, 0, 0, 0) : make_int4(o[0], o[1], o[2], o[3]);
-      if (over) // every count and offset dropped
-        *reinterpret_cast<int4 *>(in + i) = make_int4(0, 0, 0, 0);
+      *reinterpret_cast<int4 *>(out + i) = make_int4(o[0], o[1], o[2], o[3]);
     } else {
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        if (i + j < n) {
-          out[i + j] = over ? 0 : o[j];
-          if (over) in[i + j] = 0;
-        }
+        if (i + j < n) out[i + j] = o[j];
     }
   }
 }
 
-hg_status launch_small_scan(int32_t *in, int64_t n, int32_t *out, const ScanLimit &lim,
-                            cudaStream_t s) {
-  HG_LAUNCH_PDL(k_small_scan, 1, SMALL_THREADS, 0, s, in, n, out, lim);
-  HG_CHECK_LAUNCH();
-  return HG_OK;
-}
-
 } // namespace
-
-int64_t small_scan_max() { return SMALL_N; }
-
-hg_status exclusive_scan_i32_limited(int32_t *in, int32_t *out, int64_t n, const ScanLimit &lim,
-                                     cudaStream_t s) {
-  if (n <= 0 || n > small_scan_max())
-    return fail(HG_ERR_INVALID_ARGUMENT, "limited scan: size out of range");
-  return launch_small_scan(in, n, out, lim, s);
-}
 
 // out[i] = sum(in[0..i)); in and out may not alias. tmp must hold
 // scan_tmp_size(n) ints.
@@ -212,8 +183,11 @@ hg_status exclusive_scan_i32(const int32_t *in, int32_t *out, int64_t n,
     HG_CHECK_LAUNCH();
     return HG_OK;
   }
-  if (n <= small_scan_max()) // (writes to its input only when a limit is exceeded)
-    return launch_small_scan(const_cast<int32_t *>(in), n, out, ScanLimit{}, s);
+  if (n <= SMALL_N) {
+    HG_LAUNCH_PDL(k_small_scan, 1, SMALL_THREADS, 0, s, in, n, out);
+    HG_CHECK_LAUNCH();
+    return HG_OK;
+  }
   const int64_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
   int32_t *sums = tmp;
   int32_t *sums_scanned = tmp + tiles;

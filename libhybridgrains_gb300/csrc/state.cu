@@ -288,6 +288,8 @@ hg_status dem_state_load(hg_dem *d, const void *src, int64_t bytes) {
   std::memcpy(&d->cell_h, &h.meta[3], sizeof(double));
   d->ncontacts_host = h.meta[4];
   d->inv_valid = false;
+  d->desc_valid = false; // the blob keeps no list offsets
+  dem_bodies_changed(d);
   return HG_OK;
 }
 
