@@ -539,13 +539,14 @@ hg_status hg_mpm_create(hg_context *ctx, const hg_mpm_desc *d, hg_mpm **out) {
     if ((st = m->q.alloc(2 * m->cap)) || (st = m->v.alloc(2 * m->cap)) ||
         (st = m->m.alloc(m->cap)) || (st = m->vol.alloc(m->cap)) ||
         (st = m->hl.alloc(m->cap)) || (st = m->be.alloc(4 * m->cap)) ||
-        (st = m->J.alloc(m->cap)) || (st = m->sigma.alloc(4 * m->cap)) ||
+        (st = m->J.alloc(m->cap)) ||
         (st = m->jh.alloc(m->cap)) || (st = m->kin.alloc(m->cap)) ||
         (st = m->g_mass.alloc(nn)) || (st = m->g_mom.alloc(2 * nn)) ||
         (st = m->g_mom_new.alloc(2 * nn)) || (st = m->g_force.alloc(2 * nn)) ||
         (st = m->g_vel.alloc(2 * nn)) || (st = m->g_acc.alloc(2 * nn)) ||
         (st = m->g_cforce.alloc(2 * nn)) || (st = m->g_homog.alloc(nn)) ||
-        (st = m->g_hyb.alloc(nn))) {
+        (st = m->g_hyb.alloc(nn)) || (st = m->g_mass_next.alloc(nn)) ||
+        (st = m->g_mom_next.alloc(2 * nn)) || (st = m->g_force_next.alloc(2 * nn))) {
     } else {
       cudaStream_t s = ctx->stream;
       cudaMemsetAsync(m->g_cforce.p, 0, sizeof(double) * 2 * nn, s);
@@ -773,7 +774,6 @@ static hg_status upload_impl(hg_mpm *m, int64_t n, const double *q, const double
     } else {
       HG_CUDA_TRY(cudaMemsetAsync(m->kin.p, 0, n, s));
     }
-    HG_CUDA_TRY(cudaMemsetAsync(m->sigma.p, 0, sizeof(double) * 4 * n, s));
   } else {
     // stage in upload order, then convert and sort on the device (the
     // half-widths only with the uGIMP basis)
@@ -888,8 +888,8 @@ hg_status hg_mpm_estimate_bytes(const hg_mpm_desc *d, int64_t *bytes) {
   const int64_t nn = (int64_t)(P.nx + 1) * (P.ny + 1), cap = d->capacity;
   int64_t b = 4; // status word
   if (d->precision == HG_PRECISION_FP64) {
-    b += cap * (2 * 16 + 3 * 8 + 32 + 8 + 32 + 4 + 1); // q v | m vol hl | be | J | sigma | jh | kin
-    b += nn * (8 + 6 * 16 + 8 + 4);                    // grid fields
+    b += cap * (2 * 16 + 3 * 8 + 32 + 8 + 4 + 1);  // q v | m vol hl | be | J | jh | kin
+    b += nn * (8 + 6 * 16 + 8 + 4 + 8 + 2 * 16); // grid fields, the other accumulators
   } else {
     const bool ugimp = d->basis == HG_BASIS_UGIMP;
     b += mixed_device_bytes(P.nx, P.ny, cap);
@@ -962,9 +962,8 @@ hg_status hg_mpm_step(hg_mpm *m, double dt, int32_t nsteps) {
   DeviceGuard g(m->ctx);
   if (m->p.precision == HG_PRECISION_MIXED) return mixed_step(m, dt, nsteps);
   for (int k = 0; k < nsteps; ++k) {
-    hg_status st;
-    if ((st = mpm64_phase0(m)) || (st = mpm64_phase1(m, dt)) || (st = mpm64_phase2(m, dt)))
-      return st;
+    const hg_status st = mpm64_step(m, dt);
+    if (st != HG_OK) return st;
   }
   return HG_OK;
 }

@@ -424,7 +424,7 @@ hg_status hybrid_step_impl(hg_hybrid *h, double dt, int flags) {
       h->hl0_value = v;
     }
     hl0 = h->hl0.p;
-  } else if ((st = mpm64_phase0(m))) {
+  } else if ((st = mpm64_to_grid(m))) {
     return st;
   }
   // rasterizeGrainMass (pre-step positions, no partially filled cells)

@@ -40,6 +40,7 @@
 // contacts each, FP64, 68.3 -> 39.0 us; 1,000,000 such disks, mixed, 889 ->
 // 434 us.
 #include "hg_internal.cuh"
+#include "fp64_tools.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -73,11 +74,6 @@ __device__ __forceinline__ D2 dnormalized(D2 a) {
   return a;
 }
 __device__ __forceinline__ double dcross(D2 a, D2 b) { return a.x * b.y - a.y * b.x; }
-// isfinite on the bit pattern (integer pipe; FP64 compares are scarce here)
-__device__ __forceinline__ bool finite_bits(double x) {
-  return ((__double_as_longlong(x) >> 52) & 0x7FF) != 0x7FF;
-}
-
 __device__ __forceinline__ uint32_t cell_hash(int cx, int cy, uint32_t mask) {
   return ((uint32_t)cx * 73856093u ^ (uint32_t)cy * 19349663u) & mask;
 }
@@ -128,62 +124,6 @@ __device__ __forceinline__ void sort_small(int *keys, int n) {
     }
     keys[j + 1] = k;
   }
-}
-
-// ---- FP64 values through the integer pipe -----------------------------------
-//
-// FP64 instructions, conversions to and from FP64 included, issue at about two
-// lanes per cycle and SM on this part (17-21 cycles per warp instruction
-// measured, with 65 cycles of latency; a 32-bit integer instruction takes
-// 0.3), so conversions and decisions that integer arithmetic can make exactly
-// are made there.
-
-// (float)x, rounded to nearest even, for a double in FP32's normal range;
-// other values take the conversion instruction.
-__device__ __noinline__ float narrow_slow(double x) { return (float)x; }
-__device__ __forceinline__ float narrow(double x) {
-  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
-  const uint32_t e = (hi >> 20) & 0x7FFu;
-  if (e - 897u < 253u) { // 2^-126 <= |x| < 2^127
-    const uint64_t b = ((uint64_t)(hi & 0x7FFFFFFFu) << 32) | lo;
-    const uint64_t r = b + 0x0FFFFFFFull + ((b >> 29) & 1u); // ties to even at bit 29
-    return __uint_as_float(((uint32_t)(r >> 29) - (896u << 23)) | (hi & 0x80000000u));
-  }
-  if (((hi << 1) | lo) == 0u) return __uint_as_float(hi); // a zero keeps its sign
-  return narrow_slow(x);
-}
-// The same truncated, for FP32 estimates.
-__device__ __forceinline__ float narrow_trunc(double x) {
-  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
-  const uint32_t e = (hi >> 20) & 0x7FFu;
-  if (e - 897u < 253u)
-    return __uint_as_float((((hi & 0x7FFFFFFFu) - (896u << 20)) << 3) | (lo >> 29) |
-                           (hi & 0x80000000u));
-  if (((hi << 1) | lo) == 0u) return 0.0f;
-  return narrow_slow(x);
-}
-// (double)f
-__device__ __noinline__ double widen_slow(float f) { return (double)f; }
-__device__ __forceinline__ double widen(float f) {
-  const uint32_t b = __float_as_uint(f), m = b & 0x7FFFFFFFu;
-  if (m - 0x00800000u < 0x7F000000u) // normal
-    return __hiloint2double((int)(((m >> 3) + (896u << 20)) | (b & 0x80000000u)), (int)(b << 29));
-  if (m == 0u) return __hiloint2double((int)b, 0);
-  return widen_slow(f);
-}
-// (double)i for 0 <= i < 2^30
-__device__ __forceinline__ double index_f64(int i) {
-  if (i == 0) return 0.0;
-  const int e = 31 - __clz(i);
-  const uint64_t m = (uint64_t)(uint32_t)i << (52 - e); // leading bit at 52
-  return __longlong_as_double((int64_t)(m + ((uint64_t)(e + 1022) << 52)));
-}
-// min(0, x); 0 for a NaN
-__device__ __forceinline__ double min_zero(double x) {
-  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
-  const bool nan = (hi & 0x7FFFFFFFu) > 0x7FF00000u ||
-                   ((hi & 0x7FFFFFFFu) == 0x7FF00000u && lo != 0u);
-  return (hi >> 31) && !nan ? x : 0.0;
 }
 
 // Per body, for the pair search: the home cell (the cell of its centre) and,
@@ -740,30 +680,6 @@ __device__ __forceinline__ double second_root(double a, double b, double c, doub
   return (-b + ds) / (2.0 * a);
 }
 
-// Quotients by one divisor. With y = 1 / b rounded to nearest, the multiply
-// q = a y followed by the residual correction q + (a - q b) y in two FMAs
-// gives a / b rounded to nearest (P. Markstein, "Computation of elementary
-// functions on the IBM RISC System/6000 processor", 1990), three FP64
-// instructions in place of a division's eight. Operands near the ends of the
-// exponent range are divided.
-struct Divisor {
-  double b, y;
-  bool ok;
-};
-__device__ __forceinline__ Divisor divisor(double b) {
-  const uint32_t e = ((uint32_t)__double2hiint(b) >> 20) & 0x7FFu;
-  return {b, 1.0 / b, e - 823u <= 400u};
-}
-__device__ __noinline__ double divide(double a, double b) { return a / b; }
-__device__ __forceinline__ double quot(double a, const Divisor &d) {
-  const uint32_t hi = (uint32_t)__double2hiint(a);
-  const double q = a * d.y;
-  const double z = fma(fma(-q, d.b, a), d.y, q);
-  if (d.ok && ((hi >> 20) & 0x7FFu) - 300u <= 1400u) return z;
-  if (d.ok && (((hi << 1) | (uint32_t)__double2loint(a)) == 0u)) return q; // a zero's sign
-  return divide(a, d.b);
-}
-
 constexpr int CONTACT_THREADS = 128;
 constexpr int CONTACT_WARPS = CONTACT_THREADS / 32;
 constexpr int RW2 = RW / 2; // a record in 16-byte pieces
@@ -1117,8 +1033,8 @@ __global__ void __launch_bounds__(CONTACT_THREADS) kdx_contacts(const __grid_con
       depth = g2 < 0.0 ? narrow(g2) / (fnrm(e) + narrow(g)) : 0.0f;
       weight = C.weighted ? narrow(C.w[a]) : 1.0f;
       r0 = fscl(-ra, n);
-      cpx = qax + widen(r0.x);
-      cpy = qay + widen(r0.y);
+      cpx = qax + widen_f32(r0.x);
+      cpy = qay + widen_f32(r0.y);
       vrel = fadd(va, fscl(wa, F2{-r0.y, r0.x})); // the drum is static
     } else if (kind == K_PLANE) { // PenaltyImpactFrictionMap.cpp:316-359
       n = F2{narrow(C.pn[b][0]), narrow(C.pn[b][1])};
@@ -1127,8 +1043,8 @@ __global__ void __launch_bounds__(CONTACT_THREADS) kdx_contacts(const __grid_con
       depth = narrow(min_zero(dist - C.r[a]));
       weight = C.weighted ? narrow(C.w[a]) : 1.0f;
       r0 = fscl(-ra, n);
-      cpx = qax + widen(r0.x);
-      cpy = qay + widen(r0.y);
+      cpx = qax + widen_f32(r0.x);
+      cpy = qay + widen_f32(r0.y);
       vrel = fadd(va, fscl(wa, F2{-r0.y, r0.x})); // the plane is static
     } else {
       const double qbx = C.q[3 * b], qby = C.q[3 * b + 1];
@@ -1155,8 +1071,8 @@ __global__ void __launch_bounds__(CONTACT_THREADS) kdx_contacts(const __grid_con
         const F2 vk = fadd(vb, fscl(wb, F2{-arm.y, arm.x}));
         vrel = fsub(fadd(va, fscl(wa, F2{-r0.y, r0.x})), vk);
       }
-      cpx = qax + widen(r0.x);
-      cpy = qay + widen(r0.y);
+      cpx = qax + widen_f32(r0.x);
+      cpy = qay + widen_f32(r0.y);
     }
     // tangential spring carry
     F2 ds;
@@ -1191,16 +1107,16 @@ __global__ void __launch_bounds__(CONTACT_THREADS) kdx_contacts(const __grid_con
     const F2 f = fadd(fn, ft);
     reinterpret_cast<float4 *>(C.load)[k] = make_float4(f.x, f.y, fcross(r0, f), fcross(r1, f));
     put2(out, 0, index_f64(kind), index_f64(a));
-    put2(out, 1, index_f64(b), widen(depth));
-    put2(out, 2, widen(n.x), widen(n.y));
-    put2(out, 3, widen(ds.x), widen(ds.y));
-    put2(out, 4, widen(vrel.x), widen(vrel.y));
-    put2(out, 5, widen(r0.x), widen(r0.y));
-    put2(out, 6, widen(r1.x), widen(r1.y));
-    put2(out, 7, widen(weight), cpx);
-    put2(out, 8, cpy, widen(fn.x));
-    put2(out, 9, widen(fn.y), widen(ft.x));
-    put2(out, 10, widen(ft.y), 0.0);
+    put2(out, 1, index_f64(b), widen_f32(depth));
+    put2(out, 2, widen_f32(n.x), widen_f32(n.y));
+    put2(out, 3, widen_f32(ds.x), widen_f32(ds.y));
+    put2(out, 4, widen_f32(vrel.x), widen_f32(vrel.y));
+    put2(out, 5, widen_f32(r0.x), widen_f32(r0.y));
+    put2(out, 6, widen_f32(r1.x), widen_f32(r1.y));
+    put2(out, 7, widen_f32(weight), cpx);
+    put2(out, 8, cpy, widen_f32(fn.x));
+    put2(out, 9, widen_f32(fn.y), widen_f32(ft.x));
+    put2(out, 10, widen_f32(ft.y), 0.0);
   });
 }
 
@@ -1228,7 +1144,7 @@ __global__ void kdx_integrate(const __grid_constant__ IntegrateArgs A,
   const float v0 = narrow(A.v[3 * j]) + narrow(bt.z) * Fx;
   const float v1 = narrow(A.v[3 * j + 1]) + narrow(bt.z) * Fy;
   const float v2 = narrow(A.v[3 * j + 2]) + narrow(bt.w) * T;
-  const double w0 = widen(v0), w1 = widen(v1), w2 = widen(v2);
+  const double w0 = widen_f32(v0), w1 = widen_f32(v1), w2 = widen_f32(v2);
   A.v[3 * j] = w0;
   A.v[3 * j + 1] = w1;
   A.v[3 * j + 2] = w2;

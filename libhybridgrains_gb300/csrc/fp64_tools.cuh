@@ -1,0 +1,123 @@
+// FP64 values through the integer pipe, and cheaper exact quotients.
+//
+// FP64 instructions, conversions to and from FP64 included, issue at about
+// two lanes per cycle and SM on this part (17-21 cycles per warp instruction
+// measured, 65 cycles of latency; a division costs 145 cycles, a square root
+// 156), a 32-bit integer instruction 0.3 cycles. Conversions, comparisons and
+// decisions that integer or FP32 arithmetic can make exactly are made there.
+#pragma once
+
+#include <stdint.h>
+
+namespace hg {
+
+__device__ __forceinline__ uint32_t f64_hi(double x) { return (uint32_t)__double2hiint(x); }
+__device__ __forceinline__ uint32_t f64_lo(double x) { return (uint32_t)__double2loint(x); }
+// x is +0 or -0
+__device__ __forceinline__ bool f64_zero(double x) { return ((f64_hi(x) << 1) | f64_lo(x)) == 0u; }
+// a < b for values that are not negative (nor NaN)
+__device__ __forceinline__ bool f64_less(double a, double b) {
+  return __double_as_longlong(a) < __double_as_longlong(b);
+}
+// isfinite
+__device__ __forceinline__ bool finite_bits(double x) { return (f64_hi(x) & 0x7FF00000u) != 0x7FF00000u; }
+// min(0, x); 0 for a NaN
+__device__ __forceinline__ double min_zero(double x) {
+  const uint32_t hi = f64_hi(x), lo = f64_lo(x);
+  const bool nan = (hi & 0x7FFFFFFFu) > 0x7FF00000u ||
+                   ((hi & 0x7FFFFFFFu) == 0x7FF00000u && lo != 0u);
+  return (hi >> 31) && !nan ? x : 0.0;
+}
+
+// (float)x, rounded to nearest even, for a double in FP32's normal range;
+// other values take the conversion instruction.
+static __device__ __noinline__ float narrow_slow(double x) { return (float)x; }
+__device__ __forceinline__ float narrow(double x) {
+  const uint32_t hi = f64_hi(x), lo = f64_lo(x);
+  const uint32_t e = (hi >> 20) & 0x7FFu;
+  if (e - 897u < 253u) { // 2^-126 <= |x| < 2^127
+    const uint64_t b = ((uint64_t)(hi & 0x7FFFFFFFu) << 32) | lo;
+    const uint64_t r = b + 0x0FFFFFFFull + ((b >> 29) & 1u); // ties to even at bit 29
+    return __uint_as_float(((uint32_t)(r >> 29) - (896u << 23)) | (hi & 0x80000000u));
+  }
+  if (((hi << 1) | lo) == 0u) return __uint_as_float(hi); // a zero keeps its sign
+  return narrow_slow(x);
+}
+// The same truncated, for FP32 estimates.
+__device__ __forceinline__ float narrow_trunc(double x) {
+  const uint32_t hi = f64_hi(x), lo = f64_lo(x);
+  const uint32_t e = (hi >> 20) & 0x7FFu;
+  if (e - 897u < 253u)
+    return __uint_as_float((((hi & 0x7FFFFFFFu) - (896u << 20)) << 3) | (lo >> 29) |
+                           (hi & 0x80000000u));
+  if (((hi << 1) | lo) == 0u) return 0.0f;
+  return narrow_slow(x);
+}
+// (double)f
+static __device__ __noinline__ double widen_f32_slow(float f) { return (double)f; }
+__device__ __forceinline__ double widen_f32(float f) {
+  const uint32_t b = __float_as_uint(f), m = b & 0x7FFFFFFFu;
+  if (m - 0x00800000u < 0x7F000000u) // normal
+    return __hiloint2double((int)(((m >> 3) + (896u << 20)) | (b & 0x80000000u)), (int)(b << 29));
+  if (m == 0u) return __hiloint2double((int)b, 0);
+  return widen_f32_slow(f);
+}
+// (double)i for 0 <= i < 2^31
+__device__ __forceinline__ double index_f64(int i) {
+  if (i == 0) return 0.0;
+  const int e = 31 - __clz(i);
+  const uint64_t m = (uint64_t)(uint32_t)i << (52 - e); // leading bit at 52
+  return __longlong_as_double((int64_t)(m + ((uint64_t)(e + 1022) << 52)));
+}
+// (int)floor(x) and (int)ceil(x); values outside [1, 2^31) take the FP64
+// instructions.
+static __device__ __noinline__ int floor_slow(double x) { return (int)floor(x); }
+static __device__ __noinline__ int ceil_slow(double x) { return (int)ceil(x); }
+__device__ __forceinline__ int floor_int(double x, bool *whole = nullptr) {
+  const uint32_t hi = f64_hi(x), lo = f64_lo(x);
+  const uint32_t e = (hi >> 20) - 1023u; // a sign bit gives 1025 or more
+  if (e < 31u) {
+    const uint64_t m = ((uint64_t)((hi & 0xFFFFFu) | 0x100000u) << 32) | lo;
+    if (whole) *whole = (m << (12 + e)) == 0u;
+    return (int)(m >> (52u - e));
+  }
+  if (whole) *whole = x == floor(x);
+  return floor_slow(x);
+}
+__device__ __forceinline__ int ceil_int(double x) {
+  const uint32_t e = (f64_hi(x) >> 20) - 1023u;
+  if (e < 30u) {
+    bool whole;
+    const int i = floor_int(x, &whole);
+    return i + (whole ? 0 : 1);
+  }
+  return ceil_slow(x);
+}
+
+// Quotients by one divisor. With y = 1 / b rounded to nearest, the multiply
+// q = a y followed by the residual correction q + (a - q b) y in two FMAs
+// gives a / b rounded to nearest (P. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", 1990), three FP64
+// instructions in place of a division's eight. Operands near the ends of the
+// exponent range are divided.
+struct Divisor {
+  double b, y;
+  bool ok;
+};
+// y: 1 / b rounded to nearest
+__device__ __forceinline__ Divisor divisor(double b, double y) {
+  const uint32_t e = (f64_hi(b) >> 20) & 0x7FFu;
+  return {b, y, e - 823u <= 400u};
+}
+__device__ __forceinline__ Divisor divisor(double b) { return divisor(b, 1.0 / b); }
+static __device__ __noinline__ double divide(double a, double b) { return a / b; }
+__device__ __forceinline__ double quot(double a, const Divisor &d) {
+  const uint32_t hi = f64_hi(a);
+  const double q = a * d.y;
+  const double z = fma(fma(-q, d.b, a), d.y, q);
+  if (d.ok && ((hi >> 20) & 0x7FFu) - 300u <= 1400u) return z;
+  if (d.ok && ((hi << 1) | f64_lo(a)) == 0u) return q; // a zero's sign
+  return divide(a, d.b);
+}
+
+} // namespace hg

@@ -289,12 +289,15 @@ struct hg_mpm {
   int64_t cap = 0, n = 0;
   hg::DevBuf<uint32_t> status;
   // ---- FP64 state (reference layouts: q, v interleaved; be 4 per point) ----
-  hg::DevBuf<double> q, v, m, vol, hl, be, J, sigma;
+  hg::DevBuf<double> q, v, m, vol, hl, be, J;
   hg::DevBuf<int32_t> jh;
   hg::DevBuf<uint8_t> kin;
   hg::DevBuf<double> g_mass, g_mom, g_mom_new, g_force, g_vel, g_acc, g_cforce,
       g_homog;
   hg::DevBuf<int32_t> g_hyb;
+  // the other set of accumulators; next_clear: cleared by the last G2P
+  hg::DevBuf<double> g_mass_next, g_mom_next, g_force_next;
+  bool next_clear = false;
   // ---- MIXED state ----
   hg::DevBuf<double2> mu_[2];
   hg::DevBuf<float2> mv_[2], mmv_[2];
@@ -351,6 +354,10 @@ struct hg_mpm {
 
 namespace hg {
 
+// a whole step, and the reference's phases; mpm64_to_grid is phase 0 without
+// the clearing of the fields that the later phases overwrite
+hg_status mpm64_step(hg_mpm *m, double dt);
+hg_status mpm64_to_grid(hg_mpm *m);
 hg_status mpm64_phase0(hg_mpm *m);
 hg_status mpm64_phase1(hg_mpm *m, double dt);
 hg_status mpm64_phase2(hg_mpm *m, double dt);

@@ -1,25 +1,42 @@
-// Plain FP64 MPM step: the drop-in for ExplicitIntegrator::flow with the
-// reference's arithmetic in double precision.
+// Plain FP64 MPM step: the drop-in for ExplicitIntegrator::flow in double
+// precision.
 //
-// This translation unit is compiled with --fmad=false so that each multiply
-// and add rounds separately, in the order the reference's Eigen expressions
-// evaluate them (the CPU oracle is built the same way with
-// -ffp-contract=off). Grid accumulation uses FP64 atomics, so node sums differ
-// from the serial reference only in summation order.
+// Bound by the FP64 pipe (about two lanes per cycle and SM: fp64_tools.cuh), so
+// each kernel evaluates what the reference evaluates in as few FP64
+// instructions as keep its accuracy. Positions, cells, stencil offsets, strains
+// and plane tests, where a last bit decides or survives a cancellation, keep
+// the reference's operations one by one (this translation unit is compiled
+// with --fmad=false);
+// sums and products elsewhere use fma() explicitly, quotients by a common
+// divisor share its reciprocal (fp64_tools.cuh), 1-D factors are divided once
+// per axis, and sign, range and yield decisions are made on the integer and
+// FP32 pipes with an FP64 test for the close calls. Grid accumulation uses
+// FP64 atomics, so node sums differ from the serial reference in order too;
+// both stay within a few units in the last place (tests: 1e-12).
+// Measured per step against the reference's expressions instruction for
+// instruction (six memsets and four launches a step, now three launches):
+// 12,800 points, linear, one call per step 84.5 -> 30.6 us; 100,000 points,
+// uGIMP, 439 -> 180 us (425 FP64 instructions per warp of points in k64_g2p,
+// 85% of the FP64 pipe; it was about 1,100).
 //
 // Kernels:
 //   k64_p2g         rasterizePointMasses + rasterizePointMomentum
 //                   (PhysicsGrid.cpp:168-411), computeHyperelasticCauchyStress
 //                   (MaterialPoints.cpp:183-202) and the particle part of
 //                   computeForces (PhysicsGrid.cpp:413-471)
-//   k64_grid_phase1 node part of computeForces (PhysicsGrid.cpp:459-471),
-//                   updateMomentum (565-586), resolvePlaneCollisions (611-673)
-//   k64_grid_phase2 lumpedMassVelocityAndAccelerationUpdate (588-609)
+//   k64_grid        node part of computeForces (PhysicsGrid.cpp:459-471),
+//                   updateMomentum (565-586), resolvePlaneCollisions
+//                   (611-673) and lumpedMassVelocityAndAccelerationUpdate
+//                   (588-609); as two launches where a caller acts in between
 //   k64_g2p         computeVelGrad, elasticPrediction, plasticCorrection,
 //                   updateVelocities, updatePositions, resolvePlaneCollisions
-//                   (MaterialPoints.cpp:204-423), fused per material point.
+//                   (MaterialPoints.cpp:204-423), fused per material point;
+//                   clears the accumulators of the next step.
 #include "hg_internal.cuh"
+#include "fp64_tools.cuh"
 #include "mpm_basis.cuh"
+
+#include <utility>
 
 namespace hg {
 
@@ -55,27 +72,6 @@ __device__ __forceinline__ double m_norm(M2d a) {
 }
 __device__ __forceinline__ M2d m_id(double s) { return {s, 0.0, 0.0, s}; }
 
-__device__ __forceinline__ M2d load_m(const double *a, int64_t p) {
-  return {a[4 * p], a[4 * p + 1], a[4 * p + 2], a[4 * p + 3]};
-}
-__device__ __forceinline__ void store_m(double *a, int64_t p, M2d m) {
-  a[4 * p] = m.a00;
-  a[4 * p + 1] = m.a10;
-  a[4 * p + 2] = m.a01;
-  a[4 * p + 3] = m.a11;
-}
-
-// ConstitutiveModel.cpp:83-97
-__device__ M2d compute_tau(M2d be, double kappa, double mu, int jh) {
-  if (jh != 0) return {0.0, 0.0, 0.0, 0.0};
-  const double J = sqrt(m_det(be));
-  const M2d be_bar = m_div(be, sqrt(m_det(be)));
-  const double tr = m_tr(be_bar);
-  const M2d dev = m_sub(be_bar, M2d{tr / 2.0, 0.0, 0.0, tr / 2.0});
-  const double s = kappa * 0.5 * (J + 1.0) * (J - 1.0);
-  return m_add(m_id(s), m_scl(mu, dev));
-}
-
 // ConstitutiveModel.cpp:26-81
 __device__ M2d plastic_correction(M2d b, double kappa, double mu, double alpha,
                                   int &jh) {
@@ -98,323 +94,665 @@ __device__ M2d plastic_correction(M2d b, double kappa, double mu, double alpha,
   return b;
 }
 
-__device__ __forceinline__ bool finite2(double a, double b) {
-  return isfinite(a) && isfinite(b);
+// x with its sign flipped where neg is the sign bit (0 or 0x80000000)
+__device__ __forceinline__ double flip(double x, uint32_t neg) {
+  return __hiloint2double((int)(f64_hi(x) ^ neg), (int)f64_lo(x));
 }
 
-__global__ void k64_p2g(MpmParams P, int64_t n, const double *__restrict__ q,
-                        const double *__restrict__ v,
-                        const double *__restrict__ m,
-                        const double *__restrict__ vol,
-                        const double *__restrict__ hl,
-                        const double *__restrict__ be,
-                        const double *__restrict__ J,
-                        const int32_t *__restrict__ jh, double *sigma,
-                        double *g_mass, double *g_mom, double *g_force,
-                        uint32_t *status) {
-  const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  const double x = q[2 * p], y = q[2 * p + 1];
-  const double h = hl[p];
-  int x0, y0, x1, y1;
-  stencil64(P.basis, x, y, h, P.gmin[0], P.gmin[1], P.h, x0, y0, x1, y1);
-  // Stress (MaterialPoints.cpp:183-202)
-  M2d tau{0.0, 0.0, 0.0, 0.0};
-  const double Jp = J[p];
-  if (Jp <= 1.0) tau = compute_tau(m_scl(Jp, load_m(be, p)), P.kappa, P.mu, jh[p]);
-  const M2d sg = m_div(tau, Jp);
-  store_m(sigma, p, sg);
-  if (x0 < 0 || y0 < 0 || x1 > P.nx || y1 > P.ny) {
-    atomicOr(status, (uint32_t)HG_STATUS_OUT_OF_GRID);
-    return;
+// The 2-D weights and gradients of a point's stencil as products of 1-D
+// factors: node (kx, ky) has weight wx[kx] wy[ky] and gradient (dx[kx] vy[ky],
+// vx[kx] dy[ky]), where v is the factor across a gradient's axis (over h for
+// the linear basis, whose own derivative factor is a sign).
+constexpr uint32_t NO_SLOPE = 1u; // linear: derivative 0 (else the sign bit of it)
+template <int BASIS> struct Axis;
+
+// LinearBasisFunctions.cpp:6-22, 53-59, 81-136: nodes i, i + 1 at offsets
+// d = ((x - h i) - g) / h; w = 1 - |d|, dw/dx = -sign(d) / h.
+template <> struct Axis<HG_BASIS_LINEAR> {
+  int i0, n;
+  double w[2], v[2]; // weight, weight / h
+  uint32_t sg[2];
+  __device__ __forceinline__ void set(double x, double, double g, const Divisor &H) {
+    i0 = floor_int(quot(x - g, H));
+    n = 2;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int i = i0 + k;
+      const double hi = i >= 0 ? H.b * index_f64(i) : H.b * (double)i;
+      const double d = quot((x - hi) - g, H);
+      const double a = flip(d, f64_hi(d) & 0x80000000u);
+      const bool in = f64_less(a, 1.0);
+      w[k] = in ? 1.0 - a : 0.0;
+      v[k] = in ? quot(w[k], H) : 0.0;
+      // -1 for d >= 0 (a zero's sign apart), 1 for d < 0, 0 beyond 1
+      sg[k] = f64_less(1.0, a) ? NO_SLOPE
+                               : (f64_hi(d) >> 31 && !f64_zero(d) ? 0u : 0x80000000u);
+    }
   }
-  const double mp = m[p];
-  const double pmx = mp * v[2 * p], pmy = mp * v[2 * p + 1];
-  const double c = -vol[p] * Jp;
-  auto node = [&](int ix, int iy, double w, double gx, double gy) {
-    const int64_t i = (int64_t)iy * (P.nx + 1) + ix;
-    atomicAdd(&g_mass[i], w * mp);
-    atomicAdd(&g_mom[2 * i], w * pmx);
-    atomicAdd(&g_mom[2 * i + 1], w * pmy);
-    if (w == 0.0) return;
-    const double swx = sg.a00 * gx + sg.a01 * gy;
-    const double swy = sg.a10 * gx + sg.a11 * gy;
-    atomicAdd(&g_force[2 * i], c * swx);
-    atomicAdd(&g_force[2 * i + 1], c * swy);
-  };
-  const int nxs = x1 - x0 + 1, nys = y1 - y0 + 1;
-  if (nxs <= STENCIL_AXIS && nys <= STENCIL_AXIS) {
-    double ax[STENCIL_AXIS], bx[STENCIL_AXIS], ay[STENCIL_AXIS], by[STENCIL_AXIS];
-    axis_factors(P.basis, x, h, x0, nxs, P.gmin[0], P.h, ax, bx);
-    axis_factors(P.basis, y, h, y0, nys, P.gmin[1], P.h, ay, by);
+};
+
+// uGIMPLinearBasisFunctions.cpp:6-42, 71-94, 110-156. With a = |x - x_i|,
+// L = half-width and q one quotient by h:
+//   a >= h + L      0
+//   a >= h - L      q = (h + L - a)^2 / h: q / 2,       slope (h + L - a) / h
+//   a >= L          q = a / h: 2 L (1 - q),             slope 2 L / h
+//   else            q = (L^2 + a^2) / h: 2 L - q,       slope 2 a / h
+// The cases are selected, not branched on: FP64 instructions issue once per
+// warp and case taken.
+template <> struct Axis<HG_BASIS_UGIMP> {
+  int i0, n;
+  double w[STENCIL_AXIS], d[STENCIL_AXIS];
+  __device__ __forceinline__ void set(double x, double L, double g, const Divisor &H) {
+    i0 = floor_int(quot((x - L) - g, H));
+    n = ceil_int(quot((x + L) - g, H)) - i0 + 1;
+    const double wide = H.b + L, narrow_ = H.b - L, two = 2.0 * L, sq = L * L;
+#pragma unroll
+    for (int k = 0; k < STENCIL_AXIS; ++k) {
+      w[k] = 0.0;
+      d[k] = 0.0;
+      if (k >= n) continue;
+      const int i = i0 + k;
+      const double xi = (i >= 0 ? H.b * index_f64(i) : H.b * (double)i) + g;
+      const double s = x - xi;
+      const uint32_t neg = f64_hi(s) & 0x80000000u;
+      const double a = flip(s, neg);
+      if (!f64_less(a, wide)) continue;
+      const bool edge = !f64_less(a, narrow_), mid = !f64_less(a, L);
+      const double t = wide - a;
+      const double m = edge ? t : a;
+      const double m2 = m * m;
+      const double q = quot(edge ? m2 : (mid ? a : sq + m2), H);
+      const double z = (mid ? 1.0 : two) - q;
+      w[k] = edge ? 0.5 * q : (mid ? two * z : z);
+      const double slope = quot(edge ? t : (mid ? two : a + a), H);
+      d[k] = flip(slope, neg ^ 0x80000000u); // (a zero offset: slope 0 either way)
+    }
+  }
+};
+
+template <int BASIS> struct Stencil;
+template <> struct Stencil<HG_BASIS_LINEAR> {
+  Axis<HG_BASIS_LINEAR> X, Y;
+  __device__ __forceinline__ void set(const MpmParams &P, double x, double y, double hl,
+                                      const Divisor &H) {
+    X.set(x, hl, P.gmin[0], H);
+    Y.set(y, hl, P.gmin[1], H);
+  }
+  template <class F> __device__ __forceinline__ void each(int row, F &&f) const {
+#pragma unroll
+    for (int ky = 0; ky < 2; ++ky)
+#pragma unroll
+      for (int kx = 0; kx < 2; ++kx)
+        f((Y.i0 + ky) * (int64_t)row + X.i0 + kx, X.w[kx] * Y.w[ky],
+          X.sg[kx] == NO_SLOPE ? 0.0 : flip(Y.v[ky], X.sg[kx]),
+          Y.sg[ky] == NO_SLOPE ? 0.0 : flip(X.v[kx], Y.sg[ky]));
+  }
+};
+template <> struct Stencil<HG_BASIS_UGIMP> {
+  Axis<HG_BASIS_UGIMP> X, Y;
+  __device__ __forceinline__ void set(const MpmParams &P, double x, double y, double hl,
+                                      const Divisor &H) {
+    X.set(x, hl, P.gmin[0], H);
+    Y.set(y, hl, P.gmin[1], H);
+    // over the point's volume 4 hl^2, once per node of one axis
+    const Divisor V = divisor(4.0 * hl * hl);
+#pragma unroll
+    for (int k = 0; k < STENCIL_AXIS; ++k)
+      if (k < Y.n) {
+        Y.w[k] = quot(Y.w[k], V);
+        Y.d[k] = quot(Y.d[k], V);
+      }
+  }
+  template <class F> __device__ __forceinline__ void each(int row, F &&f) const {
 #pragma unroll
     for (int ky = 0; ky < STENCIL_AXIS; ++ky) {
-      if (ky >= nys) break;
+      if (ky >= Y.n) break;
 #pragma unroll
       for (int kx = 0; kx < STENCIL_AXIS; ++kx) {
-        if (kx >= nxs) break;
-        double gx, gy;
-        grad_ax(P.basis, ax[kx], bx[kx], ay[ky], by[ky], h, P.h, gx, gy);
-        node(x0 + kx, y0 + ky, weight_ax(P.basis, ax[kx], ay[ky], h), gx, gy);
+        if (kx >= X.n) break;
+        f((Y.i0 + ky) * (int64_t)row + X.i0 + kx, X.w[kx] * Y.w[ky], X.d[kx] * Y.w[ky],
+          X.w[kx] * Y.d[ky]);
       }
     }
-    return;
   }
+};
+
+// The stencil's inclusive node range (stencil64) leaves the grid, or is wider
+// than the kernels' stencils hold.
+template <int BASIS>
+__device__ __forceinline__ bool off_grid(const MpmParams &P, const Stencil<BASIS> &S) {
+  return S.X.i0 < 0 || S.Y.i0 < 0 || S.X.i0 + S.X.n - 1 > P.nx || S.Y.i0 + S.Y.n - 1 > P.ny;
+}
+template <int BASIS> __device__ __forceinline__ bool too_wide(const Stencil<BASIS> &S) {
+  return BASIS == HG_BASIS_UGIMP && (S.X.n > STENCIL_AXIS || S.Y.n > STENCIL_AXIS);
+}
+
+struct P2gArgs {
+  int64_t n;
+  const double *q, *v, *m, *vol, *hl, *be, *J;
+  const int32_t *jh;
+  double *g_mass, *g_mom, *g_force;
+  uint32_t *status;
+  double half_kappa;
+};
+
+// Strains are stored as be_bar and J near 1, so the last bit of each is the
+// last bit of the stress: what forms them (products with J, determinants,
+// roots, quotients, traces) keeps the reference's operations one by one.
+__device__ __forceinline__ double det_sym(double b00, double b01, double b11) {
+  return b00 * b11 - b01 * b01;
+}
+
+// -vol tau, the Kirchhoff stress as it enters the node forces
+// (-vol J sigma with sigma = tau / J), ConstitutiveModel.cpp:83-97.
+__device__ __forceinline__ M2d node_stress(const MpmParams &P, const P2gArgs &A, int64_t p) {
+  const double Jp = A.J[p];
+  if (!(Jp <= 1.0) || A.jh[p] != 0) return {0.0, 0.0, 0.0, 0.0};
+  const double2 c0 = reinterpret_cast<const double2 *>(A.be)[2 * p];
+  const double2 c1 = reinterpret_cast<const double2 *>(A.be)[2 * p + 1];
+  const M2d be = m_scl(Jp, M2d{c0.x, c0.y, c1.x, c1.y});
+  const double J = sqrt(m_det(be));
+  const Divisor D = divisor(J);
+  const double a00 = quot(be.a00, D), a10 = quot(be.a10, D), a11 = quot(be.a11, D);
+  const double a01 = __double_as_longlong(c0.y) == __double_as_longlong(c1.x) ? a10 : quot(be.a01, D);
+  const double half_tr = (a00 + a11) * 0.5;
+  const double s = A.half_kappa * (J + 1.0) * (J - 1.0);
+  const double c = -A.vol[p], cm = c * P.mu;
+  return {c * fma(P.mu, a00 - half_tr, s), cm * a10, cm * a01, c * fma(P.mu, a11 - half_tr, s)};
+}
+
+// General stencils (wider than STENCIL_AXIS nodes), node by node.
+__device__ __noinline__ void p2g_wide(const MpmParams &P, const P2gArgs &A, int64_t p, M2d S) {
+  const double x = A.q[2 * p], y = A.q[2 * p + 1], h = A.hl[p], mp = A.m[p];
+  const double pmx = mp * A.v[2 * p], pmy = mp * A.v[2 * p + 1];
+  int x0, y0, x1, y1;
+  stencil64(P.basis, x, y, h, P.gmin[0], P.gmin[1], P.h, x0, y0, x1, y1);
   for (int iy = y0; iy <= y1; ++iy)
     for (int ix = x0; ix <= x1; ++ix) {
       double gx, gy;
       weight_grad64(P.basis, x, y, h, ix, iy, P.gmin[0], P.gmin[1], P.h, gx, gy);
-      node(ix, iy, weight64(P.basis, x, y, h, ix, iy, P.gmin[0], P.gmin[1], P.h), gx, gy);
+      const double w = weight64(P.basis, x, y, h, ix, iy, P.gmin[0], P.gmin[1], P.h);
+      const int64_t i = (int64_t)iy * (P.nx + 1) + ix;
+      atomicAdd(&A.g_mass[i], w * mp);
+      atomicAdd(&A.g_mom[2 * i], w * pmx);
+      atomicAdd(&A.g_mom[2 * i + 1], w * pmy);
+      if (w == 0.0) continue;
+      atomicAdd(&A.g_force[2 * i], S.a00 * gx + S.a01 * gy);
+      atomicAdd(&A.g_force[2 * i + 1], S.a10 * gx + S.a11 * gy);
     }
 }
 
-__global__ void k64_grid_phase1(MpmParams P, double dt,
-                                const double *__restrict__ g_mass,
-                                const double *__restrict__ g_mom,
-                                double *g_mom_new, double *g_force,
-                                const double *__restrict__ g_cforce,
-                                const int32_t *__restrict__ g_hyb) {
-  const int64_t nn = (int64_t)(P.nx + 1) * (P.ny + 1);
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= nn) return;
-  const double mi = g_mass[i];
-  double fx = g_force[2 * i], fy = g_force[2 * i + 1];
-  if (g_hyb[i] > 0) {
-    fx += 0.5 * mi * P.g[0];
-    fy += 0.5 * mi * P.g[1];
-  } else {
-    fx += mi * P.g[0];
-    fy += mi * P.g[1];
-  }
-  fx += g_cforce[2 * i];
-  fy += g_cforce[2 * i + 1];
-  g_force[2 * i] = fx;
-  g_force[2 * i + 1] = fy;
-  double pnx = g_mom_new[2 * i], pny = g_mom_new[2 * i + 1];
-  if (mi > 0.0) {
-    pnx = g_mom[2 * i] + dt * fx;
-    pny = g_mom[2 * i + 1] + dt * fy;
-  }
-  // PhysicsGrid::resolvePlaneCollisions
-  const int ix = (int)(i % (P.nx + 1)), iy = (int)(i / (P.nx + 1));
-  const double px = P.gmin[0] + P.h * (double)ix;
-  const double py = P.gmin[1] + P.h * (double)iy;
-  for (int k = 0; k < P.nplanes; ++k) {
-    const MpmPlaneDev &pl = P.planes[k];
-    if (py < pl.lower_bound) continue;
-    const double d = pl.n[0] * (px - pl.x[0]) + pl.n[1] * (py - pl.x[1]);
-    if (d > 0.0) continue;
-    if (!pl.sticking) {
-      if (mi <= 0.0) continue;
-      double vx = pnx / mi, vy = pny / mi;
-      const double vn = pl.n[0] * vx + pl.n[1] * vy;
-      if (vn > 0.0) continue;
-      vx = vx - vn * pl.n[0];
-      vy = vy - vn * pl.n[1];
-      pnx = mi * vx;
-      pny = mi * vy;
-    } else {
-      pnx = 0.0;
-      pny = 0.0;
-    }
-  }
-  g_mom_new[2 * i] = pnx;
-  g_mom_new[2 * i + 1] = pny;
-}
-
-__global__ void k64_grid_phase2(MpmParams P, double dt,
-                                const double *__restrict__ g_mass,
-                                const double *__restrict__ g_mom,
-                                const double *__restrict__ g_mom_new,
-                                double *g_vel, double *g_acc) {
-  const int64_t nn = (int64_t)(P.nx + 1) * (P.ny + 1);
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= nn) return;
-  const double mi = g_mass[i];
-  if (mi > 0.0) {
-    g_vel[2 * i] = g_mom_new[2 * i] / mi;
-    g_vel[2 * i + 1] = g_mom_new[2 * i + 1] / mi;
-    const double dm = dt * mi;
-    g_acc[2 * i] = (g_mom_new[2 * i] - g_mom[2 * i]) / dm;
-    g_acc[2 * i + 1] = (g_mom_new[2 * i + 1] - g_mom[2 * i + 1]) / dm;
-  } else {
-    g_vel[2 * i] = 0.0;
-    g_vel[2 * i + 1] = 0.0;
-    g_acc[2 * i] = 0.0;
-    g_acc[2 * i + 1] = 0.0;
-  }
-}
-
-__global__ void k64_g2p(MpmParams P, double dt, int64_t n, double *q, double *v,
-                        const double *__restrict__ hl, double *be, double *J,
-                        int32_t *jh, const uint8_t *__restrict__ kin,
-                        const double *__restrict__ g_vel,
-                        const double *__restrict__ g_acc, uint32_t *status) {
+template <int BASIS>
+__global__ void k64_p2g(const __grid_constant__ MpmParams P, const __grid_constant__ P2gArgs A) {
+  pdl_wait();
+  pdl_trigger();
   const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  double x = q[2 * p], y = q[2 * p + 1];
-  const double h = hl[p];
-  int x0, y0, x1, y1;
-  stencil64(P.basis, x, y, h, P.gmin[0], P.gmin[1], P.h, x0, y0, x1, y1);
-  if (x0 < 0 || y0 < 0 || x1 > P.nx || y1 > P.ny) {
-    atomicOr(status, (uint32_t)HG_STATUS_OUT_OF_GRID);
+  if (p >= A.n) return;
+  const double2 x = reinterpret_cast<const double2 *>(A.q)[p];
+  const Divisor H = divisor(P.h, P.inv_h);
+  Stencil<BASIS> St;
+  St.set(P, x.x, x.y, BASIS == HG_BASIS_UGIMP ? A.hl[p] : 0.0, H);
+  if (off_grid<BASIS>(P, St)) {
+    atomicOr(A.status, (uint32_t)HG_STATUS_OUT_OF_GRID);
     return;
   }
-  const int64_t row = P.nx + 1;
-  // axis factors of the start-of-step position (when the stencil fits)
-  const int nxs = x1 - x0 + 1, nys = y1 - y0 + 1;
-  const bool fits = nxs <= STENCIL_AXIS && nys <= STENCIL_AXIS;
-  double ax[STENCIL_AXIS], bx[STENCIL_AXIS], ay[STENCIL_AXIS], by[STENCIL_AXIS];
-  if (fits) {
-    axis_factors(P.basis, x, h, x0, nxs, P.gmin[0], P.h, ax, bx);
-    axis_factors(P.basis, y, h, y0, nys, P.gmin[1], P.h, ay, by);
+  const M2d S = node_stress(P, A, p);
+  if (too_wide<BASIS>(St)) {
+    p2g_wide(P, A, p, S);
+    return;
   }
-  // visits the stencil's nodes in the reference's order with their weight
-  // and weight gradient
-  auto each_node = [&](auto &&f) {
-    if (fits) {
-#pragma unroll
-      for (int ky = 0; ky < STENCIL_AXIS; ++ky) {
-        if (ky >= nys) break;
-#pragma unroll
-        for (int kx = 0; kx < STENCIL_AXIS; ++kx) {
-          if (kx >= nxs) break;
-          double gx, gy;
-          grad_ax(P.basis, ax[kx], bx[kx], ay[ky], by[ky], h, P.h, gx, gy);
-          f((int64_t)(y0 + ky) * row + (x0 + kx), weight_ax(P.basis, ax[kx], ay[ky], h), gx,
-            gy);
+  const double mp = A.m[p];
+  const double2 v = reinterpret_cast<const double2 *>(A.v)[p];
+  const double pmx = mp * v.x, pmy = mp * v.y;
+  St.each(P.nx + 1, [&](int64_t i, double w, double gx, double gy) {
+    // nodes of zero weight get nothing (PhysicsGrid.cpp:439-441)
+    if (f64_zero(w)) return;
+    atomicAdd(&A.g_mass[i], w * mp);
+    atomicAdd(&A.g_mom[2 * i], w * pmx);
+    atomicAdd(&A.g_mom[2 * i + 1], w * pmy);
+    atomicAdd(&A.g_force[2 * i], fma(S.a00, gx, S.a01 * gy));
+    atomicAdd(&A.g_force[2 * i + 1], fma(S.a10, gx, S.a11 * gy));
+  });
+}
+
+struct GridArgs {
+  int64_t nn;
+  double dt;
+  const double *mass, *mom;
+  double *mom_new, *force;
+  const double *cforce;
+  const int32_t *hyb;
+  double *vel, *acc;
+};
+
+// True when the plane acts on node (ix, iy) (PhysicsGrid.cpp:614-629): in FP32
+// grid units away from the plane and its lower bound, within pmargin cells of
+// either by the reference's own FP64 test.
+__device__ __forceinline__ bool node_hit(const MpmParams &P, const MpmPlaneDev &pl, float pmargin,
+                                         int ix, int iy) {
+  const float fx = (float)ix, fy = (float)iy;
+  if (fy < pl.fulb - pmargin) return false;
+  const float d32 = pl.fn[0] * (fx - pl.fux[0]) + pl.fn[1] * (fy - pl.fux[1]);
+  if (fabsf(d32) > pmargin && fabsf(fy - pl.fulb) > pmargin) return d32 < 0.0f;
+  const double px = P.gmin[0] + P.h * (double)ix, py = P.gmin[1] + P.h * (double)iy;
+  if (py < pl.lower_bound) return false;
+  return !(pl.n[0] * (px - pl.x[0]) + pl.n[1] * (py - pl.x[1]) > 0.0);
+}
+
+// FORCES: the node forces and new momenta; UPDATE: velocities and
+// accelerations from them. Nodes without mass take no FP64 arithmetic.
+template <bool FORCES, bool UPDATE>
+__global__ void __launch_bounds__(128) k64_grid(const __grid_constant__ MpmParams P,
+                                                const __grid_constant__ GridArgs A) {
+  pdl_wait();
+  pdl_trigger();
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= A.nn) return;
+  double2 *mom_new = reinterpret_cast<double2 *>(A.mom_new);
+  const double mi = A.mass[i];
+  const bool has = mi > 0.0;
+  const double2 zero = make_double2(0.0, 0.0);
+  double2 pn = zero, pm = zero;
+  if (has) pm = reinterpret_cast<const double2 *>(A.mom)[i];
+  if (FORCES) {
+    double2 *force = reinterpret_cast<double2 *>(A.force);
+    const double2 cf = reinterpret_cast<const double2 *>(A.cforce)[i];
+    if (has) {
+      double2 f = force[i];
+      const double half = A.hyb[i] > 0 ? 0.5 * mi : mi;
+      f.x = fma(half, P.g[0], f.x) + cf.x;
+      f.y = fma(half, P.g[1], f.y) + cf.y;
+      force[i] = f;
+      pn = make_double2(fma(A.dt, f.x, pm.x), fma(A.dt, f.y, pm.y));
+      const int ix = (int)(i % (P.nx + 1)), iy = (int)(i / (P.nx + 1));
+      const float pmargin = 0.01f + 4.0e-7f * (float)(P.nx + P.ny);
+      for (int k = 0; k < P.nplanes; ++k) { // PhysicsGrid::resolvePlaneCollisions
+        const MpmPlaneDev &pl = P.planes[k];
+        if (!node_hit(P, pl, pmargin, ix, iy)) continue;
+        if (!pl.sticking) {
+          double vx = pn.x / mi, vy = pn.y / mi;
+          const double vn = pl.n[0] * vx + pl.n[1] * vy;
+          if (vn > 0.0) continue;
+          vx = vx - vn * pl.n[0];
+          vy = vy - vn * pl.n[1];
+          pn = make_double2(mi * vx, mi * vy);
+        } else {
+          pn = zero;
         }
       }
+    } else if (!f64_zero(cf.x) || !f64_zero(cf.y)) {
+      const double2 f = force[i];
+      force[i] = make_double2(f.x + cf.x, f.y + cf.y);
+    }
+    mom_new[i] = pn;
+  } else if (has) {
+    pn = mom_new[i];
+  }
+  if (UPDATE) {
+    double2 v = zero, a = zero;
+    if (has) {
+      const Divisor M = divisor(mi), D = divisor(A.dt * mi);
+      v = make_double2(quot(pn.x, M), quot(pn.y, M));
+      a = make_double2(quot(pn.x - pm.x, D), quot(pn.y - pm.y, D));
+    }
+    reinterpret_cast<double2 *>(A.vel)[i] = v;
+    reinterpret_cast<double2 *>(A.acc)[i] = a;
+  }
+}
+
+struct G2pArgs {
+  int64_t n, nn;
+  double dt;
+  double *q, *v;
+  const double *hl;
+  double *be, *J;
+  int32_t *jh;
+  const uint8_t *kin;
+  const double *g_vel, *g_acc;
+  double *next_mass, *next_mom, *next_force; // the next step's accumulators, cleared
+  uint32_t *status;
+  // constants of every point
+  double yield; // alpha kappa / 2
+  double pic;   // 1 - flip_alpha
+  float mu32, yield32;
+  float px[HG_MAX_PLANES][2];
+};
+
+// What the grid gives a point: its velocity gradient, velocity, acceleration.
+struct PointGrid {
+  double L00, L10, L01, L11, vx, vy, ax, ay;
+};
+
+__device__ __noinline__ PointGrid g2p_wide(const MpmParams &P, const G2pArgs &A, double x, double y,
+                                           double h) {
+  PointGrid g{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  int x0, y0, x1, y1;
+  stencil64(P.basis, x, y, h, P.gmin[0], P.gmin[1], P.h, x0, y0, x1, y1);
+  for (int iy = y0; iy <= y1; ++iy)
+    for (int ix = x0; ix <= x1; ++ix) {
+      double gx, gy;
+      weight_grad64(P.basis, x, y, h, ix, iy, P.gmin[0], P.gmin[1], P.h, gx, gy);
+      const double w = weight64(P.basis, x, y, h, ix, iy, P.gmin[0], P.gmin[1], P.h);
+      const int64_t i = (int64_t)iy * (P.nx + 1) + ix;
+      const double vx = A.g_vel[2 * i], vy = A.g_vel[2 * i + 1];
+      g.L00 += vx * gx;
+      g.L10 += vy * gx;
+      g.L01 += vx * gy;
+      g.L11 += vy * gy;
+      g.vx += w * vx;
+      g.vy += w * vy;
+      g.ax += w * A.g_acc[2 * i];
+      g.ay += w * A.g_acc[2 * i + 1];
+    }
+  return g;
+}
+
+// elasticPrediction and plasticCorrection of a be_bar that is not symmetric
+// (MaterialPoints.cpp:324-369, ConstitutiveModel.cpp:19-81), component by
+// component.
+struct PointStrain {
+  M2d b;
+  double J;
+  int jh;
+};
+__device__ __noinline__ PointStrain strain_general(const MpmParams &P, double dt, const PointGrid &g,
+                                                   PointStrain s) {
+  const M2d L{g.L00, g.L10, g.L01, g.L11};
+  const M2d ben = m_scl(s.J, s.b);
+  const M2d bs = m_add(ben, m_scl(dt, m_add(m_mul(L, ben), m_mul(ben, m_T(L)))));
+  const double J1 = sqrt(m_det(bs));
+  int jh = s.jh;
+  const M2d bn = plastic_correction(m_scl(J1, m_div(bs, J1)), P.kappa, P.mu, P.dp_alpha, jh);
+  const double J2 = sqrt(m_det(bn));
+  return {m_div(bn, J2), J2, jh};
+}
+
+// The same for a symmetric be_bar, which stays symmetric to the bit. The
+// yield test is decided in FP32 except within 1e-5 of the yield surface, so
+// that elastic points need neither |dev be| nor the yield stress in FP64.
+__device__ __forceinline__ void strain_symmetric(const MpmParams &P, const G2pArgs &A,
+                                                 const PointGrid &g, double &b00, double &b01,
+                                                 double &b11, double &Jp, int &jh) {
+  b00 *= Jp;
+  b01 *= Jp;
+  b11 *= Jp;
+  const double l00 = fma(g.L00, b00, g.L01 * b01), l01 = fma(g.L00, b01, g.L01 * b11);
+  const double l10 = fma(g.L10, b00, g.L11 * b01), l11 = fma(g.L10, b01, g.L11 * b11);
+  b00 = fma(A.dt, l00 + l00, b00);
+  b01 = fma(A.dt, l01 + l10, b01);
+  b11 = fma(A.dt, l11 + l11, b11);
+  Jp = sqrt(det_sym(b00, b01, b11));
+  {
+    const Divisor D = divisor(Jp);
+    b00 = Jp * quot(b00, D);
+    b01 = Jp * quot(b01, D);
+    b11 = Jp * quot(b11, D);
+  }
+  double det = det_sym(b00, b01, b11);
+  Jp = sqrt(det);
+  bool grown = false;
+  if (jh != 0) {
+    grown = Jp > 1.0;
+    if (!grown) jh = 0;
+  }
+  if (grown) { // be = J I (ConstitutiveModel.cpp:28-35)
+    b00 = b11 = Jp;
+    b01 = 0.0;
+    Jp = sqrt(Jp * Jp);
+  } else {
+    const double half_tr = 0.5 * (b00 + b11);
+    const double d0 = b00 - half_tr, d1 = b11 - half_tr;
+    const double up = 1.0 + Jp, down = 1.0 - Jp;
+    const float d32 = narrow_trunc(d0), o32 = narrow_trunc(b01);
+    const float n2 = 2.0f * (d32 * d32 + o32 * o32);
+    const float limit =
+        fmaxf(0.0f, A.yield32 * narrow_trunc(up) * narrow_trunc(down)) * narrow_trunc(Jp) / A.mu32;
+    // elastic for sure, where the estimate of |dev be| is well above the
+    // rounding of d0 and FP32's smallest squares
+    const bool elastic = n2 > 1.0e-18f && sqrtf(n2) < limit * 0.99999f;
+    if (!elastic) {
+      const double ys = fmax(0.0, A.yield * up * down);
+      const double t = P.mu * (sqrt(fma(d0, d0, fma(d1, d1, 2.0 * (b01 * b01)))) / Jp);
+      if (t > ys) {
+        const double l2 = ys / t;
+        const double l1 = sqrt(fma(-(l2 * l2), d0 * d1 - b01 * b01, det));
+        b00 = fma(l2, d0, l1);
+        b11 = fma(l2, d1, l1);
+        b01 = l2 * b01;
+        Jp = sqrt(det_sym(b00, b01, b11));
+      }
+    }
+  }
+  const Divisor D = divisor(Jp);
+  b00 = quot(b00, D);
+  b01 = quot(b01, D);
+  b11 = quot(b11, D);
+}
+
+template <int BASIS>
+__global__ void k64_g2p(const __grid_constant__ MpmParams P, const __grid_constant__ G2pArgs A) {
+  pdl_wait();
+  pdl_trigger();
+  const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  for (int64_t i = p; i < A.nn; i += (int64_t)gridDim.x * blockDim.x) {
+    const double2 zero = make_double2(0.0, 0.0);
+    A.next_mass[i] = 0.0;
+    reinterpret_cast<double2 *>(A.next_mom)[i] = zero;
+    reinterpret_cast<double2 *>(A.next_force)[i] = zero;
+  }
+  if (p >= A.n) return;
+  double2 x = reinterpret_cast<const double2 *>(A.q)[p];
+  const double hl = BASIS == HG_BASIS_UGIMP ? A.hl[p] : 0.0;
+  PointGrid g{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  {
+    const Divisor H = divisor(P.h, P.inv_h);
+    Stencil<BASIS> St;
+    St.set(P, x.x, x.y, hl, H);
+    if (off_grid<BASIS>(P, St)) {
+      atomicOr(A.status, (uint32_t)HG_STATUS_OUT_OF_GRID);
       return;
     }
-    for (int iy = y0; iy <= y1; ++iy)
-      for (int ix = x0; ix <= x1; ++ix) {
-        double gx, gy;
-        weight_grad64(P.basis, x, y, h, ix, iy, P.gmin[0], P.gmin[1], P.h, gx, gy);
-        f((int64_t)iy * row + ix, weight64(P.basis, x, y, h, ix, iy, P.gmin[0], P.gmin[1], P.h),
-          gx, gy);
-      }
-  };
-  // computeVelGrad (MaterialPoints.cpp:296-322)
-  M2d L{0.0, 0.0, 0.0, 0.0};
-  each_node([&](int64_t i, double, double gx, double gy) {
-    const double vx = g_vel[2 * i], vy = g_vel[2 * i + 1];
-    L = m_add(L, M2d{vx * gx, vy * gx, vx * gy, vy * gy});
-  });
-  // elasticPrediction (MaterialPoints.cpp:324-348, ConstitutiveModel.cpp:19-22)
-  double Jp = J[p];
-  M2d bb = load_m(be, p);
-  {
-    const M2d ben = m_scl(Jp, bb);
-    const M2d bs = m_add(ben, m_scl(dt, m_add(m_mul(L, ben), m_mul(ben, m_T(L)))));
-    Jp = sqrt(m_det(bs));
-    bb = m_div(bs, sqrt(m_det(bs)));
-  }
-  // plasticCorrection (MaterialPoints.cpp:350-369)
-  int jhp = jh[p];
-  {
-    const M2d bn = plastic_correction(m_scl(Jp, bb), P.kappa, P.mu, P.dp_alpha, jhp);
-    Jp = sqrt(m_det(bn));
-    bb = m_div(bn, sqrt(m_det(bn)));
-  }
-  // updateVelocities (MaterialPoints.cpp:204-245) and updatePositions
-  // (247-288); both read the grid at the start-of-step position.
-  double vpx = 0.0, vpy = 0.0, apx = 0.0, apy = 0.0, gvx = 0.0, gvy = 0.0;
-  each_node([&](int64_t i, double w, double, double) {
-    vpx = vpx + w * g_vel[2 * i];
-    vpy = vpy + w * g_vel[2 * i + 1];
-    apx = apx + w * g_acc[2 * i];
-    apy = apy + w * g_acc[2 * i + 1];
-  });
-  gvx = vpx;
-  gvy = vpy;
-  double vx = v[2 * p], vy = v[2 * p + 1];
-  const bool kinem = kin[p] != 0;
-  if (!kinem) {
-    const double a = P.flip_alpha;
-    const double fx = vx + apx * dt, fy = vy + apy * dt;
-    vx = (1.0 - a) * vpx + a * fx;
-    vy = (1.0 - a) * vpy + a * fy;
-    x += dt * gvx;
-    y += dt * gvy;
-  } else {
-    x += dt * vx;
-    y += dt * vy;
-  }
-  // MaterialPoints::resolvePlaneCollisions (MaterialPoints.cpp:371-423)
-  for (int k = 0; k < P.nplanes; ++k) {
-    const MpmPlaneDev &pl = P.planes[k];
-    if (y < pl.lower_bound) continue;
-    const double d = pl.n[0] * (x - pl.x[0]) + pl.n[1] * (y - pl.x[1]);
-    if (d > 0.0) continue;
-    x += -d * pl.n[0];
-    y += -d * pl.n[1];
-    if (!pl.sticking) {
-      const double vn = pl.n[0] * vx + pl.n[1] * vy;
-      if (vn > 0.0) continue;
-      vx = vx - vn * pl.n[0];
-      vy = vy - vn * pl.n[1];
+    if (too_wide<BASIS>(St)) {
+      g = g2p_wide(P, A, x.x, x.y, hl);
     } else {
-      vx = 0.0;
-      vy = 0.0;
+      // computeVelGrad (MaterialPoints.cpp:296-322), and the interpolations of
+      // updateVelocities (204-245) and updatePositions (247-288)
+      St.each(P.nx + 1, [&](int64_t i, double w, double gx, double gy) {
+        const double2 v = reinterpret_cast<const double2 *>(A.g_vel)[i];
+        const double2 a = reinterpret_cast<const double2 *>(A.g_acc)[i];
+        g.L00 = fma(v.x, gx, g.L00);
+        g.L10 = fma(v.y, gx, g.L10);
+        g.L01 = fma(v.x, gy, g.L01);
+        g.L11 = fma(v.y, gy, g.L11);
+        g.vx = fma(w, v.x, g.vx);
+        g.vy = fma(w, v.y, g.vy);
+        g.ax = fma(w, a.x, g.ax);
+        g.ay = fma(w, a.y, g.ay);
+      });
     }
   }
-  if (!finite2(x, y) || !finite2(vx, vy) || !isfinite(Jp))
-    atomicOr(status, (uint32_t)HG_STATUS_NONFINITE);
-  q[2 * p] = x;
-  q[2 * p + 1] = y;
-  v[2 * p] = vx;
-  v[2 * p + 1] = vy;
-  store_m(be, p, bb);
-  J[p] = Jp;
-  jh[p] = jhp;
+  double Jp = A.J[p];
+  int jh = A.jh[p];
+  double2 c0 = reinterpret_cast<const double2 *>(A.be)[2 * p];
+  double2 c1 = reinterpret_cast<const double2 *>(A.be)[2 * p + 1];
+  if (__double_as_longlong(c0.y) == __double_as_longlong(c1.x)) {
+    strain_symmetric(P, A, g, c0.x, c0.y, c1.y, Jp, jh);
+    c1.x = c0.y;
+  } else {
+    const PointStrain s = strain_general(P, A.dt, g, {{c0.x, c0.y, c1.x, c1.y}, Jp, jh});
+    c0 = make_double2(s.b.a00, s.b.a10);
+    c1 = make_double2(s.b.a01, s.b.a11);
+    Jp = s.J;
+    jh = s.jh;
+  }
+  double2 v = reinterpret_cast<const double2 *>(A.v)[p];
+  if (A.kin[p] == 0) {
+    const double a = P.flip_alpha, b = A.pic;
+    v.x = fma(a, fma(g.ax, A.dt, v.x), b * g.vx);
+    v.y = fma(a, fma(g.ay, A.dt, v.y), b * g.vy);
+    x.x += A.dt * g.vx;
+    x.y += A.dt * g.vy;
+  } else {
+    x.x += A.dt * v.x;
+    x.y += A.dt * v.y;
+  }
+  // MaterialPoints::resolvePlaneCollisions (MaterialPoints.cpp:371-423): FP32
+  // leaves out the planes a point is clearly in front of (the coordinates'
+  // truncation and FP32 sums err by less than 1e-6 of the terms)
+  for (int k = 0; k < P.nplanes; ++k) {
+    const MpmPlaneDev &pl = P.planes[k];
+    {
+      const float fx = narrow_trunc(x.x), fy = narrow_trunc(x.y);
+      const float px = A.px[k][0], py = A.px[k][1];
+      const float d32 = pl.fn[0] * (fx - px) + pl.fn[1] * (fy - py);
+      if (d32 > 1.0e-6f * (fabsf(fx) + fabsf(px) + fabsf(fy) + fabsf(py))) continue;
+    }
+    if (x.y < pl.lower_bound) continue;
+    const double d = pl.n[0] * (x.x - pl.x[0]) + pl.n[1] * (x.y - pl.x[1]);
+    if (d > 0.0) continue;
+    x.x += -d * pl.n[0];
+    x.y += -d * pl.n[1];
+    if (!pl.sticking) {
+      const double vn = pl.n[0] * v.x + pl.n[1] * v.y;
+      if (vn > 0.0) continue;
+      v.x = v.x - vn * pl.n[0];
+      v.y = v.y - vn * pl.n[1];
+    } else {
+      v = make_double2(0.0, 0.0);
+    }
+  }
+  if (!finite_bits(x.x) || !finite_bits(x.y) || !finite_bits(v.x) || !finite_bits(v.y) ||
+      !finite_bits(Jp))
+    atomicOr(A.status, (uint32_t)HG_STATUS_NONFINITE);
+  reinterpret_cast<double2 *>(A.q)[p] = x;
+  reinterpret_cast<double2 *>(A.v)[p] = v;
+  reinterpret_cast<double2 *>(A.be)[2 * p] = c0;
+  reinterpret_cast<double2 *>(A.be)[2 * p + 1] = c1;
+  A.J[p] = Jp;
+  A.jh[p] = jh;
 }
 
 inline int blocks_for(int64_t n, int t) { return (int)((n + t - 1) / t); }
 
+// Threads per CTA of the point kernels: one warp while the points are few, so
+// that their warps spread over all SMs' FP64 pipes (12,800 points: 400 warps,
+// at most 3 per SM against 4 with CTAs of four warps).
+int point_threads(const hg_mpm *m) {
+  return m->n < (int64_t)m->ctx->num_sms * 32 * 16 ? 32 : 128;
+}
+
+template <bool FORCES, bool UPDATE> hg_status grid_pass(hg_mpm *m, double dt) {
+  GridArgs A;
+  A.nn = (int64_t)(m->p.nx + 1) * (m->p.ny + 1);
+  A.dt = dt;
+  A.mass = m->g_mass.p;
+  A.mom = m->g_mom.p;
+  A.mom_new = m->g_mom_new.p;
+  A.force = m->g_force.p;
+  A.cforce = m->g_cforce.p;
+  A.hyb = m->g_hyb.p;
+  A.vel = m->g_vel.p;
+  A.acc = m->g_acc.p;
+  auto kernel = k64_grid<FORCES, UPDATE>;
+  HG_LAUNCH_PDL(kernel, blocks_for(A.nn, 128), 128, 0, m->ctx->stream, m->p, A);
+  HG_CHECK_LAUNCH();
+  return HG_OK;
+}
+
+hg_status to_points(hg_mpm *m, double dt) {
+  if (m->n <= 0) return HG_OK;
+  G2pArgs A;
+  A.n = m->n;
+  A.nn = (int64_t)(m->p.nx + 1) * (m->p.ny + 1);
+  A.dt = dt;
+  A.q = m->q.p;
+  A.v = m->v.p;
+  A.hl = m->hl.p;
+  A.be = m->be.p;
+  A.J = m->J.p;
+  A.jh = m->jh.p;
+  A.kin = m->kin.p;
+  A.g_vel = m->g_vel.p;
+  A.g_acc = m->g_acc.p;
+  A.next_mass = m->g_mass_next.p;
+  A.next_mom = m->g_mom_next.p;
+  A.next_force = m->g_force_next.p;
+  A.status = m->status.p;
+  A.yield = 0.5 * m->p.dp_alpha * m->p.kappa;
+  A.pic = 1.0 - m->p.flip_alpha;
+  A.mu32 = (float)m->p.mu;
+  A.yield32 = (float)A.yield;
+  for (int k = 0; k < HG_MAX_PLANES; ++k)
+    for (int c = 0; c < 2; ++c) A.px[k][c] = (float)m->p.planes[k].x[c];
+  auto kernel = m->p.basis == HG_BASIS_UGIMP ? k64_g2p<HG_BASIS_UGIMP> : k64_g2p<HG_BASIS_LINEAR>;
+  const int t = point_threads(m);
+  HG_LAUNCH_PDL(kernel, blocks_for(m->n, t), t, 0, m->ctx->stream, m->p, A);
+  HG_CHECK_LAUNCH();
+  m->next_clear = true;
+  return HG_OK;
+}
+
 } // namespace
+
+// The accumulators of P2G (mass, momentum, force) are a pair: the last G2P
+// cleared the other set, which becomes this step's.
+hg_status mpm64_to_grid(hg_mpm *m) {
+  cudaStream_t s = m->ctx->stream;
+  const int64_t nn = (int64_t)(m->p.nx + 1) * (m->p.ny + 1);
+  if (m->next_clear) {
+    std::swap(m->g_mass.p, m->g_mass_next.p);
+    std::swap(m->g_mom.p, m->g_mom_next.p);
+    std::swap(m->g_force.p, m->g_force_next.p);
+    m->next_clear = false;
+  } else {
+    HG_CUDA_TRY(cudaMemsetAsync(m->g_mass.p, 0, sizeof(double) * nn, s));
+    HG_CUDA_TRY(cudaMemsetAsync(m->g_mom.p, 0, sizeof(double) * 2 * nn, s));
+    HG_CUDA_TRY(cudaMemsetAsync(m->g_force.p, 0, sizeof(double) * 2 * nn, s));
+  }
+  if (m->n <= 0) return HG_OK;
+  P2gArgs A;
+  A.n = m->n;
+  A.q = m->q.p;
+  A.v = m->v.p;
+  A.m = m->m.p;
+  A.vol = m->vol.p;
+  A.hl = m->hl.p;
+  A.be = m->be.p;
+  A.J = m->J.p;
+  A.jh = m->jh.p;
+  A.g_mass = m->g_mass.p;
+  A.g_mom = m->g_mom.p;
+  A.g_force = m->g_force.p;
+  A.status = m->status.p;
+  A.half_kappa = m->p.kappa * 0.5;
+  auto kernel = m->p.basis == HG_BASIS_UGIMP ? k64_p2g<HG_BASIS_UGIMP> : k64_p2g<HG_BASIS_LINEAR>;
+  const int t = point_threads(m);
+  HG_LAUNCH_PDL(kernel, blocks_for(m->n, t), t, 0, s, m->p, A);
+  HG_CHECK_LAUNCH();
+  return HG_OK;
+}
+
+hg_status mpm64_step(hg_mpm *m, double dt) {
+  hg_status st;
+  if ((st = mpm64_to_grid(m)) || (st = grid_pass<true, true>(m, dt))) return st;
+  return to_points(m, dt);
+}
 
 hg_status mpm64_phase0(hg_mpm *m) {
   cudaStream_t s = m->ctx->stream;
   const int64_t nn = (int64_t)(m->p.nx + 1) * (m->p.ny + 1);
   // clearRasterizedData (PhysicsGrid.cpp:107-114)
-  HG_CUDA_TRY(cudaMemsetAsync(m->g_mass.p, 0, sizeof(double) * nn, s));
-  HG_CUDA_TRY(cudaMemsetAsync(m->g_mom.p, 0, sizeof(double) * 2 * nn, s));
   HG_CUDA_TRY(cudaMemsetAsync(m->g_mom_new.p, 0, sizeof(double) * 2 * nn, s));
-  HG_CUDA_TRY(cudaMemsetAsync(m->g_force.p, 0, sizeof(double) * 2 * nn, s));
   HG_CUDA_TRY(cudaMemsetAsync(m->g_vel.p, 0, sizeof(double) * 2 * nn, s));
   HG_CUDA_TRY(cudaMemsetAsync(m->g_acc.p, 0, sizeof(double) * 2 * nn, s));
-  if (m->n > 0) {
-    HG_LAUNCH(k64_p2g, blocks_for(m->n, 128), 128, 0, s, m->p, m->n, m->q.p,
-              m->v.p, m->m.p, m->vol.p, m->hl.p, m->be.p, m->J.p, m->jh.p,
-              m->sigma.p, m->g_mass.p, m->g_mom.p, m->g_force.p, m->status.p);
-    HG_CHECK_LAUNCH();
-  }
-  return HG_OK;
+  return mpm64_to_grid(m);
 }
 
-hg_status mpm64_phase1(hg_mpm *m, double dt) {
-  const int64_t nn = (int64_t)(m->p.nx + 1) * (m->p.ny + 1);
-  HG_LAUNCH(k64_grid_phase1, blocks_for(nn, 256), 256, 0, m->ctx->stream, m->p,
-            dt, m->g_mass.p, m->g_mom.p, m->g_mom_new.p, m->g_force.p,
-            m->g_cforce.p, m->g_hyb.p);
-  HG_CHECK_LAUNCH();
-  return HG_OK;
-}
+hg_status mpm64_phase1(hg_mpm *m, double dt) { return grid_pass<true, false>(m, dt); }
 
 hg_status mpm64_phase2(hg_mpm *m, double dt) {
-  const int64_t nn = (int64_t)(m->p.nx + 1) * (m->p.ny + 1);
-  cudaStream_t s = m->ctx->stream;
-  HG_LAUNCH(k64_grid_phase2, blocks_for(nn, 256), 256, 0, s, m->p, dt,
-            m->g_mass.p, m->g_mom.p, m->g_mom_new.p, m->g_vel.p, m->g_acc.p);
-  HG_CHECK_LAUNCH();
-  if (m->n > 0) {
-    HG_LAUNCH(k64_g2p, blocks_for(m->n, 128), 128, 0, s, m->p, dt, m->n, m->q.p,
-              m->v.p, m->hl.p, m->be.p, m->J.p, m->jh.p, m->kin.p, m->g_vel.p,
-              m->g_acc.p, m->status.p);
-    HG_CHECK_LAUNCH();
-  }
-  return HG_OK;
+  const hg_status st = grid_pass<false, true>(m, dt);
+  return st != HG_OK ? st : to_points(m, dt);
 }
 
 } // namespace hg
