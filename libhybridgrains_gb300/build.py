@@ -38,7 +38,8 @@ SOURCES = [
     ("resampling.cu", True),  # host code (resampling)
     ("state.cu", False),  # checkpoint / resume blobs
 ]
-HEADERS = ["hg_internal.cuh", "fp64_tools.cuh", "mpm_basis.cuh", "scan_block.cuh", "zones_internal.cuh"]
+HEADERS = ["hg_internal.cuh", "fp64_tools.cuh", "mpm_basis.cuh",
+           "mpm_axis.cuh", "scan_block.cuh", "zones_internal.cuh"]
 
 
 def _nvcc():

@@ -782,7 +782,9 @@ __global__ void __launch_bounds__(CONTACT_THREADS) kd_contacts(const __grid_cons
       n = d;
       if (d2 > 0.0) {
         const Divisor len = divisor(dist);
-        n = D2{quot(d.x, len), quot(d.y, len)};
+        bool ok = len.ok;
+        n = D2{quot(d.x, len, ok), quot(d.y, len, ok)};
+        if (!ok) n = D2{divide(d.x, dist), divide(d.y, dist)};
       }
       depth = min_zero(dist - ra - rb);
       const D2 vb{C.v[3 * b], C.v[3 * b + 1]};
@@ -927,6 +929,7 @@ struct IntegrateArgs {
   int64_t n, ccap;
   double dt;
   double *q, *v;
+  double *q_before; // receives the positions before the step, or nullptr
   const double4 *terms;
   const uint8_t *fixed;
   const int4 *desc;
@@ -972,8 +975,13 @@ __global__ void kd_integrate(const __grid_constant__ IntegrateArgs A,
   A.v[3 * j] = v0;
   A.v[3 * j + 1] = v1;
   A.v[3 * j + 2] = v2;
-  const double q0 = A.q[3 * j] + A.dt * v0, q1 = A.q[3 * j + 1] + A.dt * v1,
-               q2 = A.q[3 * j + 2] + A.dt * v2;
+  const double p0 = A.q[3 * j], p1 = A.q[3 * j + 1], p2 = A.q[3 * j + 2];
+  if (A.q_before) {
+    A.q_before[3 * j] = p0;
+    A.q_before[3 * j + 1] = p1;
+    A.q_before[3 * j + 2] = p2;
+  }
+  const double q0 = p0 + A.dt * v0, q1 = p1 + A.dt * v1, q2 = p2 + A.dt * v2;
   A.q[3 * j] = q0;
   A.q[3 * j + 1] = q1;
   A.q[3 * j + 2] = q2;
@@ -1148,8 +1156,13 @@ __global__ void kdx_integrate(const __grid_constant__ IntegrateArgs A,
   A.v[3 * j] = w0;
   A.v[3 * j + 1] = w1;
   A.v[3 * j + 2] = w2;
-  const double q0 = A.q[3 * j] + A.dt * w0, q1 = A.q[3 * j + 1] + A.dt * w1,
-               q2 = A.q[3 * j + 2] + A.dt * w2;
+  const double p0 = A.q[3 * j], p1 = A.q[3 * j + 1], p2 = A.q[3 * j + 2];
+  if (A.q_before) {
+    A.q_before[3 * j] = p0;
+    A.q_before[3 * j + 1] = p1;
+    A.q_before[3 * j + 2] = p2;
+  }
+  const double q0 = p0 + A.dt * w0, q1 = p1 + A.dt * w1, q2 = p2 + A.dt * w2;
   A.q[3 * j] = q0;
   A.q[3 * j + 1] = q1;
   A.q[3 * j + 2] = q2;
@@ -1309,7 +1322,7 @@ void dem_set_launch_shapes(hg_dem *d) {
   d->contact_grid = d->ctx->num_sms * per_sm;
 }
 
-hg_status dem_step(hg_dem *d, double dt, int weighted, bool bin_next) {
+hg_status dem_step(hg_dem *d, double dt, int weighted, bool bin_next, double *q_before) {
   cudaStream_t s = dem_stream(d);
   const int64_t n = d->n;
   if (n == 0) return HG_OK;
@@ -1456,6 +1469,7 @@ hg_status dem_step(hg_dem *d, double dt, int weighted, bool bin_next) {
   I.dt = dt;
   I.q = d->q.p;
   I.v = d->v.p;
+  I.q_before = q_before;
   I.terms = reinterpret_cast<const double4 *>(d->minv.p);
   I.fixed = d->fixed.p;
   I.desc = d->desc[nb].p;

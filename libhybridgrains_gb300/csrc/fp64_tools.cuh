@@ -1,10 +1,12 @@
 // FP64 values through the integer pipe, and cheaper exact quotients.
 //
-// FP64 instructions, conversions to and from FP64 included, issue at about
-// two lanes per cycle and SM on this part (17-21 cycles per warp instruction
-// measured, 65 cycles of latency; a division costs 145 cycles, a square root
-// 156), a 32-bit integer instruction 0.3 cycles. Conversions, comparisons and
-// decisions that integer or FP32 arithmetic can make exactly are made there.
+// An FP64 instruction, conversions to and from FP64 included, takes a warp 64
+// cycles of its SM sub-partition on this part, whatever the number of active
+// lanes and independent or not (measured: 1.8 thread instructions per cycle and
+// SM; a division 8 of them, a reciprocal 5, a square root 9), a 32-bit integer
+// instruction about 1. So the count of FP64 instructions is the time of these
+// kernels, and conversions, comparisons, powers of two and decisions that
+// integer or FP32 arithmetic can make exactly are made there.
 #pragma once
 
 #include <stdint.h>
@@ -21,6 +23,18 @@ __device__ __forceinline__ bool f64_less(double a, double b) {
 }
 // isfinite
 __device__ __forceinline__ bool finite_bits(double x) { return (f64_hi(x) & 0x7FF00000u) != 0x7FF00000u; }
+// 2 x and x / 2
+static __device__ __noinline__ double scale_slow(double x, double by) { return x * by; }
+__device__ __forceinline__ double twice(double x) {
+  const uint32_t hi = f64_hi(x), e = (hi >> 20) & 0x7FFu;
+  if (e - 1u < 2045u) return __hiloint2double((int)(hi + 0x100000u), (int)f64_lo(x));
+  return f64_zero(x) ? x : scale_slow(x, 2.0);
+}
+__device__ __forceinline__ double halved(double x) {
+  const uint32_t hi = f64_hi(x), e = (hi >> 20) & 0x7FFu;
+  if (e - 2u < 2045u) return __hiloint2double((int)(hi - 0x100000u), (int)f64_lo(x));
+  return f64_zero(x) ? x : scale_slow(x, 0.5);
+}
 // min(0, x); 0 for a NaN
 __device__ __forceinline__ double min_zero(double x) {
   const uint32_t hi = f64_hi(x), lo = f64_lo(x);
@@ -99,7 +113,8 @@ __device__ __forceinline__ int ceil_int(double x) {
 // gives a / b rounded to nearest (P. Markstein, "Computation of elementary
 // functions on the IBM RISC System/6000 processor", 1990), three FP64
 // instructions in place of a division's eight. Operands near the ends of the
-// exponent range are divided.
+// exponent range clear ok; the caller then takes true divisions, one branch for
+// a group of quotients.
 struct Divisor {
   double b, y;
   bool ok;
@@ -110,14 +125,46 @@ __device__ __forceinline__ Divisor divisor(double b, double y) {
   return {b, y, e - 823u <= 400u};
 }
 __device__ __forceinline__ Divisor divisor(double b) { return divisor(b, 1.0 / b); }
-static __device__ __noinline__ double divide(double a, double b) { return a / b; }
-__device__ __forceinline__ double quot(double a, const Divisor &d) {
-  const uint32_t hi = f64_hi(a);
+__device__ __forceinline__ double quot(double a, const Divisor &d, bool &ok) {
+  const uint32_t e = (f64_hi(a) >> 20) & 0x7FFu;
+  ok = ok && (e - 300u <= 1400u || f64_zero(a));
   const double q = a * d.y;
-  const double z = fma(fma(-q, d.b, a), d.y, q);
-  if (d.ok && ((hi >> 20) & 0x7FFu) - 300u <= 1400u) return z;
-  if (d.ok && ((hi << 1) | f64_lo(a)) == 0u) return q; // a zero's sign
-  return divide(a, d.b);
+  return fma(fma(-q, d.b, a), d.y, q); // (a zero comes out as +0)
+}
+static __device__ __noinline__ double divide(double a, double b) { return a / b; }
+// a single quotient
+__device__ __forceinline__ double quot(double a, const Divisor &d) {
+  bool ok = d.ok;
+  const double z = quot(a, d, ok);
+  return ok ? z : divide(a, d.b);
+}
+// SAFE: by division
+template <bool SAFE>
+__device__ __forceinline__ double quot_or(double a, const Divisor &d, bool &ok) {
+  return SAFE ? a / d.b : quot(a, d, ok);
+}
+
+// sqrt(a) and its reciprocal by Goldschmidt's iteration (R. Goldschmidt, 1964;
+// P. Markstein, "Software division and square root using Goldschmidt's
+// algorithms", 2004) from an FP32 estimate: one iteration to about 2^-43 and a
+// residual correction of each, which leaves both rounded to nearest but for
+// one argument in 2^32 or so (then within one unit). 8 FP64 instructions (6
+// where the reciprocal is not used) in place of 14 (9).
+static __device__ __noinline__ double2 root_slow(double a) {
+  const double g = sqrt(a);
+  return make_double2(g, 1.0 / g);
+}
+__device__ __forceinline__ double2 root(double a) {
+  const uint32_t e = (f64_hi(a) >> 20) - 898u; // a sign bit makes it large
+  if (e > 250u) return root_slow(a);
+  const double y0 = widen_f32(rsqrtf(narrow_trunc(a)));
+  double g = a * y0, h = halved(y0);
+  const double r = fma(-g, h, 0.5);
+  g = fma(g, r, g);
+  h = fma(h, r, h);
+  g = fma(fma(-g, g, a), h, g);
+  const double y = twice(h);
+  return make_double2(g, fma(y, fma(-g, y, 1.0), y));
 }
 
 } // namespace hg

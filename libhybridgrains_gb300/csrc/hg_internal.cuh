@@ -295,6 +295,7 @@ struct hg_mpm {
   hg::DevBuf<double> g_mass, g_mom, g_mom_new, g_force, g_vel, g_acc, g_cforce,
       g_homog;
   hg::DevBuf<int32_t> g_hyb;
+  bool hyb_loaded = false; // g_hyb came with a loaded state (else it is zero)
   // the other set of accumulators; next_clear: cleared by the last G2P
   hg::DevBuf<double> g_mass_next, g_mom_next, g_force_next;
   bool next_clear = false;
@@ -566,7 +567,8 @@ hg_status dem_edit(hg_dem *d, int64_t n_old, const int32_t *old_to_new, int64_t 
                    const double *m, const double *I, const uint8_t *fixed);
 // bin_next: bin the bodies for the next step (wasted when they are moved in
 // between, as the hybrid step does)
-hg_status dem_step(hg_dem *d, double dt, int weighted, bool bin_next);
+// q_before: receives the positions before the step (3 per body), or nullptr
+hg_status dem_step(hg_dem *d, double dt, int weighted, bool bin_next, double *q_before = nullptr);
 void dem_bodies_changed(hg_dem *d);
 void dem_set_launch_shapes(hg_dem *d);
 // per-body terms that dem_step needs and that only change with the bodies
@@ -598,8 +600,10 @@ struct hg_hybrid {
   hg_context *ctx = nullptr;
   hg_mpm *m = nullptr;
   hg_dem *d = nullptr;
-  hg::DevBuf<double> dem_mass, dem_mom, v_after, a_after, pos_before,
-      hstress, hvel, hmom, hmass;
+  // dem_mass and dem_mom of the last step; the other set is that of the step
+  // before, or clear
+  hg::DevBuf<double> dem_mass, dem_mom, old_mass, old_mom;
+  hg::DevBuf<double> v_after, a_after, pos_before, hstress, hvel, hmom, hmass;
   hg::DevBuf<int32_t> coupled, packed_dem, packed_mpm, flag_tmp, scan_tmp,
       node_flag, node_pos, counts; // counts[2]: packed sizes
   int64_t n_packed_dem = 0, n_packed_mpm = 0;

@@ -1,23 +1,24 @@
 // Plain FP64 MPM step: the drop-in for ExplicitIntegrator::flow in double
 // precision.
 //
-// Bound by the FP64 pipe (about two lanes per cycle and SM: fp64_tools.cuh), so
-// each kernel evaluates what the reference evaluates in as few FP64
-// instructions as keep its accuracy. Positions, cells, stencil offsets, strains
-// and plane tests, where a last bit decides or survives a cancellation, keep
-// the reference's operations one by one (this translation unit is compiled
-// with --fmad=false);
-// sums and products elsewhere use fma() explicitly, quotients by a common
-// divisor share its reciprocal (fp64_tools.cuh), 1-D factors are divided once
-// per axis, and sign, range and yield decisions are made on the integer and
-// FP32 pipes with an FP64 test for the close calls. Grid accumulation uses
-// FP64 atomics, so node sums differ from the serial reference in order too;
-// both stay within a few units in the last place (tests: 1e-12).
+// Bound by the FP64 pipe: an FP64 instruction takes a warp 64 cycles whatever
+// it does (fp64_tools.cuh), so each kernel evaluates what the reference
+// evaluates in as few FP64 instructions as keep its accuracy. Positions, cells,
+// stencil offsets, strains and plane tests, where a last bit decides or
+// survives a cancellation, keep the reference's operations one by one (this
+// translation unit is compiled with --fmad=false); sums and products elsewhere
+// use fma() explicitly, quotients by a common divisor share its reciprocal,
+// roots come with theirs, 1-D factors are divided once per axis, and sign,
+// range and yield decisions are made on the integer and FP32 pipes with an FP64
+// test for the close calls. Grid accumulation uses FP64 atomics, so node sums
+// differ from the serial reference in order too; both stay within a few units
+// in the last place (tests: 1e-12).
 // Measured per step against the reference's expressions instruction for
 // instruction (six memsets and four launches a step, now three launches):
-// 12,800 points, linear, one call per step 84.5 -> 30.6 us; 100,000 points,
-// uGIMP, 439 -> 180 us (425 FP64 instructions per warp of points in k64_g2p,
-// 85% of the FP64 pipe; it was about 1,100).
+// 12,800 points, linear, one call per step 84.5 -> 22.4 us; 100,000 points,
+// uGIMP, 439 -> 118 us (k64_g2p 214 -> 65 us: 286 FP64 instructions per warp
+// of points where there were about 1,100, 81% of the FP64 pipe; k64_p2g 170 ->
+// 50 us).
 //
 // Kernels:
 //   k64_p2g         rasterizePointMasses + rasterizePointMomentum
@@ -33,8 +34,8 @@
 //                   (MaterialPoints.cpp:204-423), fused per material point;
 //                   clears the accumulators of the next step.
 #include "hg_internal.cuh"
-#include "fp64_tools.cuh"
 #include "mpm_basis.cuh"
+#include "mpm_axis.cuh"
 
 #include <utility>
 
@@ -94,89 +95,19 @@ __device__ M2d plastic_correction(M2d b, double kappa, double mu, double alpha,
   return b;
 }
 
-// x with its sign flipped where neg is the sign bit (0 or 0x80000000)
-__device__ __forceinline__ double flip(double x, uint32_t neg) {
-  return __hiloint2double((int)(f64_hi(x) ^ neg), (int)f64_lo(x));
-}
-
-// The 2-D weights and gradients of a point's stencil as products of 1-D
-// factors: node (kx, ky) has weight wx[kx] wy[ky] and gradient (dx[kx] vy[ky],
-// vx[kx] dy[ky]), where v is the factor across a gradient's axis (over h for
-// the linear basis, whose own derivative factor is a sign).
-constexpr uint32_t NO_SLOPE = 1u; // linear: derivative 0 (else the sign bit of it)
-template <int BASIS> struct Axis;
-
-// LinearBasisFunctions.cpp:6-22, 53-59, 81-136: nodes i, i + 1 at offsets
-// d = ((x - h i) - g) / h; w = 1 - |d|, dw/dx = -sign(d) / h.
-template <> struct Axis<HG_BASIS_LINEAR> {
-  int i0, n;
-  double w[2], v[2]; // weight, weight / h
-  uint32_t sg[2];
-  __device__ __forceinline__ void set(double x, double, double g, const Divisor &H) {
-    i0 = floor_int(quot(x - g, H));
-    n = 2;
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int i = i0 + k;
-      const double hi = i >= 0 ? H.b * index_f64(i) : H.b * (double)i;
-      const double d = quot((x - hi) - g, H);
-      const double a = flip(d, f64_hi(d) & 0x80000000u);
-      const bool in = f64_less(a, 1.0);
-      w[k] = in ? 1.0 - a : 0.0;
-      v[k] = in ? quot(w[k], H) : 0.0;
-      // -1 for d >= 0 (a zero's sign apart), 1 for d < 0, 0 beyond 1
-      sg[k] = f64_less(1.0, a) ? NO_SLOPE
-                               : (f64_hi(d) >> 31 && !f64_zero(d) ? 0u : 0x80000000u);
-    }
-  }
-};
-
-// uGIMPLinearBasisFunctions.cpp:6-42, 71-94, 110-156. With a = |x - x_i|,
-// L = half-width and q one quotient by h:
-//   a >= h + L      0
-//   a >= h - L      q = (h + L - a)^2 / h: q / 2,       slope (h + L - a) / h
-//   a >= L          q = a / h: 2 L (1 - q),             slope 2 L / h
-//   else            q = (L^2 + a^2) / h: 2 L - q,       slope 2 a / h
-// The cases are selected, not branched on: FP64 instructions issue once per
-// warp and case taken.
-template <> struct Axis<HG_BASIS_UGIMP> {
-  int i0, n;
-  double w[STENCIL_AXIS], d[STENCIL_AXIS];
-  __device__ __forceinline__ void set(double x, double L, double g, const Divisor &H) {
-    i0 = floor_int(quot((x - L) - g, H));
-    n = ceil_int(quot((x + L) - g, H)) - i0 + 1;
-    const double wide = H.b + L, narrow_ = H.b - L, two = 2.0 * L, sq = L * L;
-#pragma unroll
-    for (int k = 0; k < STENCIL_AXIS; ++k) {
-      w[k] = 0.0;
-      d[k] = 0.0;
-      if (k >= n) continue;
-      const int i = i0 + k;
-      const double xi = (i >= 0 ? H.b * index_f64(i) : H.b * (double)i) + g;
-      const double s = x - xi;
-      const uint32_t neg = f64_hi(s) & 0x80000000u;
-      const double a = flip(s, neg);
-      if (!f64_less(a, wide)) continue;
-      const bool edge = !f64_less(a, narrow_), mid = !f64_less(a, L);
-      const double t = wide - a;
-      const double m = edge ? t : a;
-      const double m2 = m * m;
-      const double q = quot(edge ? m2 : (mid ? a : sq + m2), H);
-      const double z = (mid ? 1.0 : two) - q;
-      w[k] = edge ? 0.5 * q : (mid ? two * z : z);
-      const double slope = quot(edge ? t : (mid ? two : a + a), H);
-      d[k] = flip(slope, neg ^ 0x80000000u); // (a zero offset: slope 0 either way)
-    }
-  }
-};
-
+// A point's stencil: the 2-D weight of node (kx, ky) is wx[kx] wy[ky] and its
+// gradient (dx[kx] wy[ky], wx[kx] dy[ky]).
 template <int BASIS> struct Stencil;
 template <> struct Stencil<HG_BASIS_LINEAR> {
-  Axis<HG_BASIS_LINEAR> X, Y;
+  using Ax = Axis<HG_BASIS_LINEAR>;
+  Ax X, Y;
+  template <bool SAFE>
   __device__ __forceinline__ void set(const MpmParams &P, double x, double y, double hl,
-                                      const Divisor &H) {
-    X.set(x, hl, P.gmin[0], H);
-    Y.set(y, hl, P.gmin[1], H);
+                                      const Divisor &H, bool &ok) {
+    X.template range<SAFE>(x, hl, P.gmin[0], H, ok);
+    Y.template range<SAFE>(y, hl, P.gmin[1], H, ok);
+    X.template factors<true, SAFE>(x, P.gmin[0], H, ok);
+    Y.template factors<true, SAFE>(y, P.gmin[1], H, ok);
   }
   template <class F> __device__ __forceinline__ void each(int row, F &&f) const {
 #pragma unroll
@@ -184,41 +115,50 @@ template <> struct Stencil<HG_BASIS_LINEAR> {
 #pragma unroll
       for (int kx = 0; kx < 2; ++kx)
         f((Y.i0 + ky) * (int64_t)row + X.i0 + kx, X.w[kx] * Y.w[ky],
-          X.sg[kx] == NO_SLOPE ? 0.0 : flip(Y.v[ky], X.sg[kx]),
-          Y.sg[ky] == NO_SLOPE ? 0.0 : flip(X.v[kx], Y.sg[ky]));
+          X.sg[kx] == Ax::NO_SLOPE ? 0.0 : flip(Y.v[ky], X.sg[kx]),
+          Y.sg[ky] == Ax::NO_SLOPE ? 0.0 : flip(X.v[kx], Y.sg[ky]));
   }
 };
 template <> struct Stencil<HG_BASIS_UGIMP> {
   Axis<HG_BASIS_UGIMP> X, Y;
+  template <bool SAFE>
   __device__ __forceinline__ void set(const MpmParams &P, double x, double y, double hl,
-                                      const Divisor &H) {
-    X.set(x, hl, P.gmin[0], H);
-    Y.set(y, hl, P.gmin[1], H);
+                                      const Divisor &H, bool &ok) {
+    Extent E;
+    E.set(hl, H);
+    X.template range<SAFE>(x, hl, P.gmin[0], H, ok);
+    Y.template range<SAFE>(y, hl, P.gmin[1], H, ok);
+    X.factors<true>(x, E, P.gmin[0], H);
+    Y.factors<true>(y, E, P.gmin[1], H);
     // over the point's volume 4 hl^2, once per node of one axis
-    const Divisor V = divisor(4.0 * hl * hl);
+    const double inv = 1.0 / (4.0 * hl * hl);
 #pragma unroll
     for (int k = 0; k < STENCIL_AXIS; ++k)
       if (k < Y.n) {
-        Y.w[k] = quot(Y.w[k], V);
-        Y.d[k] = quot(Y.d[k], V);
+        Y.w[k] *= inv;
+        Y.d[k] *= inv;
       }
-  }
-  template <class F> __device__ __forceinline__ void each(int row, F &&f) const {
-#pragma unroll
-    for (int ky = 0; ky < STENCIL_AXIS; ++ky) {
-      if (ky >= Y.n) break;
-#pragma unroll
-      for (int kx = 0; kx < STENCIL_AXIS; ++kx) {
-        if (kx >= X.n) break;
-        f((Y.i0 + ky) * (int64_t)row + X.i0 + kx, X.w[kx] * Y.w[ky], X.d[kx] * Y.w[ky],
-          X.w[kx] * Y.d[ky]);
-      }
-    }
   }
 };
 
-// The stencil's inclusive node range (stencil64) leaves the grid, or is wider
-// than the kernels' stencils hold.
+template <int BASIS>
+__device__ __noinline__ Stencil<BASIS> stencil_safe(const MpmParams &P, double x, double y,
+                                                    double hl) {
+  Stencil<BASIS> S;
+  bool ok = true;
+  S.template set<true>(P, x, y, hl, divisor(P.h, P.inv_h), ok);
+  return S;
+}
+template <int BASIS>
+__device__ __forceinline__ void stencil(Stencil<BASIS> &S, const MpmParams &P, double x, double y,
+                                        double hl) {
+  const Divisor H = divisor(P.h, P.inv_h);
+  bool ok = H.ok;
+  S.template set<false>(P, x, y, hl, H, ok);
+  if (!ok) S = stencil_safe<BASIS>(P, x, y, hl);
+}
+
+// The node range leaves the grid, or is wider than the kernels' stencils hold.
 template <int BASIS>
 __device__ __forceinline__ bool off_grid(const MpmParams &P, const Stencil<BASIS> &S) {
   return S.X.i0 < 0 || S.Y.i0 < 0 || S.X.i0 + S.X.n - 1 > P.nx || S.Y.i0 + S.Y.n - 1 > P.ny;
@@ -251,11 +191,20 @@ __device__ __forceinline__ M2d node_stress(const MpmParams &P, const P2gArgs &A,
   const double2 c0 = reinterpret_cast<const double2 *>(A.be)[2 * p];
   const double2 c1 = reinterpret_cast<const double2 *>(A.be)[2 * p + 1];
   const M2d be = m_scl(Jp, M2d{c0.x, c0.y, c1.x, c1.y});
-  const double J = sqrt(m_det(be));
-  const Divisor D = divisor(J);
-  const double a00 = quot(be.a00, D), a10 = quot(be.a10, D), a11 = quot(be.a11, D);
-  const double a01 = __double_as_longlong(c0.y) == __double_as_longlong(c1.x) ? a10 : quot(be.a01, D);
-  const double half_tr = (a00 + a11) * 0.5;
+  const double2 r = root(m_det(be));
+  const double J = r.x;
+  const Divisor D = divisor(J, r.y);
+  bool ok = D.ok;
+  double a00 = quot(be.a00, D, ok), a10 = quot(be.a10, D, ok), a11 = quot(be.a11, D, ok);
+  double a01 = a10;
+  if (__double_as_longlong(c0.y) != __double_as_longlong(c1.x)) a01 = quot(be.a01, D, ok);
+  if (!ok) {
+    a00 = divide(be.a00, J);
+    a10 = divide(be.a10, J);
+    a01 = divide(be.a01, J);
+    a11 = divide(be.a11, J);
+  }
+  const double half_tr = halved(a00 + a11);
   const double s = A.half_kappa * (J + 1.0) * (J - 1.0);
   const double c = -A.vol[p], cm = c * P.mu;
   return {c * fma(P.mu, a00 - half_tr, s), cm * a10, cm * a01, c * fma(P.mu, a11 - half_tr, s)};
@@ -289,9 +238,8 @@ __global__ void k64_p2g(const __grid_constant__ MpmParams P, const __grid_consta
   const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (p >= A.n) return;
   const double2 x = reinterpret_cast<const double2 *>(A.q)[p];
-  const Divisor H = divisor(P.h, P.inv_h);
   Stencil<BASIS> St;
-  St.set(P, x.x, x.y, BASIS == HG_BASIS_UGIMP ? A.hl[p] : 0.0, H);
+  stencil(St, P, x.x, x.y, BASIS == HG_BASIS_UGIMP ? A.hl[p] : 0.0);
   if (off_grid<BASIS>(P, St)) {
     atomicOr(A.status, (uint32_t)HG_STATUS_OUT_OF_GRID);
     return;
@@ -304,20 +252,46 @@ __global__ void k64_p2g(const __grid_constant__ MpmParams P, const __grid_consta
   const double mp = A.m[p];
   const double2 v = reinterpret_cast<const double2 *>(A.v)[p];
   const double pmx = mp * v.x, pmy = mp * v.y;
-  St.each(P.nx + 1, [&](int64_t i, double w, double gx, double gy) {
-    // nodes of zero weight get nothing (PhysicsGrid.cpp:439-441)
-    if (f64_zero(w)) return;
-    atomicAdd(&A.g_mass[i], w * mp);
-    atomicAdd(&A.g_mom[2 * i], w * pmx);
-    atomicAdd(&A.g_mom[2 * i + 1], w * pmy);
-    atomicAdd(&A.g_force[2 * i], fma(S.a00, gx, S.a01 * gy));
-    atomicAdd(&A.g_force[2 * i + 1], fma(S.a10, gx, S.a11 * gy));
-  });
+  const int row = P.nx + 1;
+  // (nodes of zero weight get nothing, PhysicsGrid.cpp:439-441)
+  if constexpr (BASIS == HG_BASIS_LINEAR) {
+    St.each(row, [&](int64_t i, double w, double gx, double gy) {
+      if (f64_zero(w)) return;
+      atomicAdd(&A.g_mass[i], w * mp);
+      atomicAdd(&A.g_mom[2 * i], w * pmx);
+      atomicAdd(&A.g_mom[2 * i + 1], w * pmy);
+      atomicAdd(&A.g_force[2 * i], fma(S.a00, gx, S.a01 * gy));
+      atomicAdd(&A.g_force[2 * i + 1], fma(S.a10, gx, S.a11 * gy));
+    });
+  } else {
+    // the factors of a row of nodes once per row
+#pragma unroll
+    for (int ky = 0; ky < STENCIL_AXIS; ++ky) {
+      if (ky >= St.Y.n) break;
+      const double wy = St.Y.w[ky], dy = St.Y.d[ky];
+      if (f64_zero(wy)) continue;
+      const double rm = wy * mp, rx = wy * pmx, ry = wy * pmy;
+      const double f00 = S.a00 * wy, f10 = S.a10 * wy, f01 = S.a01 * dy, f11 = S.a11 * dy;
+      const int64_t base = (St.Y.i0 + ky) * (int64_t)row + St.X.i0;
+#pragma unroll
+      for (int kx = 0; kx < STENCIL_AXIS; ++kx) {
+        if (kx >= St.X.n) break;
+        const double wx = St.X.w[kx], dx = St.X.d[kx];
+        if (f64_zero(wx)) continue;
+        const int64_t i = base + kx;
+        atomicAdd(&A.g_mass[i], wx * rm);
+        atomicAdd(&A.g_mom[2 * i], wx * rx);
+        atomicAdd(&A.g_mom[2 * i + 1], wx * ry);
+        atomicAdd(&A.g_force[2 * i], fma(dx, f00, wx * f01));
+        atomicAdd(&A.g_force[2 * i + 1], fma(dx, f10, wx * f11));
+      }
+    }
+  }
 }
 
 struct GridArgs {
   int64_t nn;
-  double dt;
+  double dt, inv_dt;
   const double *mass, *mom;
   double *mom_new, *force;
   const double *cforce;
@@ -360,8 +334,10 @@ __global__ void __launch_bounds__(128) k64_grid(const __grid_constant__ MpmParam
     if (has) {
       double2 f = force[i];
       const double half = A.hyb[i] > 0 ? 0.5 * mi : mi;
-      f.x = fma(half, P.g[0], f.x) + cf.x;
-      f.y = fma(half, P.g[1], f.y) + cf.y;
+      f.x = fma(half, P.g[0], f.x);
+      f.y = fma(half, P.g[1], f.y);
+      if (!f64_zero(cf.x)) f.x += cf.x;
+      if (!f64_zero(cf.y)) f.y += cf.y;
       force[i] = f;
       pn = make_double2(fma(A.dt, f.x, pm.x), fma(A.dt, f.y, pm.y));
       const int ix = (int)(i % (P.nx + 1)), iy = (int)(i / (P.nx + 1));
@@ -391,9 +367,10 @@ __global__ void __launch_bounds__(128) k64_grid(const __grid_constant__ MpmParam
   if (UPDATE) {
     double2 v = zero, a = zero;
     if (has) {
-      const Divisor M = divisor(mi), D = divisor(A.dt * mi);
+      const Divisor M = divisor(mi);
+      const double per = M.y * A.inv_dt;
       v = make_double2(quot(pn.x, M), quot(pn.y, M));
-      a = make_double2(quot(pn.x - pm.x, D), quot(pn.y - pm.y, D));
+      a = make_double2((pn.x - pm.x) * per, (pn.y - pm.y) * per);
     }
     reinterpret_cast<double2 *>(A.vel)[i] = v;
     reinterpret_cast<double2 *>(A.acc)[i] = a;
@@ -412,7 +389,7 @@ struct G2pArgs {
   double *next_mass, *next_mom, *next_force; // the next step's accumulators, cleared
   uint32_t *status;
   // constants of every point
-  double yield; // alpha kappa / 2
+  double yield_mu; // alpha kappa / (2 mu)
   double pic;   // 1 - flip_alpha
   float mu32, yield32;
   float px[HG_MAX_PLANES][2];
@@ -470,63 +447,66 @@ __device__ __noinline__ PointStrain strain_general(const MpmParams &P, double dt
 // The same for a symmetric be_bar, which stays symmetric to the bit. The
 // yield test is decided in FP32 except within 1e-5 of the yield surface, so
 // that elastic points need neither |dev be| nor the yield stress in FP64.
-__device__ __forceinline__ void strain_symmetric(const MpmParams &P, const G2pArgs &A,
-                                                 const PointGrid &g, double &b00, double &b01,
-                                                 double &b11, double &Jp, int &jh) {
-  b00 *= Jp;
-  b01 *= Jp;
-  b11 *= Jp;
+// False when a quotient did not pass its check.
+__device__ __forceinline__ bool strain_symmetric(const MpmParams &P, const G2pArgs &A,
+                                                 const PointGrid &g, PointStrain &s) {
+  bool ok = true;
+  double b00 = s.J * s.b.a00, b01 = s.J * s.b.a01, b11 = s.J * s.b.a11;
   const double l00 = fma(g.L00, b00, g.L01 * b01), l01 = fma(g.L00, b01, g.L01 * b11);
   const double l10 = fma(g.L10, b00, g.L11 * b01), l11 = fma(g.L10, b01, g.L11 * b11);
-  b00 = fma(A.dt, l00 + l00, b00);
+  b00 = fma(A.dt, twice(l00), b00);
   b01 = fma(A.dt, l01 + l10, b01);
-  b11 = fma(A.dt, l11 + l11, b11);
-  Jp = sqrt(det_sym(b00, b01, b11));
+  b11 = fma(A.dt, twice(l11), b11);
   {
-    const Divisor D = divisor(Jp);
-    b00 = Jp * quot(b00, D);
-    b01 = Jp * quot(b01, D);
-    b11 = Jp * quot(b11, D);
+    const double2 r = root(det_sym(b00, b01, b11));
+    const Divisor D = divisor(r.x, r.y);
+    ok = D.ok;
+    b00 = r.x * quot(b00, D, ok);
+    b01 = r.x * quot(b01, D, ok);
+    b11 = r.x * quot(b11, D, ok);
   }
-  double det = det_sym(b00, b01, b11);
-  Jp = sqrt(det);
-  bool grown = false;
-  if (jh != 0) {
-    grown = Jp > 1.0;
-    if (!grown) jh = 0;
-  }
+  const double det = det_sym(b00, b01, b11);
+  double2 r = root(det); // J and 1 / J
+  double J = r.x;
+  int jh = s.jh;
+  const bool grown = jh != 0 && J > 1.0;
+  if (!grown) jh = 0;
   if (grown) { // be = J I (ConstitutiveModel.cpp:28-35)
-    b00 = b11 = Jp;
+    b00 = b11 = J;
     b01 = 0.0;
-    Jp = sqrt(Jp * Jp);
+    r = root(J * J);
   } else {
-    const double half_tr = 0.5 * (b00 + b11);
+    const double half_tr = halved(b00 + b11);
     const double d0 = b00 - half_tr, d1 = b11 - half_tr;
-    const double up = 1.0 + Jp, down = 1.0 - Jp;
+    const double up = 1.0 + J, down = 1.0 - J;
     const float d32 = narrow_trunc(d0), o32 = narrow_trunc(b01);
     const float n2 = 2.0f * (d32 * d32 + o32 * o32);
     const float limit =
-        fmaxf(0.0f, A.yield32 * narrow_trunc(up) * narrow_trunc(down)) * narrow_trunc(Jp) / A.mu32;
+        fmaxf(0.0f, A.yield32 * narrow_trunc(up) * narrow_trunc(down)) * narrow_trunc(J) / A.mu32;
     // elastic for sure, where the estimate of |dev be| is well above the
     // rounding of d0 and FP32's smallest squares
     const bool elastic = n2 > 1.0e-18f && sqrtf(n2) < limit * 0.99999f;
     if (!elastic) {
-      const double ys = fmax(0.0, A.yield * up * down);
-      const double t = P.mu * (sqrt(fma(d0, d0, fma(d1, d1, 2.0 * (b01 * b01)))) / Jp);
-      if (t > ys) {
-        const double l2 = ys / t;
-        const double l1 = sqrt(fma(-(l2 * l2), d0 * d1 - b01 * b01, det));
+      // l2 = ys / (mu |dev be| / J), below 1 beyond the yield surface; no
+      // deviator gives infinity or NaN
+      const double o2 = b01 * b01;
+      double l2 = A.yield_mu * up * down * J * rsqrt(fma(d0, d0, fma(d1, d1, twice(o2))));
+      if (f64_hi(l2) >> 31) l2 = 0.0; // J > 1: no yield stress
+      if (l2 < 1.0) {
+        const double l1 = root(fma(-(l2 * l2), fma(d0, d1, -o2), det)).x;
         b00 = fma(l2, d0, l1);
         b11 = fma(l2, d1, l1);
         b01 = l2 * b01;
-        Jp = sqrt(det_sym(b00, b01, b11));
+        r = root(det_sym(b00, b01, b11));
       }
     }
   }
-  const Divisor D = divisor(Jp);
-  b00 = quot(b00, D);
-  b01 = quot(b01, D);
-  b11 = quot(b11, D);
+  J = r.x;
+  const Divisor D = divisor(J, r.y);
+  ok = ok && D.ok;
+  const double a00 = quot(b00, D, ok), a01 = quot(b01, D, ok), a11 = quot(b11, D, ok);
+  if (ok) s = {{a00, a01, a01, a11}, J, jh};
+  return ok;
 }
 
 template <int BASIS>
@@ -545,9 +525,8 @@ __global__ void k64_g2p(const __grid_constant__ MpmParams P, const __grid_consta
   const double hl = BASIS == HG_BASIS_UGIMP ? A.hl[p] : 0.0;
   PointGrid g{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   {
-    const Divisor H = divisor(P.h, P.inv_h);
     Stencil<BASIS> St;
-    St.set(P, x.x, x.y, hl, H);
+    stencil(St, P, x.x, x.y, hl);
     if (off_grid<BASIS>(P, St)) {
       atomicOr(A.status, (uint32_t)HG_STATUS_OUT_OF_GRID);
       return;
@@ -557,34 +536,62 @@ __global__ void k64_g2p(const __grid_constant__ MpmParams P, const __grid_consta
     } else {
       // computeVelGrad (MaterialPoints.cpp:296-322), and the interpolations of
       // updateVelocities (204-245) and updatePositions (247-288)
-      St.each(P.nx + 1, [&](int64_t i, double w, double gx, double gy) {
-        const double2 v = reinterpret_cast<const double2 *>(A.g_vel)[i];
-        const double2 a = reinterpret_cast<const double2 *>(A.g_acc)[i];
-        g.L00 = fma(v.x, gx, g.L00);
-        g.L10 = fma(v.y, gx, g.L10);
-        g.L01 = fma(v.x, gy, g.L01);
-        g.L11 = fma(v.y, gy, g.L11);
-        g.vx = fma(w, v.x, g.vx);
-        g.vy = fma(w, v.y, g.vy);
-        g.ax = fma(w, a.x, g.ax);
-        g.ay = fma(w, a.y, g.ay);
-      });
+      const double2 *gv = reinterpret_cast<const double2 *>(A.g_vel);
+      const double2 *ga = reinterpret_cast<const double2 *>(A.g_acc);
+      const int row = P.nx + 1;
+      if constexpr (BASIS == HG_BASIS_LINEAR) {
+        St.each(row, [&](int64_t i, double w, double gx, double gy) {
+          const double2 v = gv[i], a = ga[i];
+          g.L00 = fma(v.x, gx, g.L00);
+          g.L10 = fma(v.y, gx, g.L10);
+          g.L01 = fma(v.x, gy, g.L01);
+          g.L11 = fma(v.y, gy, g.L11);
+          g.vx = fma(w, v.x, g.vx);
+          g.vy = fma(w, v.y, g.vy);
+          g.ax = fma(w, a.x, g.ax);
+          g.ay = fma(w, a.y, g.ay);
+        });
+      } else {
+        // row by row: the sums over x, then their factors along y
+#pragma unroll
+        for (int ky = 0; ky < STENCIL_AXIS; ++ky) {
+          if (ky >= St.Y.n) break;
+          const int64_t base = (St.Y.i0 + ky) * (int64_t)row + St.X.i0;
+          double vx = 0.0, vy = 0.0, dvx = 0.0, dvy = 0.0, ax = 0.0, ay = 0.0;
+#pragma unroll
+          for (int kx = 0; kx < STENCIL_AXIS; ++kx) {
+            if (kx >= St.X.n) break;
+            const double2 v = gv[base + kx], a = ga[base + kx];
+            const double w = St.X.w[kx], d = St.X.d[kx];
+            vx = fma(w, v.x, vx);
+            vy = fma(w, v.y, vy);
+            dvx = fma(d, v.x, dvx);
+            dvy = fma(d, v.y, dvy);
+            ax = fma(w, a.x, ax);
+            ay = fma(w, a.y, ay);
+          }
+          const double wy = St.Y.w[ky], dy = St.Y.d[ky];
+          g.L00 = fma(wy, dvx, g.L00);
+          g.L10 = fma(wy, dvy, g.L10);
+          g.L01 = fma(dy, vx, g.L01);
+          g.L11 = fma(dy, vy, g.L11);
+          g.vx = fma(wy, vx, g.vx);
+          g.vy = fma(wy, vy, g.vy);
+          g.ax = fma(wy, ax, g.ax);
+          g.ay = fma(wy, ay, g.ay);
+        }
+      }
     }
   }
-  double Jp = A.J[p];
-  int jh = A.jh[p];
-  double2 c0 = reinterpret_cast<const double2 *>(A.be)[2 * p];
-  double2 c1 = reinterpret_cast<const double2 *>(A.be)[2 * p + 1];
-  if (__double_as_longlong(c0.y) == __double_as_longlong(c1.x)) {
-    strain_symmetric(P, A, g, c0.x, c0.y, c1.y, Jp, jh);
-    c1.x = c0.y;
-  } else {
-    const PointStrain s = strain_general(P, A.dt, g, {{c0.x, c0.y, c1.x, c1.y}, Jp, jh});
-    c0 = make_double2(s.b.a00, s.b.a10);
-    c1 = make_double2(s.b.a01, s.b.a11);
-    Jp = s.J;
-    jh = s.jh;
+  PointStrain s;
+  {
+    const double2 c0 = reinterpret_cast<const double2 *>(A.be)[2 * p];
+    const double2 c1 = reinterpret_cast<const double2 *>(A.be)[2 * p + 1];
+    s = {{c0.x, c0.y, c1.x, c1.y}, A.J[p], A.jh[p]};
   }
+  if (__double_as_longlong(s.b.a10) != __double_as_longlong(s.b.a01) ||
+      !strain_symmetric(P, A, g, s))
+    s = strain_general(P, A.dt, g, s);
   double2 v = reinterpret_cast<const double2 *>(A.v)[p];
   if (A.kin[p] == 0) {
     const double a = P.flip_alpha, b = A.pic;
@@ -622,14 +629,14 @@ __global__ void k64_g2p(const __grid_constant__ MpmParams P, const __grid_consta
     }
   }
   if (!finite_bits(x.x) || !finite_bits(x.y) || !finite_bits(v.x) || !finite_bits(v.y) ||
-      !finite_bits(Jp))
+      !finite_bits(s.J))
     atomicOr(A.status, (uint32_t)HG_STATUS_NONFINITE);
   reinterpret_cast<double2 *>(A.q)[p] = x;
   reinterpret_cast<double2 *>(A.v)[p] = v;
-  reinterpret_cast<double2 *>(A.be)[2 * p] = c0;
-  reinterpret_cast<double2 *>(A.be)[2 * p + 1] = c1;
-  A.J[p] = Jp;
-  A.jh[p] = jh;
+  reinterpret_cast<double2 *>(A.be)[2 * p] = make_double2(s.b.a00, s.b.a10);
+  reinterpret_cast<double2 *>(A.be)[2 * p + 1] = make_double2(s.b.a01, s.b.a11);
+  A.J[p] = s.J;
+  A.jh[p] = s.jh;
 }
 
 inline int blocks_for(int64_t n, int t) { return (int)((n + t - 1) / t); }
@@ -645,6 +652,7 @@ template <bool FORCES, bool UPDATE> hg_status grid_pass(hg_mpm *m, double dt) {
   GridArgs A;
   A.nn = (int64_t)(m->p.nx + 1) * (m->p.ny + 1);
   A.dt = dt;
+  A.inv_dt = 1.0 / dt;
   A.mass = m->g_mass.p;
   A.mom = m->g_mom.p;
   A.mom_new = m->g_mom_new.p;
@@ -678,10 +686,11 @@ hg_status to_points(hg_mpm *m, double dt) {
   A.next_mom = m->g_mom_next.p;
   A.next_force = m->g_force_next.p;
   A.status = m->status.p;
-  A.yield = 0.5 * m->p.dp_alpha * m->p.kappa;
+  const double yield = 0.5 * m->p.dp_alpha * m->p.kappa;
+  A.yield_mu = yield / m->p.mu;
   A.pic = 1.0 - m->p.flip_alpha;
   A.mu32 = (float)m->p.mu;
-  A.yield32 = (float)A.yield;
+  A.yield32 = (float)yield;
   for (int k = 0; k < HG_MAX_PLANES; ++k)
     for (int c = 0; c < 2; ++c) A.px[k][c] = (float)m->p.planes[k].x[c];
   auto kernel = m->p.basis == HG_BASIS_UGIMP ? k64_g2p<HG_BASIS_UGIMP> : k64_g2p<HG_BASIS_LINEAR>;
