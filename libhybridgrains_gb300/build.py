@@ -39,7 +39,7 @@ SOURCES = [
     ("state.cu", False),  # checkpoint / resume blobs
 ]
 HEADERS = ["hg_internal.cuh", "fp64_tools.cuh", "mpm_basis.cuh",
-           "mpm_axis.cuh", "scan_block.cuh", "zones_internal.cuh"]
+           "mpm_axis.cuh", "dem_bins.cuh", "scan_block.cuh", "zones_internal.cuh"]
 
 
 def _nvcc():

@@ -11,8 +11,8 @@
 // shared by what it does at one position, few grains go to one-warp CTAs (a
 // CTA on every SM), and each grid is cleared by the kernel that last reads it.
 // Per step of the hybrid column (9,000 grains on 100,000 points), with eight
-// launches, four memsets and a copy before: MIXED bulk 128 -> 77 us, FP64 bulk
-// (its MPM kernels included) 367 -> 210 us.
+// launches, four memsets and a copy before: MIXED bulk 128 -> 69 us, FP64 bulk
+// (its MPM kernels included) 367 -> 201 us.
 //
 // Kernels:
 //   kc_grain_scatter  rasterizeGrainMass (Coupling.cpp:22-140) and
@@ -28,13 +28,15 @@
 //                     468-527), updatePositions_node_node (Coupling.cpp:
 //                     581-591), then the scatter of
 //                     ResamplingTools::homogenizeVelocity
-//                     (ResamplingTools.cpp:830-884)
+//                     (ResamplingTools.cpp:830-884), and the binning for the
+//                     next DEM step
 //   kc_homogenize     the rest of homogenizeVelocity over the nodes, and
 //                     ResamplingTools::homogenizeStress (ResamplingTools.cpp:
 //                     744-813) over the contacts
 #include "hg_internal.cuh"
 #include "mpm_basis.cuh"
 #include "mpm_axis.cuh"
+#include "dem_bins.cuh"
 
 #include <algorithm>
 #include <type_traits>
@@ -200,7 +202,7 @@ struct GrainArgs {
 // M: the MPM node mass type (double for an FP64 object, float for MIXED,
 // where it is the P2G sum of this step before the grid update).
 template <int BASIS, bool W32, typename M>
-__global__ void kc_grain_scatter(const __grid_constant__ GrainArgs A, const M *__restrict__ g_mass,
+__global__ void kc_grain_scatter(const __grid_constant__ GrainArgs A, const M *g_mass,
                                  double *dem_mass, double *dem_mom) {
   pdl_wait();
   pdl_trigger();
@@ -287,7 +289,7 @@ __device__ __forceinline__ bool coupled_node(const NodeArgs &A, int64_t i, doubl
 }
 
 __global__ void kc_update_nodes(const __grid_constant__ NodeArgs A,
-                                const double *__restrict__ g_mass, double *g_mom_new) {
+                                const double *g_mass, double *g_mom_new) {
   pdl_wait();
   pdl_trigger();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -314,7 +316,7 @@ __global__ void kc_update_nodes(const __grid_constant__ NodeArgs A,
 // velocity and acceleration (va: v, a) take p_new - lambda; the acceleration
 // (p_new - p) / (m dt) loses lambda / (m dt). Nodes without MPM mass keep
 // their zero velocity, as (p_new = 0) / m is never formed for them.
-__global__ void kc_update_nodes_x(const __grid_constant__ NodeArgs A, const float *__restrict__ gm,
+__global__ void kc_update_nodes_x(const __grid_constant__ NodeArgs A, const float *gm,
                                   double dt, float4 *va) {
   pdl_wait();
   pdl_trigger();
@@ -352,14 +354,19 @@ __global__ void kc_fill(double *dst, int64_t n, double v) {
 // touches the grains, updatePositions_node_node (Coupling.cpp:581-591):
 // q = q_before + dt v for every coupled grain (fixed ones are never coupled).
 // With hmom the grain, where it then is, adds to the homogenised velocity's
-// mass and momentum sums.
+// mass and momentum sums. It is binned there for the next DEM step.
 template <int BASIS, bool W32>
-__global__ void kc_transfer(const __grid_constant__ GrainArgs A, const double *__restrict__ a_after,
-                            double dt, double *hmom, double *hmass) {
+__global__ void kc_transfer(const __grid_constant__ GrainArgs A, const __grid_constant__ BinArgs B,
+                            const double *a_after, double dt, double *hmom,
+                            double *hmass) {
   pdl_wait();
   pdl_trigger();
   const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (b >= A.nb || A.fixed[b]) return;
+  if (b >= A.nb) return;
+  if (A.fixed[b]) {
+    bin_body(B, b, A.q[3 * b], A.q[3 * b + 1]);
+    return;
+  }
   const GridGeom &G = A.G;
   double vx = A.v[3 * b], vy = A.v[3 * b + 1], qx, qy;
   GridStencil<BASIS, W32> S;
@@ -385,6 +392,7 @@ __global__ void kc_transfer(const __grid_constant__ GrainArgs A, const double *_
     qx = A.q[3 * b];
     qy = A.q[3 * b + 1];
   }
+  bin_body(B, b, qx, qy);
   if (!hmom) return;
   const double mass = A.m0[b] * A.w[b], hl = G.h * 0.25;
   const double px = mass * vx, py = mass * vy;
@@ -631,9 +639,12 @@ template <int BASIS, bool W32> hg_status hybrid_step_impl(hg_hybrid *h, double d
   const bool hs = (flags & HG_HYBRID_HOMOGENIZE_STRESS) && nb > 0;
   if (nb > 0) {
     auto kernel = kc_transfer<BASIS, W32>;
-    HG_LAUNCH_PDL(kernel, blocks_for(nb, t), t, 0, s, A, (const double *)h->a_after.p, dt,
+    BinArgs B;
+    dem_bin_args(d, &B);
+    HG_LAUNCH_PDL(kernel, blocks_for(nb, t), t, 0, s, A, B, (const double *)h->a_after.p, dt,
                   hv ? h->hmom.p : (double *)nullptr, h->hmass.p);
     HG_CHECK_LAUNCH();
+    dem_binned(d);
   }
   if ((st = W32 ? mixed_particles(m, dt) : mpm64_phase2(m, dt))) return st;
   if (hv || hs) {

@@ -36,11 +36,11 @@
 // contact law by the FP64 pipe, a million disks by the records' 176 bytes per
 // contact. Against a counting sort of the grid, scans for every offset list
 // and records stored by their lanes (14 launches per step), per step: 1,000
-// disks stepped one call at a time 63.6 -> 28.3 us; 10,000 disks at 2.8
-// contacts each, FP64, 68.3 -> 39.0 us; 1,000,000 such disks, mixed, 889 ->
-// 434 us.
+// disks stepped one call at a time 63.6 -> 25.7 us; 10,000 disks at 2.8
+// contacts each, FP64, 68.3 -> 28.5 us; 1,000,000 such disks, mixed, 889 ->
+// 398 us.
 #include "hg_internal.cuh"
-#include "fp64_tools.cuh"
+#include "dem_bins.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -52,7 +52,6 @@ namespace hg {
 
 namespace {
 
-constexpr int MAXP = 32; // partner list capacity per body and step
 enum { K_PLANE = 0, K_CC = 1, K_KIN = 2 };
 constexpr int RW = HG_DEM_RECORD_WIDTH;
 
@@ -126,126 +125,10 @@ __device__ __forceinline__ void sort_small(int *keys, int n) {
   }
 }
 
-// Per body, for the pair search: the home cell (the cell of its centre) and,
-// in FP32, the offset of the centre from the home cell's corner and the
-// radius, with the fixed flag and the active static planes
-// (StaticPlaneCircleConstraint::isActive, StaticPlaneCircleConstraint.cpp:
-// 12-17) as bits; active static drums take the bits after the planes'. Per
-// candidate pair the search needs FP32 only, except for the exact tests of
-// the pairs that survive the FP32 filter.
-//
-// The bodies of a hash bucket are a linked list (head per bucket, the next
-// body in the record), built with one exchange per body: the search needs no
-// bucket counts, so no scan and no second pass over the bodies. The order of
-// a list does not matter: the emission pass sorts what the search finds.
-struct BinArgs {
-  int64_t n;
-  double H, invH;
-  uint32_t mask;
-  int nplanes;
-  double px[HG_MAX_PLANES][2], pn[HG_MAX_PLANES][2];
-  float pxf[HG_MAX_PLANES][2], pnf[HG_MAX_PLANES][2];
-  int ndrums;
-  double dx[HG_MAX_DRUMS][2], dr[HG_MAX_DRUMS];
-  const double *r;
-  const uint8_t *fixed;
-  float4 *rec; // 2 per body: (offset x, offset y, radius, flags), (home cell x, y, next, -)
-  int32_t *heads;
-  unsigned long long *pc; // contact counts by kind (PC_*)
-  int32_t *in_count;      // contacts in which the body is the second
-  int32_t *tiles;         // sums of the four counts per tile, or nullptr
-  int tile_shift;
-};
-
-enum : uint32_t { REL_FIXED = 1u, REL_PLANE0 = 2u };
-static_assert(1 + HG_MAX_PLANES + HG_MAX_DRUMS <= 32, "static-object bits of the body record");
-
-// Contact counts of a first body in one word: static objects in bits 0-7,
-// circle-circle in 8-35, kinematic in 36-63. The search adds to it with one
-// atomic per contact, which also gives the partner's slot. The last two are
-// the partners found; at most MAXP of each kind are kept.
-constexpr int PC_CC = 8, PC_KIN = 36;
-__device__ __forceinline__ int pc_static(unsigned long long p) { return (int)(p & 0xFFu); }
-__device__ __forceinline__ int pc_found_cc(unsigned long long p) {
-  return (int)((p >> PC_CC) & 0xFFFFFFFu);
-}
-__device__ __forceinline__ int pc_found_kin(unsigned long long p) { return (int)(p >> PC_KIN); }
-__device__ __forceinline__ int pc_cc(unsigned long long p) { return min(pc_found_cc(p), MAXP); }
-__device__ __forceinline__ int pc_kin(unsigned long long p) { return min(pc_found_kin(p), MAXP); }
-
-// Cell floor(x / H) of a coordinate and the FP32 offset from the cell's lower
-// edge. x / H is formed in fixed point with 24 fraction bits by one FP64 FMA
-// (adding 3 * 2^27 leaves an ulp of 2^-24), so the split is integer work; the
-// binning only has to be the same for every body and monotone. Rounding moves
-// a coordinate by at most 2^-25 cells, and contacts are at most
-// H / (1 + 1e-6) apart, so the cells of a contact's centres differ by at most
-// one. Coordinates beyond 2^27 cells and non-finite ones take the FP64 path.
-__device__ __noinline__ float2 bin_slow(double x, double H, double invH) {
-  const int c = (int)floor(x * invH);
-  return make_float2(__int_as_float(c), (float)(x - (double)c * H));
-}
-__device__ __forceinline__ void bin_axis(double x, double H, double invH, int &c, float &off) {
-  constexpr uint32_t BIAS_HI = 0x41B80000u; // 1.5 * 2^28
-  const double u = fma(x, invH, __hiloint2double((int)BIAS_HI, 0));
-  const uint32_t hi = (uint32_t)__double2hiint(u), lo = (uint32_t)__double2loint(u);
-  if ((hi >> 20) == (BIAS_HI >> 20)) {
-    c = (int)__funnelshift_r(lo, hi - BIAS_HI, 24);
-    off = (float)(lo & 0xFFFFFFu) * (1.0f / 16777216.0f) * (float)H;
-    return;
-  }
-  const float2 s = bin_slow(x, H, invH);
-  c = __float_as_int(s.x);
-  off = s.y;
-}
-
-// The body's record and its entry in the hash grid; counters set for the
-// step's search. x, y: the centre.
-__device__ __forceinline__ void bin_body(const BinArgs &A, int64_t i, double x, double y) {
-  const double ri = A.r[i];
-  const float rf = narrow_trunc(ri), xf = narrow_trunc(x), yf = narrow_trunc(y);
-  uint32_t flags = A.fixed[i] ? REL_FIXED : 0u;
-  for (int k = 0; k < A.nplanes; ++k) {
-    // n . (x - x_plane) <= r: decided in FP32 when the margin exceeds the
-    // error of truncated coordinates and FP32 sums (under 1e-6 of the terms),
-    // else in FP64 as the reference does
-    const float ex = xf - A.pxf[k][0], ey = yf - A.pxf[k][1];
-    const float gap = A.pnf[k][0] * ex + A.pnf[k][1] * ey - rf;
-    const float err = 1.0e-6f * (fabsf(xf) + fabsf(A.pxf[k][0]) + fabsf(yf) +
-                                 fabsf(A.pxf[k][1]) + rf);
-    bool on;
-    if (fabsf(gap) > err) {
-      on = gap < 0.0f;
-    } else {
-      const double d = A.pn[k][0] * (x - A.px[k][0]) + A.pn[k][1] * (y - A.px[k][1]);
-      on = d <= ri;
-    }
-    if (on) flags |= REL_PLANE0 << k;
-  }
-  // StaticDrumCircleConstraint::isActive (StaticDrumCircleConstraint.cpp:7-13):
-  // |x_drum - x|^2 >= (r_drum - r)^2; drum k is static object nplanes + k
-  for (int k = 0; k < A.ndrums; ++k) {
-    const double ex = A.dx[k][0] - x, ey = A.dx[k][1] - y, g = A.dr[k] - ri;
-    if (ex * ex + ey * ey >= g * g) flags |= REL_PLANE0 << (A.nplanes + k);
-  }
-  int cx, cy;
-  float ox, oy;
-  bin_axis(x, A.H, A.invH, cx, ox);
-  bin_axis(y, A.H, A.invH, cy, oy);
-  const int next = atomicExch(&A.heads[cell_hash(cx, cy, A.mask)], (int)i);
-  A.rec[2 * i] = make_float4(ox, oy, rf, __uint_as_float(flags));
-  A.rec[2 * i + 1] =
-      make_float4(__int_as_float(cx), __int_as_float(cy), __int_as_float(next), 0.0f);
-  // fixed bodies have no contacts of their own
-  const int ns = (flags & REL_FIXED) ? 0 : __popc(flags >> 1);
-  A.pc[i] = (unsigned long long)ns;
-  A.in_count[i] = 0;
-  if (A.tiles && ns) atomicAdd(A.tiles + 4 * (i >> A.tile_shift), ns);
-}
-
 // Bins every body: the first step after the bodies changed. Later steps find
 // the bins made by the integration of the step before.
 __global__ void __launch_bounds__(128) kd_bin(const __grid_constant__ BinArgs A,
-                                              const double *__restrict__ q) {
+                                              const double *q) {
   pdl_wait();
   pdl_trigger();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -298,14 +181,16 @@ struct PairArgs {
 
 // The contact test of a candidate pair (a, b), b's home cell offset by
 // (dx, dy) from a's. The FP32 offsets from the home cells' corners give the
-// centre distance to within about 1e-6 of a cell; the slack tol is 1e-4 of
-// a cell. So a pair whose FP32 distance exceeds ra + rb + tol is no contact,
-// and one whose FP32 distance is below ra + rb - tol is a contact under the
-// reference's FP64 tests as well (its AABBs overlap and c0 < 0 by about
-// 2 tol (ra + rb), far beyond FP64 rounding). Only the pairs in between take
-// those tests: AABB overlap (SpatialGrid.cpp:14-19, with the AABB corners
-// x -+ r evaluated as CircleGeometry.cpp:22-30 does) and
-// ballBallCCDCollisionHappens with q0 == q1 (active iff c0 <= 0).
+// centre distance to within about 1e-6 of a cell (offsets and truncated radii
+// to 1.2e-7 each, three FP32 sums); the slack tol is 4e-6 of a cell. So a pair
+// whose FP32 distance exceeds ra + rb + tol is no contact, and one whose FP32
+// distance is below ra + rb - tol is a contact under the reference's FP64
+// tests as well (its AABBs overlap and c0 < 0 by about 2 tol (ra + rb), far
+// beyond FP64 rounding). Only the pairs in between take those tests: AABB
+// overlap (SpatialGrid.cpp:14-19, with the AABB corners x -+ r evaluated as
+// CircleGeometry.cpp:22-30 does) and ballBallCCDCollisionHappens with q0 == q1
+// (active iff c0 <= 0). A pair in between costs its warp a microsecond (a dozen
+// FP64 instructions after four dependent loads), so the slack is small.
 __device__ __forceinline__ bool is_contact(const PairArgs &A, float4 pa, float4 pb, int dx,
                                            int dy, int a, int b) {
   const float ex = (float)dx * A.Hf + (pb.x - pa.x);
@@ -323,11 +208,11 @@ __device__ __forceinline__ bool is_contact(const PairArgs &A, float4 pa, float4 
   return c0 <= 0.0;
 }
 
-// Walks the bucket list of cell (cx, cy) over the bodies whose home cell it
-// is (a bucket may be shared by other cells).
+// Walks the bucket list from body b over the bodies whose home cell is (cx, cy)
+// (a bucket may be shared by other cells).
 template <class F>
-__device__ __forceinline__ void for_each_in_cell(const PairArgs &A, int cx, int cy, F &&body) {
-  int b = A.heads[cell_hash(cx, cy, A.mask)];
+__device__ __forceinline__ void for_each_in_cell(const PairArgs &A, int b, int cx, int cy,
+                                                 F &&body) {
   // (a list holds each body once: the bound on the steps is never reached)
   for (int64_t left = A.n; b >= 0 && left > 0; --left) {
     if (!HG_INDEX_OK(b, A.n, A.status)) return;
@@ -345,14 +230,15 @@ template <class F>
 __device__ __forceinline__ void for_each_partner(const PairArgs &A, int a, F &&found) {
   const float4 pa = A.rec[2 * a], ca = A.rec[2 * a + 1];
   for (int dy = -1; dy <= 1; ++dy)
-    for (int dx = -1; dx <= 1; ++dx)
-      for_each_in_cell(A, __float_as_int(ca.x) + dx, __float_as_int(ca.y) + dy,
-                       [&](int b, float4 pb) {
-                         if (b == a) return;
-                         const bool bf = (__float_as_uint(pb.w) & REL_FIXED) != 0u;
-                         if (!(b > a || bf)) return;
-                         if (is_contact(A, pa, pb, dx, dy, a, b)) found(b, bf);
-                       });
+    for (int dx = -1; dx <= 1; ++dx) {
+      const int cx = __float_as_int(ca.x) + dx, cy = __float_as_int(ca.y) + dy;
+      for_each_in_cell(A, A.heads[cell_bucket(cx, cy, A.mask)], cx, cy, [&](int b, float4 pb) {
+        if (b == a) return;
+        const bool bf = (__float_as_uint(pb.w) & REL_FIXED) != 0u;
+        if (!(b > a || bf)) return;
+        if (is_contact(A, pa, pb, dx, dy, a, b)) found(b, bf);
+      });
+    }
 }
 
 // Search over half of each neighbourhood: the home cell and the four cells
@@ -365,72 +251,124 @@ __device__ __forceinline__ void for_each_partner(const PairArgs &A, int a, F &&f
 // plist (in no particular order; the emission pass sorts them).
 // Circle-circle contacts also count as incoming at their second body.
 
-__device__ __forceinline__ void credit(const PairArgs &A, int first, int second, bool kin,
-                                       bool &overflow) {
-  if (!HG_INDEX_OK(first, A.n, A.status)) return;
-  const unsigned long long p = atomicAdd(A.pc + first, 1ull << (kin ? PC_KIN : PC_CC));
-  const int ncc = pc_found_cc(p), nkin = pc_found_kin(p);
-  const bool kept = (kin ? nkin : ncc) < MAXP;
-  overflow |= !kept;
-  if (ncc + nkin < PW)
-    A.plist[(int64_t)first * PW + ncc + nkin] = (uint32_t)second | (kin ? 0x80000000u : 0u);
-  if (!kin) atomicAdd(A.in_count + second, 1);
-  if (A.add_tiles) {
-    if (kept) atomicAdd(A.tiles + 4 * (int64_t)(first >> A.tile_shift) + (kin ? 2 : 1), 1);
-    if (!kin) atomicAdd(A.tiles + 4 * (int64_t)(second >> A.tile_shift) + 3, 1);
+// Contacts found by a thread: kept until HELD of them can be credited together
+// (an atomic's return is a round trip to L2: they overlap).
+constexpr int HELD = 4;
+struct Found {
+  int first[HELD];
+  uint32_t second[HELD]; // a kinematic (fixed) second flagged by bit 31
+  int n;
+  bool overflow;
+};
+
+// Adds one to tile t's count of kind comp for every calling lane with on set:
+// one atomic per distinct count among the lanes of mask. (With one atomic per
+// contact, 180 on each address at 10,000 disks, the search took 11.0 us instead
+// of 8.0.)
+__device__ __forceinline__ void add_tile(int32_t *tiles, unsigned mask, int t, int comp, bool on) {
+  const int at = 4 * t + comp;
+  const unsigned same = __match_any_sync(mask, at);
+  const unsigned add = same & __ballot_sync(mask, on);
+  const int lane = threadIdx.x & 31;
+  if (add && lane == __ffs(same) - 1) atomicAdd(tiles + at, __popc(add));
+}
+
+__device__ __forceinline__ void credit(const PairArgs &A, Found &f) {
+  unsigned long long p[HELD];
+#pragma unroll
+  for (int k = 0; k < HELD; ++k)
+    if (k < f.n)
+      p[k] = atomicAdd(A.pc + f.first[k], 1ull << (f.second[k] >> 31 ? PC_KIN : PC_CC));
+#pragma unroll
+  for (int k = 0; k < HELD; ++k) {
+    if (k >= f.n) break;
+    const int first = f.first[k], second = (int)(f.second[k] & 0x7FFFFFFFu);
+    const bool kin = f.second[k] >> 31;
+    const int ncc = pc_found_cc(p[k]), nkin = pc_found_kin(p[k]);
+    const bool kept = (kin ? nkin : ncc) < MAXP;
+    f.overflow |= !kept;
+    if (ncc + nkin < PW) A.plist[(int64_t)first * PW + ncc + nkin] = f.second[k];
+    if (!kin) atomicAdd(A.in_count + second, 1);
+    if (A.add_tiles) {
+      const unsigned mask = __activemask();
+      add_tile(A.tiles, mask, first >> A.tile_shift, kin ? 2 : 1, kept);
+      add_tile(A.tiles, mask, second >> A.tile_shift, 3, !kin);
+    }
   }
+  f.n = 0;
 }
 
 // cell c of the half neighbourhood: (0, 0), (1, 0), (-1, 1), (0, 1), (1, 1)
 __device__ __forceinline__ int half_dx(int c) { return c == 0 ? 0 : (c == 1 ? 1 : c - 3); }
 __device__ __forceinline__ int half_dy(int c) { return c >= 2 ? 1 : 0; }
 
-__device__ __forceinline__ void search_cell(const PairArgs &A, int a, int c, float4 pa, float4 ca,
-                                            bool &overflow) {
+__device__ __forceinline__ void search_cell(const PairArgs &A, int a, int c, float4 pa, int hx,
+                                            int hy, int head, Found &f) {
   const bool af = (__float_as_uint(pa.w) & REL_FIXED) != 0u;
   const int dx = half_dx(c), dy = half_dy(c);
-  for_each_in_cell(A, __float_as_int(ca.x) + dx, __float_as_int(ca.y) + dy,
-                   [&](int b, float4 pb) {
-                     if (b == a || (c == 0 && b < a)) return;
-                     const bool bf = (__float_as_uint(pb.w) & REL_FIXED) != 0u;
-                     if (af && bf) return;
-                     if (!is_contact(A, pa, pb, dx, dy, a, b)) return;
-                     if (af) credit(A, b, a, true, overflow);
-                     else if (bf) credit(A, a, b, true, overflow);
-                     else credit(A, min(a, b), max(a, b), false, overflow);
-                   });
+  for_each_in_cell(A, head, hx + dx, hy + dy, [&](int b, float4 pb) {
+    if (b == a || (c == 0 && b < a)) return;
+    const bool bf = (__float_as_uint(pb.w) & REL_FIXED) != 0u;
+    if (af && bf) return;
+    if (!is_contact(A, pa, pb, dx, dy, a, b)) return;
+    const int first = af ? b : (bf ? a : min(a, b));
+    const uint32_t second = af ? (uint32_t)a | 0x80000000u
+                               : (bf ? (uint32_t)b | 0x80000000u : (uint32_t)max(a, b));
+    if (!HG_INDEX_OK(first, A.n, A.status)) return;
+    if (f.n == HELD) credit(A, f);
+#pragma unroll
+    for (int k = 0; k < HELD; ++k)
+      if (k == f.n) {
+        f.first[k] = first;
+        f.second[k] = second;
+      }
+    ++f.n;
+  });
 }
 
 // One thread per body over its five cells: fewer loads of the body's own
 // record than kd_pairs when the bodies alone fill the GPU.
-__global__ void kd_pairs_body(PairArgs A) {
+__global__ void __launch_bounds__(128) kd_pairs_body(const __grid_constant__ PairArgs A) {
   // (launched with programmatic dependence on the kernel before it)
   pdl_wait();
   pdl_trigger();
   const int a = (int)(blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
   if (a >= A.n) return;
   const float4 pa = A.rec[2 * a], ca = A.rec[2 * a + 1];
-  bool overflow = false;
+  const int hx = __float_as_int(ca.x), hy = __float_as_int(ca.y);
+  Found f;
+  f.n = 0;
+  f.overflow = false;
+  int head[5];
 #pragma unroll
-  for (int c = 0; c < 5; ++c) search_cell(A, a, c, pa, ca, overflow);
-  if (overflow) atomicOr(A.status, (uint32_t)HG_STATUS_CELL_OVERFLOW);
+  for (int c = 0; c < 5; ++c)
+    head[c] = A.heads[cell_bucket(hx + half_dx(c), hy + half_dy(c), A.mask)];
+#pragma unroll
+  for (int c = 0; c < 5; ++c) search_cell(A, a, c, pa, hx, hy, head[c], f);
+  credit(A, f);
+  if (f.overflow) atomicOr(A.status, (uint32_t)HG_STATUS_CELL_OVERFLOW);
 }
 
 // One thread per (body, cell of the half neighbourhood): thread t takes cell
 // t / n of body t % n, so a warp's lanes read consecutive bodies' records and
 // each thread follows one list instead of five.
-__global__ void kd_pairs(PairArgs A) {
+__global__ void __launch_bounds__(128) kd_pairs(const __grid_constant__ PairArgs A) {
   // (launched with programmatic dependence on the kernel before it)
   pdl_wait();
   pdl_trigger();
-  const int64_t n = A.n;
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int n = (int)A.n;
+  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x); // 5 n < 2^31 here
   if (t >= 5 * n) return;
-  const int c = (int)(t / n);
-  const int a = (int)(t - (int64_t)c * n);
-  bool overflow = false;
-  search_cell(A, a, c, A.rec[2 * a], A.rec[2 * a + 1], overflow);
-  if (overflow) atomicOr(A.status, (uint32_t)HG_STATUS_CELL_OVERFLOW);
+  const int c = t / n, a = t - c * n;
+  const float4 pa = A.rec[2 * a], ca = A.rec[2 * a + 1];
+  const int hx = __float_as_int(ca.x), hy = __float_as_int(ca.y);
+  Found f;
+  f.n = 0;
+  f.overflow = false;
+  search_cell(A, a, c, pa, hx, hy, A.heads[cell_bucket(hx + half_dx(c), hy + half_dy(c), A.mask)],
+              f);
+  credit(A, f);
+  if (f.overflow) atomicOr(A.status, (uint32_t)HG_STATUS_CELL_OVERFLOW);
 }
 
 __device__ __forceinline__ int warp_sum(int x) {
@@ -442,8 +380,8 @@ __device__ __forceinline__ int warp_sum(int x) {
 // Sums of the contact counts (static, circle-circle, kinematic, incoming)
 // over tiles of 2^shift bodies, one CTA per tile.
 __global__ void __launch_bounds__(256) kd_tile_sums(int64_t n, int shift,
-                                                    const unsigned long long *__restrict__ pc,
-                                                    const int32_t *__restrict__ in_count,
+                                                    const unsigned long long *pc,
+                                                    const int32_t *in_count,
                                                     int32_t *tiles) {
   // (launched with programmatic dependence on the kernel before it)
   pdl_wait();
@@ -625,6 +563,8 @@ struct ContactArgs {
   double dt;
   int weighted;
   double kn, kt, gn, gt, mu;
+  double half_gn, half_gt;
+  float mu2_32; // mu^2
   int nplanes;
   double px[HG_MAX_PLANES][2], pn[HG_MAX_PLANES][2];
   int ndrums; // static objects nplanes .. nplanes + ndrums - 1
@@ -714,11 +654,15 @@ __device__ __forceinline__ void for_each_contact(const ContactArgs &C, Law &&law
       const int b = (int)(key & 0x3FFFFFFF);
       if (HG_INDEX_OK(a, C.n, C.status) &&
           HG_INDEX_OK(b, kind == K_PLANE ? (int64_t)(C.nplanes + C.ndrums) : C.n, C.status)) {
-        if (kind == K_CC) { // the second body's list of incoming contacts
-          const int64_t o = (int64_t)C.desc[b].w + atomicAdd(&C.in_cursor[b], 1);
-          if (o < C.ccap) C.in_list[o] = (int32_t)k;
+        // the second body's list of incoming contacts (the slot arrives while
+        // the law runs)
+        int slot = 0, list = 0;
+        if (kind == K_CC) {
+          slot = atomicAdd(&C.in_cursor[b], 1);
+          list = C.desc[b].w;
         }
         law(k, key, kind, a, b, out);
+        if (kind == K_CC && (int64_t)list + slot < C.ccap) C.in_list[list + slot] = (int32_t)k;
       }
     }
     __syncwarp();
@@ -734,6 +678,19 @@ __device__ __forceinline__ void put2(double *out, int i, double x, double y) {
   reinterpret_cast<double2 *>(out)[i] = make_double2(x, y);
 }
 
+// FP32 estimate of |a|^2 from truncated components (0 for those below FP32's
+// range); top: the largest exponent word met.
+__device__ __forceinline__ float square_est(D2 a, uint32_t &top) {
+  auto est = [&](double x) {
+    const uint32_t hi = f64_hi(x) & 0x7FFFFFFFu;
+    top = max(top, hi);
+    const uint32_t f = __funnelshift_l(f64_lo(x), hi, 3) - (896u << 23);
+    return __uint_as_float(hi < 897u << 20 ? 0u : f);
+  };
+  const float x = est(a.x), y = est(a.y);
+  return x * x + y * y;
+}
+
 __global__ void __launch_bounds__(CONTACT_THREADS) kd_contacts(const __grid_constant__ ContactArgs C) {
   // (launched with programmatic dependence on the kernel before it)
   pdl_wait();
@@ -745,6 +702,7 @@ __global__ void __launch_bounds__(CONTACT_THREADS) kd_contacts(const __grid_cons
     double depth, weight;
     D2 n, cp{0.0, 0.0}, r0, r1{0.0, 0.0}, vrel;
     const double ra = C.r[a];
+    const int o = find_old(C, key, kind, a); // (its loads overlap the bodies')
     if (kind == K_PLANE && b >= C.nplanes) { // PenaltyImpactFrictionMap.cpp:361-401
       // StaticDrumCircleConstraint.cpp:100-159: the normal points from the
       // disk's centre to the drum's; the contact point is the disk's point
@@ -780,7 +738,7 @@ __global__ void __launch_bounds__(CONTACT_THREADS) kd_contacts(const __grid_cons
       const D2 d = dsub(qa, qb);
       const double d2 = dsq(d), dist = sqrt(d2);
       n = d;
-      if (d2 > 0.0) {
+      if (!f64_zero(d2)) {
         const Divisor len = divisor(dist);
         bool ok = len.ok;
         n = D2{quot(d.x, len, ok), quot(d.y, len, ok)};
@@ -809,7 +767,6 @@ __global__ void __launch_bounds__(CONTACT_THREADS) kd_contacts(const __grid_cons
     }
     // tangential spring carry
     D2 ds;
-    const int o = find_old(C, key, kind, a);
     if (o >= 0) {
       const double2 old = *reinterpret_cast<const double2 *>(C.old_rec + (int64_t)o * RW + 6);
       ds = dadd(D2{old.x, old.y}, dscl(C.dt, vrel));
@@ -820,29 +777,32 @@ __global__ void __launch_bounds__(CONTACT_THREADS) kd_contacts(const __grid_cons
     // penalty force (PenaltyImpactFrictionMap.cpp:616-1081)
     const double w = weight;
     // (products with a weight of 1 are the products without it)
-    const bool one = w == 1.0;
-    const double nkn = one ? -C.kn : -C.kn * w, nkt = one ? -C.kt : -C.kt * w;
-    const double hgn = 0.5 * C.gn * w, hgt = 0.5 * C.gt * w;
+    double nkn = -C.kn, nkt = -C.kt, hgn = C.half_gn, hgt = C.half_gt;
+    if (__double_as_longlong(w) != __double_as_longlong(1.0)) {
+      nkn = nkn * w;
+      nkt = nkt * w;
+      hgn = hgn * w;
+      hgt = hgt * w;
+    }
     const D2 vt = dsub(vrel, dscl(ddot(n, vrel), n));
     const D2 vn = dsub(vrel, vt);
     const D2 fn = dsub(dscl(nkn * depth, n), dscl(hgn, vn));
     D2 ft = dsub(dscl(nkt, ds), dscl(hgt, vt));
     // Coulomb's law compares gamma_t w / 2 |vt| and |ft| with mu |fn|. FP32
-    // estimates of the three, within 1e-6 of them, decide all but close calls:
-    // a sticking contact then needs none of the three square roots, a sliding
-    // one none but the root of its quadratic.
-    const float vt2 = narrow_trunc(vt.x) * narrow_trunc(vt.x) + narrow_trunc(vt.y) * narrow_trunc(vt.y);
-    const float fn2 = narrow_trunc(fn.x) * narrow_trunc(fn.x) + narrow_trunc(fn.y) * narrow_trunc(fn.y);
-    const float ft2 = narrow_trunc(ft.x) * narrow_trunc(ft.x) + narrow_trunc(ft.y) * narrow_trunc(ft.y);
-    const float cap32 = narrow_trunc(C.mu) * sqrtf(fn2);
-    const float drag32 = narrow_trunc(hgt) * sqrtf(vt2), ft32 = sqrtf(ft2);
-    const bool sure = fn2 > 1.0e-24f && fn2 < 1.0e24f && vt2 > 1.0e-24f && vt2 < 1.0e24f &&
-                      ft2 > 1.0e-24f && ft2 < 1.0e24f && cap32 > 1.0e-12f;
-    const bool stick_drag = sure && drag32 < cap32 * 0.99999f; // not slipping
-    if (!(stick_drag && ft32 < cap32 * 0.99999f)) {
+    // estimates of their squares, within 1e-6 of them, decide all but close
+    // calls (2e-5): a sticking contact then needs none of the three square
+    // roots, a sliding one none but the root of its quadratic.
+    uint32_t top = 0u;
+    const float vt2 = square_est(vt, top), fn2 = square_est(fn, top), ft2 = square_est(ft, top);
+    const float half_gt32 = narrow_trunc(hgt);
+    const float cap2 = C.mu2_32 * fn2, drag2 = half_gt32 * half_gt32 * vt2;
+    const float low = fminf(fminf(vt2, fn2), fminf(ft2, cap2));
+    const bool sure = top < 1063u << 20 && low > 1.0e-24f; // squares within FP32
+    const bool stick_drag = sure && drag2 < cap2 * 0.99998f; // not slipping
+    if (!(stick_drag && ft2 < cap2 * 0.99998f)) {
       bool slip = false, slide = true;
       double mu_fn = 0.0;
-      if (!(stick_drag && ft32 > cap32 * 1.00001f)) {
+      if (!(stick_drag && ft2 > cap2 * 1.00002f)) {
         mu_fn = C.mu * dnorm(fn);
         slip = hgt * dnorm(vt) > mu_fn;
         slide = dnorm(ft) > mu_fn;
@@ -883,31 +843,42 @@ __global__ void __launch_bounds__(CONTACT_THREADS) kd_contacts(const __grid_cons
 // Body j's contacts in the reference's order: with static objects, as the
 // second body of circle-circle contacts (their first indices lie below j, so
 // they come before j's own list in the reference's loop), as the first body,
-// and with fixed disks. apply(contact, as_second). The incoming list, filled
-// in no particular order, is sorted first.
-template <class F>
-__device__ __forceinline__ void for_each_load(int j, int4 d, int counts, int nin, int32_t *in_list,
-                                              int64_t ccap, uint32_t *status, F &&apply) {
-  for (int k = 0; k < (counts & 0xFF); ++k) apply(d.x + k, false);
+// and with fixed disks. apply(load, as_second). The incoming list, filled in
+// no particular order, is sorted first. The first four incoming and own loads
+// are fetched together: the sums are a chain, their loads need not be.
+template <class L, class F>
+__device__ __forceinline__ void for_each_load(const L *load, int4 d, int counts,
+                                              int nin, int32_t *in_list, int64_t ccap,
+                                              uint32_t *status, F &&apply) {
+  const int ns = counts & 0xFF, ncc = (counts >> 8) & 0xFF, nkin = (counts >> 16) & 0xFF;
   nin = (int)min((int64_t)nin, max((int64_t)0, ccap - d.w));
   int32_t *lst = in_list + d.w;
-  if (nin <= 4) {
-    int L[4];
+  int in[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) L[k] = k < nin ? lst[k] : 0x7FFFFFFF;
+  for (int k = 0; k < 4; ++k) in[k] = k < nin ? lst[k] : 0x7FFFFFFF;
+  L own[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (k < ncc) own[k] = load[d.y + k];
+  for (int k = 0; k < ns; ++k) apply(load[d.x + k], false);
+  if (nin <= 4) {
     auto order = [&](int x, int y) {
-      const int lo = min(L[x], L[y]), hi = max(L[x], L[y]);
-      L[x] = lo;
-      L[y] = hi;
+      const int lo = min(in[x], in[y]), hi = max(in[x], in[y]);
+      in[x] = lo;
+      in[y] = hi;
     };
     order(0, 1);
     order(2, 3);
     order(0, 2);
     order(1, 3);
     order(1, 2);
+    L got[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      if (k < nin && HG_INDEX_OK(L[k], ccap, status)) apply(L[k], true);
+      if (k < nin && HG_INDEX_OK(in[k], ccap, status)) got[k] = load[in[k]];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (k < nin && HG_INDEX_OK(in[k], ccap, status)) apply(got[k], true);
   } else {
     for (int i = 1; i < nin; ++i) {
       const int key = lst[i];
@@ -919,10 +890,13 @@ __device__ __forceinline__ void for_each_load(int j, int4 d, int counts, int nin
       lst[t + 1] = key;
     }
     for (int i = 0; i < nin; ++i)
-      if (HG_INDEX_OK(lst[i], ccap, status)) apply(lst[i], true);
+      if (HG_INDEX_OK(lst[i], ccap, status)) apply(load[lst[i]], true);
   }
-  for (int k = 0; k < ((counts >> 8) & 0xFF); ++k) apply(d.y + k, false);
-  for (int k = 0; k < ((counts >> 16) & 0xFF); ++k) apply(d.z + k, false);
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (k < ncc) apply(own[k], false);
+  for (int k = 4; k < ncc; ++k) apply(load[d.y + k], false);
+  for (int k = 0; k < nkin; ++k) apply(load[d.z + k], false);
 }
 
 struct IntegrateArgs {
@@ -952,11 +926,12 @@ __global__ void kd_integrate(const __grid_constant__ IntegrateArgs A,
   if (j >= A.n) return;
   // gravity and dt / M, dt / Mi from kd_body_terms
   const double4 bt = A.terms[j];
-  const double4 *load = reinterpret_cast<const double4 *>(A.load);
+  const double u0 = A.v[3 * j], u1 = A.v[3 * j + 1], u2 = A.v[3 * j + 2];
+  const double p0 = A.q[3 * j], p1 = A.q[3 * j + 1], p2 = A.q[3 * j + 2];
+  const bool fixed = A.fixed[j] != 0;
   double Fx = bt.x, Fy = bt.y, T = 0.0;
-  for_each_load((int)j, A.desc[j], A.descn[j], A.in_cursor[j], A.in_list, A.ccap, A.status,
-                [&](int k, bool second) {
-                  const double4 f = load[k];
+  for_each_load(reinterpret_cast<const double4 *>(A.load), A.desc[j], A.descn[j], A.in_cursor[j],
+                A.in_list, A.ccap, A.status, [&](const double4 &f, bool second) {
                   if (second) {
                     Fx -= f.x;
                     Fy -= f.y;
@@ -967,15 +942,14 @@ __global__ void kd_integrate(const __grid_constant__ IntegrateArgs A,
                     T += f.z;
                   }
                 });
-  if (A.fixed[j]) Fx = Fy = T = 0.0;
+  if (fixed) Fx = Fy = T = 0.0;
   // v1 = v0 + dt Minv F ; q1 = q0 + dt v1
-  const double v0 = A.v[3 * j] + bt.z * Fx;
-  const double v1 = A.v[3 * j + 1] + bt.z * Fy;
-  const double v2 = A.v[3 * j + 2] + bt.w * T;
+  const double v0 = u0 + bt.z * Fx;
+  const double v1 = u1 + bt.z * Fy;
+  const double v2 = u2 + bt.w * T;
   A.v[3 * j] = v0;
   A.v[3 * j + 1] = v1;
   A.v[3 * j + 2] = v2;
-  const double p0 = A.q[3 * j], p1 = A.q[3 * j + 1], p2 = A.q[3 * j + 2];
   if (A.q_before) {
     A.q_before[3 * j] = p0;
     A.q_before[3 * j + 1] = p1;
@@ -1026,6 +1000,7 @@ __global__ void __launch_bounds__(CONTACT_THREADS) kdx_contacts(const __grid_con
     const F2 va{narrow(C.v[3 * a]), narrow(C.v[3 * a + 1])};
     const float wa = narrow(C.v[3 * a + 2]);
     const float ra = narrow(C.r[a]);
+    const int o = find_old(C, key, kind, a); // (its loads overlap the bodies')
     float depth, weight;
     F2 n, r0, r1{0.0f, 0.0f}, vrel;
     double cpx, cpy;
@@ -1084,7 +1059,6 @@ __global__ void __launch_bounds__(CONTACT_THREADS) kdx_contacts(const __grid_con
     }
     // tangential spring carry
     F2 ds;
-    const int o = find_old(C, key, kind, a);
     if (o >= 0) {
       const double2 old = *reinterpret_cast<const double2 *>(C.old_rec + (int64_t)o * RW + 6);
       ds = fadd(F2{narrow(old.x), narrow(old.y)}, fscl(dt, vrel));
@@ -1139,24 +1113,24 @@ __global__ void kdx_integrate(const __grid_constant__ IntegrateArgs A,
   const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (j >= A.n) return;
   const double4 bt = A.terms[j];
-  const float4 *load = reinterpret_cast<const float4 *>(A.load);
+  const double u0 = A.v[3 * j], u1 = A.v[3 * j + 1], u2 = A.v[3 * j + 2];
+  const double p0 = A.q[3 * j], p1 = A.q[3 * j + 1], p2 = A.q[3 * j + 2];
+  const bool fixed = A.fixed[j] != 0;
   float Fx = narrow(bt.x), Fy = narrow(bt.y), T = 0.0f;
-  for_each_load((int)j, A.desc[j], A.descn[j], A.in_cursor[j], A.in_list, A.ccap, A.status,
-                [&](int k, bool second) {
-                  const float4 f = load[k];
+  for_each_load(reinterpret_cast<const float4 *>(A.load), A.desc[j], A.descn[j], A.in_cursor[j],
+                A.in_list, A.ccap, A.status, [&](const float4 &f, bool second) {
                   Fx += second ? -f.x : f.x;
                   Fy += second ? -f.y : f.y;
                   T += second ? -f.w : f.z;
                 });
-  if (A.fixed[j]) Fx = Fy = T = 0.0f;
-  const float v0 = narrow(A.v[3 * j]) + narrow(bt.z) * Fx;
-  const float v1 = narrow(A.v[3 * j + 1]) + narrow(bt.z) * Fy;
-  const float v2 = narrow(A.v[3 * j + 2]) + narrow(bt.w) * T;
+  if (fixed) Fx = Fy = T = 0.0f;
+  const float v0 = narrow(u0) + narrow(bt.z) * Fx;
+  const float v1 = narrow(u1) + narrow(bt.z) * Fy;
+  const float v2 = narrow(u2) + narrow(bt.w) * T;
   const double w0 = widen_f32(v0), w1 = widen_f32(v1), w2 = widen_f32(v2);
   A.v[3 * j] = w0;
   A.v[3 * j + 1] = w1;
   A.v[3 * j + 2] = w2;
-  const double p0 = A.q[3 * j], p1 = A.q[3 * j + 1], p2 = A.q[3 * j + 2];
   if (A.q_before) {
     A.q_before[3 * j] = p0;
     A.q_before[3 * j + 1] = p1;
@@ -1217,6 +1191,7 @@ __global__ void kd_box_pairs(BroadArgs B, const int2 *__restrict__ home,
 inline int blocks_for(int64_t n, int t) { return (int)std::max<int64_t>(1, (n + t - 1) / t); }
 
 
+// Hash table sizes: at least two buckets per box or body, and 16
 uint32_t table_bits(int64_t n) {
   uint32_t bits = 4;
   while (((int64_t)1 << bits) < 2 * n && bits < 30) ++bits;
@@ -1253,11 +1228,17 @@ int tile_shift_for(int64_t n) {
 
 } // namespace
 
+// Below about one body per thread slot of the GPU, five threads per body
+// hide the buckets' latency, and the search adds to the tile sums as it
+// goes (a launch less); above it, one thread per body reads each body's
+// record once, and the sums take a pass of their own (at a million disks
+// under contact load the added atomics cost more than the pass).
+static bool search_by_cells(const hg_dem *d) { return d->n < (int64_t)d->ctx->num_sms * 1024; }
+
 hg_status dem_alloc(hg_dem *d) {
   const int64_t N = std::max<int64_t>(d->cap, 1);
   const int64_t C = std::max<int64_t>(d->ccap, 1);
-  const uint32_t bits = table_bits(N);
-  d->mask = (1u << bits) - 1u;
+  d->mask = (1u << table_bits(N)) - 1u;
   const int64_t T = (int64_t)d->mask + 1;
   const bool mixed = d->p.precision == HG_PRECISION_MIXED;
   hg_status st;
@@ -1322,27 +1303,13 @@ void dem_set_launch_shapes(hg_dem *d) {
   d->contact_grid = d->ctx->num_sms * per_sm;
 }
 
-hg_status dem_step(hg_dem *d, double dt, int weighted, bool bin_next, double *q_before) {
-  cudaStream_t s = dem_stream(d);
-  const int64_t n = d->n;
-  if (n == 0) return HG_OK;
-  hg_status st;
-  if ((st = dem_prepare(d, dt))) return st;
-  // the hash table grows with the live body count (at most the capacity's)
-  const uint32_t mask = (1u << table_bits(n)) - 1u;
-  const int shift = tile_shift_for(n);
-  const int ntiles = (int)(((n - 1) >> shift) + 1);
-  // Below about one body per thread slot of the GPU, five threads per body
-  // hide the list walks' latency, and the search adds to the tile sums as it
-  // goes (a launch less); above it, one thread per body reads each body's
-  // record once, and the sums take a pass of their own (at a million disks
-  // under contact load the added atomics cost more than the pass).
-  const bool few = n < (int64_t)d->ctx->num_sms * 1024;
-  BinArgs H;
-  H.n = n;
+void dem_bin_args(const hg_dem *d, BinArgs *out) {
+  BinArgs &H = *out;
+  H.n = d->n;
   H.H = d->cell_h;
   H.invH = 1.0 / d->cell_h;
-  H.mask = mask;
+  // the hash table grows with the live body count (at most the capacity's)
+  H.mask = (1u << table_bits(d->n)) - 1u;
   H.nplanes = d->p.nplanes;
   H.ndrums = d->p.ndrums;
   for (int k = 0; k < HG_MAX_DRUMS; ++k) {
@@ -1363,8 +1330,26 @@ hg_status dem_step(hg_dem *d, double dt, int weighted, bool bin_next, double *q_
   H.heads = d->heads.p;
   H.pc = d->pc.p;
   H.in_count = d->in_count.p;
-  H.tiles = few ? d->tiles.p : nullptr;
-  H.tile_shift = shift;
+  H.tiles = search_by_cells(d) ? d->tiles.p : nullptr;
+  H.tile_shift = tile_shift_for(d->n);
+}
+
+void dem_binned(hg_dem *d) {
+  if (d->bins == hg_dem::BINS_CLEAR) d->bins = hg_dem::BINS_FILLED;
+}
+
+hg_status dem_step(hg_dem *d, double dt, int weighted, bool bin_next, double *q_before) {
+  cudaStream_t s = dem_stream(d);
+  const int64_t n = d->n;
+  if (n == 0) return HG_OK;
+  hg_status st;
+  if ((st = dem_prepare(d, dt))) return st;
+  const int shift = tile_shift_for(n);
+  const int ntiles = (int)(((n - 1) >> shift) + 1);
+  const bool few = search_by_cells(d);
+  BinArgs H;
+  dem_bin_args(d, &H);
+  const uint32_t mask = H.mask;
   const int bins = d->bins;
   d->bins = hg_dem::BINS_DIRTY; // until the step is queued
   if (bins == hg_dem::BINS_DIRTY) {
@@ -1381,7 +1366,7 @@ hg_status dem_step(hg_dem *d, double dt, int weighted, bool bin_next, double *q_
   A.mask = mask;
   A.rec = d->brec.p;
   A.Hf = (float)d->cell_h;
-  A.tol = (float)(1.0e-4 * d->cell_h);
+  A.tol = (float)(4.0e-6 * d->cell_h);
   A.heads = d->heads.p;
   A.q = d->q.p;
   A.r = d->r.p;
@@ -1422,6 +1407,9 @@ hg_status dem_step(hg_dem *d, double dt, int weighted, bool bin_next, double *q_
   Cg.gn = d->p.gn;
   Cg.gt = d->p.gt;
   Cg.mu = d->p.mu;
+  Cg.half_gn = 0.5 * d->p.gn;
+  Cg.half_gt = 0.5 * d->p.gt;
+  Cg.mu2_32 = (float)(d->p.mu * d->p.mu);
   Cg.nplanes = d->p.nplanes;
   Cg.ndrums = d->p.ndrums;
   for (int k = 0; k < HG_MAX_DRUMS; ++k) {

@@ -75,7 +75,9 @@ struct TraceRange {
 // access to global memory, which returns once the previous kernel has
 // completed and its writes are visible, and pdl_trigger() to let the next
 // kernel be scheduled in turn. After a copy, a memset or an ordinary launch
-// the wait returns at once and the ordering is the stream's.
+// the wait returns at once and the ordering is the stream's. Such kernels take
+// plain pointers: a load from a const __restrict__ parameter counts as constant
+// for the whole kernel and may be moved ahead of the wait.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                               cudaStream_t stream, Args &&...args) {
@@ -508,7 +510,7 @@ struct hg_dem {
   bool inv_valid = false;  // minv matches m0, I0, w and terms_dt
   double terms_dt = 0.0;
   hg::DevBuf<uint8_t> fixed;
-  // broadphase: hash grid of cell width H over the centres, linked lists
+  // broadphase: hash grid of cell width H over the centres (dem_bins.cuh)
   double cell_h = 0.0;
   uint32_t mask = 0; // hash table size - 1 at the capacity
   // per body, 32 bytes: FP32 offset from the home cell, radius, flags; home
@@ -570,6 +572,11 @@ hg_status dem_edit(hg_dem *d, int64_t n_old, const int32_t *old_to_new, int64_t 
 // q_before: receives the positions before the step (3 per body), or nullptr
 hg_status dem_step(hg_dem *d, double dt, int weighted, bool bin_next, double *q_before = nullptr);
 void dem_bodies_changed(hg_dem *d);
+// for a kernel that moves the bodies after a step that binned none: the bins'
+// arguments, and the note that it has filled them
+struct BinArgs;
+void dem_bin_args(const hg_dem *d, BinArgs *out);
+void dem_binned(hg_dem *d);
 void dem_set_launch_shapes(hg_dem *d);
 // per-body terms that dem_step needs and that only change with the bodies
 // or the time step; called before a step is captured into a graph

@@ -5,6 +5,9 @@
 // scan of the tile sums, and a per-tile scan that adds the tile offset. Tiles
 // are read with coalesced 32-bit loads; the whole pass streams the counts
 // twice, which is the floor for a scan that does not fuse into its producer.
+// The kernels are launched with programmatic dependence, so their inputs are
+// plain pointers: a load marked read-only for the whole kernel (const
+// __restrict__) may be moved ahead of the wait for the kernel that writes it.
 #include "hg_internal.cuh"
 #include "scan_block.cuh"
 
@@ -17,8 +20,8 @@ constexpr int SCAN_ITEMS = 8;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 static_assert(SCAN_TILE == SCAN_TILE_ELEMS, "scan_tmp_size assumes this tile size");
 
-__global__ void k_tile_sums(const int32_t *__restrict__ in, int64_t n,
-                            int32_t *__restrict__ sums) {
+__global__ void k_tile_sums(const int32_t *in, int64_t n,
+                            int32_t *sums) {
   // (launched with programmatic dependence on the kernel before it)
   pdl_wait();
   pdl_trigger();
@@ -34,9 +37,9 @@ __global__ void k_tile_sums(const int32_t *__restrict__ in, int64_t n,
   if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
-__global__ void k_tile_scan(const int32_t *__restrict__ in, int64_t n,
-                            const int32_t *__restrict__ tile_off,
-                            int32_t *__restrict__ out) {
+__global__ void k_tile_scan(const int32_t *in, int64_t n,
+                            const int32_t *tile_off,
+                            int32_t *out) {
   // (launched with programmatic dependence on the kernel before it)
   pdl_wait();
   pdl_trigger();
@@ -66,9 +69,9 @@ __global__ void k_tile_scan(const int32_t *__restrict__ in, int64_t n,
 // sums needs no launch of its own.
 constexpr int64_t FUSED_TILES = 2048;
 
-__global__ void k_tile_scan_summed(const int32_t *__restrict__ in, int64_t n,
-                                   const int32_t *__restrict__ sums,
-                                   int32_t *__restrict__ out) {
+__global__ void k_tile_scan_summed(const int32_t *in, int64_t n,
+                                   const int32_t *sums,
+                                   int32_t *out) {
   // (launched with programmatic dependence on the kernel before it)
   pdl_wait();
   pdl_trigger();
@@ -110,7 +113,7 @@ constexpr int SMALL_N = SMALL_THREADS * SMALL_ITEMS;
 static_assert(SMALL_ITEMS % 4 == 0, "runs are read as int4");
 
 __global__ void __launch_bounds__(SMALL_THREADS)
-    k_small_scan(const int32_t *__restrict__ in, int64_t n64, int32_t *__restrict__ out) {
+    k_small_scan(const int32_t *in, int64_t n64, int32_t *out) {
   // (launched with programmatic dependence on the kernel before it)
   pdl_wait();
   pdl_trigger();
