@@ -892,7 +892,7 @@ hg_status hg_mpm_estimate_bytes(const hg_mpm_desc *d, int64_t *bytes) {
     b += nn * (8 + 6 * 16 + 8 + 4 + 8 + 2 * 16); // grid fields, the other accumulators
   } else {
     const bool ugimp = d->basis == HG_BASIS_UGIMP;
-    b += mixed_device_bytes(P.nx, P.ny, cap);
+    b += mixed_device_bytes(P.nx, P.ny, cap, !ugimp);
     if (ugimp) b += 2 * 4 * cap; // per-point half-widths, both buffers
     b += 8 * std::max<int64_t>((ugimp ? 12 : 11) * cap, 5 * nn) + cap; // upload / download staging
   }

@@ -316,9 +316,13 @@ struct hg_mpm {
   hg::DevBuf<float> accm;  // mass accumulated for the next update
   hg::DevBuf<float4> va;   // (vx, vy, ax, ay) of the last update
   hg::DevBuf<float> gm;    // mass of the last update
+  // on small grids: two more sets of (acc4, accm) for kx_step_small
+  hg::DevBuf<float4> small_4[2];
+  hg::DevBuf<float> small_m[2];
   int ntx = 0, nty = 0;    // tiles in x, y
   hg::DevBuf<int32_t> keys, counts, offsets, cursor, scan_tmp;
   hg::DevBuf<int32_t> active_bins, active_tiles, nactive; // nactive[2]
+  hg::DevBuf<int32_t> claimed; // [1]: tiles that CTAs have taken from the list
   hg::DevBuf<uint32_t> outside; // particles outside their window last step
   uint32_t *h_outside = nullptr; // pinned mirror
   cudaEvent_t outside_ev = nullptr;
@@ -393,7 +397,7 @@ hg_status mixed_step(hg_mpm *m, double dt, int nsteps);
 hg_status mixed_download_grid(hg_mpm *m, double *mass, double *vel,
                               double *acc);
 // device bytes mixed_alloc plus the staging of an upload allocate
-int64_t mixed_device_bytes(int nx, int ny, int64_t cap);
+int64_t mixed_device_bytes(int nx, int ny, int64_t cap, bool linear);
 hg_status mixed_autotune(hg_mpm *m, double dt, int steps, hg_tune_report *report);
 hg_status batch_autotune(hg_batch *b, int steps, hg_tune_report *report);
 hg_status mpm_state_bytes(hg_mpm *m, int64_t *bytes);

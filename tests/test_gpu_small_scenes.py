@@ -1,0 +1,122 @@
+"""MIXED linear scenes stepped several steps per call, where one launch does a
+whole step (small scenes) or tiles are cut into strips (a last round that leaves
+CTAs idle): point counts on both sides of each choice, one to sixteen points per
+cell, ragged columns, calls of one step to more than a chunk, re-sorts, points
+that leave their tile's window. Against the FP64 path at the bounds that the
+MIXED path has against the oracle over 20 steps (1e-9 m on positions, 1e-6 on J
+and be_bar, 1e-4 relative on velocities; grid velocities 1e-5 and masses 1e-6
+relative)."""
+import numpy as np
+import pytest
+
+import libhybridgrains_gb300 as hg
+from libhybridgrains_gb300 import scenes
+
+pytestmark = pytest.mark.gpu
+
+H = 5.0e-3
+
+
+def column(wc, hc, ppc, x0, seed=2):
+    """wc x hc cells from column x0, ppc = k^2 points per cell, in motion."""
+    rng = np.random.default_rng(seed)
+    k = int(round(np.sqrt(ppc)))
+    off = (np.arange(k) + 0.5) / k
+    gx, gy = np.meshgrid((np.arange(x0, x0 + wc)[:, None] + off).ravel(),
+                         (np.arange(hc)[:, None] + off).ravel())
+    q = np.stack([gx.ravel(), gy.ravel()], axis=1)
+    n = len(q)
+    q = (q + rng.uniform(-0.2, 0.2, (n, 2)) / k) * H
+    vol = np.full(n, (H / k) ** 2)
+    return dict(q=q, v=rng.normal(0.0, 0.02, (n, 2)), m=1550.0 * vol, vol=vol,
+                hl=np.full(n, 0.5 * H / k))
+
+
+def make(ctx, precision, nx, ny, n, planes=True, stiff=True):
+    mat = scenes.mpm_material()
+    k = 1.0 if stiff else 0.0
+    pl = [((0.0, 0.0), (0.0, 1.0), True, -np.inf), ((nx * H, 0.0), (-1.0, 0.0), False, -np.inf)]
+    return hg.MPM(ctx, (0.0, 0.0), (nx * H, ny * H), H, k * mat["shear_modulus"],
+                  k * mat["bulk_modulus"], mat["dp_alpha"], mat["flip_alpha"], scenes.GRAVITY,
+                  pl if planes else [], precision=precision, capacity=n)
+
+
+def same(a, b, steps_so_far):
+    A, B = a.download(), b.download()
+    assert np.abs(A["q"] - B["q"]).max() <= 1e-9
+    assert np.abs(A["J"] - B["J"]).max() <= 1e-6
+    assert np.abs(A["be"] - B["be"]).max() <= 1e-6
+    assert np.linalg.norm(A["v"] - B["v"]) <= 1e-4 * np.linalg.norm(B["v"])
+    G, F = a.grid(), b.grid()
+    act = F["mass"] > 0
+    assert np.abs(G["mass"] - F["mass"]).max() <= 1e-6 * F["mass"].max()
+    if steps_so_far == 1:
+        d = np.linalg.norm(G["vel"][act] - F["vel"][act])
+        assert d <= 1e-5 * np.linalg.norm(F["vel"][act])
+    assert a.status() == 0 and b.status() == 0
+
+
+# strips of a quarter, of half a tile, whole tiles in a round; points at and
+# above the limit; the two-launch path's quarters, halves, two rounds with a cut
+# second one, and without
+@pytest.mark.parametrize("wc,hc,ppc,x0", [
+    (1, 1, 1, 15), (17, 9, 4, 7), (40, 80, 4, 20), (61, 67, 16, 3), (125, 150, 4, 0),
+    (151, 125, 4, 5), (250, 300, 1, 9), (160, 200, 1, 2), (150, 200, 4, 0), (200, 260, 4, 1),
+    (320, 420, 4, 6), (300, 340, 4, 0)])
+def test_several_steps_per_call_match_fp64(ctx, wc, hc, ppc, x0):
+    p = column(wc, hc, ppc, x0)
+    n = len(p["m"])
+    objs = [make(ctx, prec, x0 + wc + 13, hc + 11, n) for prec in (hg.MIXED, hg.FP64)]
+    for o in objs:
+        o.upload(p["q"], p["v"], p["m"], p["vol"], p["hl"])
+    done = 0
+    for steps in (1, 4, 3, 12):
+        for o in objs:
+            o.flow(2.0e-5, steps)
+        done += steps
+        same(*objs, done)
+
+
+def test_chunks_and_single_steps_mix(ctx):
+    """Chunks, the steps after them, re-sorts in between and single steps, on one
+    object; the same steps one call each on another."""
+    p = column(45, 61, 4, 11)
+    n = len(p["m"])
+    a, b, f = (make(ctx, prec, 96, 80, n) for prec in (hg.MIXED, hg.MIXED, hg.FP64))
+    for o in (a, b, f):
+        o.upload(p["q"], p["v"], p["m"], p["vol"], p["hl"])
+    for steps in (16, 1, 21, 2, 7):
+        a.flow(2.0e-5, steps)
+        f.flow(2.0e-5, steps)
+        for _ in range(steps):
+            b.flow(2.0e-5, 1)
+    A, B, F = (o.download() for o in (a, b, f))
+    for X in (A, B):  # 47 steps: the 20-step bounds, by steps
+        assert np.abs(X["q"] - F["q"]).max() <= 2.5e-9
+        assert np.abs(X["J"] - F["J"]).max() <= 2.5e-6
+        assert np.linalg.norm(X["v"] - F["v"]) <= 2.5e-4 * np.linalg.norm(F["v"])
+    assert a.status() == 0 and b.status() == 0
+
+
+def test_fast_points_leave_their_windows(ctx):
+    """Points without stiffness at 0.2 cells per step, clusters one behind the
+    other in two bands that pass each other: they cross tiles within a chunk, add
+    to nodes outside the active tiles and enter tiles that others have left.
+    Bound: FP32 velocities over 0.2 cells a step."""
+    rng = np.random.default_rng(5)
+    n = 400
+    band = np.arange(n) % 2
+    q = np.stack([0.1 + 0.1 * (np.arange(n) // 2 % 4) + rng.uniform(0.0, 0.02, n),
+                  0.3 + 0.3 * band + rng.uniform(0.0, 0.02, n)], axis=1)
+    q[band == 1, 0] += 0.4
+    v = np.where(band == 0, 1.0, -1.0)[:, None] * np.array([[2.0, 0.0]])
+    m, vol, hl = np.full(n, 1e-3), np.full(n, 1e-6), np.full(n, 1.25e-3)
+    a, f = (make(ctx, prec, 200, 200, n, planes=False, stiff=False)
+            for prec in (hg.MIXED, hg.FP64))
+    for o in (a, f):
+        o.upload(q, v, m, vol, hl)
+        for steps in (40, 9, 32, 16):
+            o.flow(5.0e-4, steps)
+    assert np.abs(a.download()["q"] - f.download()["q"]).max() <= 97 / 40 * 2e-8
+    assert a.status() == 0
+    assert a.rebin_count() >= 2
