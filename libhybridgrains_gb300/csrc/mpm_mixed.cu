@@ -940,59 +940,43 @@ __global__ void __launch_bounds__(THREADS, 3) kb_g2p2g(const MixedArgs *__restri
 // nodes c-1 (f < hl), c, c+1 and c+2 (f > 1 - hl). The kernel below shares
 // the linear path's sorting, active tiles, grid update and chunk graphs.
 
-// Weights and derivatives along one axis of the three nodes b .. b+2 that
-// can carry weight when hl <= 1/2: b = c - 1 for f < 1/2 (node c+2 then has
-// none, |f - 2| >= 1 + hl) and b = c otherwise (node c-1 has none). Each
-// node's offset is f - k as in the reference's stencil over c-1 .. c+2.
-// False if a node of non-zero weight lies outside 0 .. n (the reference's
-// stencil would leave its grid).
-__device__ __forceinline__ bool ugimp_axis(int c, float f, float hl, int n, int &b, float w[3],
-                                           float g[3]) {
-  const int up = f >= 0.5f ? 1 : 0;
-  b = c - 1 + up;
-  // With a = |d|, d = u - x_i, and i2 = 1 / (2 hl) (lin_integral and
-  // lin_integral_grad with unit weight): w = 0 for a >= 1 + hl;
-  // w = (1 + hl - a)^2 i2 / 2, dw/du = -sign(d) (1 + hl - a) i2 for
-  // a >= 1 - hl; w = 2 hl (1 - a) i2, dw/du = -sign(d) 2 hl i2 for a >= hl;
-  // else w = (2 hl - (hl^2 + a^2)) i2, dw/du = -2 d i2. The middle node lies
-  // within 1/2 of the point and the outer two at least 1/2 away (>= hl), so
-  // each takes only the cases it can reach. The cases are selected, not
-  // branched on (the lanes of a warp take different ones).
-  const float i2 = 0.5f / hl, h2 = 2.0f * hl, h2i2 = h2 * i2;
-#pragma unroll
-  for (int m = 0; m < 3; m += 2) {
-    const float d = f - (float)(m - 1 + up);
-    const float a = fabsf(d), sg = d >= 0.0f ? 1.0f : -1.0f;
-    const float t = 1.0f + hl - a;
-    const bool out = a >= 1.0f + hl, edge = a >= 1.0f - hl;
-    w[m] = out ? 0.0f : (edge ? 0.5f * t * t * i2 : (1.0f - a) * h2i2);
-    g[m] = out ? 0.0f : (edge ? -sg * t * i2 : -sg * h2i2);
-  }
-  {
-    const float d = f - (float)up;
-    const float a = fabsf(d), sg = d >= 0.0f ? 1.0f : -1.0f;
-    // (at a = 1 - hl = hl = 1/2 the two cases agree)
-    const bool far = a >= hl;
-    w[1] = far ? (1.0f - a) * h2i2 : (h2 - (hl * hl + a * a)) * i2;
-    g[1] = far ? -sg * h2i2 : -2.0f * d * i2;
-  }
-  if (c >= 1 && c + 2 <= n) return true; // nodes c-1 .. c+2 all on the grid
-  bool ok = true;
-#pragma unroll
-  for (int m = 0; m < 3; ++m) {
-    const int i = b + m;
-    if ((w[m] != 0.0f || g[m] != 0.0f) && (i < 0 || i > n)) ok = false;
-  }
-  return ok;
-}
+// Weights and derivatives along one axis of the three nodes around node c that
+// can carry weight when hl <= 1/2: c is the nearest node, r the point's offset
+// from it, |r| <= 1/2 (the reference's stencil over c-1 .. c+2 of the point's
+// cell has one node more, of weight 0). With i2 = 1 / (2 hl) (lin_integral and
+// lin_integral_grad with unit weight), for a node at distance a: 0 for
+// a >= 1 + hl; (1 + hl - a)^2 i2 / 2 with derivative -+(1 + hl - a) i2 for
+// a >= 1 - hl; 1 - a with -+1 for a >= hl; else (2 hl - (hl^2 + a^2)) i2 with
+// -2 (u - x_i) i2. The middle node lies within 1/2 of the point and the outer
+// two at a = 1 + r and 1 - r, at least 1/2 (>= hl) away, so each takes only the
+// cases it can reach. The cases are selected, not branched on (the lanes of a
+// warp take different ones).
+struct UgimpAxis {
+  int c;
+  float w[3], g[3];
+  bool lo, hi; // nodes c - 1, c + 1 carry weight
 
-// Nodes of a 3-node axis that carry weight or derivative (a node is in the
-// point's support when it does along both axes; outside it, it may lie off
-// the grid)
-__device__ __forceinline__ unsigned ugimp_support(const float w[3], const float g[3]) {
-  return (w[0] != 0.0f || g[0] != 0.0f ? 1u : 0u) | (w[1] != 0.0f || g[1] != 0.0f ? 2u : 0u) |
-         (w[2] != 0.0f || g[2] != 0.0f ? 4u : 0u);
-}
+  // False if a node of non-zero weight lies outside 0 .. n (the reference's
+  // stencil would leave its grid).
+  __device__ __forceinline__ bool set(int cell, float f, float hl, int n) {
+    const bool up = f >= 0.5f;
+    c = cell + (up ? 1 : 0);
+    const float r = up ? f - 1.0f : f, i2 = 0.5f / hl;
+    const float t0 = fmaxf(hl - r, 0.0f), t2 = fmaxf(hl + r, 0.0f); // 1 + hl - a, or 0
+    const float u0 = t0 * i2, u2 = t2 * i2;
+    const bool near0 = r < -hl, near2 = r > hl;
+    w[0] = near0 ? -r : 0.5f * t0 * u0;
+    g[0] = near0 ? -1.0f : -u0;
+    w[2] = near2 ? r : 0.5f * t2 * u2;
+    g[2] = near2 ? 1.0f : u2;
+    const bool far = near0 || near2;
+    w[1] = far ? 1.0f - fabsf(r) : (2.0f * hl - (hl * hl + r * r)) * i2;
+    g[1] = far ? (near0 ? 1.0f : -1.0f) : -2.0f * r * i2;
+    lo = t0 > 0.0f;
+    hi = t2 > 0.0f;
+    return (c > 0 || !lo) && (c < n || !hi);
+  }
+};
 
 // One thread per point, in the sorted order: a warp's points lie in a few
 // neighbouring cells, so its gathers from the grid and its P2G atomics (one
@@ -1003,8 +987,17 @@ __device__ __forceinline__ unsigned ugimp_support(const float w[3], const float 
 // this kernel, with shared-memory G2P and P2G, was slower: five shared
 // atomics per node against two global reductions, at a third of the
 // occupancy.)
+//
+// Bound by the reductions' way out of the SM and by latency: of 33.0 us per
+// step of 611,648 points 6 are the grid update and 12 go with the reductions.
+// 900 instructions per warp and point where the weights took both their cases
+// and the sums were not taken row by row (1,165; 37.7 us). A CTA of 128 per
+// 128 points: 33.0 us, CTAs of 256 that walk the points 36.1 (64 registers
+// instead of 72); 350,556 points 23.0 and 24.0, 110,592 12.0 and 11.3, 6,360
+// 6.7 and 7.3.
+constexpr int UGIMP_THREADS = 128;
 template <bool PRIME>
-__global__ void __launch_bounds__(THREADS) kxu_step(const __grid_constant__ MixedArgs A) {
+__global__ void __launch_bounds__(UGIMP_THREADS) kxu_step(const __grid_constant__ MixedArgs A) {
   // launched with programmatic dependence on the grid update before it
   pdl_wait();
   pdl_trigger();
@@ -1027,36 +1020,34 @@ __global__ void __launch_bounds__(THREADS) kxu_step(const __grid_constant__ Mixe
     split_u(un.y, cy, fy);
     far_edge(A.nx, cx, fx);
     far_edge(A.ny, cy, fy);
-    int bx, by;
-    float wx[3], gx[3], wy[3], gy[3];
-    if (!in_grid_cell(A, cx, cy) || !ugimp_axis(cx, fx, hl, A.nx, bx, wx, gx) ||
-        !ugimp_axis(cy, fy, hl, A.ny, by, wy, gy)) {
+    UgimpAxis X, Y;
+    if (!in_grid_cell(A, cx, cy) || !X.set(cx, fx, hl, A.nx) || !Y.set(cy, fy, hl, A.ny)) {
       atomicOr(A.status, (uint32_t)HG_STATUS_OUT_OF_GRID);
       continue;
     }
     if (!PRIME) {
       // ---- G2P of this step at the start-of-step position ----
+      // row by row; the place of a node without weight is taken by its
+      // neighbour with weight (loaded anyway), its terms are zeros
       float Lxx = 0.f, Lxy = 0.f, Lyx = 0.f, Lyy = 0.f, vpx = 0.f, vpy = 0.f, apx = 0.f,
             apy = 0.f;
-      const unsigned sx = ugimp_support(wx, gx), sy = ugimp_support(wy, gy);
+      const int center = Y.c * row + X.c, left = X.lo ? -1 : 0, right = X.hi ? 1 : 0;
 #pragma unroll
-      for (int ky = 0; ky < 3; ++ky) {
-#pragma unroll
-        for (int kx = 0; kx < 3; ++kx) {
-          if (!((sx >> kx) & (sy >> ky) & 1u)) continue; // outside the support
-          const float w = wx[kx] * wy[ky], dX = gx[kx] * wy[ky], dY = wx[kx] * gy[ky];
-          const int node = (by + ky) * row + (bx + kx); // MIXED grids have < 2^30 nodes
-          if (!HG_INDEX_OK(node, nn, A.status)) continue;
-          const float4 nv = A.va[node];
-          Lxx += nv.x * dX;
-          Lxy += nv.x * dY;
-          Lyx += nv.y * dX;
-          Lyy += nv.y * dY;
-          vpx += w * nv.x;
-          vpy += w * nv.y;
-          apx += w * nv.z;
-          apy += w * nv.w;
-        }
+      for (int k = 0; k < 3; ++k) {
+        const int at = center + (k == 0 ? (Y.lo ? -row : 0) : k == 2 ? (Y.hi ? row : 0) : 0);
+        if (!HG_INDEX_OK(at + left, nn, A.status) || !HG_INDEX_OK(at + right, nn, A.status))
+          continue;
+        const float4 a = A.va[at + left], b = A.va[at], c = A.va[at + right];
+        const float vx = X.w[0] * a.x + X.w[1] * b.x + X.w[2] * c.x;
+        const float vy = X.w[0] * a.y + X.w[1] * b.y + X.w[2] * c.y;
+        Lxx += Y.w[k] * (X.g[0] * a.x + X.g[1] * b.x + X.g[2] * c.x);
+        Lyx += Y.w[k] * (X.g[0] * a.y + X.g[1] * b.y + X.g[2] * c.y);
+        Lxy += Y.g[k] * vx;
+        Lyy += Y.g[k] * vy;
+        vpx += Y.w[k] * vx;
+        vpy += Y.w[k] * vy;
+        apx += Y.w[k] * (X.w[0] * a.z + X.w[1] * b.z + X.w[2] * c.z);
+        apy += Y.w[k] * (X.w[0] * a.w + X.w[1] * b.w + X.w[2] * c.w);
       }
       const float ih = A.inv_h;
       constitutive_update(st, jh, Lxx * ih, Lxy * ih, Lyx * ih, Lyy * ih, A.dt, A.kappa, A.mu,
@@ -1124,8 +1115,8 @@ __global__ void __launch_bounds__(THREADS) kxu_step(const __grid_constant__ Mixe
       A.strain[p] = st;
       A.flags[p] = (uint8_t)((fl & ~1) | jh);
       moved += (ncx != cx) | (ncy != cy);
-      if (!in_grid_cell(A, ncx, ncy) || !ugimp_axis(ncx, nfx, hl, A.nx, bx, wx, gx) ||
-          !ugimp_axis(ncy, nfy, hl, A.ny, by, wy, gy)) {
+      if (!in_grid_cell(A, ncx, ncy) || !X.set(ncx, nfx, hl, A.nx) ||
+          !Y.set(ncy, nfy, hl, A.ny)) {
         atomicOr(A.status, (uint32_t)HG_STATUS_OUT_OF_GRID);
         continue;
       }
@@ -1134,23 +1125,24 @@ __global__ void __launch_bounds__(THREADS) kxu_step(const __grid_constant__ Mixe
     float s00, s01, s11;
     stress_factor(st, jh, mv.y, A.inv_h, A.kappa, A.mu, s00, s01, s11);
     const float mvx = mv.x * vel.x, mvy = mv.x * vel.y;
-    const unsigned sx = ugimp_support(wx, gx), sy = ugimp_support(wy, gy);
+    // (a node of weight 0 is not in the support, so that it gets no force, as
+    // in PhysicsGrid.cpp:439-441)
+    const int center = Y.c * row + X.c; // MIXED grids have < 2^30 nodes
 #pragma unroll
     for (int ky = 0; ky < 3; ++ky) {
+      if (ky == 0 ? !Y.lo : ky == 2 && !Y.hi) continue;
+      const float wy = Y.w[ky], gy = Y.g[ky];
+      const float m = mv.x * wy, px = mvx * wy, py = mvy * wy;
+      const float s00w = s00 * wy, s01g = s01 * gy, s01w = s01 * wy, s11g = s11 * gy;
 #pragma unroll
       for (int kx = 0; kx < 3; ++kx) {
-        if (!((sx >> kx) & (sy >> ky) & 1u)) continue; // outside the support
-        const float w = wx[kx] * wy[ky];
-        const float dX = gx[kx] * wy[ky], dY = wx[kx] * gy[ky];
-        const int node = (by + ky) * row + (bx + kx); // MIXED grids have < 2^30 nodes
+        if (kx == 0 ? !X.lo : kx == 2 && !X.hi) continue;
+        const float wx = X.w[kx], gx = X.g[kx];
+        const int node = center + (ky - 1) * row + (kx - 1);
         if (!HG_INDEX_OK(node, nn, A.status)) continue;
-        float4 add = make_float4(w * mvx, w * mvy, 0.0f, 0.0f);
-        if (w != 0.0f) { // nodes of zero weight get no force (PhysicsGrid.cpp:439-441)
-          add.z = s00 * dX + s01 * dY;
-          add.w = s01 * dX + s11 * dY;
-        }
-        atomicAdd(&A.accm[node], w * mv.x);
-        atomicAdd(&A.acc4[node], add);
+        atomicAdd(&A.accm[node], m * wx);
+        atomicAdd(&A.acc4[node],
+                  make_float4(px * wx, py * wx, s00w * gx + s01g * wx, s01w * gx + s11g * wx));
       }
     }
   }
@@ -1889,16 +1881,12 @@ int update_per_sm(const hg_launch_shape &s) {
   return s.update_ctas_per_sm > 0 ? s.update_ctas_per_sm : DEFAULT_UPDATE_CTAS;
 }
 int fused_blocks(hg_mpm *m) { return m->ctx->num_sms * fused_per_sm(m->shape); }
-// the uGIMP kernel walks the points: up to 8 CTAs per SM
-int ugimp_blocks(hg_mpm *m) {
-  const int64_t b = (m->n + THREADS - 1) / THREADS;
-  return (int)std::max<int64_t>(1, std::min<int64_t>(b, (int64_t)m->ctx->num_sms * 8));
-}
+int ugimp_blocks(hg_mpm *m) { return blocks_for(std::max<int64_t>(m->n, 1), UGIMP_THREADS); }
 // G2P of this step fused with P2G of the next (or the first P2G, PRIME)
 template <bool PRIME>
 void launch_particle_kernel(hg_mpm *m, const MixedArgs &A, cudaStream_t s) {
   if (m->p.basis == HG_BASIS_UGIMP) {
-    HG_LAUNCH_PDL(kxu_step<PRIME>, ugimp_blocks(m), THREADS, 0, s, A);
+    HG_LAUNCH_PDL(kxu_step<PRIME>, ugimp_blocks(m), UGIMP_THREADS, 0, s, A);
   } else {
     HG_LAUNCH_PDL(kx_g2p2g<PRIME>, fused_blocks(m), THREADS, fused_smem_bytes(), s, A);
   }

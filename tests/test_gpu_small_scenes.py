@@ -120,3 +120,44 @@ def test_fast_points_leave_their_windows(ctx):
     assert np.abs(a.download()["q"] - f.download()["q"]).max() <= 97 / 40 * 2e-8
     assert a.status() == 0
     assert a.rebin_count() >= 2
+
+
+@pytest.mark.parametrize("n", [1, 127, 129, 4001])
+@pytest.mark.parametrize("hl", [0.03, 0.25, 0.4375, 0.5])
+def test_ugimp_weights_at_their_joints_match_fp64(ctx, n, hl):
+    """MIXED with the uGIMP basis on both sides of where a node's weight changes
+    its form (points about +-hl and half-way around a node, on nodes) and at the
+    first and last node that a point may touch, against the FP64 path: masses
+    and momenta 1e-6 of the largest, positions 1e-12 m after one step and J 1e-6
+    (the MIXED path's bounds for one step)."""
+    rng = np.random.default_rng(8)
+    # (not on +-hl: whether a node of weight 0 there is touched is rounding, and
+    # what it adds to the gradient, force over mass, does not go to 0 with it)
+    near = hl + np.array([-1e-2, 1e-2])
+    joints = np.concatenate([[0.0, 0.5, -0.5, 0.5 * hl, 0.3], near, -near])
+    lo, hi = 1, 39  # nodes whose neighbours are on the 40-cell grid
+    u = rng.integers(lo, hi + 1, (n, 2)) + joints[rng.integers(0, len(joints), (n, 2))]
+    u = np.clip(u, hl + 1e-3, 40.0 - hl - 1e-3)  # no point moves off the grid
+    q = u * H
+    vol = np.full(n, (2.0 * hl * H) ** 2)
+    e = rng.uniform(-0.01, 0.0, n)
+    be = np.stack([1.0 + e, np.zeros(n), np.zeros(n), 1.0 / (1.0 + e)], axis=1)
+    p = dict(q=q, v=rng.normal(0.0, 0.1, (n, 2)), m=1550.0 * vol, vol=vol,
+             hl=np.full(n, hl * H), be=be, J=1.0 + rng.uniform(-0.01, 0.0, n))
+    mat = scenes.mpm_material()
+    out = []
+    for prec in (hg.MIXED, hg.FP64):
+        o = hg.MPM(ctx, (0.0, 0.0), (40 * H, 40 * H), H, mat["shear_modulus"],
+                   mat["bulk_modulus"], mat["dp_alpha"], mat["flip_alpha"], scenes.GRAVITY, [],
+                   basis=hg.UGIMP, precision=prec, capacity=n)
+        o.upload(p["q"], p["v"], p["m"], p["vol"], p["hl"], p["be"], p["J"])
+        o.flow(1.0e-6, 1)
+        assert o.status() == 0
+        out.append((o.download(), o.grid()))
+    (A, G), (B, F) = out
+    assert np.abs(A["q"] - B["q"]).max() <= 1e-12
+    assert np.abs(A["J"] - B["J"]).max() <= 1e-6
+    assert np.abs(A["be"] - B["be"]).max() <= 1e-6
+    assert np.abs(G["mass"] - F["mass"]).max() <= 1e-6 * F["mass"].max()
+    for a, b in ((G["mass"][:, None] * G["vel"], F["mass"][:, None] * F["vel"]),):
+        assert np.abs(a - b).max() <= 1e-6 * np.abs(b).max() + 1e-6 * F["mass"].max() * 0.1
