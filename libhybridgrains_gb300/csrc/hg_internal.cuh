@@ -320,6 +320,7 @@ struct hg_mpm {
   hg::DevBuf<float4> small_4[2];
   hg::DevBuf<float> small_m[2];
   int ntx = 0, nty = 0;    // tiles in x, y
+  // (cursor: per key in a batched re-sort, else per point, its rank)
   hg::DevBuf<int32_t> keys, counts, offsets, cursor, scan_tmp;
   hg::DevBuf<int32_t> active_bins, active_tiles, nactive; // nactive[2]
   hg::DevBuf<int32_t> claimed; // [1]: tiles that CTAs have taken from the list

@@ -80,21 +80,45 @@ __global__ void k_tile_scan_summed(const int32_t *in, int64_t n,
   int tile_off;
   block_excl_scan<SCAN_THREADS>(before, &tile_off);
   const int64_t base = (int64_t)blockIdx.x * SCAN_TILE;
+  const int64_t first = base + (int64_t)threadIdx.x * SCAN_ITEMS;
+  // a thread's run in 16-byte words where it lies on them
+  static_assert(SCAN_ITEMS % 4 == 0, "runs are whole words");
+  const bool words =
+      ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0 &&
+      first + SCAN_ITEMS <= n;
   int v[SCAN_ITEMS];
   int s = 0;
+  if (words) {
 #pragma unroll
-  for (int k = 0; k < SCAN_ITEMS; ++k) {
-    const int64_t i = base + (int64_t)threadIdx.x * SCAN_ITEMS + k;
-    v[k] = i < n ? in[i] : 0;
-    s += v[k];
+    for (int k = 0; k < SCAN_ITEMS; k += 4) {
+      const int4 q = *reinterpret_cast<const int4 *>(in + first + k);
+      v[k] = q.x;
+      v[k + 1] = q.y;
+      v[k + 2] = q.z;
+      v[k + 3] = q.w;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < SCAN_ITEMS; ++k) v[k] = first + k < n ? in[first + k] : 0;
   }
+#pragma unroll
+  for (int k = 0; k < SCAN_ITEMS; ++k) s += v[k];
   int total;
   int run = block_excl_scan<SCAN_THREADS>(s, &total) + tile_off;
 #pragma unroll
   for (int k = 0; k < SCAN_ITEMS; ++k) {
-    const int64_t i = base + (int64_t)threadIdx.x * SCAN_ITEMS + k;
-    if (i < n) out[i] = run;
-    run += v[k];
+    const int c = v[k];
+    v[k] = run;
+    run += c;
+  }
+  if (words) {
+#pragma unroll
+    for (int k = 0; k < SCAN_ITEMS; k += 4)
+      *reinterpret_cast<int4 *>(out + first + k) = make_int4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < SCAN_ITEMS; ++k)
+      if (first + k < n) out[first + k] = v[k];
   }
 }
 

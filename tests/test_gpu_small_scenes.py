@@ -1,4 +1,4 @@
-"""MIXED linear scenes stepped several steps per call, where one launch does a
+"""MIXED scenes stepped several steps per call, where one launch does a
 whole step (small scenes) or tiles are cut into strips (a last round that leaves
 CTAs idle): point counts on both sides of each choice, one to sixteen points per
 cell, ragged columns, calls of one step to more than a chunk, re-sorts, points
@@ -161,3 +161,62 @@ def test_ugimp_weights_at_their_joints_match_fp64(ctx, n, hl):
     assert np.abs(G["mass"] - F["mass"]).max() <= 1e-6 * F["mass"].max()
     for a, b in ((G["mass"][:, None] * G["vel"], F["mass"][:, None] * F["vel"]),):
         assert np.abs(a - b).max() <= 1e-6 * np.abs(b).max() + 1e-6 * F["mass"].max() * 0.1
+
+
+def plain(ctx, precision, n, nx=41, ny=37):
+    return hg.MPM(ctx, (0.0, 0.0), (nx * H, ny * H), H, 1.0e3, 1.0e3, 0.0, 0.95, scenes.GRAVITY,
+                  [], precision=precision, capacity=max(n, 1))
+
+
+@pytest.mark.parametrize("n", [1, 5, 257, 5000])
+def test_sort_keys_at_the_grid_edges(ctx, n):
+    """Points on cell lines, on the grid's far edges (which belong to the last
+    cell), in its first column and next to lines by one unit in the last place:
+    the masses that the first step rasterises are those of the bilinear weights
+    (1e-6 of the largest)."""
+    rng = np.random.default_rng(3)
+    x = np.concatenate([[0.0, 41.0, 1.0, 16.0, 40.0], 41.0 * rng.random(n)])[:n]
+    y = np.concatenate([[37.0, 37.0, 0.0, 16.0, 32.0], 37.0 * rng.random(n)])[:n]
+    k = rng.random((2, n)) < 0.3
+    x, y = np.where(k[0], np.round(x), x), np.where(k[1], np.round(y), y)
+    k = rng.random((2, n)) < 0.2
+    x, y = np.where(k[0], np.nextafter(x, 0.0), x), np.where(k[1], np.nextafter(y, 0.0), y)
+    q = np.minimum(np.stack([x, y], axis=1) * H, [41 * H, 37 * H])
+    m = rng.uniform(1.0, 2.0, n)
+    o = plain(ctx, hg.MIXED, n)
+    o.upload(q, np.zeros((n, 2)), m, np.full(n, 1e-6), np.full(n, 0.25 * H))
+    assert np.abs(o.download()["q"] - q).max() <= 1e-12  # the scatter keeps every point's place
+    assert o.status() == 0  # (the step takes the points on the low edge off the grid)
+    o.flow(1e-9, 1)
+    u = q / H
+    c = np.minimum(np.floor(u).astype(int), [40, 36])
+    f = u - c
+    mass = np.zeros((38, 42))
+    for dx in (0, 1):
+        for dy in (0, 1):
+            w = (f[:, 0] if dx else 1.0 - f[:, 0]) * (f[:, 1] if dy else 1.0 - f[:, 1])
+            np.add.at(mass, (c[:, 1] + dy, c[:, 0] + dx), w * m)
+    got = np.asarray(o.grid()["mass"]).reshape(38, 42)
+    assert np.abs(got - mass).max() <= 1e-6 * mass.max()
+
+
+@pytest.mark.parametrize("bad", [-1e-3, 42.0, np.nan, np.inf, -np.inf, 1e300])
+def test_points_off_the_grid_are_reported(ctx, bad):
+    q = np.full((40, 2), 5.5 * H)
+    q[17, 1] = bad * H
+    o = plain(ctx, hg.MIXED, 40)
+    o.upload(q, np.zeros((40, 2)), np.ones(40), np.full(40, 1e-6), np.full(40, 0.25 * H))
+    assert o.status() & 2
+
+
+def test_tiles_that_drop_out_are_cleared(ctx):
+    n = 300
+    rng = np.random.default_rng(4)
+    o = plain(ctx, hg.MIXED, n, 200, 100)
+    for x0 in (3.0, 150.0, 60.0):
+        q = (rng.random((n, 2)) * 10.0 + [x0, 40.0]) * H
+        o.upload(q, np.zeros((n, 2)), np.ones(n), np.full(n, 1e-6), np.full(n, 0.25 * H))
+        o.flow(1e-9, 17)
+        mass = np.asarray(o.grid()["mass"]).reshape(101, 201)
+        assert abs(mass.sum() - n) <= 1e-5 * n
+        assert np.all(mass[:, : int(x0)] == 0.0) and np.all(mass[:, int(x0) + 12:] == 0.0)
