@@ -890,6 +890,10 @@ __device__ __forceinline__ void queue_done(int32_t *q) {
 // Drains the queue: tile(A, tile index) for every claimed item, the scene's
 // arguments copied into A whenever the item's scene changes. The next chunk
 // is claimed while this one runs.
+// The kernels are launched with programmatic dependence after a chunk's first
+// one: queue, tables and tile lists are older than the launch before, and are
+// read under its end (a step of 48 scenes of 2,000 to 200,000 points 74.7 us,
+// after ordinary launches 76.7).
 template <class F>
 __device__ __forceinline__ void drain_queue(const MixedArgs *slots, int nslots, const int *prefix,
                                             int32_t *q, MixedArgs &A, F &&tile) {
@@ -907,19 +911,25 @@ __device__ __forceinline__ void drain_queue(const MixedArgs *slots, int nslots, 
     const int end = min(c.x + c.y, total);
     for (int item = c.x; item < end; ++item) {
       if (s < 0 || item >= prefix[s + 1] || item < prefix[s]) {
+        const bool first = s < 0;
         s = batch_slot(prefix, nslots, item);
         load_slot(slots, s, A);
+        if (first) {
+          pdl_wait();
+          pdl_trigger();
+        }
       }
       tile(A, A.active[item - prefix[s]]);
     }
   }
+  pdl_wait();
   queue_done(q);
 }
 
 
 // All scenes of a batch in one launch: the CTAs drain (scene, tile) items.
-__global__ void __launch_bounds__(THREADS, 3) kb_g2p2g(const MixedArgs *__restrict__ slots,
-                                                     int nslots, int32_t *queue) {
+__global__ void __launch_bounds__(THREADS, 3) kb_g2p2g(const MixedArgs *slots,
+                                                       int nslots, int32_t *queue) {
   __shared__ FusedSmem<BIN> S;
   __shared__ MixedArgs A;
   __shared__ int prefix[PREFIX_LEN];
@@ -1180,7 +1190,7 @@ __global__ void __launch_bounds__(THREADS) kx_grid_update(const __grid_constant_
   }
 }
 
-__global__ void __launch_bounds__(THREADS) kb_grid_update(const MixedArgs *__restrict__ slots,
+__global__ void __launch_bounds__(THREADS) kb_grid_update(const MixedArgs *slots,
                                                           int nslots, int32_t *queue) {
   __shared__ MixedArgs A;
   __shared__ int prefix[PREFIX_LEN];
@@ -2447,8 +2457,11 @@ hg_status batch_chunk_graph(hg_batch *b, int S) {
   HG_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   hg_status st = HG_OK;
   for (int k = 0; k < CHUNK_STEPS && st == HG_OK; ++k) {
-    HG_LAUNCH(kb_grid_update, gu, THREADS, 0, s, dt, S, b->queue.p + 2);
-    HG_LAUNCH(kb_g2p2g, gf, THREADS, 0, s, db, S, b->queue.p);
+    if (k == 0) // (it reads the tables before its wait)
+      HG_LAUNCH(kb_grid_update, gu, THREADS, 0, s, dt, S, b->queue.p + 2);
+    else
+      HG_LAUNCH_PDL(kb_grid_update, gu, THREADS, 0, s, dt, S, b->queue.p + 2);
+    HG_LAUNCH_PDL(kb_g2p2g, gf, THREADS, 0, s, db, S, b->queue.p);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) st = cuda_fail(e, "kernel launch");
   }
@@ -2593,7 +2606,7 @@ hg_status batch_step(hg_batch *b, int nsteps) {
               b->queue.p + 2);
     HG_CHECK_LAUNCH();
     if (b->profile) HG_CUDA_TRY(cudaEventRecord(ev[3], s));
-    HG_LAUNCH(kb_g2p2g, nsm * fused_per_sm(b->shape), THREADS, 0, s, db, S, b->queue.p);
+    HG_LAUNCH_PDL(kb_g2p2g, nsm * fused_per_sm(b->shape), THREADS, 0, s, db, S, b->queue.p);
     HG_CHECK_LAUNCH();
     if (b->profile) HG_CUDA_TRY(cudaEventRecord(ev[4], s));
     for (hg_mpm *m : b->members) m->steps_since_rebin++;
