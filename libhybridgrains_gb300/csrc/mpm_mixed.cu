@@ -972,7 +972,12 @@ struct UgimpAxis {
     const bool up = f >= 0.5f;
     c = cell + (up ? 1 : 0);
     const float r = up ? f - 1.0f : f, i2 = 0.5f / hl;
-    const float t0 = fmaxf(hl - r, 0.0f), t2 = fmaxf(hl + r, 0.0f); // 1 + hl - a, or 0
+    // 1 + hl - a, or 0. (Not hl -+ r: rounded as here, points on the joint
+    // fall on the same side from step to step. A node that takes a weight of
+    // rounding size there adds force over mass to the point's gradient, which
+    // does not vanish with the weight.)
+    const float a0 = 1.0f + r, a2 = 1.0f - r;
+    const float t0 = fmaxf((1.0f + hl) - a0, 0.0f), t2 = fmaxf((1.0f + hl) - a2, 0.0f);
     const float u0 = t0 * i2, u2 = t2 * i2;
     const bool near0 = r < -hl, near2 = r > hl;
     w[0] = near0 ? -r : 0.5f * t0 * u0;
@@ -998,12 +1003,12 @@ struct UgimpAxis {
 // atomics per node against two global reductions, at a third of the
 // occupancy.)
 //
-// Bound by the reductions' way out of the SM and by latency: of 33.0 us per
+// Bound by the reductions' way out of the SM and by latency: of 33.5 us per
 // step of 611,648 points 6 are the grid update and 12 go with the reductions.
 // 900 instructions per warp and point where the weights took both their cases
 // and the sums were not taken row by row (1,165; 37.7 us). A CTA of 128 per
-// 128 points: 33.0 us, CTAs of 256 that walk the points 36.1 (64 registers
-// instead of 72); 350,556 points 23.0 and 24.0, 110,592 12.0 and 11.3, 6,360
+// 128 points: 33.5 us, CTAs of 256 that walk the points 36.1 (64 registers
+// instead of 72); 350,556 points 23.5 and 24.0, 110,592 12.0 and 11.3, 6,360
 // 6.7 and 7.3.
 constexpr int UGIMP_THREADS = 128;
 template <bool PRIME>
