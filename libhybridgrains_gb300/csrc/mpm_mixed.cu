@@ -27,12 +27,13 @@
 // itself rather than on the leading 1. Grid fields are dense node-major
 // float4/float arrays; only tiles near particles are touched.
 //
-// P2G is cell-major: one thread per cell accumulates the contributions of the
-// points sorted into its cell in registers (no atomics); points that left
-// their cell since the last re-sort use shared-memory atomics on the tile's
-// node window. Window sums go to global memory with one float4 + one float
-// atomic per touched node. With the uGIMP basis (up to 3 x 3 nodes per point)
-// one thread per point adds to the grid with global reductions.
+// P2G is cell-major: each point's contribution is staged in shared memory, and
+// one thread per cell adds those of the points sorted into its cell up in
+// registers (no atomics); points that left their cell since the last re-sort
+// use shared-memory atomics on the tile's node window. Window sums go to global
+// memory with one float4 + one float atomic per touched node. With the uGIMP
+// basis (up to 3 x 3 nodes per point) one thread per point adds to the grid with
+// global reductions.
 //
 // Re-sorting (counting sort by cell key) runs when a point has drifted out of
 // its tile's window, when more than 1/32 of the points have left their sorted
@@ -109,13 +110,13 @@ __device__ __noinline__ int2 split_u_slow(double u) {
 __device__ __forceinline__ void split_u(double u, int &c, float &f) {
   // 32-bit word operations only: hi = sign | exponent | mantissa[51:32]
   const unsigned hi = (unsigned)__double2hiint(u), lo = (unsigned)__double2loint(u);
-  const int e = (int)(hi >> 20) - 1023; // sign bit set gives e >= 1025
-  if (e >= 0 && e < 23) {
-    const unsigned hf = (hi & 0xFFFFFu) | 0x100000u; // 21 leading mantissa bits
-    const int sh = 52 - e;                            // 30..52
-    c = sh >= 32 ? (int)(hf >> (sh - 32)) : (int)__funnelshift_r(lo, hf, sh);
-    const unsigned f24 = __funnelshift_r(lo, hf, sh - 24) & 0xFFFFFFu;
-    f = (float)f24 * (1.0f / 16777216.0f);
+  const unsigned e = hi >> 20; // sign and exponent: 1023 .. 1045 for 1 <= u < 2^23
+  if (e - 1023u < 23u) {
+    // the mantissa with its leading 1 at bit 63; shifts take their amount
+    // modulo 32
+    const unsigned m1 = __funnelshift_l(lo, hi, 11) | 0x80000000u, m0 = lo << 11;
+    c = (int)__funnelshift_r(m1, 0u, 30u - e);                 // the upper e - 1022 bits
+    f = (float)(__funnelshift_l(m0, m1, e + 2u) >> 8) * (1.0f / 16777216.0f); // the next 24
   } else {
     const int2 s = split_u_slow(u);
     c = s.x;
@@ -230,22 +231,34 @@ __device__ __forceinline__ void scatter_global(const MixedArgs &A, int cx, int c
 // Adds the P2G contribution of one material point at cell (cx, cy) with
 // fractions (fx, fy) to 4 corner accumulators a[corner * 5 + {m, px, py, fx, fy}]
 // (corner = dx + 2 dy). The internal force is skipped where the weight is
-// zero, like PhysicsGrid::computeForces (PhysicsGrid.cpp:439-441).
+// zero, like PhysicsGrid::computeForces (PhysicsGrid.cpp:439-441, 443-445):
+// only for a point on a line of the grid.
 __device__ __forceinline__ void p2g_corners(const PRec &r, float *a) {
+  const float wx1 = r.a.x, wx0 = 1.0f - wx1, wy1 = r.a.y, wy0 = 1.0f - wy1;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    const int dx = k & 1, dy = k >> 1;
-    const float wx = dx ? r.a.x : 1.0f - r.a.x;
-    const float wy = dy ? r.a.y : 1.0f - r.a.y;
-    const float w = wx * wy;
+    const float w = (k & 1 ? wx1 : wx0) * (k >> 1 ? wy1 : wy0);
     a[5 * k + 0] += w * r.a.z;
     a[5 * k + 1] += w * r.a.w;
     a[5 * k + 2] += w * r.b.x;
-    // nodes of zero weight get no force (PhysicsGrid.cpp:443-445)
-    const bool on = w != 0.0f;
-    const float gx = on ? (dx ? wy : -wy) : 0.0f, gy = on ? (dy ? wx : -wx) : 0.0f;
-    a[5 * k + 3] += r.b.y * gx + r.b.z * gy;
-    a[5 * k + 4] += r.b.z * gx + r.b.w * gy;
+  }
+  if ((wx0 * wx1) * (wy0 * wy1) != 0.0f) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float gx = k & 1 ? (k >> 1 ? wy1 : wy0) : -(k >> 1 ? wy1 : wy0);
+      const float gy = k >> 1 ? (k & 1 ? wx1 : wx0) : -(k & 1 ? wx1 : wx0);
+      a[5 * k + 3] += r.b.y * gx + r.b.z * gy;
+      a[5 * k + 4] += r.b.z * gx + r.b.w * gy;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float wx = k & 1 ? wx1 : wx0, wy = k >> 1 ? wy1 : wy0;
+      const bool on = wx * wy != 0.0f;
+      const float gx = on ? (k & 1 ? wy : -wy) : 0.0f, gy = on ? (k >> 1 ? wx : -wx) : 0.0f;
+      a[5 * k + 3] += r.b.y * gx + r.b.z * gy;
+      a[5 * k + 4] += r.b.z * gx + r.b.w * gy;
+    }
   }
 }
 
@@ -302,52 +315,87 @@ __device__ __forceinline__ bool node_behind_plane(const MixedArgs &A, const MpmP
   return !(d > 0 && d <= 0x7FF0000000000000ll);
 }
 
-// Cell-major fused kernel. A CTA owns one tile of BIN x BIN cells at a time
-// (or a strip of its rows) and a thread (or a few) owns one cell: it updates
-// the material points sorted into that cell (G2P of this step) and accumulates
-// their P2G contributions for the next step in registers, per corner node of
-// the cell. Points that have left
+// Fused kernel over tiles. A CTA owns one tile of BIN x BIN cells at a time (or
+// a strip of its rows). Its threads take the tile's points in turn: G2P of this
+// step, the new state, and the P2G contribution for the next step as a record
+// in shared memory. Then a thread (or a few) per cell adds the records of its
+// points up in registers, per corner node of the cell. Points that have left
 // their cell since the last re-sort go through shared-memory atomics on the
 // tile's node window (or global atomics outside it). Corner sums are combined
 // per node through shared memory and flushed with one global atomic per node
 // and field.
-// (rows: of the highest strip)
-template <int ROWS> struct FusedSmem {
+//
+// Taking the points, not the cells, in turn keeps a warp's lanes equally busy
+// (four points per cell on average are up to nine in the fullest of 32 cells),
+// reads and writes them coalesced, and keeps the 20 sums out of the way of the
+// constitutive update: 64 registers and four CTAs per SM instead of 80 and
+// three. 2,000,000 points right after seeding 66.5 -> 61.0 us per step, late in
+// a collapse 77 -> 68; 48 scenes 74.7 -> 59.7 and 93 -> 74.
+//
+// CAP: points per pass; a tile of 4 points per cell (1,024) is one pass, and a
+// tile with more is flushed once per pass. (Passes of 512 with the corner sums
+// beside the records 65.3 where one of 1,152 took 62.9; of 256 in two buffers,
+// so that a pass is added up under the next one, 72.)
+template <int CAP> struct FusedSmem {
   static constexpr int VW = BIN + 2 * DRIFT + 1; // G2P node window
   static constexpr int AW = BIN + 2 * DRIFT + 3; // P2G node window
-  float4 va[VW * (ROWS + 2 * DRIFT + 1)];
-  float slow[5][AW * (ROWS + 2 * DRIFT + 3)];
-  float corner[20][BIN * ROWS];
-  unsigned out[2]; // left the tile window / left the sorted cell
-  int claimed;     // the number that the CTA drew
+  float4 va[VW * VW];
+  float slow[5][AW * AW];
+  union {
+    float corner[20][BIN_CELLS];
+    float4 rec[2][CAP]; // the pass's points (rec_slot); zeros for one that moved
+  };
+  uint8_t cell[CAP]; // their cells in the strip
+  unsigned out[2];   // left the tile window / left the sorted cell
+  int claimed;       // the number that the CTA drew
 };
+
+// as many as four CTAs per SM have room for (a batch's also hold the scene's
+// arguments and the prefix of the scenes' tiles)
+constexpr int PASS_POINTS = 1152, BATCH_PASS_POINTS = 1024;
+static_assert(4 * (sizeof(FusedSmem<PASS_POINTS>) + 16 + 1024) <= 228 * 1024, "shared memory");
+
+// Slot of point i of a pass: points four apart, which neighbouring cells read
+// together, lie in different banks.
+__device__ __forceinline__ int rec_slot(int i) { return i ^ ((i >> 3) & 3); }
 
 // One of the 2^split strips of a tile: BIN >> split rows of cells, 2^split
 // threads per cell.
 struct Strip {
   int tile, split, sy; // sy: its first row in the tile
-  int2 points;         // of the thread's cell
+  int2 all, points;    // its points, those of the thread's cell
 };
 
 __device__ __forceinline__ Strip strip_of(const MixedArgs &A, int tile, int split, int sub) {
-  Strip s = {tile, split, sub * (BIN >> split), make_int2(0, 0)};
+  Strip s = {tile, split, sub * (BIN >> split), make_int2(0, 0), make_int2(0, 0)};
   if (!HG_INDEX_OK(tile, (int64_t)A.ntx * A.nty, A.status)) return s;
-  const int key = tile * BIN_CELLS + sub * (BIN_CELLS >> split) + ((int)threadIdx.x >> split);
+  const int cells = BIN_CELLS >> split, key0 = tile * BIN_CELLS + sub * cells;
+  const int key = key0 + ((int)threadIdx.x >> split);
   const int2 r = make_int2(A.offsets[key], A.offsets[key + 1]);
-  if (HG_INDEX_OK(r.x, (int64_t)A.n + 1, A.status) && HG_INDEX_OK(r.y, (int64_t)A.n + 1, A.status))
+  const int2 all = make_int2(A.offsets[key0], A.offsets[key0 + cells]);
+  if (HG_INDEX_OK(all.x, (int64_t)A.n + 1, A.status) &&
+      HG_INDEX_OK(all.y, (int64_t)A.n + 1, A.status) &&
+      HG_INDEX_OK(r.x - all.x, (int64_t)all.y - all.x + 1, A.status) &&
+      HG_INDEX_OK(r.y - all.x, (int64_t)all.y - all.x + 1, A.status)) {
     s.points = r;
+    s.all = all;
+  }
   return s;
 }
 
 // One strip of one scene; A lives in shared memory or the constant bank.
 // nodes: where a grid node's velocity and acceleration come from. claim: a
-// counter that the CTA draws S.claimed from on the way.
-template <bool PRIME, int ROWS, class N>
+// counter that the CTA draws S.claimed from on the way. AHEAD: a point's state
+// is loaded while the one before it is processed, after that one's window
+// reads (before them its 13 registers spilled: 64.0 us), the first one's under
+// the window loads: 61.0 us, without 66. With the arguments in shared memory,
+// as in a batch, they would spill: 72.0 us, without 59.6.
+template <bool PRIME, bool AHEAD, int CAP, class N>
 __device__ __forceinline__ void fused_strip(const MixedArgs &A, const Strip &strip,
-                                            FusedSmem<ROWS> &S, const N nodes,
+                                            FusedSmem<CAP> &S, const N nodes,
                                             int32_t *claim = nullptr) {
   static_assert(THREADS == BIN_CELLS, "a whole tile has one thread per cell");
-  constexpr int VA_W = FusedSmem<ROWS>::VW, ACC_W = FusedSmem<ROWS>::AW;
+  constexpr int VA_W = FusedSmem<CAP>::VW, ACC_W = FusedSmem<CAP>::AW;
   const int split = strip.split, lanes = 1 << split, rows = BIN >> split;
   float4 *s_va = S.va;
   auto &s_slow = S.slow;
@@ -355,27 +403,11 @@ __device__ __forceinline__ void fused_strip(const MixedArgs &A, const Strip &str
   unsigned *s_out = S.out;
   const int tid = threadIdx.x;
   const int row = A.nx + 1;
-  const int cell = tid >> split, lcx = cell % BIN, lcy = cell / BIN;
+  const int cell = tid >> split;
   {
     const int X0 = (strip.tile % A.ntx) * BIN;
     const int Y0 = (strip.tile / A.ntx) * BIN + strip.sy;
     const int WX = X0 - DRIFT - 1, WY = Y0 - DRIFT - 1; // P2G window origin (node)
-    const int ps = strip.points.x + (tid & (lanes - 1)), pe = strip.points.y;
-    // the next point's state is loaded while the current one is processed;
-    // the first one's before the barrier, under the window loads
-    double2 nu = make_double2(0.0, 0.0);
-    float2 nmv = make_float2(0.f, 0.f), nvel = make_float2(0.f, 0.f);
-    float4 nst = make_float4(0.f, 0.f, 0.f, 0.f);
-    int nfl = 0;
-    const auto first = [&]() {
-      if (ps < pe) {
-        nu = A.u[ps];
-        nmv = A.mv[ps];
-        nvel = A.v[ps];
-        nst = A.strain[ps];
-        nfl = A.flags[ps];
-      }
-    };
     if (!PRIME) {
       for (int k = tid; k < VA_W * (rows + 2 * DRIFT + 1); k += THREADS) {
         const int ix = X0 - DRIFT + k % VA_W, iy = Y0 - DRIFT + k / VA_W;
@@ -387,7 +419,6 @@ __device__ __forceinline__ void fused_strip(const MixedArgs &A, const Strip &str
     // s_slow is zero here: zeroed at kernel start and by the previous
     // tile's flush
     if (tid < 2) s_out[tid] = 0;
-    const int gcx = X0 + lcx, gcy = Y0 + lcy;
     // Planes that can touch a point of this tile's window: the window corners
     // bound every position a point of the tile can take this step.
     unsigned plane_mask = 0;
@@ -401,226 +432,258 @@ __device__ __forceinline__ void fused_strip(const MixedArgs &A, const Strip &str
                                pl.fn[0] * (x1 - pl.fux[0]) + pl.fn[1] * (y1 - pl.fux[1])));
       if (dmin <= 2.0f * A.pmargin && y1 >= pl.fulb - A.pmargin) plane_mask |= 1u << k;
     }
-    first();
-    __syncthreads();
-    float acc[20];
-#pragma unroll
-    for (int k = 0; k < 20; ++k) acc[k] = 0.f;
-    // per-thread counters and flags, published once after the loop
+    // A pass: the threads that own cells name their points' cells; every thread
+    // takes points in turn; the owners add their cells' records up.
     unsigned left_window = 0, left_cell = 0;
     bool nonfinite = false;
-    for (int p = ps; p < pe; p += lanes) {
-      const double2 u = nu;
-      const float2 mv = nmv;
-      float2 vel = nvel;
-      float4 st = nst;
-      const int fl = nfl;
-      if (p + lanes < pe) { // (an unconditional reload of the last point was slower)
-        nu = A.u[p + lanes];
-        nmv = A.mv[p + lanes];
-        nvel = A.v[p + lanes];
-        nst = A.strain[p + lanes];
-        nfl = A.flags[p + lanes];
-      }
-      int cx, cy;
-      float fx, fy;
-      split_u(u.x, cx, fx);
-      split_u(u.y, cy, fy);
-      if (!in_grid_cell(A, cx, cy)) { // the grid's far edge, or outside it
-        far_edge(A.nx, cx, fx);
-        far_edge(A.ny, cy, fy);
-        if (!in_grid_cell(A, cx, cy)) {
+    for (int base = strip.all.x; base == strip.all.x || base < strip.all.y; base += CAP) {
+      const int m = min(CAP, strip.all.y - base);
+      const int p0 = max(strip.points.x, base) - base, p1 = min(strip.points.y - base, m);
+      for (int i = p0 + (tid & (lanes - 1)); i < p1; i += lanes) S.cell[i] = (uint8_t)cell;
+      double2 nu = make_double2(0.0, 0.0);
+      float2 nmv = make_float2(0.f, 0.f), nvel = make_float2(0.f, 0.f);
+      float4 nst = make_float4(0.f, 0.f, 0.f, 0.f);
+      int nfl = 0;
+      const auto load = [&](int p) {
+        nu = A.u[p];
+        nmv = A.mv[p];
+        nvel = A.v[p];
+        nst = A.strain[p];
+        nfl = A.flags[p];
+      };
+      if (AHEAD && tid < m) load(base + tid);
+      __syncthreads();
+      for (int i = tid; i < m; i += THREADS) {
+        const int p = base + i, slot = rec_slot(i);
+        const int gcx = X0 + S.cell[i] % BIN, gcy = Y0 + S.cell[i] / BIN;
+        if (!AHEAD) load(p);
+        const double2 u = nu;
+        const float2 mv = nmv;
+        float2 vel = nvel;
+        float4 st = nst;
+        const int fl = nfl;
+        if (AHEAD && PRIME && i + THREADS < m) load(p + THREADS);
+        // (a point that is not in its sorted cell adds nothing there)
+        PRec r = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+        const auto keep = [&]() {
+          S.rec[0][slot] = r.a;
+          S.rec[1][slot] = r.b;
+        };
+        int cx, cy;
+        float fx, fy;
+        split_u(u.x, cx, fx);
+        split_u(u.y, cy, fy);
+        if (!in_grid_cell(A, cx, cy)) { // the grid's far edge, or outside it
+          far_edge(A.nx, cx, fx);
+          far_edge(A.ny, cy, fy);
+          if (!in_grid_cell(A, cx, cy)) {
+            atomicOr(A.status, (uint32_t)HG_STATUS_OUT_OF_GRID);
+            keep();
+            continue;
+          }
+        }
+        int jh = fl & 1;
+        int ncx = cx, ncy = cy;
+        float nfx = fx, nfy = fy;
+        if (!PRIME) {
+          float4 n00, n10, n01, n11;
+          const int gx = cx - (X0 - DRIFT), gy = cy - (Y0 - DRIFT);
+          const bool in_window = gx >= 0 && gy >= 0 && gx <= VA_W - 2 && gy <= rows + 2 * DRIFT - 1;
+          if (in_window) {
+            const int k0 = gy * VA_W + gx;
+            n00 = s_va[k0];
+            n10 = s_va[k0 + 1];
+            n01 = s_va[k0 + VA_W];
+            n11 = s_va[k0 + VA_W + 1];
+          } else {
+            if (HG_INDEX_OK((cy + 1) * row + cx + 1, (int64_t)row * (A.ny + 1), A.status)) {
+              nodes.corners(cx, cy, n00, n10, n01, n11);
+            } else {
+              n00 = n10 = n01 = n11 = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+          }
+          const float wx0 = 1.0f - fx, wx1 = fx, wy0 = 1.0f - fy, wy1 = fy;
+          const float w00 = wx0 * wy0, w10 = wx1 * wy0, w01 = wx0 * wy1, w11 = wx1 * wy1;
+          // velocity gradient from the grid-unit weight gradients
+          const float ih = A.inv_h;
+          const float Lxx = (-wy0 * n00.x + wy0 * n10.x - wy1 * n01.x + wy1 * n11.x) * ih;
+          const float Lxy = (-wx0 * n00.x - wx1 * n10.x + wx0 * n01.x + wx1 * n11.x) * ih;
+          const float Lyx = (-wy0 * n00.y + wy0 * n10.y - wy1 * n01.y + wy1 * n11.y) * ih;
+          const float Lyy = (-wx0 * n00.y - wx1 * n10.y + wx0 * n01.y + wx1 * n11.y) * ih;
+          const float vpx = w00 * n00.x + w10 * n10.x + w01 * n01.x + w11 * n11.x;
+          const float vpy = w00 * n00.y + w10 * n10.y + w01 * n01.y + w11 * n11.y;
+          const float apx = w00 * n00.z + w10 * n10.z + w01 * n01.z + w11 * n11.z;
+          const float apy = w00 * n00.w + w10 * n10.w + w01 * n01.w + w11 * n11.w;
+          if (AHEAD && i + THREADS < m) load(p + THREADS);
+          constitutive_update(st, jh, Lxx, Lxy, Lyx, Lyy, A.dt, A.kappa, A.mu, A.dp_alpha);
+          // kinematically scripted points move with their own velocity
+          const bool kin = (fl & 2) != 0;
+          const float dtih = A.dt * A.inv_h;
+          const float dux = dtih * (kin ? vel.x : vpx);
+          const float duy = dtih * (kin ? vel.y : vpy);
+          {
+            const float a = A.flip_alpha;
+            const float fvx = (1.0f - a) * vpx + a * (vel.x + A.dt * apx);
+            const float fvy = (1.0f - a) * vpy + a * (vel.y + A.dt * apy);
+            vel.x = kin ? vel.x : fvx;
+            vel.y = kin ? vel.y : fvy;
+          }
+          double2 un = make_double2(u.x + widen(dux), u.y + widen(duy));
+          // new cell and fraction by FP32 carry of the old fraction
+          nfx = fx + dux;
+          nfy = fy + duy;
+          bool exact = !(fabsf(dux) < 1.0f && fabsf(duy) < 1.0f);
+          // the tile's plane mask bounds points that start in the window and
+          // move less than a cell; any other point tests every plane
+          const unsigned pmask = (in_window && !exact) ? plane_mask : (1u << A.nplanes) - 1u;
+          {
+            const float cx1 = floorf(nfx), cy1 = floorf(nfy); // -1, 0 or 1
+            ncx += (int)cx1;
+            ncy += (int)cy1;
+            nfx -= cx1;
+            nfy -= cy1;
+          }
+          // MaterialPoints::resolvePlaneCollisions in grid units; FP32 test
+          // first, FP64 where the point is within pmargin cells of a plane
+          const float ufx = (float)ncx + nfx, ufy = (float)ncy + nfy;
+          for (unsigned mk = pmask; mk; mk &= mk - 1) {
+            const MpmPlaneDev &pl = A.planes[__ffs(mk) - 1];
+            if (ufy < pl.fulb - A.pmargin) continue;
+            const float dapprox = pl.fn[0] * (ufx - pl.fux[0]) + pl.fn[1] * (ufy - pl.fux[1]);
+            if (dapprox > A.pmargin) continue;
+            if (un.y < pl.ulb) continue;
+            const double d = plane_distance_u(pl, un.x, un.y);
+            if (d > 0.0) continue;
+            un.x += -d * pl.n[0];
+            un.y += -d * pl.n[1];
+            exact = true;
+            if (!pl.sticking) {
+              const float vn = pl.fn[0] * vel.x + pl.fn[1] * vel.y;
+              if (vn > 0.0f) continue;
+              vel.x -= vn * pl.fn[0];
+              vel.y -= vn * pl.fn[1];
+            } else {
+              vel = make_float2(0.0f, 0.0f);
+            }
+          }
+          if (exact || !in_grid_cell(A, ncx, ncy)) {
+            // (also when the FP32 carry put a point just inside the low edge in
+            // cell -1, its fraction rounded down and its step rounded up: the
+            // FP64 position decides)
+            split_u(un.x, ncx, nfx);
+            split_u(un.y, ncy, nfy);
+            far_edge(A.nx, ncx, nfx);
+            far_edge(A.ny, ncy, nfy);
+          }
+          // the position stays finite while its increments do (it was finite
+          // and inside the grid): one test covers position, velocity and J
+          nonfinite |= !isfinite((dux + duy) + (vel.x + vel.y) + st.x);
+          A.u[p] = un;
+          A.v[p] = vel;
+          A.strain[p] = st;
+          A.flags[p] = (uint8_t)((fl & ~1) | jh);
+          if ((ncx != gcx) | (ncy != gcy)) { // a point in its sorted cell is in the window
+            // (the tile's window, whichever strip of it this is)
+            const int ngx = ncx - (X0 - DRIFT), ngy = ncy - (Y0 - strip.sy - DRIFT);
+            left_window += (ngx < 0) | (ngy < 0) | (ngx > VA_W - 2) | (ngy > VA_W - 2);
+            ++left_cell;
+          }
+        }
+        if (!in_grid_cell(A, ncx, ncy)) {
           atomicOr(A.status, (uint32_t)HG_STATUS_OUT_OF_GRID);
+          keep();
           continue;
         }
-      }
-      int jh = fl & 1;
-      int ncx = cx, ncy = cy;
-      float nfx = fx, nfy = fy;
-      if (!PRIME) {
-        float4 n00, n10, n01, n11;
-        const int gx = cx - (X0 - DRIFT), gy = cy - (Y0 - DRIFT);
-        const bool in_window = gx >= 0 && gy >= 0 && gx <= VA_W - 2 && gy <= rows + 2 * DRIFT - 1;
-        if (in_window) {
-          const int k0 = gy * VA_W + gx;
-          n00 = s_va[k0];
-          n10 = s_va[k0 + 1];
-          n01 = s_va[k0 + VA_W];
-          n11 = s_va[k0 + VA_W + 1];
-        } else {
-          if (HG_INDEX_OK((cy + 1) * row + cx + 1, (int64_t)row * (A.ny + 1), A.status)) {
-            nodes.corners(cx, cy, n00, n10, n01, n11);
+        // ---- P2G contribution for the next step ----
+        float s00, s01, s11;
+        stress_factor(st, jh, mv.y, A.inv_h, A.kappa, A.mu, s00, s01, s11);
+        r.a = make_float4(nfx, nfy, mv.x, mv.x * vel.x);
+        r.b = make_float4(mv.x * vel.y, s00, s01, s11);
+        if (ncx != gcx || ncy != gcy) {
+          const int lx = ncx - WX, ly = ncy - WY;
+          if (lx >= 0 && ly >= 0 && lx <= ACC_W - 2 && ly <= rows + 2 * DRIFT + 1) {
+            float part[20];
+#pragma unroll
+            for (int k = 0; k < 20; ++k) part[k] = 0.f;
+            p2g_corners(r, part);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const int node = (ly + (k >> 1)) * ACC_W + lx + (k & 1);
+#pragma unroll
+              for (int c = 0; c < 5; ++c) atomicAdd(&s_slow[c][node], part[5 * k + c]);
+            }
           } else {
-            n00 = n10 = n01 = n11 = make_float4(0.f, 0.f, 0.f, 0.f);
+            scatter_global(A, ncx, ncy, r);
           }
+          r = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
         }
-        const float wx0 = 1.0f - fx, wx1 = fx, wy0 = 1.0f - fy, wy1 = fy;
-        const float w00 = wx0 * wy0, w10 = wx1 * wy0, w01 = wx0 * wy1, w11 = wx1 * wy1;
-        // velocity gradient from the grid-unit weight gradients
-        const float ih = A.inv_h;
-        const float Lxx = (-wy0 * n00.x + wy0 * n10.x - wy1 * n01.x + wy1 * n11.x) * ih;
-        const float Lxy = (-wx0 * n00.x - wx1 * n10.x + wx0 * n01.x + wx1 * n11.x) * ih;
-        const float Lyx = (-wy0 * n00.y + wy0 * n10.y - wy1 * n01.y + wy1 * n11.y) * ih;
-        const float Lyy = (-wx0 * n00.y - wx1 * n10.y + wx0 * n01.y + wx1 * n11.y) * ih;
-        const float vpx = w00 * n00.x + w10 * n10.x + w01 * n01.x + w11 * n11.x;
-        const float vpy = w00 * n00.y + w10 * n10.y + w01 * n01.y + w11 * n11.y;
-        const float apx = w00 * n00.z + w10 * n10.z + w01 * n01.z + w11 * n11.z;
-        const float apy = w00 * n00.w + w10 * n10.w + w01 * n01.w + w11 * n11.w;
-        constitutive_update(st, jh, Lxx, Lxy, Lyx, Lyy, A.dt, A.kappa, A.mu, A.dp_alpha);
-        // kinematically scripted points move with their own velocity
-        const bool kin = (fl & 2) != 0;
-        const float dtih = A.dt * A.inv_h;
-        const float dux = dtih * (kin ? vel.x : vpx);
-        const float duy = dtih * (kin ? vel.y : vpy);
-        {
-          const float a = A.flip_alpha;
-          const float fvx = (1.0f - a) * vpx + a * (vel.x + A.dt * apx);
-          const float fvy = (1.0f - a) * vpy + a * (vel.y + A.dt * apy);
-          vel.x = kin ? vel.x : fvx;
-          vel.y = kin ? vel.y : fvy;
-        }
-        double2 un = make_double2(u.x + widen(dux), u.y + widen(duy));
-        // new cell and fraction by FP32 carry of the old fraction
-        nfx = fx + dux;
-        nfy = fy + duy;
-        bool exact = !(fabsf(dux) < 1.0f && fabsf(duy) < 1.0f);
-        // the tile's plane mask bounds points that start in the window and
-        // move less than a cell; any other point tests every plane
-        const unsigned pmask = (in_window && !exact) ? plane_mask : (1u << A.nplanes) - 1u;
-        {
-          const float cx1 = floorf(nfx), cy1 = floorf(nfy); // -1, 0 or 1
-          ncx += (int)cx1;
-          ncy += (int)cy1;
-          nfx -= cx1;
-          nfy -= cy1;
-        }
-        // MaterialPoints::resolvePlaneCollisions in grid units; FP32 test
-        // first, FP64 where the point is within pmargin cells of a plane
-        const float ufx = (float)ncx + nfx, ufy = (float)ncy + nfy;
-        for (unsigned mk = pmask; mk; mk &= mk - 1) {
-          const MpmPlaneDev &pl = A.planes[__ffs(mk) - 1];
-          if (ufy < pl.fulb - A.pmargin) continue;
-          const float dapprox = pl.fn[0] * (ufx - pl.fux[0]) + pl.fn[1] * (ufy - pl.fux[1]);
-          if (dapprox > A.pmargin) continue;
-          if (un.y < pl.ulb) continue;
-          const double d = plane_distance_u(pl, un.x, un.y);
-          if (d > 0.0) continue;
-          un.x += -d * pl.n[0];
-          un.y += -d * pl.n[1];
-          exact = true;
-          if (!pl.sticking) {
-            const float vn = pl.fn[0] * vel.x + pl.fn[1] * vel.y;
-            if (vn > 0.0f) continue;
-            vel.x -= vn * pl.fn[0];
-            vel.y -= vn * pl.fn[1];
-          } else {
-            vel = make_float2(0.0f, 0.0f);
-          }
-        }
-        if (exact || !in_grid_cell(A, ncx, ncy)) {
-          // (also when the FP32 carry put a point just inside the low edge in
-          // cell -1, its fraction rounded down and its step rounded up: the
-          // FP64 position decides)
-          split_u(un.x, ncx, nfx);
-          split_u(un.y, ncy, nfy);
-          far_edge(A.nx, ncx, nfx);
-          far_edge(A.ny, ncy, nfy);
-        }
-        // the position stays finite while its increments do (it was finite
-        // and inside the grid): one test covers position, velocity and J
-        nonfinite |= !isfinite((dux + duy) + (vel.x + vel.y) + st.x);
-        A.u[p] = un;
-        A.v[p] = vel;
-        A.strain[p] = st;
-        A.flags[p] = (uint8_t)((fl & ~1) | jh);
-        if ((ncx != gcx) | (ncy != gcy)) { // a point in its sorted cell is in the window
-          // (the tile's window, whichever strip of it this is)
-          const int ngx = ncx - (X0 - DRIFT), ngy = ncy - (Y0 - strip.sy - DRIFT);
-          left_window += (ngx < 0) | (ngy < 0) | (ngx > VA_W - 2) | (ngy > VA_W - 2);
-          ++left_cell;
-        }
+        keep();
       }
-      if (!in_grid_cell(A, ncx, ncy)) {
-        atomicOr(A.status, (uint32_t)HG_STATUS_OUT_OF_GRID);
-        continue;
-      }
-      // ---- P2G contribution for the next step ----
-      PRec r;
-      float s00, s01, s11;
-      stress_factor(st, jh, mv.y, A.inv_h, A.kappa, A.mu, s00, s01, s11);
-      r.a = make_float4(nfx, nfy, mv.x, mv.x * vel.x);
-      r.b = make_float4(mv.x * vel.y, s00, s01, s11);
-      if (ncx == gcx && ncy == gcy) {
+      __syncthreads();
+      float acc[20];
+#pragma unroll
+      for (int k = 0; k < 20; ++k) acc[k] = 0.f;
+      for (int i = p0 + (tid & (lanes - 1)); i < p1; i += lanes) {
+        const int slot = rec_slot(i);
+        const PRec r = {S.rec[0][slot], S.rec[1][slot]};
         p2g_corners(r, acc);
-      } else {
-        const int lx = ncx - WX, ly = ncy - WY;
-        if (lx >= 0 && ly >= 0 && lx <= ACC_W - 2 && ly <= rows + 2 * DRIFT + 1) {
-          float part[20];
+      }
+      for (int o = 1; o < lanes; o <<= 1)
 #pragma unroll
-          for (int k = 0; k < 20; ++k) part[k] = 0.f;
-          p2g_corners(r, part);
+        for (int k = 0; k < 20; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+      __syncthreads(); // the corner sums take the records' place
+      if ((tid & (lanes - 1)) == 0)
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int node = (ly + (k >> 1)) * ACC_W + lx + (k & 1);
+        for (int k = 0; k < 20; ++k) s_corner[k][cell] = acc[k];
+      const bool last = base + CAP >= strip.all.y;
+      if (last) {
+        if (nonfinite) atomicOr(A.status, (uint32_t)HG_STATUS_NONFINITE);
+        if (left_window) atomicAdd(&s_out[0], left_window);
+        if (left_cell) atomicAdd(&s_out[1], left_cell);
+      }
+      __syncthreads();
+      int claimed = 0; // (arrives under the flush)
+      if (claim && last && tid == 0) claimed = atomicAdd(claim, 1);
+      // ---- node sums of the tile window, flushed to the global accumulators ----
+      for (int k = tid; k < ACC_W * (rows + 2 * DRIFT + 3); k += THREADS) {
+        const int i = k % ACC_W, j = k / ACC_W;
+        float sum[5];
 #pragma unroll
-            for (int c = 0; c < 5; ++c) atomicAdd(&s_slow[c][node], part[5 * k + c]);
+        for (int c = 0; c < 5; ++c) {
+          sum[c] = s_slow[c][k];
+          s_slow[c][k] = 0.f; // ready for the next tile
+        }
+        const int bi = i - (DRIFT + 1), bj = j - (DRIFT + 1); // node index within the tile
+        if (bi >= 0 && bj >= 0 && bi <= BIN && bj <= rows) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int dx = q & 1, dy = q >> 1;
+            const int ci = bi - dx, cj = bj - dy;
+            if (ci < 0 || cj < 0 || ci >= BIN || cj >= rows) continue;
+            const int cell = cj * BIN + ci;
+#pragma unroll
+            for (int c = 0; c < 5; ++c) sum[c] += s_corner[5 * q + c][cell];
           }
-        } else {
-          scatter_global(A, ncx, ncy, r);
         }
+        if (sum[0] == 0.f && sum[1] == 0.f && sum[2] == 0.f && sum[3] == 0.f && sum[4] == 0.f)
+          continue;
+        const int ix = WX + i, iy = WY + j;
+        if (ix < 0 || iy < 0 || ix > A.nx || iy > A.ny) continue;
+        const int node = iy * row + ix;
+        if (!HG_INDEX_OK(node, (int64_t)row * (A.ny + 1), A.status)) continue;
+        atomicAdd(&A.accm[node], sum[0]);
+        atomicAdd(&A.acc4[node], make_float4(sum[1], sum[2], sum[3], sum[4]));
       }
+      if (claim && last && tid == 0) S.claimed = claimed;
+      __syncthreads();
     }
-    if (nonfinite) atomicOr(A.status, (uint32_t)HG_STATUS_NONFINITE);
-    if (left_window) atomicAdd(&s_out[0], left_window);
-    if (left_cell) atomicAdd(&s_out[1], left_cell);
-    for (int o = 1; o < lanes; o <<= 1)
-#pragma unroll
-      for (int k = 0; k < 20; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-    if ((tid & (lanes - 1)) == 0)
-#pragma unroll
-      for (int k = 0; k < 20; ++k) s_corner[k][cell] = acc[k];
-    __syncthreads();
-    int claimed = 0; // (arrives under the flush)
-    if (claim && tid == 0) claimed = atomicAdd(claim, 1);
-    // ---- node sums of the tile window, flushed to the global accumulators ----
-    for (int k = tid; k < ACC_W * (rows + 2 * DRIFT + 3); k += THREADS) {
-      const int i = k % ACC_W, j = k / ACC_W;
-      float sum[5];
-#pragma unroll
-      for (int c = 0; c < 5; ++c) {
-        sum[c] = s_slow[c][k];
-        s_slow[c][k] = 0.f; // ready for the next tile
-      }
-      const int bi = i - (DRIFT + 1), bj = j - (DRIFT + 1); // node index within the tile
-      if (bi >= 0 && bj >= 0 && bi <= BIN && bj <= rows) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int dx = q & 1, dy = q >> 1;
-          const int ci = bi - dx, cj = bj - dy;
-          if (ci < 0 || cj < 0 || ci >= BIN || cj >= rows) continue;
-          const int cell = cj * BIN + ci;
-#pragma unroll
-          for (int c = 0; c < 5; ++c) sum[c] += s_corner[5 * q + c][cell];
-        }
-      }
-      if (sum[0] == 0.f && sum[1] == 0.f && sum[2] == 0.f && sum[3] == 0.f && sum[4] == 0.f)
-        continue;
-      const int ix = WX + i, iy = WY + j;
-      if (ix < 0 || iy < 0 || ix > A.nx || iy > A.ny) continue;
-      const int node = iy * row + ix;
-      if (!HG_INDEX_OK(node, (int64_t)row * (A.ny + 1), A.status)) continue;
-      atomicAdd(&A.accm[node], sum[0]);
-      atomicAdd(&A.acc4[node], make_float4(sum[1], sum[2], sum[3], sum[4]));
-    }
-    if (claim && tid == 0) S.claimed = claimed;
-    __syncthreads();
     if (tid < 2 && s_out[tid]) atomicAdd(&A.outside[tid], s_out[tid]);
   }
 }
 
 // fused_strip expects the moved-point window to be zero on entry (it leaves
 // it zero); the first tile's barrier orders this against its use.
-template <int ROWS> __device__ __forceinline__ void zero_slow(FusedSmem<ROWS> &S) {
+template <int CAP> __device__ __forceinline__ void zero_slow(FusedSmem<CAP> &S) {
   float *s = &S.slow[0][0];
   for (int k = threadIdx.x; k < (int)(sizeof(S.slow) / sizeof(float)); k += THREADS) s[k] = 0.f;
 }
@@ -641,26 +704,26 @@ struct GridNodes {
   }
 };
 
-// Bound by issue slots and load latency (59 % of the slots, 585 thread
-// instructions per point) at the three CTAs per SM that 80 registers allow.
+// Bound by issue slots and load latency: 68 % of the slots, 660 instructions
+// per warp and point, 64 registers and 55 KB at four CTAs per SM.
 //
 // A CTA takes its first tile by its number and draws each further one from a
 // counter that the grid update zeroes. Dealt out by CTA number, the tiles of
 // the last round went to the CTAs of the lowest numbers, which dependent
-// launches place three to an SM: 2,000,000 points (1000 x 500 cells) 76 to 81
-// us per step, drawn 68; 1,155,200 56.6, drawn 49.
+// launches place on the same SMs: 2,000,000 points (1000 x 500 cells) 76 to 81
+// us per step, drawn 68; 1,155,200 56.6, drawn 49 (at three CTAs per SM).
 //
-// The last tiles are cut into strips with as many threads per cell more, since
-// a tile's time is that of the points its threads take one after the other.
-// Below two rounds those of a round that would leave half of the CTAs idle (or
-// three in four): 100,000 points 13.5 us per step, uncut 17.0; 204,800 17.7,
-// uncut 25.0. From two rounds on the last half round, which levels the end:
-// 1,155,200 47.7 us, uncut 49.9; 2,000,000 (500 x 1000 cells) 76.1, uncut 78.1.
-// (A quarter round in quarters took 69.8 where halves and whole tiles took 68.)
+// The last tiles are cut into strips with as many threads per cell more, for
+// the latency of a tile is that of the points its threads take one after the
+// other. Below two rounds those of a round that would leave half of the CTAs
+// idle (or three in four): 100,000 points 11.9 us per step, uncut 17.0; 204,800
+// 17.4, uncut 25.0. From two rounds on the last half round, which levels the
+// end: 1,155,200 47.7 us, uncut 49.9 (at three CTAs per SM; now 41.9).
 template <bool PRIME>
-__global__ void __launch_bounds__(THREADS, 3) kx_g2p2g(const __grid_constant__ MixedArgs A) {
+__global__ void __launch_bounds__(THREADS, 4) kx_g2p2g(const __grid_constant__ MixedArgs A) {
   // the arguments stay in the constant bank: operands need no registers
-  __shared__ FusedSmem<BIN> S;
+  extern __shared__ __align__(16) unsigned char fused_smem[];
+  FusedSmem<PASS_POINTS> &S = *reinterpret_cast<FusedSmem<PASS_POINTS> *>(fused_smem);
   __shared__ struct {
     int nitems, whole, split; // whole tiles, then strips
   } Q;
@@ -687,7 +750,7 @@ __global__ void __launch_bounds__(THREADS, 3) kx_g2p2g(const __grid_constant__ M
     const Strip strip =
         i < 0 ? strip_of(A, A.active[t], 0, 0)
               : strip_of(A, A.active[Q.whole + (i >> Q.split)], Q.split, i & ((1 << Q.split) - 1));
-    fused_strip<PRIME>(A, strip, S, GridNodes{A}, PRIME ? nullptr : A.claimed);
+    fused_strip<PRIME, true>(A, strip, S, GridNodes{A}, PRIME ? nullptr : A.claimed);
     t = PRIME ? t + gridDim.x : gridDim.x + S.claimed;
   }
 }
@@ -738,13 +801,13 @@ __device__ __forceinline__ float4 node_update(const MixedArgs &A, int ix, int iy
 // than once), so that the grid update needs no launch of its own. The sums
 // rotate through three sets: this step reads one (in), adds the next step's to
 // A's and clears the third for the step after. Per step, 4 points per cell: 200
-// points 7.1 us, in two launches over whole tiles 13.9; 12,800 8.7 and 17.5;
-// 62,468 10.3 and 18.8. What is left is the chain of one strip: about 1,600
-// instructions of a warp with few others to hide behind.
+// points 6.4 us, in two launches over whole tiles 13.9; 12,800 7.4 and 17.5;
+// 62,468 9.2 and 18.8. What is left is the chain of one strip, about 1,600
+// instructions of a warp with few others to hide behind, and the launch.
 //
 // It steps linear scenes with no more points than fit its CTAs at one per cell,
 // so that no sparse scene takes a second round of whole tiles (80,000 points at
-// one per cell: 14.6 us, in two launches 12.4; 59,858: 9.5 and 11.4), on a grid
+// one per cell: 14.6 us, in two launches 12.5; 59,858: 8.4 and 11.4), on a grid
 // that a step clears in four stores per thread.
 constexpr int SMALL_CTAS = 2; // per SM
 constexpr int64_t SMALL_POINTS = 75000, SMALL_NODES = 4 * 152 * SMALL_CTAS * THREADS;
@@ -773,7 +836,8 @@ struct SumNodes {
 
 __global__ void __launch_bounds__(THREADS, SMALL_CTAS)
     kx_step_small(const __grid_constant__ MixedArgs A, const __grid_constant__ SmallSets R) {
-  __shared__ FusedSmem<BIN> S;
+  extern __shared__ __align__(16) unsigned char fused_smem[];
+  FusedSmem<PASS_POINTS> &S = *reinterpret_cast<FusedSmem<PASS_POINTS> *>(fused_smem);
   zero_slow(S);
   // the sort's tables are older than the launch before this one: they are
   // read under its end
@@ -791,7 +855,7 @@ __global__ void __launch_bounds__(THREADS, SMALL_CTAS)
   pdl_wait();
   pdl_trigger();
   while (t < nitems) {
-    if (work) fused_strip<false>(A, strip, S, SumNodes{A, R});
+    if (work) fused_strip<false, true>(A, strip, S, SumNodes{A, R});
     t += grid;
     work = t < nitems && item();
   }
@@ -831,10 +895,11 @@ __device__ __forceinline__ void batch_prefix(const MixedArgs *slots, int nslots,
   int run = off + x - sum;
 #pragma unroll
   for (int j = 0; j < PER; ++j) {
-    prefix[threadIdx.x * PER + j] = run;
+    const int s = threadIdx.x * PER + j;
+    if (s <= nslots) prefix[s] = run;
     run += v[j];
   }
-  if (threadIdx.x == THREADS - 1) prefix[THREADS * PER] = run;
+  if (threadIdx.x == THREADS - 1 && nslots == THREADS * PER) prefix[nslots] = run;
   __syncthreads();
 }
 
@@ -928,16 +993,17 @@ __device__ __forceinline__ void drain_queue(const MixedArgs *slots, int nslots, 
 
 
 // All scenes of a batch in one launch: the CTAs drain (scene, tile) items.
-__global__ void __launch_bounds__(THREADS, 3) kb_g2p2g(const MixedArgs *slots,
+__global__ void __launch_bounds__(THREADS, 4) kb_g2p2g(const MixedArgs *slots,
                                                        int nslots, int32_t *queue) {
-  __shared__ FusedSmem<BIN> S;
+  extern __shared__ __align__(16) unsigned char fused_smem[];
+  FusedSmem<BATCH_PASS_POINTS> &S = *reinterpret_cast<FusedSmem<BATCH_PASS_POINTS> *>(fused_smem);
+  int *prefix = reinterpret_cast<int *>(fused_smem + sizeof(S)); // [nslots + 1]
   __shared__ MixedArgs A;
-  __shared__ int prefix[PREFIX_LEN];
   zero_slow(S);
   batch_prefix(slots, nslots, prefix);
   drain_queue(slots, nslots, prefix, queue, A,
               [&](const MixedArgs &a, int tile) {
-                fused_strip<false>(a, strip_of(a, tile, 0, 0), S, GridNodes{a});
+                fused_strip<false, false>(a, strip_of(a, tile, 0, 0), S, GridNodes{a});
               });
 }
 
@@ -1767,7 +1833,22 @@ MixedParticles parts(hg_mpm *m, int which) {
   return P;
 }
 
-size_t fused_smem_bytes() { return 0; } // static shared memory only
+template <int CAP> size_t fused_smem_bytes() { return sizeof(FusedSmem<CAP>); }
+// a batch's kernel holds the prefix of its scenes' tiles as well
+size_t fused_batch_smem_bytes(int nslots) {
+  return sizeof(FusedSmem<BATCH_PASS_POINTS>) + sizeof(int) * ((size_t)nslots + 1);
+}
+// more than 48 KB of shared memory is asked for by kernel
+hg_status fused_smem_setup() {
+  const auto ask = [](const void *kernel, size_t bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
+  HG_CUDA_TRY(ask((const void *)kx_g2p2g<true>, fused_smem_bytes<PASS_POINTS>()));
+  HG_CUDA_TRY(ask((const void *)kx_g2p2g<false>, fused_smem_bytes<PASS_POINTS>()));
+  HG_CUDA_TRY(ask((const void *)kx_step_small, fused_smem_bytes<PASS_POINTS>()));
+  HG_CUDA_TRY(ask((const void *)kb_g2p2g, fused_batch_smem_bytes(MAX_BATCH)));
+  return HG_OK;
+}
 
 MixedArgs make_args(hg_mpm *m, double dt, bool tiles) {
   MixedArgs A;
@@ -1926,9 +2007,9 @@ hg_status rebin_batch(hg_context *ctx, const std::vector<hg_mpm *> &R, unsigned 
   return HG_OK;
 }
 
-// CTAs per SM of the two kernels: the launch shape, else 3 (the fused
-// kernel's occupancy at 80 registers) and 8
-constexpr int DEFAULT_FUSED_CTAS = 3, DEFAULT_UPDATE_CTAS = 8;
+// CTAs per SM of the two kernels: the launch shape, else the fused kernel's
+// occupancy and 8
+constexpr int DEFAULT_FUSED_CTAS = 4, DEFAULT_UPDATE_CTAS = 8;
 int fused_per_sm(const hg_launch_shape &s) {
   return s.fused_ctas_per_sm > 0 ? s.fused_ctas_per_sm : DEFAULT_FUSED_CTAS;
 }
@@ -1943,7 +2024,8 @@ void launch_particle_kernel(hg_mpm *m, const MixedArgs &A, cudaStream_t s) {
   if (m->p.basis == HG_BASIS_UGIMP) {
     HG_LAUNCH_PDL(kxu_step<PRIME>, ugimp_blocks(m), UGIMP_THREADS, 0, s, A);
   } else {
-    HG_LAUNCH_PDL(kx_g2p2g<PRIME>, fused_blocks(m), THREADS, fused_smem_bytes(), s, A);
+    HG_LAUNCH_PDL(kx_g2p2g<PRIME>, fused_blocks(m), THREADS,
+                  fused_smem_bytes<PASS_POINTS>(), s, A);
   }
 }
 int update_blocks(hg_mpm *m) { return m->ctx->num_sms * update_per_sm(m->shape); }
@@ -1985,7 +2067,7 @@ void tune_store(const TuneKey &k, const hg_launch_shape &s) {
 // CTAs per SM tried for (fused, update): fewer, the default, and more CTAs
 // than are resident (finer shares of the tiles, later ones fill in behind
 // the first wave)
-constexpr hg_launch_shape TUNE_CANDIDATES[HG_TUNE_CANDIDATES] = {{2, 4}, {3, 8}, {6, 16},
+constexpr hg_launch_shape TUNE_CANDIDATES[HG_TUNE_CANDIDATES] = {{2, 4}, {4, 8}, {8, 16},
                                                                  {12, 32}};
 static_assert(HG_TUNE_CANDIDATES == 4, "candidate list");
 
@@ -2022,10 +2104,12 @@ hg_status mixed_alloc(hg_mpm *m) {
     if (m->p.basis == HG_BASIS_UGIMP && (st = m->mhl_[b].alloc(m->cap))) return st;
   }
   hg_status st;
-  if ((st = m->acc4.alloc(nn)) || (st = m->accm.alloc(nn)) || (st = m->va.alloc(nn)) ||
+  if ((st = fused_smem_setup()) || (st = m->acc4.alloc(nn)) || (st = m->accm.alloc(nn)) ||
+      (st = m->va.alloc(nn)) ||
       (st = m->gm.alloc(nn)) || (st = m->keys.alloc(m->cap)) ||
       (st = m->counts.alloc(nkeys + 1)) || (st = m->offsets.alloc(nkeys + 1)) ||
-      (st = m->cursor.alloc(std::max(nkeys, m->cap))) || (st = m->scan_tmp.alloc(scan_tmp_size(nkeys + 1))) ||
+      (st = m->cursor.alloc(std::max(nkeys, m->cap))) ||
+      (st = m->scan_tmp.alloc(scan_tmp_size(nkeys + 1))) ||
       (st = m->active_bins.alloc((int64_t)m->ntx * m->nty)) ||
       (st = m->active_tiles.alloc((int64_t)m->ntx * m->nty)) ||
       (st = m->nactive.alloc(2)) || (st = m->claimed.alloc(1)) || (st = m->outside.alloc(2)))
@@ -2061,7 +2145,7 @@ int64_t mixed_device_bytes(int nx, int ny, int64_t cap, bool linear) {
   int64_t b = 2 * cap * per_point + cap * 4 * 3;             // particle pairs, keys, order tables
   b += nn * (2 * sizeof(float4) + 2 * sizeof(float));       // acc4, va, accm, gm
   if (linear && nn <= SMALL_NODES) b += 2 * nn * (sizeof(float4) + sizeof(float));
-  b += 4 * (2 * nkeys + std::max(nkeys, cap) + 2 + scan_tmp_size(nkeys + 1)); // counts, offsets, cursor
+  b += 4 * (2 * nkeys + 2 + std::max(nkeys, cap) + scan_tmp_size(nkeys + 1)); // counts, offsets ...
   b += 4 * (2 * ntx * nty + 5);                             // active lists, counters
   return b;
 }
@@ -2221,6 +2305,7 @@ void launch_small_steps(hg_mpm *m, double dt, int n, cudaStream_t s) {
   MixedArgs A = make_args(m, dt, false);
   SmallSets R;
   const int blocks = m->ctx->num_sms * SMALL_CTAS;
+  const size_t smem = fused_smem_bytes<PASS_POINTS>();
   for (int k = 0; k < n; ++k) {
     R.in4 = set4[k % 3];
     R.inm = setm[k % 3];
@@ -2229,9 +2314,9 @@ void launch_small_steps(hg_mpm *m, double dt, int n, cudaStream_t s) {
     R.clear4 = set4[(k + 2) % 3];
     R.clearm = setm[(k + 2) % 3];
     if (k == 0)
-      HG_LAUNCH(kx_step_small, blocks, THREADS, 0, s, A, R);
+      HG_LAUNCH(kx_step_small, blocks, THREADS, smem, s, A, R);
     else
-      HG_LAUNCH_PDL(kx_step_small, blocks, THREADS, 0, s, A, R);
+      HG_LAUNCH_PDL(kx_step_small, blocks, THREADS, smem, s, A, R);
   }
 }
 
@@ -2466,7 +2551,7 @@ hg_status batch_chunk_graph(hg_batch *b, int S) {
       HG_LAUNCH(kb_grid_update, gu, THREADS, 0, s, dt, S, b->queue.p + 2);
     else
       HG_LAUNCH_PDL(kb_grid_update, gu, THREADS, 0, s, dt, S, b->queue.p + 2);
-    HG_LAUNCH_PDL(kb_g2p2g, gf, THREADS, 0, s, db, S, b->queue.p);
+    HG_LAUNCH_PDL(kb_g2p2g, gf, THREADS, fused_batch_smem_bytes(S), s, db, S, b->queue.p);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) st = cuda_fail(e, "kernel launch");
   }
@@ -2611,7 +2696,8 @@ hg_status batch_step(hg_batch *b, int nsteps) {
               b->queue.p + 2);
     HG_CHECK_LAUNCH();
     if (b->profile) HG_CUDA_TRY(cudaEventRecord(ev[3], s));
-    HG_LAUNCH_PDL(kb_g2p2g, nsm * fused_per_sm(b->shape), THREADS, 0, s, db, S, b->queue.p);
+    HG_LAUNCH_PDL(kb_g2p2g, nsm * fused_per_sm(b->shape), THREADS,
+                  fused_batch_smem_bytes(S), s, db, S, b->queue.p);
     HG_CHECK_LAUNCH();
     if (b->profile) HG_CUDA_TRY(cudaEventRecord(ev[4], s));
     for (hg_mpm *m : b->members) m->steps_since_rebin++;
