@@ -264,7 +264,7 @@ hg_status hg_batch_profile_read(hg_batch *b, double *resort_ms, double *table_ms
  * The MIXED kernels run as grids of CTAs that walk the active tiles (single
  * scene) or contiguous shares of the (scene, tile) items (batch). A launch
  * shape gives the CTAs per SM of the fused G2P/P2G kernel and of the grid
- * update; 0 keeps the built-in choice (4 and 8). The autotuner times
+ * update; 0 keeps the built-in choice (4, in a batch 8, and 8). The autotuner times
  * HG_TUNE_CANDIDATES shapes on the live object with CUDA events, each for
  * steps_per_candidate steps (the scene advances by all of them: a shape only
  * changes the order of FP32 atomic sums). A batch keeps the fastest shape for
