@@ -1274,7 +1274,7 @@ hg_status dem_reset_history(hg_dem *d) {
 // The bodies' positions, radii, flags or number changed outside dem_step: the
 // next step bins them anew.
 void dem_bodies_changed(hg_dem *d) {
-  if (d->bins == hg_dem::BINS_FILLED) d->bins = hg_dem::BINS_DIRTY;
+  d->bins = hg_dem::BINS_DIRTY;
 }
 
 hg_status dem_prepare(hg_dem *d, double dt) {
