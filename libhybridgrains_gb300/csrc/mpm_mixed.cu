@@ -479,6 +479,8 @@ __device__ __forceinline__ void fused_strip(const MixedArgs &A, const Strip &str
           if (!in_grid_cell(A, cx, cy)) {
             atomicOr(A.status, (uint32_t)HG_STATUS_OUT_OF_GRID);
             keep();
+            // (the load ahead below is the next point's only source)
+            if (AHEAD && !PRIME && i + THREADS < m) load(p + THREADS);
             continue;
           }
         }
