@@ -37,6 +37,7 @@
 #include "mpm_basis.cuh"
 #include "mpm_axis.cuh"
 
+#include <cmath>
 #include <utility>
 
 namespace hg {
@@ -297,17 +298,19 @@ struct GridArgs {
   const double *cforce;
   const int32_t *hyb;
   double *vel, *acc;
+  // cells about each plane and its lower bound within which FP64 decides
+  float margin[HG_MAX_PLANES], bound_margin[HG_MAX_PLANES];
 };
 
 // True when the plane acts on node (ix, iy) (PhysicsGrid.cpp:614-629): in FP32
-// grid units away from the plane and its lower bound, within pmargin cells of
-// either by the reference's own FP64 test.
-__device__ __forceinline__ bool node_hit(const MpmParams &P, const MpmPlaneDev &pl, float pmargin,
-                                         int ix, int iy) {
+// grid units away from the plane and its lower bound, within margin and
+// bound_margin cells of them by the reference's own FP64 test.
+__device__ __forceinline__ bool node_hit(const MpmParams &P, const MpmPlaneDev &pl, float margin,
+                                         float bound_margin, int ix, int iy) {
   const float fx = (float)ix, fy = (float)iy;
-  if (fy < pl.fulb - pmargin) return false;
+  if (fy < pl.fulb - bound_margin) return false;
   const float d32 = pl.fn[0] * (fx - pl.fux[0]) + pl.fn[1] * (fy - pl.fux[1]);
-  if (fabsf(d32) > pmargin && fabsf(fy - pl.fulb) > pmargin) return d32 < 0.0f;
+  if (fabsf(d32) > margin && fabsf(fy - pl.fulb) > bound_margin) return d32 < 0.0f;
   const double px = P.gmin[0] + P.h * (double)ix, py = P.gmin[1] + P.h * (double)iy;
   if (py < pl.lower_bound) return false;
   return !(pl.n[0] * (px - pl.x[0]) + pl.n[1] * (py - pl.x[1]) > 0.0);
@@ -341,10 +344,9 @@ __global__ void __launch_bounds__(128) k64_grid(const __grid_constant__ MpmParam
       force[i] = f;
       pn = make_double2(fma(A.dt, f.x, pm.x), fma(A.dt, f.y, pm.y));
       const int ix = (int)(i % (P.nx + 1)), iy = (int)(i / (P.nx + 1));
-      const float pmargin = 0.01f + 4.0e-7f * (float)(P.nx + P.ny);
       for (int k = 0; k < P.nplanes; ++k) { // PhysicsGrid::resolvePlaneCollisions
         const MpmPlaneDev &pl = P.planes[k];
-        if (!node_hit(P, pl, pmargin, ix, iy)) continue;
+        if (!node_hit(P, pl, A.margin[k], A.bound_margin[k], ix, iy)) continue;
         if (!pl.sticking) {
           double vx = pn.x / mi, vy = pn.y / mi;
           const double vn = pl.n[0] * vx + pl.n[1] * vy;
@@ -662,6 +664,18 @@ template <bool FORCES, bool UPDATE> hg_status grid_pass(hg_mpm *m, double dt) {
   A.hyb = m->g_hyb.p;
   A.vel = m->g_vel.p;
   A.acc = m->g_acc.p;
+  // A normal's component, an anchor's coordinate, their difference, product and
+  // sum each round by 2^-24 of a term, the terms being at most the grid's extent
+  // and the anchor's distance: five of them are 3e-7 of the terms. (The FP64 test
+  // itself rounds at the grid's distance from the origin: well below 0.01 cells
+  // of any grid whose nodes are distinct numbers by that much.)
+  for (int k = 0; k < m->p.nplanes; ++k) {
+    const MpmPlaneDev &pl = m->p.planes[k];
+    const double size = (double)m->p.nx + m->p.ny;
+    A.margin[k] = (float)(0.01 + 4.0e-7 * (size + std::fabs(pl.ux[0]) + std::fabs(pl.ux[1])));
+    A.bound_margin[k] =
+        std::isfinite(pl.ulb) ? (float)(0.01 + 4.0e-7 * (size + std::fabs(pl.ulb))) : 0.01f;
+  }
   auto kernel = k64_grid<FORCES, UPDATE>;
   HG_LAUNCH_PDL(kernel, blocks_for(A.nn, 128), 128, 0, m->ctx->stream, m->p, A);
   HG_CHECK_LAUNCH();
