@@ -16,6 +16,9 @@
 namespace hg {
 
 std::atomic<int64_t> g_launches{0};
+#ifdef HG_BOUNDS_CHECK
+std::atomic<int64_t> g_fail_launch{0};
+#endif
 std::atomic<int> g_host_threads{0};
 thread_local cudaStream_t t_alloc_stream = nullptr;
 
@@ -329,6 +332,10 @@ const char *hg_status_string(hg_status s) {
 const char *hg_last_error(void) { return hg::last_error_cstr(); }
 
 int64_t hg_kernel_launch_count(void) { return g_launches.load(); }
+#ifdef HG_BOUNDS_CHECK
+// the n-th launch check from now reports a failure (0: none); what is left of n
+int64_t hg_check_fail_launch(int64_t n) { return g_fail_launch.exchange(n); }
+#endif
 
 hg_status hg_set_host_threads(int32_t n) {
   if (n < 0 || n > 1024) return fail(HG_ERR_INVALID_ARGUMENT, "host threads must be 0 .. 1024");

@@ -470,6 +470,17 @@ __global__ void __launch_bounds__(128) kc_homogenize(const __grid_constant__ Hom
 
 inline int blocks_for(int64_t n, int t) { return (int)std::max<int64_t>(1, (n + t - 1) / t); }
 
+// the exchange's grids and the homogenisation's sums as before a first step
+hg_status clear_grids(hg_hybrid *h) {
+  const size_t bytes = sizeof(double) * (size_t)(h->m->p.nx + 1) * (h->m->p.ny + 1);
+  for (double *p : {h->dem_mass.p, h->old_mass.p, h->hmass.p})
+    HG_CUDA_TRY(cudaMemsetAsync(p, 0, bytes, h->ctx->stream));
+  for (double *p : {h->dem_mom.p, h->old_mom.p, h->hmom.p, h->v_after.p, h->a_after.p})
+    HG_CUDA_TRY(cudaMemsetAsync(p, 0, 2 * bytes, h->ctx->stream));
+  h->grids_kept = true;
+  return HG_OK;
+}
+
 } // namespace
 
 hg_status hybrid_alloc(hg_hybrid *h) {
@@ -498,14 +509,7 @@ hg_status hybrid_alloc(hg_hybrid *h) {
     HG_CHECK_LAUNCH();
   }
   HG_CUDA_TRY(cudaMemsetAsync(h->counts.p, 0, 2 * sizeof(int32_t), s));
-  HG_CUDA_TRY(cudaMemsetAsync(h->dem_mass.p, 0, sizeof(double) * nn, s));
-  HG_CUDA_TRY(cudaMemsetAsync(h->dem_mom.p, 0, sizeof(double) * 2 * nn, s));
-  HG_CUDA_TRY(cudaMemsetAsync(h->old_mass.p, 0, sizeof(double) * nn, s));
-  HG_CUDA_TRY(cudaMemsetAsync(h->old_mom.p, 0, sizeof(double) * 2 * nn, s));
-  HG_CUDA_TRY(cudaMemsetAsync(h->hmass.p, 0, sizeof(double) * nn, s));
-  HG_CUDA_TRY(cudaMemsetAsync(h->hmom.p, 0, sizeof(double) * 2 * nn, s));
-  HG_CUDA_TRY(cudaMemsetAsync(h->v_after.p, 0, sizeof(double) * 2 * nn, s));
-  HG_CUDA_TRY(cudaMemsetAsync(h->a_after.p, 0, sizeof(double) * 2 * nn, s));
+  if ((st = clear_grids(h))) return st;
   hg_status r = hybrid_clear_homogenized(h);
   if (r != HG_OK) return r;
   HG_CUDA_TRY(cudaStreamSynchronize(s));
@@ -562,6 +566,9 @@ template <int BASIS, bool W32> hg_status hybrid_step_impl(hg_hybrid *h, double d
   const int64_t nn = (int64_t)(m->p.nx + 1) * (m->p.ny + 1);
   const int64_t nb = d->n;
   hg_status st;
+  // (what a failed step scattered, and which set it had taken, is dropped)
+  if (!h->grids_kept && (st = clear_grids(h))) return st;
+  h->grids_kept = false;
   // A MIXED MPM object (FP32 bulk, FP64 positions) runs the same sequence on
   // its FP32 grid: its P2G for this step was done by the previous particle
   // launch (or the upload), its grid update and G2P are separate launches.
@@ -666,6 +673,7 @@ template <int BASIS, bool W32> hg_status hybrid_step_impl(hg_hybrid *h, double d
     HG_LAUNCH_PDL(kernel, H.node_blocks + contact_blocks, 128, 0, s, H);
     HG_CHECK_LAUNCH();
   }
+  h->grids_kept = true;
   return HG_OK;
 }
 

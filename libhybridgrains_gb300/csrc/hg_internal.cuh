@@ -105,9 +105,22 @@ __device__ __forceinline__ void pdl_trigger() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// The launch error, if any. In the bounds-checking build a test can have the
+// n-th check from now report one (hg_check_fail_launch), for what follows a
+// failed call.
+#ifdef HG_BOUNDS_CHECK
+extern std::atomic<int64_t> g_fail_launch;
+inline cudaError_t launch_error() {
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess || g_fail_launch.load() <= 0) return e;
+  return g_fail_launch.fetch_sub(1) == 1 ? cudaErrorLaunchOutOfResources : cudaSuccess;
+}
+#else
+inline cudaError_t launch_error() { return cudaGetLastError(); }
+#endif
 #define HG_CHECK_LAUNCH()                                                     \
   do {                                                                        \
-    cudaError_t e_ = cudaGetLastError();                                      \
+    cudaError_t e_ = ::hg::launch_error();                                    \
     if (e_ != cudaSuccess) return ::hg::cuda_fail(e_, "kernel launch");       \
   } while (0)
 
@@ -613,7 +626,9 @@ struct hg_hybrid {
   hg_mpm *m = nullptr;
   hg_dem *d = nullptr;
   // dem_mass and dem_mom of the last step; the other set is that of the step
-  // before, or clear
+  // before, or clear. grids_kept: they and the sums below are as a whole step
+  // leaves them (false in a step, and after one that failed)
+  bool grids_kept = false;
   hg::DevBuf<double> dem_mass, dem_mom, old_mass, old_mom;
   hg::DevBuf<double> v_after, a_after, pos_before, hstress, hvel, hmom, hmass;
   hg::DevBuf<int32_t> coupled, packed_dem, packed_mpm, flag_tmp, scan_tmp,
