@@ -330,8 +330,10 @@ struct hg_mpm {
   hg::DevBuf<float4> va;   // (vx, vy, ax, ay) of the last update
   hg::DevBuf<float> gm;    // mass of the last update
   // on small grids: two more sets of (acc4, accm) for kx_step_small
+  // (small_kept: the first is clear, as a run of such steps leaves it)
   hg::DevBuf<float4> small_4[2];
   hg::DevBuf<float> small_m[2];
+  bool small_kept = false;
   int ntx = 0, nty = 0;    // tiles in x, y
   // (cursor: per key in a batched re-sort, else per point, its rank)
   hg::DevBuf<int32_t> keys, counts, offsets, cursor, scan_tmp;

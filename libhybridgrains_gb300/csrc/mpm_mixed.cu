@@ -2147,13 +2147,9 @@ hg_status mixed_alloc(hg_mpm *m) {
   HG_CUDA_TRY(cudaMemsetAsync(m->nactive.p, 0, sizeof(int32_t) * 2, s));
   if ((st = m->inv.alloc(m->cap)) || (st = m->skey.alloc(m->cap)) || (st = m->d_flag.alloc(1)))
     return st;
-  if (m->p.basis == HG_BASIS_LINEAR && nn <= SMALL_NODES) {
-    for (int k = 0; k < 2; ++k) {
+  if (m->p.basis == HG_BASIS_LINEAR && nn <= SMALL_NODES)
+    for (int k = 0; k < 2; ++k)
       if ((st = m->small_4[k].alloc(nn)) || (st = m->small_m[k].alloc(nn))) return st;
-      HG_CUDA_TRY(cudaMemsetAsync(m->small_4[k].p, 0, sizeof(float4) * nn, s));
-      HG_CUDA_TRY(cudaMemsetAsync(m->small_m[k].p, 0, sizeof(float) * nn, s));
-    }
-  }
   m->h_outside = context_pinned_pair(m->ctx);
   m->h_flag = context_pinned_pair(m->ctx);
   if (!m->h_outside || !m->h_flag) return fail(HG_ERR_OUT_OF_MEMORY, "page-locked host memory");
@@ -2319,12 +2315,23 @@ hg_status end_chunk_capture(cudaStream_t s, hg_status st, int64_t l0, cudaGraphE
 
 bool small_scene(const hg_mpm *m) { return m->small_m[0].p && m->n <= SMALL_POINTS; }
 
-// n (a multiple of three) steps of a small scene. A regular step has to follow:
-// it leaves the grid's outputs, and the sums are again in the object's own set
-// (acc4, accm). The second set is clear before and after; the first step clears
-// the third. That step waits for all that came before: the kernel reads the
-// sort's tables before its own wait.
-void launch_small_steps(hg_mpm *m, double dt, int n, cudaStream_t s) {
+// The second set of sums is clear before and after a run of one-launch steps;
+// here before the first run, and after one that failed half-way.
+hg_status small_ready(hg_mpm *m) {
+  if (m->small_kept) return HG_OK;
+  const int64_t nn = (int64_t)(m->p.nx + 1) * (m->p.ny + 1);
+  HG_CUDA_TRY(cudaMemsetAsync(m->small_4[0].p, 0, sizeof(float4) * nn, m->ctx->stream));
+  HG_CUDA_TRY(cudaMemsetAsync(m->small_m[0].p, 0, sizeof(float) * nn, m->ctx->stream));
+  m->small_kept = true;
+  return HG_OK;
+}
+
+// n (a multiple of three) steps of a small scene, after small_ready. A regular
+// step has to follow: it leaves the grid's outputs, and the sums are again in
+// the object's own set (acc4, accm). The first step clears the third set. That
+// step waits for all that came before: the kernel reads the sort's tables before
+// its own wait.
+hg_status launch_small_steps(hg_mpm *m, double dt, int n, cudaStream_t s) {
   float4 *set4[3] = {m->acc4.p, m->small_4[0].p, m->small_4[1].p};
   float *setm[3] = {m->accm.p, m->small_m[0].p, m->small_m[1].p};
   MixedArgs A = make_args(m, dt, false);
@@ -2342,7 +2349,9 @@ void launch_small_steps(hg_mpm *m, double dt, int n, cudaStream_t s) {
       HG_LAUNCH(kx_step_small, blocks, THREADS, smem, s, A, R);
     else
       HG_LAUNCH_PDL(kx_step_small, blocks, THREADS, smem, s, A, R);
+    HG_CHECK_LAUNCH();
   }
+  return HG_OK;
 }
 
 // The graph of CHUNK_STEPS steps of one scene for its live buffer: the two
@@ -2364,7 +2373,7 @@ hg_status mixed_chunk_graph(hg_mpm *m, double dt) {
   const int64_t l0 = g_launches.load();
   HG_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   static_assert((CHUNK_STEPS - 1) % 3 == 0, "the accumulator sets come full circle");
-  if (small) launch_small_steps(m, dt, CHUNK_STEPS - 1, s);
+  if (small) st = launch_small_steps(m, dt, CHUNK_STEPS - 1, s);
   for (int k = small ? CHUNK_STEPS - 1 : 0; k < CHUNK_STEPS && st == HG_OK; ++k) {
     HG_LAUNCH_PDL(kx_grid_update, update_blocks(m), THREADS, 0, s, At);
     launch_particle_kernel<false>(m, Ab, s);
@@ -2390,6 +2399,10 @@ hg_status mixed_step(hg_mpm *m, double dt, int nsteps) {
   cudaStream_t s = m->ctx->stream;
   if (!m->primed) {
     hg_status st = prime(m);
+    if (st != HG_OK) return st;
+  }
+  if (small_scene(m)) {
+    hg_status st = small_ready(m);
     if (st != HG_OK) return st;
   }
   int k = 0;
@@ -2426,8 +2439,10 @@ hg_status mixed_step(hg_mpm *m, double dt, int nsteps) {
     }
     if (small_scene(m) && !m->profile && nsteps - k > 3) {
       const int few = (nsteps - k - 1) / 3 * 3;
-      launch_small_steps(m, dt, few, s);
-      HG_CHECK_LAUNCH();
+      m->small_kept = false;
+      hg_status st = launch_small_steps(m, dt, few, s);
+      if (st != HG_OK) return st;
+      m->small_kept = true;
       m->steps_since_rebin += few;
       k += few;
     }

@@ -19,6 +19,10 @@ def test_hybrid_steps_after_a_failed_one():
     run("hybrid")
 
 
+def test_small_mixed_scenes_after_a_failed_step():
+    run("small")
+
+
 def run(case):
     from libhybridgrains_gb300 import build
     build.build(bounds_check=True)
@@ -82,13 +86,46 @@ def hybrid(hg, fail):
         assert failed >= 8, failed
 
 
+def small(hg, fail):
+    """A MIXED scene stepped several steps in one launch each: the masses after
+    a step are the points' to 1e-6 of the largest (FP32 sums)."""
+    from libhybridgrains_gb300 import scenes
+    rng = np.random.default_rng(6)
+    n, h, mat = 3000, 5.0e-3, scenes.mpm_material()
+    vol = np.full(n, 0.25 * h * h)
+    pts = (rng.uniform([0.02, 0.02], [0.2, 0.1], (n, 2)), rng.normal(0.0, 0.3, (n, 2)),
+           1550.0 * vol, vol, np.full(n, 0.25 * h))
+    ctx = hg.Context(0)
+    a, b = (hg.MPM(ctx, (0.0, 0.0), (0.25, 0.15), h, mat["shear_modulus"], mat["bulk_modulus"],
+                   mat["dp_alpha"], mat["flip_alpha"], scenes.GRAVITY, [], precision=hg.MIXED,
+                   capacity=n) for _ in range(2))
+    b.upload(*pts)
+    b.flow(1.0e-5, 10)
+    want = b.grid()["mass"]
+    failed = 0
+    for k in range(1, 40):
+        a.upload(*pts)
+        a.flow(1.0e-5, 1)
+        fail(k)
+        try:
+            a.flow(1.0e-5, 10)
+        except hg.HGError:
+            failed += 1
+        if fail(0) > 0:
+            break
+        a.upload(*pts)
+        a.flow(1.0e-5, 10)
+        assert np.abs(a.grid()["mass"] - want).max() <= 1e-6 * want.max(), k
+    assert failed >= 10, failed
+
+
 def main(case):
     sys.path.insert(0, ROOT)
     import libhybridgrains_gb300 as hg
     from libhybridgrains_gb300 import _capi
     fail = _capi.load().hg_check_fail_launch
     fail.argtypes, fail.restype = [ctypes.c_int64], ctypes.c_int64
-    {"hybrid": hybrid}[case](hg, fail)
+    {"hybrid": hybrid, "small": small}[case](hg, fail)
 
 
 if __name__ == "__main__":
