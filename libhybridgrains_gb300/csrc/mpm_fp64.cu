@@ -391,10 +391,9 @@ struct G2pArgs {
   double *next_mass, *next_mom, *next_force; // the next step's accumulators, cleared
   uint32_t *status;
   // constants of every point
-  double yield_mu; // alpha kappa / (2 mu)
+  double yield_mu; // alpha kappa / (2 mu); NaN without a shear modulus
   double pic;   // 1 - flip_alpha
-  float yield_mu32;
-  bool yields; // a shear modulus above 0: without one mu |dev be| exceeds no yield stress
+  float mu32, yield32;
   float px[HG_MAX_PLANES][2];
 };
 
@@ -485,13 +484,14 @@ __device__ __forceinline__ bool strain_symmetric(const MpmParams &P, const G2pAr
     const float d32 = narrow_trunc(d0), o32 = narrow_trunc(b01);
     const float n2 = 2.0f * (d32 * d32 + o32 * o32);
     const float limit =
-        fmaxf(0.0f, A.yield_mu32 * narrow_trunc(up) * narrow_trunc(down)) * narrow_trunc(J);
+        fmaxf(0.0f, A.yield32 * narrow_trunc(up) * narrow_trunc(down)) * narrow_trunc(J) / A.mu32;
     // elastic for sure, where the estimate of |dev be| is well above the
     // rounding of d0 and FP32's smallest squares
-    const bool elastic = !A.yields || (n2 > 1.0e-18f && sqrtf(n2) < limit * 0.99999f);
+    const bool elastic = n2 > 1.0e-18f && sqrtf(n2) < limit * 0.99999f;
     if (!elastic) {
       // l2 = ys / (mu |dev be| / J), below 1 beyond the yield surface; no
-      // deviator gives infinity or NaN
+      // deviator gives infinity or NaN, no shear modulus NaN (arithmetic's, whose
+      // sign bit is clear): neither is below 1
       const double o2 = b01 * b01;
       double l2 = A.yield_mu * up * down * J * rsqrt(fma(d0, d0, fma(d1, d1, twice(o2))));
       if (f64_hi(l2) >> 31) l2 = 0.0; // J > 1: no yield stress
@@ -701,10 +701,14 @@ hg_status to_points(hg_mpm *m, double dt) {
   A.next_mom = m->g_mom_next.p;
   A.next_force = m->g_force_next.p;
   A.status = m->status.p;
-  A.yields = m->p.mu > 0.0;
-  A.yield_mu = A.yields ? 0.5 * m->p.dp_alpha * m->p.kappa / m->p.mu : 0.0;
-  A.yield_mu32 = (float)A.yield_mu;
+  const double yield = 0.5 * m->p.dp_alpha * m->p.kappa;
+  // (without a shear modulus mu |dev be| exceeds no yield stress; a test of its
+  // own on the device cost 12,800 to 52,000 points 7 to 28 % of the step, through
+  // the registers and so the places of the next kernel's CTAs)
+  A.yield_mu = m->p.mu > 0.0 ? yield / m->p.mu : std::nan("");
   A.pic = 1.0 - m->p.flip_alpha;
+  A.mu32 = m->p.mu > 0.0 ? (float)m->p.mu : 0.0f;
+  A.yield32 = (float)yield;
   for (int k = 0; k < HG_MAX_PLANES; ++k)
     for (int c = 0; c < 2; ++c) A.px[k][c] = (float)m->p.planes[k].x[c];
   auto kernel = m->p.basis == HG_BASIS_UGIMP ? k64_g2p<HG_BASIS_UGIMP> : k64_g2p<HG_BASIS_LINEAR>;
