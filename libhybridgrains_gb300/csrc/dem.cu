@@ -840,28 +840,58 @@ __global__ void __launch_bounds__(CONTACT_THREADS) kd_contacts(const __grid_cons
   });
 }
 
+struct IntegrateArgs {
+  int64_t n, ccap;
+  double dt;
+  double *q, *v;
+  double *q_before; // receives the positions before the step, or nullptr
+  const double4 *terms;
+  const uint8_t *fixed;
+  const int4 *desc;
+  const int32_t *descn, *in_cursor;
+  int32_t *in_list;
+  const void *load;
+  const int64_t *keys; // the contacts, and the circle-circle ones' range
+  const int2 *range;
+  uint32_t *status;
+};
+
 // Body j's contacts in the reference's order: with static objects, as the
 // second body of circle-circle contacts (their first indices lie below j, so
 // they come before j's own list in the reference's loop), as the first body,
 // and with fixed disks. apply(load, as_second). The incoming list, filled in
 // no particular order, is sorted first. The first four incoming and own loads
 // are fetched together: the sums are a chain, their loads need not be.
+// The lists have room for every contact found, so with more than MAXP on a body
+// they can go past the buffer, which holds the contacts kept; such a body's are
+// looked up among all circle-circle contacts (by second body, in order).
 template <class L, class F>
-__device__ __forceinline__ void for_each_load(const L *load, int4 d, int counts,
-                                              int nin, int32_t *in_list, int64_t ccap,
-                                              uint32_t *status, F &&apply) {
+__device__ __forceinline__ void for_each_load(const IntegrateArgs &A, int64_t j, F &&apply) {
+  const L *load = reinterpret_cast<const L *>(A.load);
+  const int4 d = A.desc[j];
+  const int counts = A.descn[j];
+  int nin = A.in_cursor[j];
+  const int64_t ccap = A.ccap;
+  uint32_t *status = A.status;
   const int ns = counts & 0xFF, ncc = (counts >> 8) & 0xFF, nkin = (counts >> 16) & 0xFF;
-  nin = (int)min((int64_t)nin, max((int64_t)0, ccap - d.w));
-  int32_t *lst = in_list + d.w;
+  const bool listed = (int64_t)d.w + nin <= ccap;
+  int32_t *lst = A.in_list + d.w;
   int in[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) in[k] = k < nin ? lst[k] : 0x7FFFFFFF;
+  for (int k = 0; k < 4; ++k) in[k] = k < nin && listed ? lst[k] : 0x7FFFFFFF;
   L own[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k)
     if (k < ncc) own[k] = load[d.y + k];
   for (int k = 0; k < ns; ++k) apply(load[d.x + k], false);
-  if (nin <= 4) {
+  if (!listed) {
+    const int2 r = *A.range;
+    for (int64_t k = r.x; k < r.y && nin > 0; ++k)
+      if ((int64_t)(A.keys[k] & 0x3FFFFFFF) == j) {
+        apply(load[k], true);
+        --nin;
+      }
+  } else if (nin <= 4) {
     auto order = [&](int x, int y) {
       const int lo = min(in[x], in[y]), hi = max(in[x], in[y]);
       in[x] = lo;
@@ -899,20 +929,6 @@ __device__ __forceinline__ void for_each_load(const L *load, int4 d, int counts,
   for (int k = 0; k < nkin; ++k) apply(load[d.z + k], false);
 }
 
-struct IntegrateArgs {
-  int64_t n, ccap;
-  double dt;
-  double *q, *v;
-  double *q_before; // receives the positions before the step, or nullptr
-  const double4 *terms;
-  const uint8_t *fixed;
-  const int4 *desc;
-  const int32_t *descn, *in_cursor;
-  int32_t *in_list;
-  const void *load;
-  uint32_t *status;
-};
-
 // Force gather and symplectic Euler. With BIN the body is binned at its new
 // position for the next step's search (the tables were cleared by the contact
 // law), which saves that step a pass over the bodies.
@@ -930,18 +946,17 @@ __global__ void kd_integrate(const __grid_constant__ IntegrateArgs A,
   const double p0 = A.q[3 * j], p1 = A.q[3 * j + 1], p2 = A.q[3 * j + 2];
   const bool fixed = A.fixed[j] != 0;
   double Fx = bt.x, Fy = bt.y, T = 0.0;
-  for_each_load(reinterpret_cast<const double4 *>(A.load), A.desc[j], A.descn[j], A.in_cursor[j],
-                A.in_list, A.ccap, A.status, [&](const double4 &f, bool second) {
-                  if (second) {
-                    Fx -= f.x;
-                    Fy -= f.y;
-                    T -= f.w;
-                  } else {
-                    Fx += f.x;
-                    Fy += f.y;
-                    T += f.z;
-                  }
-                });
+  for_each_load<double4>(A, j, [&](const double4 &f, bool second) {
+    if (second) {
+      Fx -= f.x;
+      Fy -= f.y;
+      T -= f.w;
+    } else {
+      Fx += f.x;
+      Fy += f.y;
+      T += f.z;
+    }
+  });
   if (fixed) Fx = Fy = T = 0.0;
   // v1 = v0 + dt Minv F ; q1 = q0 + dt v1
   const double v0 = u0 + bt.z * Fx;
@@ -1117,12 +1132,11 @@ __global__ void kdx_integrate(const __grid_constant__ IntegrateArgs A,
   const double p0 = A.q[3 * j], p1 = A.q[3 * j + 1], p2 = A.q[3 * j + 2];
   const bool fixed = A.fixed[j] != 0;
   float Fx = narrow(bt.x), Fy = narrow(bt.y), T = 0.0f;
-  for_each_load(reinterpret_cast<const float4 *>(A.load), A.desc[j], A.descn[j], A.in_cursor[j],
-                A.in_list, A.ccap, A.status, [&](const float4 &f, bool second) {
-                  Fx += second ? -f.x : f.x;
-                  Fy += second ? -f.y : f.y;
-                  T += second ? -f.w : f.z;
-                });
+  for_each_load<float4>(A, j, [&](const float4 &f, bool second) {
+    Fx += second ? -f.x : f.x;
+    Fy += second ? -f.y : f.y;
+    T += second ? -f.w : f.z;
+  });
   if (fixed) Fx = Fy = T = 0.0f;
   const float v0 = narrow(u0) + narrow(bt.z) * Fx;
   const float v1 = narrow(u1) + narrow(bt.z) * Fy;
@@ -1465,6 +1479,8 @@ hg_status dem_step(hg_dem *d, double dt, int weighted, bool bin_next, double *q_
   I.in_cursor = d->in_cursor.p;
   I.in_list = d->in_list.p;
   I.load = d->load.p;
+  I.keys = d->ckey[nb].p;
+  I.range = d->cc_range.p;
   I.status = d->status.p;
   auto integrate = d->p.precision == HG_PRECISION_MIXED
                        ? (bin_next ? kdx_integrate<true> : kdx_integrate<false>)
