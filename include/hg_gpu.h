@@ -270,7 +270,10 @@ hg_status hg_batch_profile_read(hg_batch *b, double *resort_ms, double *table_ms
  * changes the order of FP32 atomic sums). A batch keeps the fastest shape for
  * each kernel. A single scene then times the whole step, replayed as graphs
  * in which the two kernels overlap, for every pair of a fused and an update
- * shape (48 more steps each) and keeps the fastest pair. The result is
+ * shape (48 more steps each) and keeps the fastest pair. (Small linear scenes
+ * step in one launch but for the last step of a call; timed are the two kernels,
+ * for the larger scenes of the class. The uGIMP particle kernel takes no shape:
+ * such scenes choose the grid update's, in classes of their own.) The result is
  * recorded in a process-wide table under the object's size
  * class: the device's SM count, the tile count (single scenes) and the point
  * count, both rounded up to powers of two. MIXED objects and batches look up

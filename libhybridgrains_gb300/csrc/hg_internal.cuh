@@ -350,13 +350,15 @@ struct hg_mpm {
   // the autotuner, else looked up in the tuning table at priming
   hg_launch_shape shape{0, 0};
   bool shape_set = false;
+  bool tuning = false; // the launch shapes are being timed
   // CHUNK_STEPS steps captured as a CUDA graph, one per live buffer; rebuilt
   // when dt, the point count or the launch shape changes
   cudaGraphExec_t chunk_exec[2] = {nullptr, nullptr};
   double chunk_dt[2] = {0.0, 0.0};
   int64_t chunk_n[2] = {-1, -1};
   hg_launch_shape chunk_shape[2] = {{-1, -1}, {-1, -1}};
-  int64_t chunk_launches = 0;
+  bool chunk_small[2] = {false, false}; // captured as one-launch steps
+  int64_t chunk_launches[2] = {0, 0};
   // per-kernel event timing (hg_mpm_profile)
   bool profile = false;
   std::vector<cudaEvent_t> prof_events; // 3 per recorded step

@@ -2062,7 +2062,9 @@ bool same_shape(const hg_launch_shape &a, const hg_launch_shape &b) {
 // ---- the tuning table -------------------------------------------------------
 //
 // Keyed by (kind, SMs, tiles, points), tiles and points rounded up to powers
-// of two: kind 0 is a single scene, kind 1 a batch (tiles 0).
+// of two: kind 0 is a single linear scene, kind 1 a batch (tiles 0), kind 2 a
+// single uGIMP scene (its particle kernel takes no shape, so that what was timed
+// for one is no choice for a linear scene).
 using TuneKey = std::array<int64_t, 4>;
 std::mutex g_tune_mu;
 std::map<TuneKey, hg_launch_shape> g_tune;
@@ -2073,7 +2075,8 @@ int64_t ceil_pow2(int64_t x) {
   return p;
 }
 TuneKey mixed_key(const hg_mpm *m) {
-  return {0, m->ctx->num_sms, ceil_pow2((int64_t)m->ntx * m->nty), ceil_pow2(std::max<int64_t>(m->n, 1))};
+  return {m->p.basis == HG_BASIS_UGIMP ? 2 : 0, m->ctx->num_sms,
+          ceil_pow2((int64_t)m->ntx * m->nty), ceil_pow2(std::max<int64_t>(m->n, 1))};
 }
 TuneKey batch_key(const hg_batch *b, int64_t points) {
   return {1, b->ctx->num_sms, 0, ceil_pow2(std::max<int64_t>(points, 1))};
@@ -2089,9 +2092,10 @@ void tune_store(const TuneKey &k, const hg_launch_shape &s) {
   std::lock_guard<std::mutex> lock(g_tune_mu);
   g_tune[k] = s;
 }
-// CTAs per SM tried for (fused, update): fewer, the default, and more CTAs
-// than are resident (finer shares of the tiles, later ones fill in behind
-// the first wave)
+// CTAs per SM tried for (fused, update): fewer, a single scene's default, and
+// more CTAs than are resident (finer shares of the tiles, later ones fill in
+// behind the first wave; 8 is a batch's default for its fused kernel, which is
+// chosen apart from the update's)
 constexpr hg_launch_shape TUNE_CANDIDATES[HG_TUNE_CANDIDATES] = {{2, 4}, {4, 8}, {8, 16},
                                                                  {12, 32}};
 static_assert(HG_TUNE_CANDIDATES == 4, "candidate list");
@@ -2313,7 +2317,11 @@ hg_status end_chunk_capture(cudaStream_t s, hg_status st, int64_t l0, cudaGraphE
   return HG_OK;
 }
 
-bool small_scene(const hg_mpm *m) { return m->small_m[0].p && m->n <= SMALL_POINTS; }
+// (The autotuner times the two kernels of the launch shapes, which larger scenes
+// of the class step by and small ones end each call with.)
+bool small_scene(const hg_mpm *m) {
+  return m->small_m[0].p && m->n <= SMALL_POINTS && !m->tuning;
+}
 
 // The second set of sums is clear before and after a run of one-launch steps;
 // here before the first run, and after one that failed half-way.
@@ -2359,8 +2367,9 @@ hg_status launch_small_steps(hg_mpm *m, double dt, int n, cudaStream_t s) {
 // out-of-window counters.
 hg_status mixed_chunk_graph(hg_mpm *m, double dt) {
   const int c = m->cur;
+  const bool small = small_scene(m);
   if (m->chunk_exec[c] && m->chunk_dt[c] == dt && m->chunk_n[c] == m->n &&
-      same_shape(m->chunk_shape[c], m->shape))
+      m->chunk_small[c] == small && same_shape(m->chunk_shape[c], m->shape))
     return HG_OK;
   if (m->chunk_exec[c]) {
     cudaGraphExecDestroy(m->chunk_exec[c]);
@@ -2368,7 +2377,6 @@ hg_status mixed_chunk_graph(hg_mpm *m, double dt) {
   }
   cudaStream_t s = m->ctx->stream;
   const MixedArgs At = make_args(m, dt, true), Ab = make_args(m, dt, false);
-  const bool small = small_scene(m);
   hg_status st = HG_OK;
   const int64_t l0 = g_launches.load();
   HG_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
@@ -2390,8 +2398,9 @@ hg_status mixed_chunk_graph(hg_mpm *m, double dt) {
   if (st != HG_OK) return st;
   m->chunk_dt[c] = dt;
   m->chunk_n[c] = m->n;
+  m->chunk_small[c] = small;
   m->chunk_shape[c] = m->shape;
-  m->chunk_launches = launches;
+  m->chunk_launches[c] = launches;
   return HG_OK;
 }
 
@@ -2421,7 +2430,7 @@ hg_status mixed_step(hg_mpm *m, double dt, int nsteps) {
     hg_status st = mixed_chunk_graph(m, dt);
     if (st != HG_OK) return st;
     HG_CUDA_TRY(cudaGraphLaunch(m->chunk_exec[m->cur], s));
-    g_launches.fetch_add(m->chunk_launches, std::memory_order_relaxed);
+    g_launches.fetch_add(m->chunk_launches[m->cur], std::memory_order_relaxed);
     HG_CUDA_TRY(cudaEventRecord(m->outside_ev, s));
     m->outside_pending = true;
     m->steps_since_rebin += CHUNK_STEPS;
@@ -2777,6 +2786,7 @@ hg_status mixed_autotune(hg_mpm *m, double dt, int steps, hg_tune_report *report
   const bool prof0 = m->profile;
   hg_status st = HG_OK;
   if (!m->primed) st = prime(m);
+  m->tuning = true;
   for (int i = 0; i < HG_TUNE_CANDIDATES && st == HG_OK; ++i) {
     r.tried[i] = TUNE_CANDIDATES[i];
     m->shape = TUNE_CANDIDATES[i];
@@ -2827,6 +2837,7 @@ hg_status mixed_autotune(hg_mpm *m, double dt, int steps, hg_tune_report *report
     }
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
+  m->tuning = false;
   m->profile = prof0;
   if (st != HG_OK) {
     m->shape = hg_launch_shape{0, 0};
