@@ -383,17 +383,22 @@ __device__ __forceinline__ Strip strip_of(const MixedArgs &A, int tile, int spli
   return s;
 }
 
+struct NoClaim {
+  __device__ __forceinline__ bool due() const { return false; }
+  __device__ __forceinline__ int draw() const { return 0; }
+};
+
 // One strip of one scene; A lives in shared memory or the constant bank.
-// nodes: where a grid node's velocity and acceleration come from. claim: a
-// counter that the CTA draws S.claimed from on the way. AHEAD: a point's state
-// is loaded while the one before it is processed, after that one's window
-// reads (before them its 13 registers spilled: 64.0 us), the first one's under
-// the window loads: 61.0 us, without 66. With the arguments in shared memory,
-// as in a batch, they would spill: 72.0 us, without 59.6.
-template <bool PRIME, bool AHEAD, int CAP, class N>
+// nodes: where a grid node's velocity and acceleration come from. claim: draws
+// S.claimed, the CTA's next work, under the last flush if it is due. AHEAD: a
+// point's state is loaded while the one before it is processed, after that one's
+// window reads (before them its 13 registers spilled: 64.0 us), the first one's
+// under the window loads: 61.0 us, without 66. With the arguments in shared
+// memory, as in a batch, they would spill: 72.0 us, without 59.6.
+template <bool PRIME, bool AHEAD, int CAP, class N, class C = NoClaim>
 __device__ __forceinline__ void fused_strip(const MixedArgs &A, const Strip &strip,
                                             FusedSmem<CAP> &S, const N nodes,
-                                            int32_t *claim = nullptr) {
+                                            const C claim = C{}) {
   static_assert(THREADS == BIN_CELLS, "a whole tile has one thread per cell");
   constexpr int VA_W = FusedSmem<CAP>::VW, ACC_W = FusedSmem<CAP>::AW;
   const int split = strip.split, lanes = 1 << split, rows = BIN >> split;
@@ -644,8 +649,8 @@ __device__ __forceinline__ void fused_strip(const MixedArgs &A, const Strip &str
         if (left_cell) atomicAdd(&s_out[1], left_cell);
       }
       __syncthreads();
-      int claimed = 0; // (arrives under the flush)
-      if (claim && last && tid == 0) claimed = atomicAdd(claim, 1);
+      int claimed = -1; // (arrives under the flush)
+      if (last && tid == 0 && claim.due()) claimed = claim.draw();
       // ---- node sums of the tile window, flushed to the global accumulators ----
       for (int k = tid; k < ACC_W * (rows + 2 * DRIFT + 3); k += THREADS) {
         const int i = k % ACC_W, j = k / ACC_W;
@@ -676,7 +681,7 @@ __device__ __forceinline__ void fused_strip(const MixedArgs &A, const Strip &str
         atomicAdd(&A.accm[node], sum[0]);
         atomicAdd(&A.acc4[node], make_float4(sum[1], sum[2], sum[3], sum[4]));
       }
-      if (claim && last && tid == 0) S.claimed = claimed;
+      if (claimed >= 0) S.claimed = claimed;
       __syncthreads();
     }
     if (tid < 2 && s_out[tid]) atomicAdd(&A.outside[tid], s_out[tid]);
@@ -704,6 +709,12 @@ struct GridNodes {
     n01 = A.va[k0 + row];
     n11 = A.va[k0 + row + 1];
   }
+};
+
+struct TileClaim {
+  int32_t *at;
+  __device__ __forceinline__ bool due() const { return true; }
+  __device__ __forceinline__ int draw() const { return atomicAdd(at, 1); }
 };
 
 // Bound by issue slots and load latency: 68 % of the slots, 660 instructions
@@ -752,8 +763,13 @@ __global__ void __launch_bounds__(THREADS, 4) kx_g2p2g(const __grid_constant__ M
     const Strip strip =
         i < 0 ? strip_of(A, A.active[t], 0, 0)
               : strip_of(A, A.active[Q.whole + (i >> Q.split)], Q.split, i & ((1 << Q.split) - 1));
-    fused_strip<PRIME, true>(A, strip, S, GridNodes{A}, PRIME ? nullptr : A.claimed);
-    t = PRIME ? t + gridDim.x : gridDim.x + S.claimed;
+    if (PRIME) {
+      fused_strip<PRIME, true>(A, strip, S, GridNodes{A});
+      t += gridDim.x;
+    } else {
+      fused_strip<PRIME, true>(A, strip, S, GridNodes{A}, TileClaim{A.claimed});
+      t = gridDim.x + S.claimed;
+    }
   }
 }
 
@@ -940,9 +956,9 @@ __device__ __forceinline__ int batch_slot(const int *prefix, int nslots, int ite
 // static split by item count cannot balance.
 constexpr int QUEUE_MAX_CHUNK = 8;
 
-__device__ __forceinline__ int2 queue_claim(int32_t *q, int total, int seen) {
-  const int g = max(1, min(QUEUE_MAX_CHUNK, (total - seen) / (2 * (int)gridDim.x)));
-  return make_int2(atomicAdd(q, g), g);
+__device__ __forceinline__ int queue_chunk(int total, int seen) {
+  const int left = total - seen, ctas = (int)gridDim.x;
+  return left < 4 * ctas ? 1 : min(QUEUE_MAX_CHUNK, left / (2 * ctas));
 }
 
 __device__ __forceinline__ void queue_done(int32_t *q) {
@@ -954,29 +970,50 @@ __device__ __forceinline__ void queue_done(int32_t *q) {
   }
 }
 
-// Drains the queue: tile(A, tile index) for every claimed item, the scene's
-// arguments copied into A whenever the item's scene changes. The next chunk
-// is claimed while this one runs.
+// (thread 0's view of its place in the queue, in shared memory: the strip has
+// no registers to spare)
+struct QueuePlace {
+  int total, end; // items in all, the end of its chunk
+  bool more, due; // items beyond the first claims, in the chunk's last item
+};
+struct QueueClaim {
+  int32_t *q;
+  const QueuePlace &at;
+  __device__ __forceinline__ bool due() const { return at.due; }
+  __device__ __forceinline__ int draw() const { return atomicAdd(q, queue_chunk(at.total, at.end)); }
+};
+
+// Drains the queue: tile(A, tile index, claim) for every claimed item, the
+// scene's arguments copied into A whenever the item's scene changes. The next
+// chunk is claimed under the end of this one's last tile: claimed at its start,
+// the CTAs first to run hold two tiles each where others find none (36 scenes of
+// 2,000 to 16,000 points 50.5 us per step, now 36.9; 28 of 2,000 to 40,000 49
+// and 37.5). Where half of the CTAs (at twice the resident ones, a round) have a
+// tile for each, the first claims take all and no CTA waits for another.
 // The kernels are launched with programmatic dependence after a chunk's first
 // one: queue, tables and tile lists are older than the launch before, and are
 // read under its end (a step of 48 scenes of 2,000 to 100,000 points 74.7 us,
 // after ordinary launches 76.7).
 template <class F>
 __device__ __forceinline__ void drain_queue(const MixedArgs *slots, int nslots, const int *prefix,
-                                            int32_t *q, MixedArgs &A, F &&tile) {
-  __shared__ int2 s_claim;
-  const int total = prefix[nslots];
-  int2 claim = threadIdx.x == 0 ? queue_claim(q, total, 0) : make_int2(0, 0);
-  int s = -1;
-  for (;;) {
-    if (threadIdx.x == 0) s_claim = claim;
-    __syncthreads();
-    const int2 c = s_claim;
-    __syncthreads();
-    if (c.x >= total) break;
-    if (threadIdx.x == 0) claim = queue_claim(q, total, c.x + c.y);
-    const int end = min(c.x + c.y, total);
-    for (int item = c.x; item < end; ++item) {
+                                            int32_t *q, MixedArgs &A, int &claimed,
+                                            F &&tile) {
+  __shared__ int s_first;
+  __shared__ QueuePlace at;
+  if (threadIdx.x == 0) {
+    claimed = at.total = prefix[nslots];
+    at.more = at.total > (int)gridDim.x / 2;
+    s_first = atomicAdd(q, queue_chunk(at.total, 0));
+  }
+  __syncthreads();
+  int s = -1, seen = 0; // seen: the end of the chunk before
+  for (int begin = s_first; begin < prefix[nslots]; begin = claimed) {
+    const int end = min(begin + queue_chunk(prefix[nslots], seen), prefix[nslots]);
+    for (int item = begin; item < end; ++item) {
+      if (threadIdx.x == 0) {
+        at.end = end;
+        at.due = at.more && item + 1 == end;
+      }
       if (s < 0 || item >= prefix[s + 1] || item < prefix[s]) {
         const bool first = s < 0;
         s = batch_slot(prefix, nslots, item);
@@ -986,8 +1023,9 @@ __device__ __forceinline__ void drain_queue(const MixedArgs *slots, int nslots, 
           pdl_trigger();
         }
       }
-      tile(A, A.active[item - prefix[s]]);
+      tile(A, A.active[item - prefix[s]], QueueClaim{q, at});
     }
+    seen = end;
   }
   pdl_wait();
   queue_done(q);
@@ -1003,9 +1041,9 @@ __global__ void __launch_bounds__(THREADS, 4) kb_g2p2g(const MixedArgs *slots,
   __shared__ MixedArgs A;
   zero_slow(S);
   batch_prefix(slots, nslots, prefix);
-  drain_queue(slots, nslots, prefix, queue, A,
-              [&](const MixedArgs &a, int tile) {
-                fused_strip<false, false>(a, strip_of(a, tile, 0, 0), S, GridNodes{a});
+  drain_queue(slots, nslots, prefix, queue, A, S.claimed,
+              [&](const MixedArgs &a, int tile, QueueClaim claim) {
+                fused_strip<false, false>(a, strip_of(a, tile, 0, 0), S, GridNodes{a}, claim);
               });
 }
 
