@@ -350,10 +350,20 @@ template <int CAP> struct FusedSmem {
   int claimed;       // the number that the CTA drew
 };
 
-// as many as four CTAs per SM have room for (a batch's also hold the scene's
-// arguments and the prefix of the scenes' tiles)
-constexpr int PASS_POINTS = 1152, BATCH_PASS_POINTS = 1024;
+// As many as four CTAs per SM have room for. A batch's also hold the scene's
+// arguments and the prefix of the scenes' tiles, so in batches of more than
+// ROOMY_BATCH scenes a pass ends at 1,024 points. There a tile of four points
+// per cell takes a second pass, and a second flush, from one point more on. In
+// collapse, 28 scenes of 2,000 to 40,000 points take 37.8 us per step with passes
+// of 1,024 and 36.0 with 1,152, 36 of 2,000 to 16,000 37.9 and 35.8, four of
+// 2,000 to 9,000 25.1 and 23.7.
+constexpr int PASS_POINTS = 1152, MANY_PASS_POINTS = 1024, ROOMY_BATCH = 128;
+constexpr size_t batch_smem(size_t fused, int nslots) {
+  return fused + sizeof(int) * ((size_t)nslots + 1);
+}
 static_assert(4 * (sizeof(FusedSmem<PASS_POINTS>) + 16 + 1024) <= 228 * 1024, "shared memory");
+static_assert(4 * (batch_smem(sizeof(FusedSmem<PASS_POINTS>), ROOMY_BATCH) + sizeof(MixedArgs) +
+                   128 + 1024) <= 228 * 1024, "shared memory");
 
 // Slot of point i of a pass: points four apart, which neighbouring cells read
 // together, lie in different banks.
@@ -1033,10 +1043,11 @@ __device__ __forceinline__ void drain_queue(const MixedArgs *slots, int nslots, 
 
 
 // All scenes of a batch in one launch: the CTAs drain (scene, tile) items.
+template <int CAP>
 __global__ void __launch_bounds__(THREADS, 4) kb_g2p2g(const MixedArgs *slots,
                                                        int nslots, int32_t *queue) {
   extern __shared__ __align__(16) unsigned char fused_smem[];
-  FusedSmem<BATCH_PASS_POINTS> &S = *reinterpret_cast<FusedSmem<BATCH_PASS_POINTS> *>(fused_smem);
+  FusedSmem<CAP> &S = *reinterpret_cast<FusedSmem<CAP> *>(fused_smem);
   int *prefix = reinterpret_cast<int *>(fused_smem + sizeof(S)); // [nslots + 1]
   __shared__ MixedArgs A;
   zero_slow(S);
@@ -1890,9 +1901,15 @@ MixedParticles parts(hg_mpm *m, int which) {
 }
 
 template <int CAP> size_t fused_smem_bytes() { return sizeof(FusedSmem<CAP>); }
-// a batch's kernel holds the prefix of its scenes' tiles as well
-size_t fused_batch_smem_bytes(int nslots) {
-  return sizeof(FusedSmem<BATCH_PASS_POINTS>) + sizeof(int) * ((size_t)nslots + 1);
+// a batch's kernel, and its shared memory
+struct BatchFused {
+  void (*kernel)(const MixedArgs *, int, int32_t *);
+  size_t smem;
+};
+BatchFused batch_fused(int nslots) {
+  if (nslots <= ROOMY_BATCH)
+    return {kb_g2p2g<PASS_POINTS>, batch_smem(sizeof(FusedSmem<PASS_POINTS>), nslots)};
+  return {kb_g2p2g<MANY_PASS_POINTS>, batch_smem(sizeof(FusedSmem<MANY_PASS_POINTS>), nslots)};
 }
 // more than 48 KB of shared memory is asked for by kernel
 hg_status fused_smem_setup() {
@@ -1902,7 +1919,8 @@ hg_status fused_smem_setup() {
   HG_CUDA_TRY(ask((const void *)kx_g2p2g<true>, fused_smem_bytes<PASS_POINTS>()));
   HG_CUDA_TRY(ask((const void *)kx_g2p2g<false>, fused_smem_bytes<PASS_POINTS>()));
   HG_CUDA_TRY(ask((const void *)kx_step_small, fused_smem_bytes<PASS_POINTS>()));
-  HG_CUDA_TRY(ask((const void *)kb_g2p2g, fused_batch_smem_bytes(MAX_BATCH)));
+  for (int nslots : {ROOMY_BATCH, (int)MAX_BATCH})
+    HG_CUDA_TRY(ask((const void *)batch_fused(nslots).kernel, batch_fused(nslots).smem));
   return HG_OK;
 }
 
@@ -2630,6 +2648,7 @@ hg_status batch_chunk_graph(hg_batch *b, int S) {
   const MixedArgs *db = dt + S;
   const int nsm = b->ctx->num_sms;
   const int gu = nsm * update_per_sm(b->shape), gf = nsm * batch_fused_per_sm(b->shape);
+  const BatchFused fused = batch_fused(S);
   const int64_t l0 = g_launches.load();
   HG_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   hg_status st = HG_OK;
@@ -2638,7 +2657,7 @@ hg_status batch_chunk_graph(hg_batch *b, int S) {
       HG_LAUNCH(kb_grid_update, gu, THREADS, 0, s, dt, S);
     else
       HG_LAUNCH_PDL(kb_grid_update, gu, THREADS, 0, s, dt, S);
-    HG_LAUNCH_PDL(kb_g2p2g, gf, THREADS, fused_batch_smem_bytes(S), s, db, S, b->queue.p);
+    HG_LAUNCH_PDL(fused.kernel, gf, THREADS, fused.smem, s, db, S, b->queue.p);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) st = cuda_fail(e, "kernel launch");
   }
@@ -2782,8 +2801,9 @@ hg_status batch_step(hg_batch *b, int nsteps) {
     HG_LAUNCH(kb_grid_update, nsm * update_per_sm(b->shape), THREADS, 0, s, dt, S);
     HG_CHECK_LAUNCH();
     if (b->profile) HG_CUDA_TRY(cudaEventRecord(ev[3], s));
-    HG_LAUNCH_PDL(kb_g2p2g, nsm * batch_fused_per_sm(b->shape), THREADS,
-                  fused_batch_smem_bytes(S), s, db, S, b->queue.p);
+    const BatchFused fused = batch_fused(S);
+    HG_LAUNCH_PDL(fused.kernel, nsm * batch_fused_per_sm(b->shape), THREADS, fused.smem, s, db, S,
+                  b->queue.p);
     HG_CHECK_LAUNCH();
     if (b->profile) HG_CUDA_TRY(cudaEventRecord(ev[4], s));
     for (hg_mpm *m : b->members) m->steps_since_rebin++;

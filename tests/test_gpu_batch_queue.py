@@ -1,6 +1,7 @@
-"""Batches over the forms that their work queue takes (1,216 CTAs on 152 SMs):
-fewer tiles than half of the CTAs, more tiles than CTAs, so many that several are
-claimed at a time. Each member ends where it ends stepped alone, at the bounds of
+"""Batches over the forms that their work queue and their kernel take (1,216 CTAs
+on 152 SMs): fewer tiles than half of the CTAs, more tiles than CTAs, so many
+that several are claimed at a time; as many members as the long passes have room
+for and one more; a tile with one point more than a pass. Each member ends where it ends stepped alone, at the bounds of
 test_gpu_batch."""
 import numpy as np
 import pytest
@@ -30,7 +31,7 @@ def make(ctx, tiles, crowd, seed):
 
 
 @pytest.mark.parametrize("members,tiles,crowd", [
-    (20, 4, 1025), (20, 8, 1025), (20, 16, 1025)])
+    (20, 4, 1025), (20, 8, 1025), (20, 16, 1025), (128, 2, 1153), (129, 2, 1025), (1, 2, 2305)])
 def test_members_step_as_alone(ctx, members, tiles, crowd):
     alone = [make(ctx, tiles, crowd, k) for k in range(members)]
     together = [make(ctx, tiles, crowd, k) for k in range(members)]
