@@ -1467,8 +1467,10 @@ static hg_status dem_upload_impl(hg_dem *d, int64_t n, const double *q, const do
   }
   DeviceGuard g(d->ctx);
   AllocScope dem_scope(dem_stream(d)); // temporaries on the DEM's stream
-  // Broadphase cell width: the widest disk AABB plus a relative margin, so a
-  // disk's partners lie in the 3x3 cells around the cell of its AABB minimum.
+  // Broadphase cell width: the largest diameter plus a relative margin. Centres
+  // of disks that touch are at most that diameter apart, so with the margin over
+  // the binning's rounding a disk's partners lie in the 3x3 cells around the cell
+  // of its centre.
   d->cell_h = 2.0 * rmax * (1.0 + 1.0e-6);
   cudaStream_t s = dem_stream(d);
   d->n = n;

@@ -521,8 +521,8 @@ hg_status hybrid_pack_lists(hg_hybrid *h) {
   cudaStream_t s = h->ctx->stream;
   const int64_t nn = (int64_t)(h->m->p.nx + 1) * (h->m->p.ny + 1), nb = h->step_bodies;
   hg_status st;
-  // std::stable_partition of the grains (Coupling.cpp:113-127): kc_grain_mass
-  // flagged them
+  // std::stable_partition of the grains (Coupling.cpp:113-127):
+  // kc_grain_scatter flagged them
   HG_CUDA_TRY(cudaMemsetAsync(h->coupled.p + nb, 0, sizeof(int32_t), s));
   if ((st = exclusive_scan_i32(h->coupled.p, h->flag_tmp.p, nb + 1, h->scan_tmp.p, s))) return st;
   HG_LAUNCH(kc_pack, blocks_for(nb + 1, 256), 256, 0, s, nb, h->coupled.p, h->flag_tmp.p,

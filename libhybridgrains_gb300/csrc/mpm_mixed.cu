@@ -833,12 +833,14 @@ __device__ __forceinline__ float4 node_update(const MixedArgs &A, int ix, int iy
 // 62,468 9.2 and 18.8. What is left is the chain of one strip, about 1,600
 // instructions of a warp with few others to hide behind, and the launch.
 //
-// It steps linear scenes with no more points than fit its CTAs at one per cell,
-// so that no sparse scene takes a second round of whole tiles (80,000 points at
-// one per cell: 14.6 us, in two launches 12.5; 59,858: 8.4 and 11.4), on a grid
-// that a step clears in four stores per thread.
+// It steps linear scenes with nearly as many points as its CTAs have cells (247
+// of 256: a column's edges leave tiles partly filled), so that no scene of a point
+// per cell takes a second round of whole tiles (80,000 points at one per cell:
+// 14.6 us, in two launches 12.5; 59,858: 8.4 and 11.4). The grid has at most
+// SMALL_NODES nodes, which 152 SMs clear in four stores per thread (a constant:
+// the estimate of a scene's memory knows no device).
 constexpr int SMALL_CTAS = 2; // per SM
-constexpr int64_t SMALL_POINTS = 75000, SMALL_NODES = 4 * 152 * SMALL_CTAS * THREADS;
+constexpr int64_t SMALL_POINTS_PER_CTA = 247, SMALL_NODES = 4 * 152 * SMALL_CTAS * THREADS;
 struct SmallSets {
   const float4 *in4;
   const float *inm;
@@ -1678,7 +1680,8 @@ __global__ void kr_active(const RebinArgs *__restrict__ R, RebinPrefix P) {
   }
 }
 
-// kx_clear_inactive over (member, tile) items, one block per item
+// The outputs of the grid update on tiles without points, over (member, tile)
+// items, one block per item (a single scene's: kx_tiles)
 __global__ void __launch_bounds__(BIN_CELLS) kr_clear_inactive(const RebinArgs *__restrict__ R,
                                                                RebinPrefix P) {
   const int64_t total = P.bins[P.nmem];
@@ -2376,7 +2379,8 @@ hg_status end_chunk_capture(cudaStream_t s, hg_status st, int64_t l0, cudaGraphE
 // (The autotuner times the two kernels of the launch shapes, which larger scenes
 // of the class step by and small ones end each call with.)
 bool small_scene(const hg_mpm *m) {
-  return m->small_m[0].p && m->n <= SMALL_POINTS && !m->tuning;
+  const int64_t ctas = (int64_t)m->ctx->num_sms * SMALL_CTAS;
+  return m->small_m[0].p && m->n <= ctas * SMALL_POINTS_PER_CTA && !m->tuning;
 }
 
 // The second set of sums is clear before and after a run of one-launch steps;
