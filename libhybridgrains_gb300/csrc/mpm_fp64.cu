@@ -188,7 +188,11 @@ __device__ __forceinline__ double det_sym(double b00, double b01, double b11) {
 // (-vol J sigma with sigma = tau / J), ConstitutiveModel.cpp:83-97.
 __device__ __forceinline__ M2d node_stress(const MpmParams &P, const P2gArgs &A, int64_t p) {
   const double Jp = A.J[p];
-  if (!(Jp <= 1.0) || A.jh[p] != 0) return {0.0, 0.0, 0.0, 0.0};
+  if (!(Jp <= 1.0) || A.jh[p] != 0) {
+    // (no stress is 0 / J: a J that is not a number reaches the nodes)
+    const double none = finite_bits(Jp) && !f64_zero(Jp) ? 0.0 : __hiloint2double(0x7FF80000, 0);
+    return {none, none, none, none};
+  }
   const double2 c0 = reinterpret_cast<const double2 *>(A.be)[2 * p];
   const double2 c1 = reinterpret_cast<const double2 *>(A.be)[2 * p + 1];
   const M2d be = m_scl(Jp, M2d{c0.x, c0.y, c1.x, c1.y});
